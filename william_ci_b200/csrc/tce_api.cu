@@ -78,6 +78,17 @@ void mapped_gauss_legendre(int n, std::vector<double> &t, std::vector<double> &w
     }
 }
 
+// smallest and largest t^2 of n nodes, widened to the neighbouring floats; (inf, -inf) when n = 0
+float2 node_range(const double *t, int n)
+{
+    double lo = HUGE_VAL, hi = -HUGE_VAL;
+    for (int k = 0; k < n; ++k) {
+        lo = std::min(lo, t[k] * t[k]);
+        hi = std::max(hi, t[k] * t[k]);
+    }
+    return make_float2(std::nextafterf((float)lo, 0.0f), std::nextafterf((float)hi, n > 0 ? HUGE_VALF : -HUGE_VALF));
+}
+
 int mod_pos(int a, int m) { int r = a % m; return r < 0 ? r + m : r; }
 
 // index shifted by -(cell of ref), cells x fastest (translate_to_unit_cell)
@@ -122,8 +133,8 @@ int route(const Handle *h, const int4 &q)
                         if (h->lxyz[3 * (h->sh_first[S] + c) + d] != (c == d ? 1 : 0)) sp = false;
         }
     }
-    if (cls == 0 && sp && (h->nq == 32 || h->nq == 40)) return 1 * 16;
-    if (sp && tce_r1_supported(h->ndp, h->nq, cls)) return 2 * 16 + cls;
+    if (cls == 0 && sp) return 1 * 16;
+    if (sp && h->ndp == 1 && __builtin_popcount(cls) <= 2) return 2 * 16 + cls;
     // generic kernel: one list per number of shells above p, each launched with
     // its own largest block (buffers sized for the list, not for (dd|dd))
     return (l[0] > 1) + (l[1] > 1) + (l[2] > 1) + (l[3] > 1);
@@ -423,6 +434,13 @@ int build(Handle *h, const tce_system *sys)
         for (int d = 0; d < 3; ++d)
             for (int g = 0; g < TCE_MAXG; ++g) gm[d * TCE_MAXG + g] = S.gmax[d][g];
         if ((s = upload(h, &h->d_gmax, gm))) return s;
+        S.rule_gmax = h->d_gmax;
+        std::vector<float2> t2((size_t)TCE_MAXG);
+        for (int g = 0; g < TCE_MAXG; ++g)
+            t2[(size_t)g] = node_range(h->tnode.data() + std::min(8 * g, h->nq), std::max(0, std::min(8, h->nq - 8 * g)));
+        float2 *d_t2 = nullptr;
+        if ((s = upload(h, &d_t2, t2))) return s;
+        S.rule_t2 = d_t2;
     }
 
     clk.mark("t-tables");
@@ -647,7 +665,9 @@ static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStre
     if (h->method != TCE_METHOD_FIXED) return lg_jk_passes(h, dP, dJ, dK, st);
     for (const auto &w : h->lists) {
         if (w.n == 0) continue;
-        if (w.kind == 0) {   // every other class: generic kernel
+        // the CUDA-core kernels of the all-s and one-p classes are built for 32 nodes (all-s: and 40)
+        const bool core = w.kind == 1 ? (h->nq == 32 || h->nq == 40) : tce_r1_supported(h->ndp, h->nq, w.cls);
+        if (w.kind == 0 || (!h->use_tc && !core)) {   // every other class: generic kernel
             QuartetHostArgs a;
             a.items = w.d;
             a.nitems = (int)w.n;
@@ -673,8 +693,13 @@ static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStre
             b.J = dJ;
             b.K = dK;
             b.num_sms = h->num_sms;
-            if (w.kind == 1) CKS(h, tce_launch_quartets_s(h->S, b, st));
-            else CKS(h, tce_launch_quartets_r1(h->S, w.cls, b, st));
+            if (h->use_tc) {
+                if (w.kind == 1) CKS(h, tce_launch_quartets_s_tc(h->S, b, h->nq, 1, st));
+                else CKS(h, tce_launch_quartets_sp_tc(h->S, w.cls, b, h->nq, 1, st));
+            } else {
+                if (w.kind == 1) CKS(h, tce_launch_quartets_s(h->S, b, st));
+                else CKS(h, tce_launch_quartets_r1(h->S, w.cls, b, st));
+            }
         }
     }
     return TCE_OK;

@@ -67,6 +67,8 @@ struct DevSys {
     // t tables
     const double *tnode, *tweight, *Tt;   // Tt[(d*(ncap+1)+n)*nq + k]
     int gmax[3][TCE_MAXG];                // per 8-node group: last n with a nonzero entry
+    const int *rule_gmax;                 // the same on the device, [d * TCE_MAXG + g]
+    const float2 *rule_t2;                // per 8-node group: smallest and largest t^2
     // Schwarz
     const double *Q;
 };
@@ -80,6 +82,7 @@ struct RuleDev {
     int nn;            // real nodes (2n+1 of the Kronrod rule)
     int nq;            // padded node count: 32 or 64
     int gmax[3 * TCE_MAXG];
+    float2 t2[TCE_MAXG];   // per 8-node group: smallest and largest t^2 of its real nodes (inf, -inf when it has none)
 };
 
 // ---------------------------------------------------------------------------

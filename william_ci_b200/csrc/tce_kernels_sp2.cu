@@ -1,26 +1,26 @@
 // tce_kernels_sp2.cu -- the s/p tensor-core kernel (k_quartets_sp_tc,
 // tce_kernels_tc.cuh) for the six classes with two p shells of one periodic
-// direction, in its three tile shapes: 8 primitive quartets x 16, 32 or 64
-// nodes per pass (four power combinations per step loop).
+// direction (four power combinations per step loop), learned grid and system
+// rule: 8 primitive quartets x 16 (shape 1) or 8 (shapes 2 and 3) nodes per pass.
 #include "tce_kernels_tc.cuh"
 
-int tce_sp2_launch(const DevSys &S, int cls, const SArgs &A, int nq, int shape, int nsm, cudaStream_t st)
+template <int NT, bool LG>
+static int sp2_launch(const DevSys &S, int cls, const SArgs &A, int nsm, cudaStream_t st)
 {
-#define TCE_SP2(NQv, MTv, NTv)                                                     \
-    switch (cls) {                                                                 \
-    case 3: sp_tc_launch<NQv, 1, 1, 0, 0, MTv, NTv>(S, A, nsm, st); break;         \
-    case 5: sp_tc_launch<NQv, 1, 0, 1, 0, MTv, NTv>(S, A, nsm, st); break;         \
-    case 6: sp_tc_launch<NQv, 0, 1, 1, 0, MTv, NTv>(S, A, nsm, st); break;         \
-    case 9: sp_tc_launch<NQv, 1, 0, 0, 1, MTv, NTv>(S, A, nsm, st); break;         \
-    case 10: sp_tc_launch<NQv, 0, 1, 0, 1, MTv, NTv>(S, A, nsm, st); break;        \
-    case 12: sp_tc_launch<NQv, 0, 0, 1, 1, MTv, NTv>(S, A, nsm, st); break;        \
-    default: return TCE_ERR_UNSUPPORTED;                                           \
+    switch (cls) {
+    case 3: sp_tc_launch<1, 1, 0, 0, 1, NT, LG>(S, A, nsm, st); break;
+    case 5: sp_tc_launch<1, 0, 1, 0, 1, NT, LG>(S, A, nsm, st); break;
+    case 6: sp_tc_launch<0, 1, 1, 0, 1, NT, LG>(S, A, nsm, st); break;
+    case 9: sp_tc_launch<1, 0, 0, 1, 1, NT, LG>(S, A, nsm, st); break;
+    case 10: sp_tc_launch<0, 1, 0, 1, 1, NT, LG>(S, A, nsm, st); break;
+    case 12: sp_tc_launch<0, 0, 1, 1, 1, NT, LG>(S, A, nsm, st); break;
+    default: return TCE_ERR_UNSUPPORTED;
     }
-    if (nq == 32) {
-        if (shape == 1) { TCE_SP2(32, 1, 2) } else { TCE_SP2(32, 1, 4) }
-    } else {
-        if (shape == 1) { TCE_SP2(64, 1, 2) } else if (shape == 2) { TCE_SP2(64, 1, 4) } else { TCE_SP2(64, 1, 8) }
-    }
-#undef TCE_SP2
     return TCE_OK;
+}
+
+int tce_sp2_launch(const DevSys &S, int cls, const SArgs &A, int shape, int nsm, cudaStream_t st)
+{
+    if (!A.item_rule) return sp2_launch<2, false>(S, cls, A, nsm, st);
+    return shape == 1 ? sp2_launch<2, true>(S, cls, A, nsm, st) : sp2_launch<1, true>(S, cls, A, nsm, st);
 }

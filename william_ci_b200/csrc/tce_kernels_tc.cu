@@ -1,45 +1,45 @@
-// tce_kernels_tc.cu -- all-s shell quartets of one periodic direction with
-// per-quartet learned-grid rules, the node sums on the FP64 tensor cores.
+// tce_kernels_tc.cu -- all-s shell quartets, the node sums on the FP64 tensor
+// cores, with per-quartet learned-grid rules (LG) or the system's rule.
 //
 // The quartet is the one k_quartets_s evaluates (ERI_shell_block_toroidal.f90
 // :28-366 for s functions, scattered like direct_JK, eri_direct.f90:331-357).
-// For a batch of up to 16 primitive quartets pq (sorted by truncation order)
-// the periodic direction needs, per node k of the quartet's rule,
-//     I[pq][k] = sum_n F[pq][n] T[n][k],   F[pq][n] = G_n H_n cos(n phi_pq)
-// (n <= min(N_bra, N_ket); T[n][k] = c_n e^{-C_k} I_n(C_k), rows past the node
-// group's truncation order skipped).  Per pass of 32 nodes this is a
-// (16 x N) x (N x 32) product: one warp holds it as 2 x 4 tiles of 8 x 8 and
-// issues mma.sync.m8n8k4 (FP64) per tile and step of four orders n.  A
-// fragments (F) are built in registers by the lanes that own them: lane l
-// holds rows 8 m + l/4 (m = 0, 1) and order 4 s + l%4, with cos(n phi) from
-// the three-term recurrence in steps of four (re-seeded every 32 orders).
-// B fragments are T[4 s + l%4][8 g + l/4], one load per tile column.  The
-// G, H and T values of the next step are loaded before the current step's
-// mma instructions are issued.  The
-// epilogue (real directions, weights, Kronrod and Gauss sums, the judge and
-// the J/K scatter) is the one of k_quartets_s.
+// A batch of 8 MT primitive quartets pq, sorted by concentration, needs per
+// periodic direction and node k of the rule
+//     I[pq][k] = h sum_j F[pq][h j] T[h j][k],   F[pq][n] = G_n H_n cos(n phi_pq),
+// with the stride h and last order that tce_order_plan finds for the batch and
+// a pass of NT node tiles of 8 (T[n][k] = c_n e^{-C_k} I_n(C_k)): an (8 MT x J)
+// x (J x 8 NT) product per pass, mma.sync.m8n8k4 (FP64) per 8 x 8 tile and step
+// of four orders.  Lane l builds the A fragments (F) of rows 8 m + l/4 at order
+// h (4 s + l%4), cos(n phi) from the three-term recurrence in steps of 4 h
+// (re-seeded every eight steps); the B fragments are T[h (4 s + l%4)][8 g + l/4].
+// The next step's G, H and T are loaded before the current step's mma.
+//
+// What bounds it: with every order summed (about 170 per node on the 64-cell
+// chain) the mma instructions did; with 13 to 27 orders per tile the epilogue
+// (one reciprocal per two nodes), the plans and the loads' latency weigh as
+// much.  Passes of 16 nodes share one plan: 8-node passes need as many tile
+// products and twice the fragments, 32-node passes twice the tile products,
+// because the node with the smallest C sets the stride.
+// 64-cell chain, all-s 64-node list 16.4 -> 8.2 ms, 32-node list 6.5 -> 4.8 ms;
+// fixed 32-node rule, whole pass 72.7 -> 16.7 ms.
 //
 // Also here: the launch of the s/p tensor-core kernel (k_quartets_sp_tc,
 // tce_kernels_tc.cuh) for the classes with one p shell; those with two are
 // instantiated in tce_kernels_sp2.cu.
 #include "tce_kernels_tc.cuh"
 
-// MT row tiles of 8 per warp: batches of 8 MT primitive quartets; acc holds
-// the batch's 8 MT rows x 8 NT nodes of one pass (MT x NT tiles, 2 per lane).
-// The all-s and the s/p kernels take (MT, NT) as template parameters, their
-// tile shapes (tce_tc_shapes_s, tce_tc_shapes_sp) chosen per work list by
-// tce_lg_autotune.
-
-template <int NQ, int MTP, int NTP>
+// A batch is 8 MT primitive quartets, a pass NT node tiles of 8 for one set of
+// orders; (MT, NT) are template parameters, chosen per work list by
+// tce_lg_autotune (tce_tc_shapes_s, tce_tc_shapes_sp).
+template <int NDP, int MT, int NT, bool LG>
 __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
 {
-    constexpr int MT = MTP, BT = 8 * MTP;
-    constexpr int NT = (NQ / 8) < NTP ? (NQ / 8) : NTP;   // node tiles per pass
+    constexpr int BT = 8 * MT;
+    constexpr float E = tce_order_exponent(0);
     extern __shared__ double smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int rq = lane >> 2, cq = lane & 3;   // fragment row in an 8-row tile, fragment column
     const PrimPool Pool = tce_pool(smem, wib);
-    const double PI2 = PI_D * PI_D;
 
     while (true) {
         int it = 0;
@@ -47,10 +47,34 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= A.nitems) break;
         const int4 q = A.items[it];
-        const RuleDev *D = A.rules + A.item_rule[it];
-        const double *Tg = A.rule_T + D->T_off;   // direction 0: (ncap + 1) rows of NQ nodes
-        const int *gm = D->gmax;
-        const double *tn = A.rule_t + D->node_off, *wk = A.rule_wk + D->node_off, *wg = A.rule_wg + D->node_off;
+        const TcRule R = tce_tc_rule<LG>(S, A, it);
+        const int nq = R.nq, ng = nq / 8, nchunk = (ng + NT - 1) / NT;
+        // lane c holds what pass c needs to know of its nodes: 1/C = a^2 / (2 t^2), last stored order
+        float vmin[NDP], vmax[NDP];
+        int glast[NDP];
+        {
+            float lo = __int_as_float(0x7f800000), hi = -lo;
+#pragma unroll
+            for (int d = 0; d < NDP; ++d) glast[d] = -1;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const int g = lane * NT + t;
+                if (g < ng) {
+                    const float2 w = R.t2[g];
+                    lo = fminf(lo, w.x);
+                    hi = fmaxf(hi, w.y);
+#pragma unroll
+                    for (int d = 0; d < NDP; ++d) glast[d] = max(glast[d], R.gmax[d * TCE_MAXG + g]);
+                }
+            }
+#pragma unroll
+            for (int d = 0; d < NDP; ++d) {
+                const float a2 = 0.5f * (float)(S.a[d] * S.a[d]);
+                vmin[d] = a2 / hi;
+                vmax[d] = a2 / lo;
+                if (!(lo <= hi)) glast[d] = -1;   // padding nodes only
+            }
+        }
         const int cK = q.z / S.nshuc;
         const int SK0 = q.z - cK * S.nshuc;
         const int SLp = tce_shift_to(q.w, cK, S.nshuc, S.ncl);
@@ -61,153 +85,223 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
         for (int d = 0; d < 3; ++d) Tsh[d] = S.sh_r[3 * q.z + d] - S.sh_r[3 * SK0 + d];
         const int nppb = Ub.npp, nppk = Uk.npp;
         const long long total = (long long)nppb * nppk;
-        const double *Gbase = reinterpret_cast<const double *>(S.vec + Ub.vec_off);
-        const double *Hbase = reinterpret_cast<const double *>(S.vec + Uk.vec_off + (long long)Uk.Nlen * nppk);
         double blk = 0.0, blkG = 0.0;
         int np = 0;
         for (long long base = 0; base < total; base += 32) {
-            np = tce_pool_add<true>(S, A, Ub, Uk, q, base, total, lane, Pool, np);
-            const bool last = base + 32 >= total;
-            if (!(np > TCE_POOL - 32 || (last && np > 0))) continue;
-            if (np > BT) tce_pool_sort(Pool, np, lane);
-            const int nproc = last ? np : (np & ~(BT - 1));
-            for (int b0 = 0; b0 < nproc; b0 += BT) {
-                const int nb = nproc - b0 < BT ? nproc - b0 : BT;
-                const int nmax = Pool.key[b0];   // largest truncation order of the batch (sorted)
-                // this lane's fragment rows: primitive quartets 8 m + rq of the batch
-                int goff[MT], hoff[MT], nmr[MT];
+            np = tce_pool_add<true, NDP>(S, A, Ub, Uk, q, base, total, lane, Pool, np);
+            if (!(np > TCE_POOL - 32 || (base + 32 >= total && np > 0))) continue;
+            tce_pool_order(Pool, np, lane);
+            for (int b0 = 0; b0 < np; b0 += BT) {
+                // this lane's fragment rows (primitive quartets 8 m + rq of the batch; past
+                // its end the first one, with factor zero)
+                const double *Gp[NDP][MT], *Hp[NDP][MT];
+                double f[MT], pq_[MT], ps[MT], R2[MT], c1[NDP][MT], s1[NDP][MT];
+                double phi[NDP][MT];
+                float umin[NDP], umax[NDP], pmin[NDP], pmax[NDP];
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
-                    const int r = 8 * m + rq;
-                    nmr[m] = -1;
-                    goff[m] = hoff[m] = 0;
-                    if (r < nb) {
-                        const int2 pq = Pool.pq[b0 + r];
-                        nmr[m] = Pool.key[b0 + r];
-                        goff[m] = 2 * pq.x;
-                        hoff[m] = 2 * pq.y;
+                    const int r = b0 + 8 * m + rq;
+                    const int e = Pool.key[r < np ? r : b0];
+                    const int2 pq = Pool.pq[e];
+                    f[m] = r < np ? Pool.fac[e] : 0.0;
+                    const PairPrim &Pb = S.pp[Ub.pp_off + pq.x];
+                    const PairPrim &Pk = S.pp[Uk.pp_off + pq.y];
+                    pq_[m] = Pb.esum * Pk.esum;
+                    ps[m] = Pb.esum + Pk.esum;
+                    R2[m] = 0.0;
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const double x = Pb.cen[d] - (Pk.cen[d] + Tsh[d]);
+                        if (d < NDP) {
+                            phi[d < NDP ? d : 0][m] = S.a[d] * x;
+                            const float u = 1.0f / (float)Pb.A[d] + 1.0f / (float)Pk.A[d], ap = tce_fold_phase(S.a[d] * x);
+                            umin[d < NDP ? d : 0] = m == 0 ? u : fminf(umin[d < NDP ? d : 0], u);
+                            umax[d < NDP ? d : 0] = m == 0 ? u : fmaxf(umax[d < NDP ? d : 0], u);
+                            pmin[d < NDP ? d : 0] = m == 0 ? ap : fminf(pmin[d < NDP ? d : 0], ap);
+                            pmax[d < NDP ? d : 0] = m == 0 ? ap : fmaxf(pmax[d < NDP ? d : 0], ap);
+                        } else {
+                            R2[m] += x * x;
+                        }
+                    }
+#pragma unroll
+                    for (int d = 0; d < NDP; ++d) {
+                        Gp[d][m] = reinterpret_cast<const double *>(S.vec + Ub.vec_off + (long long)(2 * d) * Ub.Nlen * nppb + pq.x);
+                        Hp[d][m] = reinterpret_cast<const double *>(S.vec + Uk.vec_off + (long long)(2 * d + 1) * Uk.Nlen * nppk + pq.y);
                     }
                 }
-                // phase of row m, from the pool entry (read again where the recurrence is re-seeded)
-                auto phase = [&](int m) {
-                    const int r = 8 * m + rq;
-                    if (r >= nb) return 0.0;
-                    const int2 pq = Pool.pq[b0 + r];
-                    return S.a[0] * (S.pp[Ub.pp_off + pq.x].cen[0] - (S.pp[Uk.pp_off + pq.y].cen[0] + Tsh[0]));
-                };
+                OrderPlan plan[NDP];   // of pass `lane`
+#pragma unroll
+                for (int d = 0; d < NDP; ++d) {
+#pragma unroll
+                    for (int o = 4; o < 32; o <<= 1) {
+                        umin[d] = fminf(umin[d], __shfl_xor_sync(0xffffffffu, umin[d], o));
+                        umax[d] = fmaxf(umax[d], __shfl_xor_sync(0xffffffffu, umax[d], o));
+                        pmin[d] = fminf(pmin[d], __shfl_xor_sync(0xffffffffu, pmin[d], o));
+                        pmax[d] = fmaxf(pmax[d], __shfl_xor_sync(0xffffffffu, pmax[d], o));
+                    }
+                    const int nlast = min(glast[d], min(Ub.Nlen, Uk.Nlen) - 1);
+                    plan[d] = tce_order_plan(E, 0, umin[d], umax[d], pmin[d], pmax[d], vmin[d], vmax[d], nlast);
+                    if (glast[d] < 0) plan[d].h = 0;
+                }
+                double vK[MT], vG[MT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) vK[m] = vG[m] = 0.0;
 #pragma unroll 1
-                for (int g0 = 0; g0 < NQ / 8; g0 += NT) {
-                    int gmb[NT], nend = -1;
+                for (int c = 0; c < nchunk; ++c) {
+                    // cos, sin of h phi for four passes at a time: lane column cq computes pass c + cq's
+                    if ((c & 3) == 0) {
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) {
-                        gmb[t] = gm[g0 + t];
-                        nend = gmb[t] > nend ? gmb[t] : nend;
+                        for (int d = 0; d < NDP; ++d) {
+                            const double hd = (double)__shfl_sync(0xffffffffu, plan[d].h, c + cq);
+#pragma unroll
+                            for (int m = 0; m < MT; ++m) sincos(hd * phi[d][m], &s1[d][m], &c1[d][m]);
+                        }
                     }
-                    nend = nend < nmax ? nend : nmax;
-                    double acc[2 * MT * NT];
+                    double pr[2 * MT * NT];
+                    bool none = false;
+                    double hw = 1.0;
+                    int h[NDP], last[NDP];
 #pragma unroll
-                    for (int x = 0; x < 2 * MT * NT; ++x) acc[x] = 0.0;
-                    double cc[MT], cp[MT], c4[MT];   // cos(n phi), cos((n - 4) phi), 2 cos(4 phi)
-                    double gN[MT], hN[MT];           // G_n, H_n of the next step (prefetched)
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const double ph = phase(m);
-                        cc[m] = cos((double)cq * ph);
-                        cp[m] = cos((double)(cq - 4) * ph);
-                        c4[m] = 2.0 * cos(4.0 * ph);
-                        const bool ok = cq <= nmr[m];
-                        gN[m] = ok ? __ldg(Gbase + goff[m] + 2 * (size_t)cq * nppb) : 0.0;
-                        hN[m] = ok ? __ldg(Hbase + hoff[m] + 2 * (size_t)cq * nppk) : 0.0;
+                    for (int d = 0; d < NDP; ++d) {
+                        h[d] = __shfl_sync(0xffffffffu, plan[d].h, c);
+                        last[d] = __shfl_sync(0xffffffffu, plan[d].last, c);
+                        none = none || h[d] == 0;
+                        hw *= (double)h[d];
                     }
-                    double tN[NT];                    // T fragments of the next step
+                    if (none) continue;
+                    int col[NT];
 #pragma unroll
-                    for (int t = 0; t < NT; ++t)
-                        tN[t] = (0 <= gmb[t] && cq <= S.ncap) ? __ldg(Tg + (size_t)cq * NQ + 8 * (g0 + t) + rq) : 0.0;
-#pragma unroll 2
-                    for (int s4 = 0; s4 <= nend; s4 += 4) {
-                        const int n = s4 + cq, n1 = n + 4;
-                        double F[MT], Tb[NT];
+                    for (int t = 0; t < NT; ++t) col[t] = 8 * min(c * NT + t, ng - 1) + rq;
+#pragma unroll
+                    for (int d = 0; d < NDP; ++d) {
+                        double acc[2 * MT * NT];
+#pragma unroll
+                        for (int x = 0; x < 2 * MT * NT; ++x) acc[x] = 0.0;
+                        double cc[MT], cp[MT], c4[MT];   // cos(n phi), cos((n - 4 h) phi), 2 cos(4 h phi)
 #pragma unroll
                         for (int m = 0; m < MT; ++m) {
-                            F[m] = gN[m] * hN[m] * cc[m];
-                            const bool ok = n1 <= nmr[m];
-                            gN[m] = ok ? __ldg(Gbase + goff[m] + 2 * (size_t)n1 * nppb) : 0.0;
-                            hN[m] = ok ? __ldg(Hbase + hoff[m] + 2 * (size_t)n1 * nppk) : 0.0;
+                            const int src = (lane & ~3) | (c & 3);
+                            const double cb = __shfl_sync(0xffffffffu, c1[d][m], src);
+                            const double sb = __shfl_sync(0xffffffffu, s1[d][m], src);
+                            double u0, u1;
+                            tce_phase_start(cb, sb, cq, cc[m], u0, cp[m], u1, c4[m]);
                         }
-#pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            Tb[t] = tN[t];
-                            tN[t] = (s4 + 4 <= gmb[t] && n1 <= S.ncap)
-                                        ? __ldg(Tg + (size_t)n1 * NQ + 8 * (g0 + t) + rq) : 0.0;
-                        }
-                        if (((s4 + 4) & 31) == 0) {   // re-seed the recurrence
+                        const double *Tg = R.T + d * R.strideD;
+                        const int steps = last[d] / (4 * h[d]) + 1, h4 = 4 * h[d];
+                        int n = h[d] * cq;
+                        double gN[MT], hN[MT], tN[NT];
+                        auto load = [&]() {   // the values of order n (past the last order: T = 0)
+                            const int nn = min(n, last[d]);
 #pragma unroll
                             for (int m = 0; m < MT; ++m) {
-                                const double ph = phase(m);
-                                cp[m] = cos((double)n * ph);
-                                cc[m] = cos((double)n1 * ph);
+                                gN[m] = __ldg(Gp[d][m] + (long long)nn * (2 * nppb));
+                                hN[m] = __ldg(Hp[d][m] + (long long)nn * (2 * nppk));
                             }
-                        } else {
 #pragma unroll
-                            for (int m = 0; m < MT; ++m) {
-                                const double t = c4[m] * cc[m] - cp[m];
-                                cp[m] = cc[m];
-                                cc[m] = t;
+                            for (int t = 0; t < NT; ++t) {
+                                const double tv = __ldg(Tg + ((long long)nn * nq + col[t]));
+                                tN[t] = n <= last[d] ? tv : 0.0;
                             }
-                        }
+                            n += h4;
+                        };
+                        load();
+#pragma unroll 2
+                        for (int s = 0; s < steps; ++s) {
+                            double F[MT], Tb[NT];
 #pragma unroll
-                        for (int t = 0; t < NT; ++t)
-                            if (s4 <= gmb[t]) {
+                            for (int m = 0; m < MT; ++m) F[m] = gN[m] * hN[m] * cc[m];
+#pragma unroll
+                            for (int t = 0; t < NT; ++t) Tb[t] = tN[t];
+                            load();
+                            if ((s & 7) == 7) {   // re-seed the recurrence
+#pragma unroll
+                                for (int m = 0; m < MT; ++m) {
+                                    cp[m] = cos((double)(n - 2 * h4) * phi[d][m]);
+                                    cc[m] = cos((double)(n - h4) * phi[d][m]);
+                                }
+                            } else {
+#pragma unroll
+                                for (int m = 0; m < MT; ++m) {
+                                    const double t = c4[m] * cc[m] - cp[m];
+                                    cp[m] = cc[m];
+                                    cc[m] = t;
+                                }
+                            }
+#pragma unroll
+                            for (int t = 0; t < NT; ++t)
 #pragma unroll
                                 for (int m = 0; m < MT; ++m) tce_dmma(acc[(m * NT + t) * 2], acc[(m * NT + t) * 2 + 1], F[m], Tb[t]);
-                            }
-                    }
-                    // epilogue: acc[2 (m NT + t) + i] = I[8 m + rq][8 (g0 + t) + 2 cq + i]
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const int r = 8 * m + rq;
-                        if (r >= nb) continue;
-                        const int2 pq = Pool.pq[b0 + r];
-                        const PairPrim &Pb = S.pp[Ub.pp_off + pq.x];
-                        const PairPrim &Pk = S.pp[Uk.pp_off + pq.y];
-                        const double p = Pb.esum, qq = Pk.esum, pq_ = p * qq, ps = p + qq;
-                        double R2 = 0.0;
-#pragma unroll
-                        for (int dd = 1; dd < 3; ++dd) {
-                            const double R = Pb.cen[dd] - (Pk.cen[dd] + Tsh[dd]);
-                            R2 += R * R;
                         }
-                        double vK = 0.0, vG = 0.0;
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            if (gmb[t] < 0) continue;   // padding nodes
+                        for (int x = 0; x < 2 * MT * NT; ++x) pr[x] = d == 0 ? acc[x] : pr[x] * acc[x];
+                    }
+                    // epilogue: pr[2 (m NT + t) + i] = prod_d I_d[8 m + rq][8 (c NT + t) + 2 cq + i] / h_d
 #pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                const int k = 8 * (g0 + t) + 2 * cq + i;
-                                const double t2 = tn[k] * tn[k];
-                                const double D2 = 1.0 / (pq_ + ps * t2);
-                                const double e = (R2 == 0.0) ? 1.0 : exp(-(pq_ * t2 * D2) * R2);
-                                const double bse = acc[(m * NT + t) * 2 + i] * (PI2 * D2 * e);
-                                vK = fma(bse, wk[k], vK);
-                                vG = fma(bse, wg[k], vG);
+                    for (int t = 0; t < NT; ++t) {
+                        if (NT > 1 && c * NT + t >= ng) continue;
+                        const int k = 8 * (c * NT + t) + 2 * cq;
+                        const double2 tn = *reinterpret_cast<const double2 *>(R.t + k);
+                        double2 wk = *reinterpret_cast<const double2 *>(R.wk + k), wg = make_double2(0.0, 0.0);
+                        if (LG) {
+                            wg = *reinterpret_cast<const double2 *>(R.wg + k);
+                            wg.x *= hw;
+                            wg.y *= hw;
+                        }
+                        wk.x *= hw;
+                        wk.y *= hw;
+                        const double t20 = tn.x * tn.x, t21 = tn.y * tn.y;
+#pragma unroll
+                        for (int m = 0; m < MT; ++m) {
+                            double b0_ = pr[(m * NT + t) * 2], b1_ = pr[(m * NT + t) * 2 + 1];
+                            if (NDP < 3) {
+                                const double d0 = fma(ps[m], t20, pq_[m]), d1 = fma(ps[m], t21, pq_[m]);
+                                double D0, D1;   // 1 / d0 and 1 / d1
+                                if (NDP == 1) {
+                                    const double ri = 1.0 / (d0 * d1);
+                                    D0 = ri * d1;
+                                    D1 = ri * d0;
+                                    b0_ *= D0;
+                                    b1_ *= D1;
+                                } else {
+                                    const double r0 = rsqrt(d0), r1 = rsqrt(d1);
+                                    D0 = r0 * r0;
+                                    D1 = r1 * r1;
+                                    b0_ *= r0;
+                                    b1_ *= r1;
+                                }
+                                if (R2[m] != 0.0) {
+                                    const double w = -pq_[m] * R2[m];
+                                    b0_ *= exp(w * t20 * D0);
+                                    b1_ *= exp(w * t21 * D1);
+                                }
+                            }
+                            vK[m] = fma(b0_, wk.x, vK[m]);
+                            vK[m] = fma(b1_, wk.y, vK[m]);
+                            if (LG) {
+                                vG[m] = fma(b0_, wg.x, vG[m]);
+                                vG[m] = fma(b1_, wg.y, vG[m]);
                             }
                         }
-                        const double f = Pool.fac[b0 + r];
-                        blk = fma(f, vK, blk);
-                        blkG = fma(f, vG, blkG);
                     }
+                }
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    blk = fma(f[m], vK[m], blk);
+                    if (LG) blkG = fma(f[m], vG[m], blkG);
                 }
             }
             __syncwarp();
-            if (np > nproc) tce_pool_carry(Pool, nproc, np - nproc, lane);
-            np -= nproc;
+            np = 0;
         }
-        blk = tce_warp_sum(blk);
-        blkG = tce_warp_sum(blkG);
-        if (!tce_judge_accepts(fabs(blk - blkG), fabs(blk), A.judge_tol)) {
-            if (lane == 0) tce_queue_fallback(A, q);
-            __syncwarp();
-            continue;
+        const double rc = NDP == 1 ? PI_D * PI_D : NDP == 2 ? PI_D : 1.0;   // the real directions' pi^(3 - ndp)
+        blk = tce_warp_sum(blk) * rc;
+        if (LG) {
+            blkG = tce_warp_sum(blkG) * rc;
+            if (!tce_judge_accepts(fabs(blk - blkG), fabs(blk), A.judge_tol)) {
+                if (lane == 0) tce_queue_fallback(A, q);
+                __syncwarp();
+                continue;
+            }
         }
         if (lane == 0) {
             const int fI = S.sh_first[q.x], fJ = S.sh_first[q.y], fK = S.sh_first[q.z], fL = S.sh_first[q.w];
@@ -224,21 +318,22 @@ int tce_tc_shapes_sp(int nq)
     return nq == 64 ? 3 : nq == 32 ? 2 : 0;
 }
 
-// one p shell.  shape 1: 8 rows x 32 nodes per pass, 2: 16 x 32, 3: 8 x 64
-static int sp1_launch(const DevSys &S, int cls, const SArgs &A, int nq, int shape, int nsm, cudaStream_t st)
+// one p shell.  shape 1: 8 rows x 16 nodes per pass, 2: 16 x 16, 3: 8 x 8
+template <bool LG>
+static int sp1_launch(const DevSys &S, int cls, const SArgs &A, int shape, int nsm, cudaStream_t st)
 {
-#define TCE_SP1(NQv, MTv, NTv)                                                     \
-    switch (cls) {                                                                 \
-    case 1: sp_tc_launch<NQv, 1, 0, 0, 0, MTv, NTv>(S, A, nsm, st); break;         \
-    case 2: sp_tc_launch<NQv, 0, 1, 0, 0, MTv, NTv>(S, A, nsm, st); break;         \
-    case 4: sp_tc_launch<NQv, 0, 0, 1, 0, MTv, NTv>(S, A, nsm, st); break;         \
-    case 8: sp_tc_launch<NQv, 0, 0, 0, 1, MTv, NTv>(S, A, nsm, st); break;         \
-    default: return TCE_ERR_UNSUPPORTED;                                           \
+#define TCE_SP1(MTv, NTv)                                                              \
+    switch (cls) {                                                                     \
+    case 1: sp_tc_launch<1, 0, 0, 0, MTv, NTv, LG>(S, A, nsm, st); break;              \
+    case 2: sp_tc_launch<0, 1, 0, 0, MTv, NTv, LG>(S, A, nsm, st); break;              \
+    case 4: sp_tc_launch<0, 0, 1, 0, MTv, NTv, LG>(S, A, nsm, st); break;              \
+    case 8: sp_tc_launch<0, 0, 0, 1, MTv, NTv, LG>(S, A, nsm, st); break;              \
+    default: return TCE_ERR_UNSUPPORTED;                                               \
     }
-    if (nq == 32) {
-        if (shape == 1) { TCE_SP1(32, 1, 4) } else { TCE_SP1(32, 2, 4) }
+    if constexpr (!LG) {
+        TCE_SP1(1, 2)
     } else {
-        if (shape == 1) { TCE_SP1(64, 1, 4) } else if (shape == 2) { TCE_SP1(64, 2, 4) } else { TCE_SP1(64, 1, 8) }
+        if (shape == 1) { TCE_SP1(1, 2) } else if (shape == 2) { TCE_SP1(2, 2) } else { TCE_SP1(1, 1) }
     }
 #undef TCE_SP1
     return TCE_OK;
@@ -246,16 +341,20 @@ static int sp1_launch(const DevSys &S, int cls, const SArgs &A, int nq, int shap
 
 int tce_launch_quartets_sp_tc(const DevSys &S, int cls, const SArgsHost &h, int nq, int shape, cudaStream_t st)
 {
-    if (!h.item_rule || !h.rules || !h.rule_T || !h.fb_items || !h.fb_count) return TCE_ERR_ARG;
-    if (S.ndp != 1 || (nq != 32 && nq != 64)) return TCE_ERR_UNSUPPORTED;
-    if (shape < 1 || shape > tce_tc_shapes_sp(nq)) return TCE_ERR_ARG;
+    const bool lg = h.item_rule != nullptr;
+    if (lg && (!h.rules || !h.rule_T || !h.fb_items || !h.fb_count)) return TCE_ERR_ARG;
+    if (S.ndp != 1) return TCE_ERR_UNSUPPORTED;
+    if (lg && (nq != 32 && nq != 64)) return TCE_ERR_UNSUPPORTED;
+    if (shape < 1 || shape > 3) return TCE_ERR_ARG;
     const int np = __builtin_popcount(cls & 15);
     if (cls < 1 || cls > 15 || np > 2) return TCE_ERR_UNSUPPORTED;
     SArgs A{};
     tc_args(A, h);
     if (cudaMemsetAsync(h.next, 0, sizeof(unsigned int), st) != cudaSuccess) return TCE_ERR_CUDA;
     const int nsm = h.num_sms > 0 ? h.num_sms : 148;
-    const int s = np == 1 ? sp1_launch(S, cls, A, nq, shape, nsm, st) : tce_sp2_launch(S, cls, A, nq, shape, nsm, st);
+    const int s = np == 2 ? tce_sp2_launch(S, cls, A, shape, nsm, st)
+                  : lg    ? sp1_launch<true>(S, cls, A, shape, nsm, st)
+                          : sp1_launch<false>(S, cls, A, 1, nsm, st);
     if (s != TCE_OK) return s;
     return cudaGetLastError() == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }
@@ -265,30 +364,34 @@ int tce_tc_shapes_s(int nq)
     return (nq == 32 || nq == 64) ? 5 : 0;
 }
 
-// shape 1: 16 rows x 32 nodes per pass (the default), 2: 32 x 16, 3: 16 x 16,
-// 4: 8 rows x 64 nodes (x 32 for 32-node rules), 5: 8 x 32
+// shape 1: 16 rows x 16 nodes per pass (the default), 2: 8 x 16, 3: 16 x 8,
+// 4: 8 x 8, 5: 16 x 32
 int tce_launch_quartets_s_tc(const DevSys &S, const SArgsHost &h, int nq, int shape, cudaStream_t st)
 {
-    if (!h.item_rule || !h.rules || !h.rule_T || !h.fb_items || !h.fb_count) return TCE_ERR_ARG;
-    if (S.ndp != 1 || (nq != 32 && nq != 64)) return TCE_ERR_UNSUPPORTED;
-    if (shape < 1 || shape > tce_tc_shapes_s(nq)) return TCE_ERR_ARG;
+    const bool lg = h.item_rule != nullptr;
+    if (lg && (!h.rules || !h.rule_T || !h.fb_items || !h.fb_count)) return TCE_ERR_ARG;
+    if (lg && (nq != 32 && nq != 64)) return TCE_ERR_UNSUPPORTED;
+    if (shape < 1 || shape > 5) return TCE_ERR_ARG;
     SArgs A{};
     tc_args(A, h);
     if (cudaMemsetAsync(h.next, 0, sizeof(unsigned int), st) != cudaSuccess) return TCE_ERR_CUDA;
     const int nsm = h.num_sms > 0 ? h.num_sms : 148;
-#define TCE_S_TC(NQv)                                                              \
-    switch (shape) {                                                               \
-    case 1: tc_launch(k_quartets_s_tc<NQv, 2, 4>, S, A, nsm, st); break;           \
-    case 2: tc_launch(k_quartets_s_tc<NQv, 4, 2>, S, A, nsm, st); break;           \
-    case 3: tc_launch(k_quartets_s_tc<NQv, 2, 2>, S, A, nsm, st); break;           \
-    case 4: tc_launch(k_quartets_s_tc<NQv, 1, 8>, S, A, nsm, st); break;           \
-    default: tc_launch(k_quartets_s_tc<NQv, 1, 4>, S, A, nsm, st); break;          \
-    }
-    if (nq == 32) {
-        TCE_S_TC(32)
+    if (!lg) {
+        if (S.ndp == 1) tc_launch(k_quartets_s_tc<1, 2, 2, false>, S, A, nsm, st);
+        else if (S.ndp == 2) tc_launch(k_quartets_s_tc<2, 1, 2, false>, S, A, nsm, st);
+        else tc_launch(k_quartets_s_tc<3, 1, 2, false>, S, A, nsm, st);
+    } else if (S.ndp == 2) {
+        tc_launch(k_quartets_s_tc<2, 1, 2, true>, S, A, nsm, st);
+    } else if (S.ndp == 3) {
+        tc_launch(k_quartets_s_tc<3, 1, 2, true>, S, A, nsm, st);
     } else {
-        TCE_S_TC(64)
+        switch (shape) {
+        case 1: tc_launch(k_quartets_s_tc<1, 2, 2, true>, S, A, nsm, st); break;
+        case 2: tc_launch(k_quartets_s_tc<1, 1, 2, true>, S, A, nsm, st); break;
+        case 3: tc_launch(k_quartets_s_tc<1, 2, 1, true>, S, A, nsm, st); break;
+        case 4: tc_launch(k_quartets_s_tc<1, 1, 1, true>, S, A, nsm, st); break;
+        default: tc_launch(k_quartets_s_tc<1, 2, 4, true>, S, A, nsm, st); break;
+        }
     }
-#undef TCE_S_TC
     return cudaGetLastError() == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }

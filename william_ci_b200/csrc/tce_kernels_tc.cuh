@@ -1,10 +1,11 @@
-// tce_kernels_tc.cuh -- pieces shared by the FP64 tensor-core kernels of one
-// periodic direction (learned grid): the mma.sync.m8n8k4 (FP64) wrapper, the
-// primitive pool fill, the launch helpers, and the s/p kernel
+// tce_kernels_tc.cuh -- pieces shared by the FP64 tensor-core quartet kernels:
+// the mma.sync.m8n8k4 (FP64) wrapper, the primitive pool fill and its order, the
+// rule view, the launch helpers, and the s/p kernel of one periodic direction
 // k_quartets_sp_tc (one or two p shells), instantiated per class in
 // tce_kernels_tc.cu (one p) and tce_kernels_sp2.cu (two p).
 #pragma once
 #include "tce_kernels_s.cuh"
+#include "tce_orders.cuh"
 
 __device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, double b)
 {
@@ -16,9 +17,10 @@ __device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, doubl
 // Screen the primitive quartets base + lane of a shell quartet (as
 // k_quartets_s) and append the kept ones to the warp's pool: pair indices,
 // factor (FOLD: with the four contraction coefficients of s shells folded in)
-// and the truncation order min(N_bra, N_ket) of the periodic direction.
-// Returns the pool's new fill.
-template <bool FOLD>
+// and the sort key, the bits of u = sum over the periodic directions of
+// 1/A_bra + 1/A_ket with the entry's index in the low seven bits (positive
+// floats order like their bits).  Returns the pool's new fill.
+template <bool FOLD, int NDP>
 __device__ __forceinline__ int tce_pool_add(const DevSys &S, const SArgs &A, const UnitPair &Ub, const UnitPair &Uk,
                                             const int4 &q, long long base, long long total, int lane,
                                             const PrimPool &Pool, int np)
@@ -26,10 +28,11 @@ __device__ __forceinline__ int tce_pool_add(const DevSys &S, const SArgs &A, con
     const int nppk = Uk.npp;
     const long long idx = base + lane;
     bool keep = idx < total;
-    int ipb = 0, ipk = 0, key = 0;
+    int ipb = 0, ipk = 0;
+    float u = 0.0f;
     double fac = 0.0;
     if (keep) {
-        ipb = (int)(idx / nppk);
+        ipb = total <= 0x7fffffffLL ? (int)idx / nppk : (int)(idx / nppk);
         ipk = (int)(idx - (long long)ipb * nppk);
         const PairPrim &Pb = S.pp[Ub.pp_off + ipb];
         const PairPrim &Pk = S.pp[Uk.pp_off + ipk];
@@ -42,18 +45,117 @@ __device__ __forceinline__ int tce_pool_add(const DevSys &S, const SArgs &A, con
             if (FOLD)
                 fac *= S.sh_coef[S.sh_coff[q.x] + ipb / Ub.np2] * S.sh_coef[S.sh_coff[q.y] + ipb % Ub.np2] *
                        S.sh_coef[S.sh_coff[q.z] + ipk / Uk.np2] * S.sh_coef[S.sh_coff[q.w] + ipk % Uk.np2];
-            key = Pb.N[0] < Pk.N[0] ? Pb.N[0] : Pk.N[0];
+#pragma unroll
+            for (int d = 0; d < NDP; ++d) u += 1.0f / (float)Pb.A[d] + 1.0f / (float)Pk.A[d];
         }
     }
     const unsigned msk = __ballot_sync(0xffffffffu, keep);
-    const int pos = __popc(msk & ((1u << lane) - 1u));
+    const int at = np + __popc(msk & ((1u << lane) - 1u));
     if (keep) {
-        Pool.pq[np + pos] = make_int2(ipb, ipk);
-        Pool.fac[np + pos] = fac;
-        Pool.key[np + pos] = key;
+        Pool.pq[at] = make_int2(ipb, ipk);
+        Pool.fac[at] = fac;
+        Pool.key[at] = (int)((__float_as_uint(u) & ~127u) | (unsigned)at);
     }
     __syncwarp();
     return np + __popc(msk);
+}
+
+// Sort the keys of pool entries [0, n), n <= 32 R, ascending in registers
+// (bitonic over lane + 32 r) and write the entries' indices in that order to
+// Pool.key.  Rows of about the same concentration end up in one tile, so that
+// they need about the same orders (tce_orders.cuh).
+template <int R>
+__device__ __forceinline__ void tce_pool_order_r(const PrimPool &P, int n, int lane)
+{
+    unsigned k[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) k[r] = lane + 32 * r < n ? (unsigned)P.key[lane + 32 * r] : 0xffffffffu;
+#pragma unroll
+    for (int s = 2; s <= 32 * R; s <<= 1)
+#pragma unroll
+        for (int j = s >> 1; j > 0; j >>= 1) {
+            if (j >= 32) {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const int x = r ^ (j >> 5);
+                    if (x > r) {
+                        const bool up = ((32 * r) & s) == 0;
+                        const unsigned lo = min(k[r], k[x]), hi = max(k[r], k[x]);
+                        k[r] = up ? lo : hi;
+                        k[x] = up ? hi : lo;
+                    }
+                }
+            } else {
+#pragma unroll
+                for (int r = 0; r < R; ++r) {
+                    const unsigned o = __shfl_xor_sync(0xffffffffu, k[r], j);
+                    const bool up = ((lane + 32 * r) & s) == 0, lower = (lane & j) == 0;
+                    k[r] = up == lower ? min(k[r], o) : max(k[r], o);
+                }
+            }
+        }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+        if (lane + 32 * r < n) P.key[lane + 32 * r] = (int)(k[r] & 127u);
+    __syncwarp();
+}
+__device__ __forceinline__ void tce_pool_order(const PrimPool &P, int n, int lane)
+{
+    __syncwarp();
+    if (n <= 32) tce_pool_order_r<1>(P, n, lane);
+    else if (n <= 64) tce_pool_order_r<2>(P, n, lane);
+    else tce_pool_order_r<4>(P, n, lane);
+}
+
+// The quadrature rule of a shell quartet for the tensor-core kernels: learned
+// grid (LG) a dictionary rule with its judge weights, else the system's rule.
+struct TcRule {
+    const double *T;      // direction d at T + d * strideD, row n at + n * nq
+    long long strideD;
+    const double *t, *wk, *wg;
+    const int *gmax;
+    const float2 *t2;     // per 8-node group: smallest and largest t^2
+    int nq;
+};
+template <bool LG>
+__device__ __forceinline__ TcRule tce_tc_rule(const DevSys &S, const SArgs &A, int it)
+{
+    TcRule R;
+    if (LG) {
+        const RuleDev *D = A.rules + A.item_rule[it];
+        R.nq = D->nq;
+        R.T = A.rule_T + D->T_off;
+        R.t = A.rule_t + D->node_off;
+        R.wk = A.rule_wk + D->node_off;
+        R.wg = A.rule_wg + D->node_off;
+        R.gmax = D->gmax;
+        R.t2 = D->t2;
+    } else {
+        R.nq = S.nq;
+        R.T = S.Tt;
+        R.t = S.tnode;
+        R.wk = S.tweight;
+        R.wg = nullptr;
+        R.gmax = S.rule_gmax;
+        R.t2 = S.rule_t2;
+    }
+    R.strideD = (long long)(S.ncap + 1) * R.nq;
+    return R;
+}
+
+// cos and sin of q phi and (4 - q) phi, q = 0..3, and 2 cos(4 phi), from
+// (c, s) = (cos phi, sin phi): the start of the three-term recurrence in steps of four
+__device__ __forceinline__ void tce_phase_start(double c, double s, int q, double &cc, double &sc, double &cm, double &sm,
+                                                double &c4)
+{
+    const double c2 = fma(-2.0 * s, s, 1.0), s2 = 2.0 * s * c;
+    const double c3 = fma(c2, c, -s2 * s), s3 = fma(s2, c, c2 * s);
+    const double k4 = fma(-2.0 * s2, s2, 1.0), z4 = 2.0 * s2 * c2;
+    cc = q == 0 ? 1.0 : q == 1 ? c : q == 2 ? c2 : c3;
+    sc = q == 0 ? 0.0 : q == 1 ? s : q == 2 ? s2 : s3;
+    cm = q == 0 ? k4 : q == 1 ? c3 : q == 2 ? c2 : c;
+    sm = -(q == 0 ? z4 : q == 1 ? s3 : q == 2 ? s2 : s);
+    c4 = 2.0 * k4;
 }
 
 static inline void tc_args(SArgs &A, const SArgsHost &h)
@@ -92,17 +194,17 @@ static void tc_launch(Kern kern, const DevSys &S, const SArgs &A, int nsm, cudaS
 
 // ============================================================================
 // s/p classes with one or two p shells, one periodic direction
-// (compile-time class LA, LB | LC, LD in {0, 1}), learned grid: the quartet of
+// (compile-time class LA, LB | LC, LD in {0, 1}), learned-grid or system rule: the quartet of
 // ERI_shell_block_toroidal.f90:28-366 for these classes, scattered like
 // direct_JK (eri_direct.f90:331-357), with the node sums on the tensor cores.
 //
 // Power combinations.  The periodic direction has one row per x-power
 // combination (ia, ib | ic, id) of the p shells (2^NP of them):
 //     I_cmb[pq][k] = sum_n Re[G^(ia,ib)_n H^(ic,id)_n e^{i n phi}] T[n][k],
-// all of them in the same step loop: the zero-power vectors G^(0,0), H^(0,0)
-// are real and loaded once for every combination, and cos(n phi), sin(n phi)
-// come from one three-term recurrence in steps of four (re-seeded every 32
-// orders).  The A fragments are F = Re(G H) cos(n phi) - Im(G H) sin(n phi)
+// all of them in the same step loop over the orders of tce_order_plan: the
+// zero-power vectors G^(0,0), H^(0,0) are real and loaded once for every
+// combination, and cos(n phi), sin(n phi) come from one three-term recurrence
+// in steps of four strides (re-seeded every eight steps).  The A fragments are F = Re(G H) cos(n phi) - Im(G H) sin(n phi)
 // with the products of real factors left out.
 //
 // Epilogue by moments.  The real directions add, per node k and component c
@@ -118,19 +220,19 @@ static void tc_launch(Kern kern, const DevSys &S, const SArgs &A, int nsm, cudaS
 //     M_cmb,j = sum_k I_cmb[pq][k] D2 e^{-w R^2} w^j   (Kronrod and Gauss weights)
 // and each component follows once per row: pi^2 a^-xs sum_j P_c[j] M_cmb,j.
 //
-// A batch is 8 MT primitive quartets (rows, sorted by truncation order), a pass
-// NT node tiles of 8; per pass and step of four orders a warp issues
-// 2^NP MT NT mma.sync.m8n8k4.  Shapes with 16 or more accumulator tiles per warp
-// keep them in up to 255 registers (8 warps per SM), the others in 128 (16).
+// A batch is 8 MT primitive quartets (rows, sorted by concentration), a pass
+// NT node tiles of 8 with the orders and stride of tce_order_plan; per pass and
+// step of four orders a warp issues 2^NP MT NT mma.sync.m8n8k4.  The moments of
+// a row are kept over the passes of a batch, the components follow once.
 // ============================================================================
-template <int NQ, int LA, int LB, int LC, int LD, int MTP, int NTP,
-          int MINB = ((1 << (LA + LB + LC + LD)) * MTP * ((NQ / 8) < NTP ? (NQ / 8) : NTP) >= 16 ? 1 : 2)>
-__global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
+template <int LA, int LB, int LC, int LD, int MT, int NT, bool LG>
+__global__ void __launch_bounds__(256, LA + LB + LC + LD == 1 ? 2 : 1) k_quartets_sp_tc(DevSys S, SArgs A)
 {
     constexpr int NP = LA + LB + LC + LD;
     static_assert(NP >= 1 && NP <= 2, "one or two p shells");
-    constexpr int MT = MTP, BT = 8 * MTP;
-    constexpr int NT = (NQ / 8) < NTP ? (NQ / 8) : NTP;   // node tiles per pass
+    constexpr int BT = 8 * MT;
+    constexpr float E = tce_order_exponent(NP);
+    constexpr int SHIFT = LA + LB > LC + LD ? LA + LB : LC + LD;
     constexpr int NA = LA == 0 ? 1 : 3, NB = LB == 0 ? 1 : 3, NC = LC == 0 ? 1 : 3, ND = LD == 0 ? 1 : 3;
     constexpr int NCQ = NA * NB * NC * ND;
     constexpr int NCOMB = (LA + 1) * (LB + 1) * (LC + 1) * (LD + 1);
@@ -138,6 +240,7 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
     constexpr int NN = NP;                                // largest y + z power of a component
     constexpr int EB = tce_ecount(LA, LB), EK = tce_ecount(LC, LD);
     constexpr int AT = 2 * MT * NT;                       // accumulators per combination and lane
+    constexpr int NW = LG ? 2 : 1;                        // Kronrod sums, and Gauss sums with the judge
     extern __shared__ double smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int rq = lane >> 2, cq = lane & 3;   // fragment row in an 8-row tile, fragment column
@@ -158,10 +261,28 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= A.nitems) break;
         const int4 q = A.items[it];
-        const RuleDev *D = A.rules + A.item_rule[it];
-        const double *Tg = A.rule_T + D->T_off;
-        const int *gm = D->gmax;
-        const double *tn = A.rule_t + D->node_off, *wk = A.rule_wk + D->node_off, *wg = A.rule_wg + D->node_off;
+        const TcRule R = tce_tc_rule<LG>(S, A, it);
+        const int nq = R.nq, ng = nq / 8, nchunk = (ng + NT - 1) / NT;
+        // lane c holds what pass c needs to know of its nodes: 1/C = a^2 / (2 t^2), last stored order
+        float vmin, vmax;
+        int glast = -1;
+        {
+            float lo = __int_as_float(0x7f800000), hi = -lo;
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+                const int g = lane * NT + t;
+                if (g < ng) {
+                    const float2 w = R.t2[g];
+                    lo = fminf(lo, w.x);
+                    hi = fmaxf(hi, w.y);
+                    glast = max(glast, R.gmax[g]);
+                }
+            }
+            const float a2 = 0.5f * (float)(S.a[0] * S.a[0]);
+            vmin = a2 / hi;
+            vmax = a2 / lo;
+            if (!(lo <= hi)) glast = -1;   // padding nodes only
+        }
         const int cK = q.z / S.nshuc;
         const int SK0 = q.z - cK * S.nshuc;
         const int SLp = tce_shift_to(q.w, cK, S.nshuc, S.ncl);
@@ -171,87 +292,114 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
         const int nppb = Ub.npp, nppk = Uk.npp;
         const int npA = S.sh_np[q.x], npB = S.sh_np[q.y], npC = S.sh_np[q.z], npD = S.sh_np[q.w];
         const long long total = (long long)nppb * nppk;
-        // power vectors of the periodic direction: bra g = ia + (LA + 1) ib at
-        // Gv + 2 g gl, ket h = ic + (LC + 1) id at Hv + 2 h hl
+        // power vectors of the periodic direction: combination g = ia + (LA + 1) ib
+        // of the bra is the slab ia (LB + 1) + ib, at Gv + 2 slab gl; the ket alike
         const long long gl = (long long)Ub.Nlen * nppb, hl = (long long)Uk.Nlen * nppk;
         const double2 *Gv = S.vec + Ub.vec_off, *Hv = S.vec + Uk.vec_off + hl;
-        const double *G0 = reinterpret_cast<const double *>(Gv), *H0 = reinterpret_cast<const double *>(Hv);
 #pragma unroll
-        for (int c = 0; c < 2 * NCQ; ++c) bacc[c * 32 + lane] = 0.0;
+        for (int c = 0; c < NW * NCQ; ++c) bacc[c * 32 + lane] = 0.0;
         int np = 0;
         for (long long base = 0; base < total; base += 32) {
-            np = tce_pool_add<false>(S, A, Ub, Uk, q, base, total, lane, Pool, np);
-            const bool last = base + 32 >= total;
-            if (!(np > TCE_POOL - 32 || (last && np > 0))) continue;
-            if (np > BT) tce_pool_sort(Pool, np, lane);
-            const int nproc = last ? np : (np & ~(BT - 1));
-            for (int b0 = 0; b0 < nproc; b0 += BT) {
-                const int nb = nproc - b0 < BT ? nproc - b0 : BT;
-                const int nmax = Pool.key[b0];   // largest truncation order of the batch (sorted)
-                int nmr[MT], go[MT], ho[MT];
+            np = tce_pool_add<false, 1>(S, A, Ub, Uk, q, base, total, lane, Pool, np);
+            if (!(np > TCE_POOL - 32 || (base + 32 >= total && np > 0))) continue;
+            tce_pool_order(Pool, np, lane);
+            for (int b0 = 0; b0 < np; b0 += BT) {
+                // this lane's fragment rows (past the batch's end its first one, not used)
+                int go[MT], ho[MT];
+                double phi[MT], pq_[MT], ps[MT], R2[MT], c1[MT], s1[MT];
+                float umin = 0.0f, umax = 0.0f, pmin = 0.0f, pmax = 0.0f;
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
-                    const int r = 8 * m + rq;
-                    nmr[m] = -1;
-                    go[m] = ho[m] = 0;
-                    if (r < nb) {
-                        const int2 pq = Pool.pq[b0 + r];
-                        nmr[m] = Pool.key[b0 + r];
-                        go[m] = pq.x;
-                        ho[m] = pq.y;
-                    }
+                    const int r = b0 + 8 * m + rq;
+                    const int2 pq = Pool.pq[Pool.key[r < np ? r : b0]];
+                    const PairPrim &Pb = S.pp[Ub.pp_off + pq.x];
+                    const PairPrim &Pk = S.pp[Uk.pp_off + pq.y];
+                    go[m] = pq.x;
+                    ho[m] = pq.y;
+                    phi[m] = S.a[0] * (Pb.cen[0] - (Pk.cen[0] + Tx));
+                    pq_[m] = Pb.esum * Pk.esum;
+                    ps[m] = Pb.esum + Pk.esum;
+                    const double Ry = Pb.cen[1] - Pk.cen[1], Rz = Pb.cen[2] - Pk.cen[2];
+                    R2[m] = Ry * Ry + Rz * Rz;
+                    const float u = 1.0f / (float)Pb.A[0] + 1.0f / (float)Pk.A[0], ap = tce_fold_phase(phi[m]);
+                    umin = m == 0 ? u : fminf(umin, u);
+                    umax = m == 0 ? u : fmaxf(umax, u);
+                    pmin = m == 0 ? ap : fminf(pmin, ap);
+                    pmax = m == 0 ? ap : fmaxf(pmax, ap);
                 }
-                auto phase = [&](int m) {
-                    const int r = 8 * m + rq;
-                    if (r >= nb) return 0.0;
-                    const int2 pq = Pool.pq[b0 + r];
-                    return S.a[0] * (S.pp[Ub.pp_off + pq.x].cen[0] - (S.pp[Uk.pp_off + pq.y].cen[0] + Tx));
-                };
-                // the vectors of order n of row m (zero past the row's truncation order)
-                double g0N[MT], h0N[MT];
-                double2 gN[NGV - 1 > 0 ? NGV - 1 : 1][MT], hN[NHV - 1 > 0 ? NHV - 1 : 1][MT];
-                auto load = [&](int m, int n) {
-                    const bool ok = n <= nmr[m];
-                    g0N[m] = ok ? __ldg(G0 + 2 * ((size_t)go[m] + (size_t)n * nppb)) : 0.0;
-                    h0N[m] = ok ? __ldg(H0 + 2 * ((size_t)ho[m] + (size_t)n * nppk)) : 0.0;
 #pragma unroll
-                    for (int g = 1; g < NGV; ++g)
-                        gN[g - 1][m] = ok ? __ldg(Gv + 2 * g * gl + go[m] + (size_t)n * nppb) : make_double2(0.0, 0.0);
+                for (int o = 4; o < 32; o <<= 1) {
+                    umin = fminf(umin, __shfl_xor_sync(0xffffffffu, umin, o));
+                    umax = fmaxf(umax, __shfl_xor_sync(0xffffffffu, umax, o));
+                    pmin = fminf(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
+                    pmax = fmaxf(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+                }
+                OrderPlan plan = tce_order_plan(E, SHIFT, umin, umax, pmin, pmax, vmin, vmax,
+                                                min(glast, min(Ub.Nlen, Uk.Nlen) - 1));   // of pass `lane`
+                if (glast < 0) plan.h = 0;
+                // moments [m][cmb][j][Kronrod, Gauss], j <= NN - xsum(cmb)
+                double Mo[MT][NCOMB][NN + 1][NW];
 #pragma unroll
-                    for (int h = 1; h < NHV; ++h)
-                        hN[h - 1][m] = ok ? __ldg(Hv + 2 * h * hl + ho[m] + (size_t)n * nppk) : make_double2(0.0, 0.0);
-                };
+                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                    for (int cmb = 0; cmb < NCOMB; ++cmb)
+#pragma unroll
+                        for (int j = 0; j <= NN; ++j)
+#pragma unroll
+                            for (int w = 0; w < NW; ++w) Mo[m][cmb][j][w] = 0.0;
 #pragma unroll 1
-                for (int g0 = 0; g0 < NQ / 8; g0 += NT) {
-                    int gmb[NT], nend = -1;
+                for (int c = 0; c < nchunk; ++c) {
+                    // cos, sin of h phi for four passes at a time: lane column cq computes pass c + cq's
+                    if ((c & 3) == 0) {
+                        const double hd = (double)__shfl_sync(0xffffffffu, plan.h, c + cq);
 #pragma unroll
-                    for (int t = 0; t < NT; ++t) {
-                        gmb[t] = gm[g0 + t];
-                        nend = gmb[t] > nend ? gmb[t] : nend;
+                        for (int m = 0; m < MT; ++m) sincos(hd * phi[m], &s1[m], &c1[m]);
                     }
-                    nend = nend < nmax ? nend : nmax;
+                    const int h = __shfl_sync(0xffffffffu, plan.h, c), last = __shfl_sync(0xffffffffu, plan.last, c);
+                    if (h == 0) continue;
+                    int col[NT];
+#pragma unroll
+                    for (int t = 0; t < NT; ++t) col[t] = 8 * min(c * NT + t, ng - 1) + rq;
                     double acc[NCOMB][AT];
 #pragma unroll
                     for (int cmb = 0; cmb < NCOMB; ++cmb)
 #pragma unroll
                         for (int x = 0; x < AT; ++x) acc[cmb][x] = 0.0;
-                    // cos / sin of n phi and (n - 4) phi, 2 cos(4 phi)
+                    // cos / sin of n phi and (n - 4 h) phi, 2 cos(4 h phi)
                     double cc[MT], cp[MT], sc[MT], sp[MT], c4[MT];
 #pragma unroll
                     for (int m = 0; m < MT; ++m) {
-                        const double ph = phase(m);
-                        sincos((double)cq * ph, &sc[m], &cc[m]);
-                        sincos((double)(cq - 4) * ph, &sp[m], &cp[m]);
-                        c4[m] = 2.0 * cos(4.0 * ph);
-                        load(m, cq);
+                        const int src = (lane & ~3) | (c & 3);
+                        const double cb = __shfl_sync(0xffffffffu, c1[m], src);
+                        const double sb = __shfl_sync(0xffffffffu, s1[m], src);
+                        tce_phase_start(cb, sb, cq, cc[m], sc[m], cp[m], sp[m], c4[m]);
                     }
-                    double tN[NT];
+                    const int steps = last / (4 * h) + 1, h4 = 4 * h;
+                    int n = h * cq;
+                    double g0N[MT], h0N[MT], tN[NT];
+                    double2 gN[NGV - 1 > 0 ? NGV - 1 : 1][MT], hN[NHV - 1 > 0 ? NHV - 1 : 1][MT];
+                    auto load = [&]() {   // the values of order n (past the last order: T = 0)
+                        const int nn = min(n, last);
 #pragma unroll
-                    for (int t = 0; t < NT; ++t)
-                        tN[t] = (0 <= gmb[t] && cq <= S.ncap) ? __ldg(Tg + (size_t)cq * NQ + 8 * (g0 + t) + rq) : 0.0;
+                        for (int m = 0; m < MT; ++m) {
+                            const double2 *gp = Gv + ((long long)nn * nppb + go[m]), *hp = Hv + ((long long)nn * nppk + ho[m]);
+                            g0N[m] = __ldg(reinterpret_cast<const double *>(gp));
+                            h0N[m] = __ldg(reinterpret_cast<const double *>(hp));
+#pragma unroll
+                            for (int g = 1; g < NGV; ++g) gN[g - 1][m] = __ldg(gp + 2 * (g % (LA + 1) * (LB + 1) + g / (LA + 1)) * gl);
+#pragma unroll
+                            for (int x = 1; x < NHV; ++x) hN[x - 1][m] = __ldg(hp + 2 * (x % (LC + 1) * (LD + 1) + x / (LC + 1)) * hl);
+                        }
+#pragma unroll
+                        for (int t = 0; t < NT; ++t) {
+                            const double tv = __ldg(R.T + ((long long)nn * nq + col[t]));
+                            tN[t] = n <= last ? tv : 0.0;
+                        }
+                        n += h4;
+                    };
+                    load();
 #pragma unroll 2
-                    for (int s4 = 0; s4 <= nend; s4 += 4) {
-                        const int n = s4 + cq, n1 = n + 4;
+                    for (int s = 0; s < steps; ++s) {
                         double F[NCOMB][MT], Tb[NT];
 #pragma unroll
                         for (int m = 0; m < MT; ++m) {
@@ -272,20 +420,15 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
                                     F[cmb][m] = ar * cc[m] - ai * sc[m];
                                 }
                             }
-                            load(m, n1);
                         }
 #pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            Tb[t] = tN[t];
-                            tN[t] = (s4 + 4 <= gmb[t] && n1 <= S.ncap)
-                                        ? __ldg(Tg + (size_t)n1 * NQ + 8 * (g0 + t) + rq) : 0.0;
-                        }
-                        if (((s4 + 4) & 31) == 0) {   // re-seed the recurrences
+                        for (int t = 0; t < NT; ++t) Tb[t] = tN[t];
+                        load();
+                        if ((s & 7) == 7) {   // re-seed the recurrences
 #pragma unroll
                             for (int m = 0; m < MT; ++m) {
-                                const double ph = phase(m);
-                                sincos((double)n * ph, &sp[m], &cp[m]);
-                                sincos((double)n1 * ph, &sc[m], &cc[m]);
+                                sincos((double)(n - 2 * h4) * phi[m], &sp[m], &cp[m]);
+                                sincos((double)(n - h4) * phi[m], &sc[m], &cc[m]);
                             }
                         } else {
 #pragma unroll
@@ -299,142 +442,149 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
                         }
 #pragma unroll
                         for (int t = 0; t < NT; ++t)
-                            if (s4 <= gmb[t]) {
 #pragma unroll
-                                for (int m = 0; m < MT; ++m)
-#pragma unroll
-                                    for (int cmb = 0; cmb < NCOMB; ++cmb) {
-                                        const int x = (m * NT + t) * 2;
-                                        tce_dmma(acc[cmb][x], acc[cmb][x + 1], F[cmb][m], Tb[t]);
-                                    }
-                            }
-                    }
-                    // epilogue per fragment row: acc[cmb][2 (m NT + t) + i] = I_cmb[8 m + rq][8 (g0 + t) + 2 cq + i]
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const int r = 8 * m + rq;
-                        if (r >= nb) continue;
-                        const int2 pq = Pool.pq[b0 + r];
-                        const PairPrim &Pb = S.pp[Ub.pp_off + pq.x];
-                        const PairPrim &Pk = S.pp[Uk.pp_off + pq.y];
-                        const double p = Pb.esum, qq = Pk.esum, pq_ = p * qq, ps = p + qq;
-                        const double Ry = Pb.cen[1] - Pk.cen[1], Rz = Pb.cen[2] - Pk.cen[2];
-                        const double R2 = Ry * Ry + Rz * Rz;
-                        // moments [cmb][j][Kronrod, Gauss], j <= NN - xsum(cmb)
-                        double Mo[NCOMB][NN + 1][2];
-#pragma unroll
-                        for (int cmb = 0; cmb < NCOMB; ++cmb)
-#pragma unroll
-                            for (int j = 0; j <= NN; ++j) Mo[cmb][j][0] = Mo[cmb][j][1] = 0.0;
-#pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            if (gmb[t] < 0) continue;   // padding nodes
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                const int k = 8 * (g0 + t) + 2 * cq + i;
-                                const double t2 = tn[k] * tn[k];
-                                const double D2 = 1.0 / (pq_ + ps * t2);
-                                const double w = pq_ * t2 * D2;
-                                const double bse = (R2 == 0.0) ? D2 : D2 * exp(-w * R2);
-                                const double wkk = wk[k], wgk = wg[k];
+                            for (int m = 0; m < MT; ++m)
 #pragma unroll
                                 for (int cmb = 0; cmb < NCOMB; ++cmb) {
-                                    const double b = acc[cmb][(m * NT + t) * 2 + i] * bse;
-                                    double bk = b * wkk, bg = b * wgk;
+                                    const int x = (m * NT + t) * 2;
+                                    tce_dmma(acc[cmb][x], acc[cmb][x + 1], F[cmb][m], Tb[t]);
+                                }
+                    }
+                    // epilogue: acc[cmb][2 (m NT + t) + i] = I_cmb[8 m + rq][8 (c NT + t) + 2 cq + i] / h
+                    const double hw = (double)h;
 #pragma unroll
-                                    for (int j = 0; j <= NN - xsum(cmb); ++j) {
-                                        Mo[cmb][j][0] += bk;
-                                        Mo[cmb][j][1] += bg;
-                                        bk *= w;
-                                        bg *= w;
-                                    }
+                    for (int t = 0; t < NT; ++t) {
+                        if (NT > 1 && c * NT + t >= ng) continue;
+                        const int k = 8 * (c * NT + t) + 2 * cq;
+                        const double2 tn = *reinterpret_cast<const double2 *>(R.t + k);
+                        const double2 wk = *reinterpret_cast<const double2 *>(R.wk + k);
+                        double2 wg = make_double2(0.0, 0.0);
+                        if (LG) wg = *reinterpret_cast<const double2 *>(R.wg + k);
+#pragma unroll
+                        for (int m = 0; m < MT; ++m) {
+                            const double t20 = tn.x * tn.x, t21 = tn.y * tn.y;
+                            const double d0 = fma(ps[m], t20, pq_[m]), d1 = fma(ps[m], t21, pq_[m]);
+                            const double ri = 1.0 / (d0 * d1);
+#pragma unroll
+                            for (int i = 0; i < 2; ++i) {
+                                const double D2 = i == 0 ? ri * d1 : ri * d0;
+                                const double w = pq_[m] * (i == 0 ? t20 : t21) * D2;
+                                double bse = D2 * hw;
+                                if (R2[m] != 0.0) bse *= exp(-w * R2[m]);
+                                double wj[NN + 1][NW];   // weight x D2 e^{-w R^2} w^j
+                                wj[0][0] = bse * (i == 0 ? wk.x : wk.y);
+                                if (LG) wj[0][NW - 1] = bse * (i == 0 ? wg.x : wg.y);
+#pragma unroll
+                                for (int j = 1; j <= NN; ++j)
+#pragma unroll
+                                    for (int v = 0; v < NW; ++v) wj[j][v] = wj[j - 1][v] * w;
+#pragma unroll
+                                for (int cmb = 0; cmb < NCOMB; ++cmb) {
+                                    const double b = acc[cmb][(m * NT + t) * 2 + i];
+#pragma unroll
+                                    for (int j = 0; j <= NN - xsum(cmb); ++j)
+#pragma unroll
+                                        for (int v = 0; v < NW; ++v) Mo[m][cmb][j][v] = fma(b, wj[j][v], Mo[m][cmb][j][v]);
                                 }
                             }
                         }
-                        // Hermite E coefficients of the real directions y (dr = 0), z (dr = 1)
-                        double eb[2][EB], ek[2][EK];
-                        const double *Ebp = S.ecoef + Ub.e_off + (long long)pq.x * 2 * (LA + 1) * (LB + 1) * TCE_ECO;
-                        const double *Ekp = S.ecoef + Uk.e_off + (long long)pq.y * 2 * (LC + 1) * (LD + 1) * TCE_ECO;
+                    }
+                }
+                // the components of this lane's rows from their moments
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const int r = b0 + 8 * m + rq;
+                    if (r >= np) continue;
+                    const int e = Pool.key[r];
+                    const int2 pq = Pool.pq[e];
+                    const PairPrim &Pb = S.pp[Ub.pp_off + pq.x];
+                    const PairPrim &Pk = S.pp[Uk.pp_off + pq.y];
+                    const double Ry = Pb.cen[1] - Pk.cen[1], Rz = Pb.cen[2] - Pk.cen[2];
+                    // Hermite E coefficients of the real directions y (dr = 0), z (dr = 1)
+                    double eb[2][EB], ek[2][EK];
+                    const double *Ebp = S.ecoef + Ub.e_off + (long long)pq.x * 2 * (LA + 1) * (LB + 1) * TCE_ECO;
+                    const double *Ekp = S.ecoef + Uk.e_off + (long long)pq.y * 2 * (LC + 1) * (LD + 1) * TCE_ECO;
+#pragma unroll
+                    for (int dr = 0; dr < 2; ++dr) {
+#pragma unroll
+                        for (int a = 0; a <= LA; ++a)
+#pragma unroll
+                            for (int b = 0; b <= LB; ++b)
+#pragma unroll
+                                for (int u = 0; u <= a + b; ++u)
+                                    eb[dr][tce_eoff(LB, a, b) + u] = Ebp[((dr * (LA + 1) + a) * (LB + 1) + b) * TCE_ECO + u];
+#pragma unroll
+                        for (int a = 0; a <= LC; ++a)
+#pragma unroll
+                            for (int b = 0; b <= LD; ++b)
+#pragma unroll
+                                for (int u = 0; u <= a + b; ++u)
+                                    ek[dr][tce_eoff(LD, a, b) + u] = Ekp[((dr * (LC + 1) + a) * (LD + 1) + b) * TCE_ECO + u];
+                    }
+                    // coefficients in w of h_m(w) per real direction: hc[dr][m][j]
+                    double hc[2][NN + 1][NN + 1];
+#pragma unroll
+                    for (int dr = 0; dr < 2; ++dr) {
+                        const double Rr = dr == 0 ? Ry : Rz;
+#pragma unroll
+                        for (int mm = 0; mm <= NN; ++mm)
+#pragma unroll
+                            for (int j = 0; j <= NN; ++j) hc[dr][mm][j] = (mm == 0 && j == 0) ? 1.0 : 0.0;
+#pragma unroll
+                        for (int mm = 0; mm < NN; ++mm)
+#pragma unroll
+                            for (int j = 1; j <= NN; ++j)
+                                hc[dr][mm + 1][j] = 2.0 * Rr * hc[dr][mm][j - 1] - (mm > 0 ? 2.0 * mm * hc[dr][mm - 1][j - 1] : 0.0);
+                    }
+                    const double fac = Pool.fac[e] * PI2;
+                    const int i0 = pq.x / Ub.np2, j0 = pq.x - i0 * Ub.np2;
+                    const int k0 = pq.y / Uk.np2, l0 = pq.y - k0 * Uk.np2;
+#pragma unroll
+                    for (int c = 0; c < NCQ; ++c) {
+                        const int ca = c % NA, cb = (c / NA) % NB, cc_ = (c / (NA * NB)) % NC, cd = c / (NA * NB * NC);
+                        const int cmb = tce_pw(LA, ca, 0) + (LA + 1) * (tce_pw(LB, cb, 0) + (LB + 1) * (tce_pw(LC, cc_, 0) + (LC + 1) * tce_pw(LD, cd, 0)));
+                        const int xs = xsum(cmb);
+                        // P_d(w) = sum_{u,v} (-1)^u E_u E'_v h_{u+v}(w) per real direction
+                        double Pd[2][NN + 1];
 #pragma unroll
                         for (int dr = 0; dr < 2; ++dr) {
+                            const int pa = tce_pw(LA, ca, dr + 1), pb = tce_pw(LB, cb, dr + 1);
+                            const int pc = tce_pw(LC, cc_, dr + 1), pd = tce_pw(LD, cd, dr + 1);
 #pragma unroll
-                            for (int a = 0; a <= LA; ++a)
+                            for (int j = 0; j <= NN; ++j) Pd[dr][j] = 0.0;
 #pragma unroll
-                                for (int b = 0; b <= LB; ++b)
+                            for (int u = 0; u <= pa + pb; ++u)
 #pragma unroll
-                                    for (int u = 0; u <= a + b; ++u)
-                                        eb[dr][tce_eoff(LB, a, b) + u] = Ebp[((dr * (LA + 1) + a) * (LB + 1) + b) * TCE_ECO + u];
+                                for (int v = 0; v <= pc + pd; ++v) {
+                                    const double e1 = eb[dr][tce_eoff(LB, pa, pb) + u];
+                                    const double ee = ((u & 1) ? -e1 : e1) * ek[dr][tce_eoff(LD, pc, pd) + v];
 #pragma unroll
-                            for (int a = 0; a <= LC; ++a)
-#pragma unroll
-                                for (int b = 0; b <= LD; ++b)
-#pragma unroll
-                                    for (int u = 0; u <= a + b; ++u)
-                                        ek[dr][tce_eoff(LD, a, b) + u] = Ekp[((dr * (LC + 1) + a) * (LD + 1) + b) * TCE_ECO + u];
+                                    for (int j = 0; j <= u + v; ++j) Pd[dr][j] = fma(ee, hc[dr][u + v][j], Pd[dr][j]);
+                                }
                         }
-                        // coefficients in w of h_m(w) per real direction: hc[dr][m][j]
-                        double hc[2][NN + 1][NN + 1];
+                        double vs[NW];
 #pragma unroll
-                        for (int dr = 0; dr < 2; ++dr) {
-                            const double R = dr == 0 ? Ry : Rz;
+                        for (int v = 0; v < NW; ++v) vs[v] = 0.0;
 #pragma unroll
-                            for (int mm = 0; mm <= NN; ++mm)
+                        for (int j = 0; j <= NN - xs; ++j) {
+                            double cj = 0.0;
 #pragma unroll
-                                for (int j = 0; j <= NN; ++j) hc[dr][mm][j] = (mm == 0 && j == 0) ? 1.0 : 0.0;
+                            for (int j1 = 0; j1 <= j; ++j1) cj = fma(Pd[0][j1], Pd[1][j - j1], cj);
 #pragma unroll
-                            for (int mm = 0; mm < NN; ++mm)
-#pragma unroll
-                                for (int j = 1; j <= NN; ++j)
-                                    hc[dr][mm + 1][j] = 2.0 * R * hc[dr][mm][j - 1] - (mm > 0 ? 2.0 * mm * hc[dr][mm - 1][j - 1] : 0.0);
+                            for (int v = 0; v < NW; ++v) vs[v] = fma(cj, Mo[m][cmb][j][v], vs[v]);
                         }
-                        const double fac = Pool.fac[b0 + r] * PI2;
-                        const int i0 = pq.x / Ub.np2, j0 = pq.x - i0 * Ub.np2;
-                        const int k0 = pq.y / Uk.np2, l0 = pq.y - k0 * Uk.np2;
+                        const double sg = xs == 0 ? 1.0 : xs == 1 ? ainv : ainv * ainv;
+                        const double cf = S.sh_coef[S.sh_coff[q.x] + ca * npA + i0] * S.sh_coef[S.sh_coff[q.y] + cb * npB + j0] *
+                                          S.sh_coef[S.sh_coff[q.z] + cc_ * npC + k0] * S.sh_coef[S.sh_coff[q.w] + cd * npD + l0];
+                        const double f = fac * cf * sg;
 #pragma unroll
-                        for (int c = 0; c < NCQ; ++c) {
-                            const int ca = c % NA, cb = (c / NA) % NB, cc_ = (c / (NA * NB)) % NC, cd = c / (NA * NB * NC);
-                            const int cmb = tce_pw(LA, ca, 0) + (LA + 1) * (tce_pw(LB, cb, 0) + (LB + 1) * (tce_pw(LC, cc_, 0) + (LC + 1) * tce_pw(LD, cd, 0)));
-                            const int xs = xsum(cmb);
-                            // P_d(w) = sum_{u,v} (-1)^u E_u E'_v h_{u+v}(w) per real direction
-                            double Pd[2][NN + 1];
-#pragma unroll
-                            for (int dr = 0; dr < 2; ++dr) {
-                                const int pa = tce_pw(LA, ca, dr + 1), pb = tce_pw(LB, cb, dr + 1);
-                                const int pc = tce_pw(LC, cc_, dr + 1), pd = tce_pw(LD, cd, dr + 1);
-#pragma unroll
-                                for (int j = 0; j <= NN; ++j) Pd[dr][j] = 0.0;
-#pragma unroll
-                                for (int u = 0; u <= pa + pb; ++u)
-#pragma unroll
-                                    for (int v = 0; v <= pc + pd; ++v) {
-                                        const double e1 = eb[dr][tce_eoff(LB, pa, pb) + u];
-                                        const double ee = ((u & 1) ? -e1 : e1) * ek[dr][tce_eoff(LD, pc, pd) + v];
-#pragma unroll
-                                        for (int j = 0; j <= u + v; ++j) Pd[dr][j] = fma(ee, hc[dr][u + v][j], Pd[dr][j]);
-                                    }
-                            }
-                            double vK = 0.0, vG = 0.0;
-#pragma unroll
-                            for (int j = 0; j <= NN - xs; ++j) {
-                                double cj = 0.0;
-#pragma unroll
-                                for (int j1 = 0; j1 <= j; ++j1) cj = fma(Pd[0][j1], Pd[1][j - j1], cj);
-                                vK = fma(cj, Mo[cmb][j][0], vK);
-                                vG = fma(cj, Mo[cmb][j][1], vG);
-                            }
-                            const double sg = xs == 0 ? 1.0 : xs == 1 ? ainv : ainv * ainv;
-                            const double cf = S.sh_coef[S.sh_coff[q.x] + ca * npA + i0] * S.sh_coef[S.sh_coff[q.y] + cb * npB + j0] *
-                                              S.sh_coef[S.sh_coff[q.z] + cc_ * npC + k0] * S.sh_coef[S.sh_coff[q.w] + cd * npD + l0];
-                            const double f = fac * cf * sg;
-                            bacc[c * 32 + lane] = fma(f, vK, bacc[c * 32 + lane]);
-                            bacc[(NCQ + c) * 32 + lane] = fma(f, vG, bacc[(NCQ + c) * 32 + lane]);
-                        }
+                        for (int v = 0; v < NW; ++v)
+                            bacc[(v * NCQ + c) * 32 + lane] = fma(f, vs[v], bacc[(v * NCQ + c) * 32 + lane]);
                     }
                 }
             }
             __syncwarp();
-            if (np > nproc) tce_pool_carry(Pool, nproc, np - nproc, lane);
-            np -= nproc;
+            np = 0;
         }
         const int fI = S.sh_first[q.x], fJ = S.sh_first[q.y], fK = S.sh_first[q.z], fL = S.sh_first[q.w];
         double e = 0.0, M = 0.0;
@@ -442,11 +592,13 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
 #pragma unroll
         for (int c = 0; c < NCQ; ++c) {
             blk[c] = tce_warp_sum(bacc[c * 32 + lane]);
-            const double vg = tce_warp_sum(bacc[(NCQ + c) * 32 + lane]);
-            e = fmax(e, fabs(blk[c] - vg));
-            M = fmax(M, fabs(blk[c]));
+            if (LG) {
+                const double vg = tce_warp_sum(bacc[(NCQ + c) * 32 + lane]);
+                e = fmax(e, fabs(blk[c] - vg));
+                M = fmax(M, fabs(blk[c]));
+            }
         }
-        if (!tce_judge_accepts(e, M, A.judge_tol)) {
+        if (LG && !tce_judge_accepts(e, M, A.judge_tol)) {
             if (lane == 0) tce_queue_fallback(A, q);
             __syncwarp();
             continue;
@@ -466,13 +618,12 @@ __global__ void __launch_bounds__(256, MINB) k_quartets_sp_tc(DevSys S, SArgs A)
 }
 
 // one class of the s/p kernel in tile shape (MT, NT): ncq components
-template <int NQ, int LA, int LB, int LC, int LD, int MT, int NT>
+template <int LA, int LB, int LC, int LD, int MT, int NT, bool LG>
 static void sp_tc_launch(const DevSys &S, const SArgs &A, int nsm, cudaStream_t st)
 {
     constexpr int ncq = (LA ? 3 : 1) * (LB ? 3 : 1) * (LC ? 3 : 1) * (LD ? 3 : 1);
-    tc_launch(k_quartets_sp_tc<NQ, LA, LB, LC, LD, MT, NT>, S, A, nsm, st, ncq);
+    tc_launch(k_quartets_sp_tc<LA, LB, LC, LD, MT, NT, LG>, S, A, nsm, st, ncq);
 }
 
-// the classes with two p shells (tce_kernels_sp2.cu), as sp1_launch in
-// tce_kernels_tc.cu: shape 1: 8 rows x 16 nodes per pass, 2: 8 x 32, 3: 8 x 64
-int tce_sp2_launch(const DevSys &S, int cls, const SArgs &A, int nq, int shape, int nsm, cudaStream_t st);
+// the classes with two p shells (tce_kernels_sp2.cu), as sp1_launch in tce_kernels_tc.cu
+int tce_sp2_launch(const DevSys &S, int cls, const SArgs &A, int shape, int nsm, cudaStream_t st);

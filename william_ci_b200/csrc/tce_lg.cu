@@ -542,20 +542,16 @@ int lg_rebuild_lists(Handle *h)
     return TCE_OK;
 }
 
-// Whether a learned-grid list has a tensor-core form (one periodic direction:
-// generic rows, all-s and one-p kernels) and which form it runs by default:
-// the all-s kernel on the tensor cores for FP64 quartets, the one-p kernel on
-// the tensor cores for every list (its FP64 tensor-core form is faster than
-// the FP32-panel CUDA-core kernel too), the generic rows with 64-node rules
-// (the forms measured faster on the 64-cell chain); the other FP32-panel
-// lists keep their CUDA-core kernels unless tuned otherwise.
 // kernel forms of a list: 0 the CUDA-core kernel, 1.. the FP64 tensor-core
-// kernel (the all-s and one-p kernels in each of their tile shapes)
+// kernel (the all-s and the s/p kernels in each of their tile shapes).  By
+// default the all-s and s/p lists run on the tensor cores (FP32-panel lists
+// too: few orders in FP64 cost less than every order in FP32), the generic
+// rows with 64-node rules of one periodic direction.
 static int lg_nforms(const Handle *h, const Handle::LgList &w)
 {
     if (w.nq != 32 && w.nq != 64) return 1;
     if (w.kind == 0) return 2;               // the generic kernel's rows: every ndp
-    if (h->ndp != 1) return 1;
+    if (h->ndp != 1) return w.kind == 1 ? 2 : 1;
     return 1 + (w.kind == 1 ? tce_tc_shapes_s(w.nq) : tce_tc_shapes_sp(w.nq));
 }
 
@@ -564,10 +560,7 @@ static bool lg_tc_available(const Handle *h, const Handle::LgList &w) { return l
 static int lg_tc_default(const Handle *h, const Handle::LgList &w)
 {
     if (!lg_tc_available(h, w)) return 0;
-    if (w.kind == 2) return 1;
-    if (w.fp32) return 0;
-    if (w.kind == 0) return (h->ndp == 1 && w.nq == 64) ? 1 : 0;
-    return 1;
+    return w.kind != 0 ? 1 : (h->ndp == 1 && w.nq == 64) ? 1 : 0;
 }
 
 static int lg_tc(const Handle *h, const Handle::LgList &w)
@@ -879,6 +872,8 @@ int tce_lg_set_rules(void *handle, int32_t nrules, const int32_t *nn, const doub
                     if (k < nn[r]) m = std::max(m, tnmax[(size_t)d * R.nq + k]);
                 R.gmax[d * TCE_MAXG + g] = m;
             }
+        for (int g = 0; g < TCE_MAXG; ++g)
+            R.t2[g] = node_range(t + (size_t)r * 64 + std::min(8 * g, 56), std::max(0, std::min(8, nn[r] - 8 * g)));
     }
     dfree(h, tb);
     dfree(h, tn);
