@@ -26,6 +26,20 @@ def _system(name, ncell, spacing=None, off_axis=False):
     return s
 
 
+def _one_d_component(s):
+    """The system with dxy alone of every d shell: shells of one function whose
+    power combinations outnumber their components."""
+    keep = [f for f in range(s.nbas) if not s.labels[f].startswith("d") or s.labels[f] == "dxy"]
+    off, ex, co = [0], [], []
+    for f in keep:
+        ex.extend(s.exps[s.prim_off[f]:s.prim_off[f + 1]])
+        co.extend(s.coefs[s.prim_off[f]:s.prim_off[f + 1]])
+        off.append(len(ex))
+    return dataclasses.replace(s, nfuc=len([f for f in keep if f < s.nfuc]), ctr=s.ctr[keep], lxyz=s.lxyz[keep],
+                               prim_off=np.array(off, dtype=np.int32), exps=np.array(ex), coefs=np.array(co),
+                               labels=[s.labels[f] for f in keep], atom_of=s.atom_of[keep])
+
+
 CASES = [
     ("h2_ring", (2, 1, 1), None, False),        # antipodal pairs: Bessel argument 0
     ("h_chain64", (1, 1, 1), 3.0, False),       # one cell, small arguments
@@ -52,3 +66,17 @@ def test_strided_orders_match_every_order(name, ncell, spacing, off, nquad):
     assert np.abs(J0).max() > 0
     assert np.abs(J - J0).max() <= 1e-12 * scale, np.abs(J - J0).max() / scale
     assert np.abs(K - K0).max() <= 1e-12 * scale, np.abs(K - K0).max() / scale
+
+
+@pytest.mark.parametrize("nquad", [32, 64])
+def test_shells_of_one_d_component(nquad):
+    import pyoracle
+    from william_ci_b200.engine import Engine
+    s = _one_d_component(_system("h2_sheet", (2, 2, 1)))
+    P = random_density(s.nbas, 5) * 0.05
+    t, w = pyoracle.fast_quad(nquad)
+    J0, K0 = pyoracle.Oracle(s, t_nodes=t, t_weights=w).direct_jk(P)[:2]
+    with Engine(s, t_nodes=t, t_weights=w) as eng:
+        J, K = eng.direct_JK(P)
+    scale = np.abs(P).sum()
+    assert np.abs(J - J0).max() <= 1e-12 * scale and np.abs(K - K0).max() <= 1e-12 * scale

@@ -135,9 +135,21 @@ int route(const Handle *h, const int4 &q)
     }
     if (cls == 0 && sp) return 1 * 16;
     if (sp && h->ndp == 1 && __builtin_popcount(cls) <= 2) return 2 * 16 + cls;
-    // generic kernel: one list per number of shells above p, each launched with
-    // its own largest block (buffers sized for the list, not for (dd|dd))
-    return (l[0] > 1) + (l[1] > 1) + (l[2] > 1) + (l[3] > 1);
+    return generic_class(h, q);
+}
+
+// The generic kernel's lists, one per number of p and number of d shells
+// (0..14): each launches with its own combination count and block size, so that
+// no quartet carries the per-warp buffers of a larger class; the buffers decide
+// how many warps an SM holds (10 of 16 with the lists by d shells alone).
+int generic_class(const Handle *h, const int4 &q)
+{
+    int np = 0, nd = 0;
+    for (int S : {q.x, q.y, q.z, q.w}) {
+        np += h->sh_l[S] == 1;
+        nd += h->sh_l[S] > 1;
+    }
+    return nd * 5 - nd * (nd - 1) / 2 + np;
 }
 
 // split a list of quartets (most expensive first) into per-kernel device lists
@@ -681,7 +693,7 @@ static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStre
             a.max_ncq = w.max_ncq;
             a.fixed_gmax = h->d_gmax;
             a.num_sms = h->num_sms;
-            a.use_tc = h->use_tc && h->nq == 64;   // tensor-core rows measured faster with 64 nodes only
+            a.use_tc = h->use_tc;
             CKS(h, tce_launch_quartets(h->S, a, st));
         } else {             // register-resident kernels of the dominant classes
             SArgsHost b;

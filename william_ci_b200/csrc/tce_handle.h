@@ -52,7 +52,7 @@ struct Handle {
     // the J/K work of this shard, one list per kernel: kind 0 generic
     // (k_quartets), 1 all-s (k_quartets_s), 2 one-periodic-direction s/p class
     // `cls` (k_quartets_r1)
-    // (generic lists: cls = shells above p, 0..4; max_ncomb / max_ncq of the list's quartets)
+    // (generic lists: cls = generic_class; max_ncomb / max_ncq of the list's quartets)
     struct WorkList { int kind, cls; int4 *d = nullptr; long long n = 0; int max_ncomb = 1, max_ncq = 1; };
     std::vector<WorkList> lists;
     long long nitems_shard = 0;
@@ -84,7 +84,7 @@ struct Handle {
     // tc: kernel form chosen by tce_lg_autotune (-1: the default rule of
     // lg_tc_default, 0: CUDA cores, 1: FP64 tensor cores); tc_choice keeps the
     // choices per list key across rebuilds
-    // generic lists (kind 0): cls = shells above p (0..4), and the largest
+    // generic lists (kind 0): cls = generic_class, and the largest
     // combination count and block of the list's quartets size its buffers
     struct LgList {
         int kind, cls, nq, fp32, tc = -1;
@@ -196,6 +196,7 @@ void dfree(Handle *h, void *p);
 
 // helpers defined in tce_api.cu
 int shift_to(const Handle *h, int idx, int refcell, int nblk);
+int generic_class(const Handle *h, const int4 &q);
 float2 node_range(const double *t, int n);
 int ncomb_of(const Handle *h, int SI, int SJ, int SK, int SL);
 int make_lists(Handle *h, const std::vector<int4> &items);

@@ -401,21 +401,13 @@ static int lg_route(const Handle *h, const int4 &q)
     return 0;
 }
 
-// the generic kernel's lists by the number of shells above p (0..4): each list
-// launches with its own largest block and combination count, so that quartets
-// without d shells do not carry the per-warp buffers of (dd|dd)
-static int generic_size_class(const Handle *h, const int4 &q)
-{
-    return (h->sh_l[q.x] > 1) + (h->sh_l[q.y] > 1) + (h->sh_l[q.z] > 1) + (h->sh_l[q.w] > 1);
-}
-
 static void fill_common(Handle *h, QuartetHostArgs &a)
 {
     a.max_ncomb = h->max_ncomb;
     a.max_ncq = h->max_ncq;
     a.fixed_gmax = h->d_gmax;
     a.num_sms = h->num_sms;
-    a.use_tc = 0;   // set per launch
+    a.use_tc = h->use_tc;
     a.rules = h->d_rules;
     a.rule_T = h->d_rule_T;
     a.rule_t = h->d_rule_t;
@@ -470,7 +462,7 @@ int lg_rebuild_lists(Handle *h)
         const int4 &q = h->items_host[(size_t)i];
         if (r >= 0 && r < h->lg_nrules) {
             int route = lg_route(h, q);
-            if (route == 0) route = generic_size_class(h, q);
+            if (route == 0) route = generic_class(h, q);
             // (no FP32 form for two p shells: their CUDA-core form is the generic kernel)
             const bool f32 = h->fp32_thr > 0.0 && route >= 16 && h->ndp == 1 && h->d_rule_T32 &&
                              __builtin_popcount(route & 15) <= 1 &&
@@ -543,10 +535,9 @@ int lg_rebuild_lists(Handle *h)
 }
 
 // kernel forms of a list: 0 the CUDA-core kernel, 1.. the FP64 tensor-core
-// kernel (the all-s and the s/p kernels in each of their tile shapes).  By
-// default the all-s and s/p lists run on the tensor cores (FP32-panel lists
-// too: few orders in FP64 cost less than every order in FP32), the generic
-// rows with 64-node rules of one periodic direction.
+// kernel (the all-s and the s/p kernels in each of their tile shapes).  Every
+// list runs on the tensor cores by default, FP32-panel lists too: few orders
+// in FP64 cost less than every order in FP32.
 static int lg_nforms(const Handle *h, const Handle::LgList &w)
 {
     if (w.nq != 32 && w.nq != 64) return 1;
@@ -559,8 +550,7 @@ static bool lg_tc_available(const Handle *h, const Handle::LgList &w) { return l
 
 static int lg_tc_default(const Handle *h, const Handle::LgList &w)
 {
-    if (!lg_tc_available(h, w)) return 0;
-    return w.kind != 0 ? 1 : (h->ndp == 1 && w.nq == 64) ? 1 : 0;
+    return lg_tc_available(h, w) ? 1 : 0;
 }
 
 static int lg_tc(const Handle *h, const Handle::LgList &w)
@@ -1023,7 +1013,7 @@ int tce_rule_blocks(void *handle, int32_t rule, int32_t mode, int64_t n, const i
         a.dict_nq = h->rules_host[rule].nq;
     }
     if (rule == -2) a.method = TCE_METHOD_PLAIN;
-    a.use_tc = h->use_tc && ((rule >= 0 && a.dict_nq == 64) || (rule == -1 && h->nq == 64));
+    a.use_tc = h->use_tc;
     CKS(h, tce_launch_quartets(h->S, a, h->st));
     CK(h, cudaMemcpyAsync(K, d_K, sizeof(double) * off.back(), cudaMemcpyDeviceToHost, h->st));
     if (d_G) CK(h, cudaMemcpyAsync(G, d_G, sizeof(double) * off.back(), cudaMemcpyDeviceToHost, h->st));

@@ -81,3 +81,18 @@ __device__ __forceinline__ float tce_fold_phase(double phi)
     const double t = phi * 0.15915494309189535;   // 1 / (2 pi)
     return fabsf((float)(t - rint(t))) * 6.2831853f;
 }
+
+// cos and sin of q phi and (4 - q) phi, q = 0..3, and 2 cos(4 phi), from
+// (c, s) = (cos phi, sin phi): the start of the three-term recurrence in steps of four
+__device__ __forceinline__ void tce_phase_start(double c, double s, int q, double &cc, double &sc, double &cm, double &sm,
+                                                double &c4)
+{
+    const double c2 = fma(-2.0 * s, s, 1.0), s2 = 2.0 * s * c;
+    const double c3 = fma(c2, c, -s2 * s), s3 = fma(s2, c, c2 * s);
+    const double k4 = fma(-2.0 * s2, s2, 1.0), z4 = 2.0 * s2 * c2;
+    cc = q == 0 ? 1.0 : q == 1 ? c : q == 2 ? c2 : c3;
+    sc = q == 0 ? 0.0 : q == 1 ? s : q == 2 ? s2 : s3;
+    cm = q == 0 ? k4 : q == 1 ? c3 : q == 2 ? c2 : c;
+    sm = -(q == 0 ? z4 : q == 1 ? s3 : q == 2 ? s2 : s);
+    c4 = 2.0 * k4;
+}

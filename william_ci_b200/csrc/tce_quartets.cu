@@ -17,10 +17,12 @@
 // scatter (ERI_toroidal.f90:416-454).
 #include <map>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "tce_device.cuh"
 #include "tce_kernels.h"
+#include "tce_orders.cuh"
 
 #define PI_D 3.14159265358979323846
 #define PLAIN_PMAX 24
@@ -30,42 +32,7 @@ struct RuleView {
     long long strideD;
     const double *t, *wk, *wg;   // nodes, weights, judge weights (nullptr: no judge)
     const int *gmax;          // gmax[d * TCE_MAXG + g]: last n with a nonzero entry in node group g
-};
-
-struct QuartetArgs {
-    const int4 *items;
-    const int *prim_sel;
-    int nitems;
-    const unsigned int *nitems_dev;   // when set, the item count is read on the device
-    int mode, method;
-    int prim_screen;
-    unsigned int *next;
-    double *blk_out, *blk_out2;
-    const long long *blk_off;
-    const double *P;
-    double *J, *K;
-    double *eri;
-    int eri_size, physicist;
-    PairPrim *pp_rw;
-    int rowcap, cstride, blkcap, warp_smem_doubles;
-    int use_tc;
-    const int *fixed_gmax;
-    // learned grid
-    const RuleDev *rules;
-    const double *rule_T, *rule_t, *rule_wk, *rule_wg;
-    const int *item_rule;
-    int rule_override;
-    double judge_tol;
-    int4 *fb_items;
-    int *fb_index;
-    unsigned int *fb_count;
-    // plain
-    double *scratch;
-    long long scratch_per_warp, T_doubles;
-    double plain_tol, plain_scale;
-    int plain_max_panels;
-    const double *gk_u, *gk_wk, *gk_wg;
-    unsigned long long *node_evals;
+    const float2 *t2;         // per node group: smallest and largest t^2
 };
 
 template <bool RO>
@@ -130,30 +97,145 @@ __device__ __forceinline__ void row_dot(const RuleView &R, int d, const double2 
 
 struct QCtx {
     int SI, SJ, SK, SL, nA, nB, nC, nD, lsA, lsB, lsC, lsD, ncomb, ncq, NN, R;
-    int cqg;   // lanes per component in the component contraction (power of two)
+    int cqp;   // lanes of one primitive quartet in the component contraction: power of two >= ncq, at most 32
     UnitPair Ub, Uk;
     double Tsh[3];
+    RuleView R_;             // the quadrature rule of the evaluation at hand
 };
 
-// per-warp shared memory: [qlist rowcap int2][qfac rowcap][rows rowcap*RS]
-// [real nreal*cstride*RS][blkK blkcap][blkG blkcap][extra]; RS = 33 (rows of a
-// chunk of 32 nodes plus padding), 17 for the plain method's 16-node panels
+// Row numbering of a batch of nb primitive quartets: row d nb ncomb + p ncomb +
+// cmb is direction d, primitive quartet p, power combination cmb; tiles of 16
+// rows of one direction.
+//
+// Per-warp shared memory (WarpBuf), sized for the launch's largest class by
+// tce_warp_doubles: rows of a chunk of 32 nodes at stride RS = 34 doubles (even,
+// so that two nodes load as one double2, and 16 bytes past a multiple of 128,
+// so that eight rows fall into different banks; 18 for the plain method's
+// 16-node panels).
+constexpr int TCE_NC = 32;        // nodes of a chunk
+constexpr int TCE_GT_ROWS = 12;   // rows of g_m(t) of the real directions: (NN + 1) x primitive quartets at once
+struct RowMeta {
+    int g, h;            // first elements of the bra and ket vectors, from the unit pairs' slabs
+    double phi;
+    float u, ap;         // 1/A_bra + 1/A_ket, |phi| in [0, pi]
+};
 struct WarpBuf {
-    int2 *qlist;
-    double *qfac, *rows, *realb, *blkK, *blkG, *extra;
+    int2 *qlist;                 // primitive pairs
+    short4 *qidx;                // primitive of each of the four shells
+    double *qfac, *rows, *realb, *gt, *blkK, *blkG, *cf, *wts, *pqm, *extra;
+    RowMeta *meta;
+    int2 *plan;                  // [tile][half]: stride and last order of a tile's 16-node half
+    double2 *cs;                 // [row][half]: cos and sin of h phi
+    unsigned *cmap;              // per component: power combination of x, y, z (8 bits each)
+    unsigned char *dig;          // per power combination: ia, ib, ic, id (2 bits each)
 };
 
-__device__ __forceinline__ WarpBuf warp_buf(const QuartetArgs &A, double *ws, int nreal, int RS)
+struct WarpLayout {              // offsets in doubles
+    int qlist, qidx, qfac, rows, realb, gt, blkK, blkG, cf, wts, pqm, meta, plan, cs, cmap, dig, extra;
+};
+__host__ __device__ inline WarpLayout tce_warp_layout(int rowcap, int RS, int nreal, int cstride, int blkcap, int nhalf)
 {
+    WarpLayout o;
+    int at = ((int)(sizeof(QCtx) + 7) / 8 + 1) & ~1;   // the quartet at hand
+    auto take = [&](int n) { const int r = at; at += (n + 1) & ~1; return r; };
+    o.qlist = take(rowcap);
+    o.qidx = take(rowcap);
+    o.qfac = take(rowcap);
+    o.rows = take(rowcap * RS);
+    o.realb = take(nreal * cstride * RS);
+    o.gt = take(nreal * TCE_GT_ROWS * RS);
+    o.blkK = take(blkcap);
+    o.blkG = take(blkcap);
+    o.cf = take(72);
+    o.wts = take(64);
+    o.pqm = take(nreal > 0 ? 4 * rowcap : 0);
+    o.meta = take(rowcap * (int)(sizeof(RowMeta) / 8));
+    o.plan = take((rowcap / 16 + 3) * nhalf);
+    o.cs = take(2 * rowcap * nhalf);
+    o.cmap = take((blkcap + 1) / 2);
+    o.dig = take(12);
+    o.extra = at;
+    return o;
+}
+
+struct QuartetArgs {
+    const int4 *items;
+    const int *prim_sel;
+    int nitems;
+    const unsigned int *nitems_dev;   // when set, the item count is read on the device
+    int mode, method;
+    int prim_screen;
+    unsigned int *next;
+    double *blk_out, *blk_out2;
+    const long long *blk_off;
+    const double *P;
+    double *J, *K;
+    double *eri;
+    int eri_size, physicist;
+    PairPrim *pp_rw;
+    int rowcap, cstride, blkcap, warp_smem_doubles;
+    WarpLayout lay;
+    int use_tc;
+    const int *fixed_gmax;
+    // learned grid
+    const RuleDev *rules;
+    const double *rule_T, *rule_t, *rule_wk, *rule_wg;
+    const int *item_rule;
+    int rule_override;
+    double judge_tol;
+    int4 *fb_items;
+    int *fb_index;
+    unsigned int *fb_count;
+    // plain
+    double *scratch;
+    long long scratch_per_warp, T_doubles;
+    double plain_tol, plain_scale;
+    int plain_max_panels;
+    const double *gk_u, *gk_wk, *gk_wg;
+    unsigned long long *node_evals;
+};
+
+// Shared memory of a block: [DevSys][WarpLayout][warp buffers]; a warp buffer
+// starts with the quartet at hand (QCtx).  The device functions below get a
+// warp buffer's offset and read all of it from shared memory: what is uniform
+// over the warp stays out of the registers, and every access is known to be a
+// shared-memory one.
+constexpr int TCE_SYS_DOUBLES = ((int)(sizeof(DevSys) + 7) / 8 + 1) & ~1;
+constexpr int TCE_HDR_DOUBLES = TCE_SYS_DOUBLES + (((int)(sizeof(WarpLayout) + 7) / 8 + 1) & ~1);
+extern __shared__ __align__(16) double smem[];
+
+__device__ __forceinline__ const DevSys &blk_sys() { return *reinterpret_cast<const DevSys *>(smem); }
+__device__ __forceinline__ QCtx &warp_ctx(int wofs) { return *reinterpret_cast<QCtx *>(smem + wofs); }
+__device__ __forceinline__ WarpBuf warp_buf(int wofs)
+{
+    const WarpLayout &o = *reinterpret_cast<const WarpLayout *>(smem + TCE_SYS_DOUBLES);
+    double *ws = smem + wofs;
     WarpBuf b;
-    b.qlist = reinterpret_cast<int2 *>(ws);
-    b.qfac = ws + A.rowcap;
-    b.rows = ws + 2 * A.rowcap;
-    b.realb = b.rows + (size_t)A.rowcap * RS;
-    b.blkK = b.realb + (size_t)nreal * A.cstride * RS;
-    b.blkG = b.blkK + A.blkcap;
-    b.extra = b.blkG + A.blkcap;
+    b.qlist = reinterpret_cast<int2 *>(ws + o.qlist);
+    b.qidx = reinterpret_cast<short4 *>(ws + o.qidx);
+    b.qfac = ws + o.qfac;
+    b.rows = ws + o.rows;
+    b.realb = ws + o.realb;
+    b.gt = ws + o.gt;
+    b.blkK = ws + o.blkK;
+    b.blkG = ws + o.blkG;
+    b.cf = ws + o.cf;
+    b.wts = ws + o.wts;
+    b.pqm = ws + o.pqm;
+    b.meta = reinterpret_cast<RowMeta *>(ws + o.meta);
+    b.plan = reinterpret_cast<int2 *>(ws + o.plan);
+    b.cs = reinterpret_cast<double2 *>(ws + o.cs);
+    b.cmap = reinterpret_cast<unsigned *>(ws + o.cmap);
+    b.dig = reinterpret_cast<unsigned char *>(ws + o.dig);
+    b.extra = ws + o.extra;
     return b;
+}
+// header of the block's shared memory, by all threads
+__device__ __forceinline__ void blk_header(const DevSys &S, const WarpLayout &lay)
+{
+    if (threadIdx.x == 0) *reinterpret_cast<DevSys *>(smem) = S;
+    if (threadIdx.x == blockDim.x - 1) *reinterpret_cast<WarpLayout *>(smem + TCE_SYS_DOUBLES) = lay;
+    __syncthreads();
 }
 
 __device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, double b)
@@ -163,306 +245,430 @@ __device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, doubl
                  : "d"(a), "d"(b));
 }
 
-// The rows of row_dot for a batch and periodic direction d on the FP64 tensor
-// cores: the batch's nb * ncomb rows of direction d (primitive quartet x power
-// combination) in chunks of 32 are the A operand (32 x N, F = Re[G_n H_n
-// e^{i n phi}]), the rule's T table of direction d the B operand (N x 32
-// nodes per pass);
-// mma.sync.m8n8k4 per 8 x 8 tile and step of four orders.  Lane l builds the
-// A fragments of rows 8 m + l/4 (m = 0..3) at order 4 s + l%4, cos and sin
-// of n phi by the three-term recurrence in steps of four (re-seeded every 32
-// orders), and loads the next step's G, H and T before the current step's
-// mma instructions.  Nodes of one chunk (8-node groups g0c .. g0c + 3); output
-// as row_dot: rows[r * 33 + x] = sgn I_r(t_{8 g0c + x}).
-template <int NQ>
-__device__ void tc_rows(const DevSys &S, const RuleView &Rv, const QCtx &Q, int nb, const WarpBuf &b, int lane,
-                        int g0c, int d)
+__device__ __forceinline__ double tce_ipow(double x, int k)
 {
-    constexpr int RS = 32 + 1;
-    const int rq = lane >> 2, cq = lane & 3;
-    const int lsA = Q.lsA, lsB = Q.lsB, lsC = Q.lsC, lsD = Q.lsD, R = Q.R, nd = Q.ncomb;
+    double r = 1.0;
+    for (int i = 0; i < k; ++i) r *= x;
+    return r;
+}
+
+// What the rows of a batch need, once per batch: vector offsets and phase of
+// every row (RowMeta), and for every tile of 16 rows and every 16-node half of
+// the rule the stride and last order (tce_order_plan): lane = half + nhalf x
+// tile.  Kept out of the node chunks: index divisions, the PairPrim loads and
+// the plans cost more than a tile's mma instructions.
+template <int NQ>
+__device__ __noinline__ void row_setup(int wofs, int nb, int lane)
+{
+    const DevSys &S = blk_sys();
+    const QCtx &Q = warp_ctx(wofs);
+    const RuleView &Rv = Q.R_;
+    const WarpBuf b = warp_buf(wofs);
+    constexpr int NH = NQ / 16 + (NQ % 16 ? 1 : 0);
+    const int ndp = S.ndp, nd = Q.ncomb, per = nb * nd;
     const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
-    const int nrows = nb * nd;                 // the batch's rows of direction d
-    const double *T = Rv.T + (size_t)d * Rv.strideD;
-    const int *gm = Rv.gmax + d * TCE_MAXG;
-    // row rr = (primitive quartet p, combination cmb) of direction d -> its place in b.rows
-    auto orow = [&](int rr) {
-        const int p = rr / nd;
-        return p * R + d * nd + (rr - p * nd);
-    };
-    for (int r0 = 0; r0 < nrows; r0 += 32) {
-        int goff[4], hoff[4], nmr[4];
-        double sg[4];
-        int nmax = -1;
+    for (int r = lane; r < per * ndp; r += 32) {
+        const int d = r / per, rr = r - d * per, p = rr / nd;
+        const int dg = b.dig[rr - p * nd];
+        const int ia = dg & 3, ib = (dg >> 2) & 3, ic = (dg >> 4) & 3, id = dg >> 6;
+        const int2 pq = b.qlist[p];
+        const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
+        const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
+        RowMeta m;
+        m.g = (((d * (Q.lsA + 1) + ia) * (Q.lsB + 1) + ib) * 2 + 0) * Q.Ub.Nlen * nppb + pq.x;
+        m.h = (((d * (Q.lsC + 1) + ic) * (Q.lsD + 1) + id) * 2 + 1) * Q.Uk.Nlen * nppk + pq.y;
+        m.phi = S.a[d] * (Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]));
+        m.u = 1.0f / (float)Pb.A[d] + 1.0f / (float)Pk.A[d];
+        m.ap = tce_fold_phase(m.phi);
+        b.meta[r] = m;
+    }
+    __syncwarp();
+    const int tiles = (per + 15) / 16, shift = max(Q.lsA + Q.lsB, Q.lsC + Q.lsD);
+    const float E = tce_order_exponent(Q.NN);
+    for (int x = lane; x < tiles * ndp * NH; x += 32) {
+        const int tile = x / NH, half = x - tile * NH, d = tile / tiles, r0 = d * per + (tile - d * tiles) * 16;
+        const int r1 = min(r0 + 16, (d + 1) * per);
+        float umin = b.meta[r0].u, umax = umin, pmin = b.meta[r0].ap, pmax = pmin;
+        for (int r = r0 + 1; r < r1; ++r) {
+            const float u = b.meta[r].u, ap = b.meta[r].ap;
+            umin = fminf(umin, u);
+            umax = fmaxf(umax, u);
+            pmin = fminf(pmin, ap);
+            pmax = fmaxf(pmax, ap);
+        }
+        float lo = __int_as_float(0x7f800000), hi = -lo;
+        int glast = -1;
 #pragma unroll
-        for (int m = 0; m < 4; ++m) {
-            const int r = r0 + 8 * m + rq;
-            nmr[m] = -1;
-            goff[m] = hoff[m] = 0;
-            sg[m] = 0.0;
-            if (r < nrows) {
-                const int p = r / nd, cmb = r - p * nd;
-                const int ia = cmb % (lsA + 1), t1 = cmb / (lsA + 1);
-                const int ib = t1 % (lsB + 1), t2 = t1 / (lsB + 1);
-                const int ic = t2 % (lsC + 1), id = t2 / (lsC + 1);
-                const int2 pq = b.qlist[p];
-                const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
-                const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
-                nmr[m] = Pb.N[d] < Pk.N[d] ? Pb.N[d] : Pk.N[d];
-                goff[m] = (int)(((((long long)d * (lsA + 1) + ia) * (lsB + 1) + ib) * 2 + 0) * Q.Ub.Nlen * nppb + pq.x);
-                hoff[m] = (int)(((((long long)d * (lsC + 1) + ic) * (lsD + 1) + id) * 2 + 1) * Q.Uk.Nlen * nppk + pq.y);
-                sg[m] = pow(S.a[d], -(double)(ia + ib + ic + id));
-                nmax = nmr[m] > nmax ? nmr[m] : nmax;
+        for (int t = 0; t < 2; ++t) {
+            const int g = 2 * half + t;
+            if (g < NQ / 8) {
+                const float2 w = Rv.t2[g];
+                lo = fminf(lo, w.x);
+                hi = fmaxf(hi, w.y);
+                glast = max(glast, Rv.gmax[d * TCE_MAXG + g]);
             }
         }
+        const float a2 = 0.5f * (float)(S.a[d] * S.a[d]);
+        OrderPlan plan;
+        plan.h = 0;
+        plan.last = 0;
+        if (lo <= hi && glast >= 0)   // the half has real nodes
+            plan = tce_order_plan(E, shift, umin, umax, pmin, pmax, a2 / hi, a2 / lo, min(glast, min(Q.Ub.Nlen, Q.Uk.Nlen) - 1));
+        b.plan[x] = make_int2(plan.h, plan.last);
+    }
+    __syncwarp();
+    for (int x = lane; x < per * ndp * NH; x += 32) {
+        const int r = x / NH, half = x - r * NH, d = r / per;
+        const int h = b.plan[(d * tiles + (r - d * per) / 16) * NH + half].x;
+        double2 v;
+        sincos((double)h * b.meta[r].phi, &v.y, &v.x);
+        b.cs[x] = v;
+    }
+    __syncwarp();
+}
+
+// The rows of one chunk of 32 nodes on the FP64 tensor cores: per tile of 16
+// rows the A operand F = Re[G_n H_n e^{i n phi}], the rule's T table of the
+// direction the B operand; mma.sync.m8n8k4 per 8 x 8 tile and step of four
+// orders.  Lane l builds the A fragments of rows 8 m + l/4 (m = 0, 1) at order
+// h (4 s + l%4), e^{i n phi} by rotation, and loads the next step's G, H and T
+// before the current step's mma.  Halves of the same stride run in one loop, so that
+// they share the A fragments.  rows[r * RS + x] = a^-powers I_r(t_{8 g0c + x}).
+// Rows of one primitive quartet are next to each other, so a tile's rows share
+// phase and concentration.
+template <int NQ, bool RO, int RS>
+__device__ __noinline__ void tc_rows(int wofs, int nb, int lane, int g0c)
+{
+    const DevSys &S = blk_sys();
+    const QCtx &Q = warp_ctx(wofs);
+    const RuleView &Rv = Q.R_;
+    const WarpBuf b = warp_buf(wofs);
+    constexpr int MT = 2, NTC = (NQ < TCE_NC ? NQ : TCE_NC) / 8;
+    constexpr int NH = NQ / 16 + (NQ % 16 ? 1 : 0);
+    const int ng = NQ / 8 - g0c < NTC ? NQ / 8 - g0c : NTC;   // groups of this chunk
+    const int rq = lane >> 2, cq = lane & 3;
+    const int nd = Q.ncomb, per = nb * nd, tiles = (per + 15) / 16;
+    const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
+    const double2 *Gv = S.vec + Q.Ub.vec_off, *Hv = S.vec + Q.Uk.vec_off;
+#pragma unroll 1
+    for (int tile = 0; tile < tiles * S.ndp; ++tile) {
+        const int d = tile / tiles, r0 = d * per + (tile - d * tiles) * 16, rend = (d + 1) * per;
+        const double *T = Rv.T + (size_t)d * Rv.strideD + 8 * g0c + rq;
+        const int2 pl0 = b.plan[tile * NH + g0c / 2];
+        const int2 pl1 = NTC > 2 && g0c / 2 + 1 < NH ? b.plan[tile * NH + g0c / 2 + 1] : make_int2(0, 0);
+        const int h0 = pl0.x, l0 = pl0.y, h1 = pl1.x, l1 = pl1.y;
+        const double2 *gp[MT], *hp[MT], *cs[MT];
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) nmax = max(nmax, __shfl_xor_sync(0xffffffffu, nmax, o));
-        auto phase = [&](int m) {
-            const int r = r0 + 8 * m + rq;
-            if (r >= nrows) return 0.0;
-            const int2 pq = b.qlist[r / nd];
-            return S.a[d] * (S.pp[Q.Ub.pp_off + pq.x].cen[d] - (S.pp[Q.Uk.pp_off + pq.y].cen[d] + Q.Tsh[d]));
+        for (int m = 0; m < MT; ++m) {
+            const int r = min(r0 + 8 * m + rq, rend - 1);   // past the end: the last row again
+            gp[m] = Gv + b.meta[r].g;
+            hp[m] = Hv + b.meta[r].h;
+            cs[m] = b.cs + (r * NH + g0c / 2);
+        }
+        double acc[NTC][MT][2];
+#pragma unroll
+        for (int t = 0; t < NTC; ++t)
+#pragma unroll
+            for (int m = 0; m < MT; ++m) acc[t][m][0] = acc[t][m][1] = 0.0;
+        // node tiles [T0, T1) of the chunk over the orders 0, h, .., last
+        auto run = [&](auto t0c, auto t1c, int half, int h, int last) {
+            constexpr int T0 = decltype(t0c)::value, T1 = decltype(t1c)::value;
+            const int h4 = 4 * h;
+            int n = h * cq;
+            double2 gN[MT], hN[MT];
+            double tN[T1 - T0];
+            auto load = [&]() {   // the values of order n (past the last order: F = 0)
+                const int nn = min(n, last);
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    gN[m] = __ldg(gp[m] + (long long)nn * nppb);
+                    hN[m] = __ldg(hp[m] + (long long)nn * nppk);
+                }
+#pragma unroll
+                for (int t = T0; t < T1; ++t) tN[t - T0] = ldT<RO>(T + ((long long)nn * NQ + 8 * (t < ng ? t : 0)));
+            };
+            load();
+            // e^{i n phi} at n = h cq and the rotation by 4 h phi per step (errors add up
+            // linearly, one rounding per step, and few steps are taken: no re-seeding)
+            double cc[MT], sc[MT], c4[MT], s4[MT];
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const double2 z = cs[m][half];
+                const double c2 = fma(-2.0 * z.y, z.y, 1.0), s2 = 2.0 * z.y * z.x;
+                cc[m] = cq == 0 ? 1.0 : cq == 1 ? z.x : cq == 2 ? c2 : fma(c2, z.x, -s2 * z.y);
+                sc[m] = cq == 0 ? 0.0 : cq == 1 ? z.y : cq == 2 ? s2 : fma(s2, z.x, c2 * z.y);
+                c4[m] = fma(-2.0 * s2, s2, 1.0);
+                s4[m] = 2.0 * s2 * c2;
+            }
+#pragma unroll 1
+            for (int n0 = 0; n0 <= last; n0 += h4) {
+                double F[MT], Tb[T1 - T0];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const double ar = gN[m].x * hN[m].x - gN[m].y * hN[m].y, ai = gN[m].x * hN[m].y + gN[m].y * hN[m].x;
+                    F[m] = n <= last ? ar * cc[m] - ai * sc[m] : 0.0;
+                }
+#pragma unroll
+                for (int t = 0; t < T1 - T0; ++t) Tb[t] = tN[t];
+                n += h4;
+                load();
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const double t = cc[m];
+                    cc[m] = fma(t, c4[m], -sc[m] * s4[m]);
+                    sc[m] = fma(sc[m], c4[m], t * s4[m]);
+                }
+#pragma unroll
+                for (int t = T0; t < T1; ++t)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) tce_dmma(acc[t][m][0], acc[t][m][1], F[m], Tb[t - T0]);
+            }
         };
-        const double2 *Gv = S.vec + Q.Ub.vec_off, *Hv = S.vec + Q.Uk.vec_off;
-        {
-            const int g0 = g0c;
-            int gmb[4], nend = -1;
-#pragma unroll
-            for (int t = 0; t < 4; ++t) {
-                gmb[t] = gm[g0 + t];
-                nend = gmb[t] > nend ? gmb[t] : nend;
+        using I0 = std::integral_constant<int, 0>;
+        using I2 = std::integral_constant<int, 2>;
+        using IN = std::integral_constant<int, NTC>;
+        if constexpr (NTC > 2) {
+            if (h0 != 0 && h0 == h1) {
+                run(I0{}, IN{}, 0, h0, max(l0, l1));
+            } else {
+                if (h0 != 0) run(I0{}, I2{}, 0, h0, l0);
+                if (h1 != 0) run(I2{}, IN{}, 1, h1, l1);
             }
-            nend = nend < nmax ? nend : nmax;
-            double acc[32];
+        } else {
+            if (h0 != 0) run(I0{}, IN{}, 0, h0, l0);
+        }
 #pragma unroll
-            for (int x = 0; x < 32; ++x) acc[x] = 0.0;
-            double cc[4], cp[4], sc[4], sp[4], c4[4];
-            double2 gN[4], hN[4];
+        for (int m = 0; m < MT; ++m) {
+            const int r = r0 + 8 * m + rq;
+            if (r >= rend) continue;
 #pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const double ph = phase(m);
-                sincos((double)cq * ph, &sc[m], &cc[m]);
-                sincos((double)(cq - 4) * ph, &sp[m], &cp[m]);
-                c4[m] = 2.0 * cos(4.0 * ph);
-                const bool ok = cq <= nmr[m];
-                gN[m] = ok ? __ldg(Gv + goff[m] + (size_t)cq * nppb) : make_double2(0.0, 0.0);
-                hN[m] = ok ? __ldg(Hv + hoff[m] + (size_t)cq * nppk) : make_double2(0.0, 0.0);
-            }
-            double tN[4];
-#pragma unroll
-            for (int t = 0; t < 4; ++t)
-                tN[t] = (0 <= gmb[t] && cq <= S.ncap) ? __ldg(T + (size_t)cq * NQ + 8 * (g0 + t) + rq) : 0.0;
-            for (int s4 = 0; s4 <= nend; s4 += 4) {
-                const int n = s4 + cq, n1 = n + 4;
-                double F[4], Tb[4];
-#pragma unroll
-                for (int m = 0; m < 4; ++m) {
-                    const double2 gv = gN[m], hv = hN[m];
-                    const double ar = gv.x * hv.x - gv.y * hv.y, ai = gv.x * hv.y + gv.y * hv.x;
-                    F[m] = ar * cc[m] - ai * sc[m];
-                    const bool ok = n1 <= nmr[m];
-                    gN[m] = ok ? __ldg(Gv + goff[m] + (size_t)n1 * nppb) : make_double2(0.0, 0.0);
-                    hN[m] = ok ? __ldg(Hv + hoff[m] + (size_t)n1 * nppk) : make_double2(0.0, 0.0);
-                }
-#pragma unroll
-                for (int t = 0; t < 4; ++t) {
-                    Tb[t] = tN[t];
-                    tN[t] = (s4 + 4 <= gmb[t] && n1 <= S.ncap) ? __ldg(T + (size_t)n1 * NQ + 8 * (g0 + t) + rq) : 0.0;
-                }
-                if (((s4 + 4) & 31) == 0) {
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const double ph = phase(m);
-                        sincos((double)n * ph, &sp[m], &cp[m]);
-                        sincos((double)n1 * ph, &sc[m], &cc[m]);
-                    }
-                } else {
-#pragma unroll
-                    for (int m = 0; m < 4; ++m) {
-                        const double tc_ = c4[m] * cc[m] - cp[m], ts_ = c4[m] * sc[m] - sp[m];
-                        cp[m] = cc[m];
-                        cc[m] = tc_;
-                        sp[m] = sc[m];
-                        sc[m] = ts_;
-                    }
-                }
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-                    if (s4 <= gmb[t]) {
-#pragma unroll
-                        for (int m = 0; m < 4; ++m) tce_dmma(acc[8 * m + 2 * t], acc[8 * m + 2 * t + 1], F[m], Tb[t]);
-                    }
-            }
-#pragma unroll
-            for (int m = 0; m < 4; ++m) {
-                const int r = r0 + 8 * m + rq;
-                if (r >= nrows) continue;
-#pragma unroll
-                for (int t = 0; t < 4; ++t)
-#pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        b.rows[(size_t)orow(r) * RS + 8 * t + 2 * cq + i] = acc[8 * m + 2 * t + i] * sg[m];
+            for (int t = 0; t < NTC; ++t) {
+                if (t >= ng) continue;
+                const double w = (double)(t < 2 ? h0 : h1);
+                *reinterpret_cast<double2 *>(b.rows + (size_t)r * RS + 8 * t + 2 * cq) =
+                    make_double2(acc[t][m][0] * w, acc[t][m][1] * w);
             }
         }
     }
 }
 
-// Phases 1+2 for a batch of nb primitive quartets, accumulating into blkK (and blkG)
+// A batch of nb primitive quartets: the rows of a chunk of 32 nodes, then the
+// chunk's share of every component's node sum (the row buffer holds 32 nodes
+// instead of NQ: more warps per SM).  With at most 32 components lane l
+// accumulates component l % cqp into accK (and accG) for the primitive quartets
+// l / cqp + PW j; otherwise the lanes run over the components of one primitive
+// quartet after the other and accumulate into blkK (and blkG).
 template <int NQ, bool RO>
-__device__ void process_batch(const DevSys &S, const RuleView &Rv, const QCtx &Q, int nb, const WarpBuf &b, int lane,
-                              int cstride, bool tc)
+__device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstride, bool tc, double &accK_, double &accG_)
 {
-    // The rule's nodes in chunks of NC (32): the rows of one chunk, then its
-    // share of every component's node sum.  The row dots restart their order
-    // loop per 32 nodes anyway, so chunking costs no extra arithmetic and the
-    // per-warp row buffer holds 32 nodes instead of NQ (more warps per SM).
-    constexpr int NC = NQ < 32 ? NQ : 32;
-    constexpr int RS = NC + 1;
+    const DevSys &S = blk_sys();
+    const QCtx &Q = warp_ctx(wofs);
+    const RuleView &Rv = Q.R_;
+    const WarpBuf b = warp_buf(wofs);
+    constexpr int NC = NQ < TCE_NC ? NQ : TCE_NC;
+    constexpr int RS = NC + 2;
     const int ndp = S.ndp, nreal = 3 - ndp;
-    const int lsA = Q.lsA, lsB = Q.lsB, lsC = Q.lsC, lsD = Q.lsD, ncomb = Q.ncomb, R = Q.R;
-    const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
-    const int nrows = nb * R;
-    const int npA = S.sh_np[Q.SI], npB = S.sh_np[Q.SJ], npC = S.sh_np[Q.SK], npD = S.sh_np[Q.SL];
+    const int ncomb = Q.ncomb, per = nb * ncomb, NN = Q.NN;
     const bool judge = Rv.wg != nullptr;
+    const bool few = Q.ncq <= 32;
+    const int nAB = Q.nA * Q.nB, nCD = Q.nC * Q.nD;
+    int PW = 1, pl = 0, cl = lane;                   // primitive quartets at once; this lane's, its component
+    if (few) {
+        PW = 32 / Q.cqp;
+        pl = lane / Q.cqp;
+        cl = lane - pl * Q.cqp;
+    }
+    // primitive quartets whose real-direction tables are built together
+    const int RP = nreal > 0 ? max(1, min(cstride / ncomb, TCE_GT_ROWS / (NN + 1))) : nb;
+    const double *coA = S.sh_coef + S.sh_coff[Q.SI], *coB = S.sh_coef + S.sh_coff[Q.SJ];
+    const double *coC = S.sh_coef + S.sh_coff[Q.SK], *coD = S.sh_coef + S.sh_coff[Q.SL];
+    const int npA = S.sh_np[Q.SI], npB = S.sh_np[Q.SJ], npC = S.sh_np[Q.SK], npD = S.sh_np[Q.SL];
+    // 1/a per power of the periodic directions (the rows leave it out), by function
+    auto apow = [&](int shell, int comp) {
+        const int *pw = S.fn_pw + 3 * (S.sh_first[shell] + comp);
+        double f = 1.0;
+        for (int d = 0; d < ndp; ++d) f *= tce_ipow(1.0 / S.a[d], pw[d]);
+        return f;
+    };
+    unsigned cm0 = 0;
+    double f0 = 1.0;
+    if (few && cl < Q.ncq) {                         // this lane's component
+        const int ca = cl % Q.nA, r1 = cl / Q.nA, cb = r1 % Q.nB, r2 = r1 / Q.nB, cc = r2 % Q.nC, cd = r2 / Q.nC;
+        coA += ca * npA;
+        coB += cb * npB;
+        coC += cc * npC;
+        coD += cd * npD;
+        cm0 = b.cmap[cl];
+        f0 = apow(Q.SI, ca) * apow(Q.SJ, cb) * apow(Q.SK, cc) * apow(Q.SL, cd);
+    }
+    double accK = 0.0, accG = 0.0;
+    if (nreal > 0)   // exponents and real distances of every primitive quartet of the batch
+        for (int p = lane; p < nb; p += 32) {
+            const int2 pq = b.qlist[p];
+            const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
+            const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
+            b.pqm[4 * p] = Pb.esum * Pk.esum;
+            b.pqm[4 * p + 1] = Pb.esum + Pk.esum;
+            for (int dr = 0; dr < nreal; ++dr) b.pqm[4 * p + 2 + dr] = Pb.cen[ndp + dr] - (Pk.cen[ndp + dr] + Q.Tsh[ndp + dr]);
+        }
+    if (tc) row_setup<NQ>(wofs, nb, lane);
 #pragma unroll 1
     for (int k0 = 0; k0 < NQ; k0 += NC) {
         const int g0c = k0 / 8, kn = NQ - k0 < NC ? NQ - k0 : NC;
-        bool rows_done = false;
-        // tensor-core rows when the launch asks for them (32- and 64-node rules)
-        if constexpr (RO && (NQ == 32 || NQ == 64)) {
-            if (tc) {
-                for (int d = 0; d < ndp; ++d) tc_rows<NQ>(S, Rv, Q, nb, b, lane, g0c, d);
-                rows_done = true;
+        if (tc) {
+            tc_rows<NQ, RO, RS>(wofs, nb, lane, g0c);
+        } else {
+            const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
+            for (int r = lane; r < per * ndp; r += 32) {
+                const int d = r / per, rr = r - d * per, p = rr / ncomb;
+                const int dg = b.dig[rr - p * ncomb];
+                const int ia = dg & 3, ib = (dg >> 2) & 3, ic = (dg >> 4) & 3, id = dg >> 6;
+                int2 pq = b.qlist[p];
+                const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
+                const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
+                const double2 *G = S.vec + Q.Ub.vec_off +
+                                   ((((long long)d * (Q.lsA + 1) + ia) * (Q.lsB + 1) + ib) * 2 + 0) * (long long)Q.Ub.Nlen * nppb;
+                const double2 *H = S.vec + Q.Uk.vec_off +
+                                   ((((long long)d * (Q.lsC + 1) + ic) * (Q.lsD + 1) + id) * 2 + 1) * (long long)Q.Uk.Nlen * nppk;
+                int nm = Pb.N[d] < Pk.N[d] ? Pb.N[d] : Pk.N[d];
+                double phi = S.a[d] * (Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]));
+                row_dot<NQ, RO>(Rv, d, G, nppb, pq.x, H, nppk, pq.y, nm, phi, 1.0, g0c, b.rows + (size_t)r * RS);
             }
         }
-        for (int r = lane; r < (rows_done ? 0 : nrows); r += 32) {
-            int p = r / R, rem = r - p * R;
-            int d = rem / ncomb, cmb = rem - d * ncomb;
-            int ia = cmb % (lsA + 1), t1 = cmb / (lsA + 1);
-            int ib = t1 % (lsB + 1), t2 = t1 / (lsB + 1);
-            int ic = t2 % (lsC + 1), id = t2 / (lsC + 1);
-            int2 pq = b.qlist[p];
-            const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
-            const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
-            const double2 *G = S.vec + Q.Ub.vec_off +
-                               ((((long long)d * (lsA + 1) + ia) * (lsB + 1) + ib) * 2 + 0) * (long long)Q.Ub.Nlen * nppb;
-            const double2 *H = S.vec + Q.Uk.vec_off +
-                               ((((long long)d * (lsC + 1) + ic) * (lsD + 1) + id) * 2 + 1) * (long long)Q.Uk.Nlen * nppk;
-            int nm = Pb.N[d] < Pk.N[d] ? Pb.N[d] : Pk.N[d];
-            double phi = S.a[d] * (Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]));
-            double sgn = pow(S.a[d], -(double)(ia + ib + ic + id));
-            row_dot<NQ, RO>(Rv, d, G, nppb, pq.x, H, nppk, pq.y, nm, phi, sgn, g0c, b.rows + (size_t)r * RS);
+        for (int k = lane; k < 2 * kn; k += 32) {   // the chunk's weights: Kronrod, then Gauss
+            const int kk = k < kn ? k : k - kn;
+            b.wts[(k < kn ? 0 : 32) + kk] = k < kn ? Rv.wk[k0 + kk] : (judge ? Rv.wg[k0 + kk] : 0.0);
         }
         __syncwarp();
-        for (int p = 0; p < nb; ++p) {
-            int2 pq = b.qlist[p];
-            const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
-            const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
-            const double pp_ = Pb.esum, qq = Pk.esum;
+#pragma unroll 1
+        for (int q0 = 0; q0 < nb; q0 += RP) {
+            const int qn = nb - q0 < RP ? nb - q0 : RP;
             if (nreal > 0) {
-                const double *Eb = S.ecoef + Q.Ub.e_off + (long long)pq.x * nreal * (lsA + 1) * (lsB + 1) * TCE_ECO;
-                const double *Ek = S.ecoef + Q.Uk.e_off + (long long)pq.y * nreal * (lsC + 1) * (lsD + 1) * TCE_ECO;
-                for (int k = lane; k < kn; k += 32) {
-                    double t = Rv.t[k0 + k], t2 = t * t;
-                    const double rr = rsqrt(pp_ * qq + (pp_ + qq) * t2), D2 = rr * rr;
-                    double w = pp_ * qq * t2 * D2, rs = PI_D * rr;
+                // g_m(t) of the real directions, then every combination's
+                // sum_{u,v} (-1)^u E_u E'_v g_{u+v}: the products of E by order first
+                for (int x = lane; x < qn * kn; x += 32) {
+                    const int pi = x / kn, k = x - pi * kn;
+                    const double *pm = b.pqm + 4 * (q0 + pi);
+                    const double t = Rv.t[k0 + k], t2 = t * t;
+                    const double rr = rsqrt(fma(pm[1], t2, pm[0])), D2 = rr * rr;
+                    const double w2 = 2.0 * (pm[0] * t2 * D2), rs = PI_D * rr;
                     for (int dr = 0; dr < nreal; ++dr) {
-                        int d = ndp + dr;
-                        double Rr = Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]);
-                        double gt[4 * TCE_LMAX + 2];
-                        gt[0] = (Rr == 0.0) ? rs : rs * exp(-w * Rr * Rr);
-                        double gm1 = 0.0, g0 = gt[0];
-                        for (int n = 0; n < Q.NN; ++n) {
-                            double gp1 = 2.0 * w * Rr * g0 - 2.0 * (double)n * w * gm1;
-                            gt[n + 1] = gp1;
+                        const double Rr = pm[2 + dr], wR = w2 * Rr;
+                        double *g = b.gt + (size_t)(dr * TCE_GT_ROWS + pi * (NN + 1)) * RS + k;
+                        double gm1 = 0.0, g0 = (Rr == 0.0) ? rs : rs * exp(-0.5 * wR * Rr);
+                        g[0] = g0;
+                        for (int n = 0; n < NN; ++n) {
+                            const double gp1 = wR * g0 - (double)n * w2 * gm1;
+                            g += RS;
+                            g[0] = gp1;
                             gm1 = g0;
                             g0 = gp1;
-                        }
-                        for (int cmb = 0; cmb < ncomb; ++cmb) {
-                            int ia = cmb % (lsA + 1), u1 = cmb / (lsA + 1);
-                            int ib = u1 % (lsB + 1), u2 = u1 / (lsB + 1);
-                            int ic = u2 % (lsC + 1), id = u2 / (lsC + 1);
-                            const double *eb = Eb + ((dr * (lsA + 1) + ia) * (lsB + 1) + ib) * TCE_ECO;
-                            const double *ek = Ek + ((dr * (lsC + 1) + ic) * (lsD + 1) + id) * TCE_ECO;
-                            double val = 0.0;
-                            for (int n = 0; n <= ia + ib; ++n) {
-                                double sb = (n & 1) ? -eb[n] : eb[n];
-                                for (int kk = 0; kk <= ic + id; ++kk) val += sb * ek[kk] * gt[n + kk];
-                            }
-                            b.realb[((size_t)dr * cstride + cmb) * RS + k] = val;
                         }
                     }
                 }
                 __syncwarp();
+                const int nrow = qn * ncomb * nreal;
+                const int sp = nrow <= 8 ? 4 : nrow <= 16 ? 2 : 1, kp = ((kn >> 1) + sp - 1) / sp;   // lanes per row, node pairs each
+                for (int xs = lane; xs < nrow * sp; xs += 32) {
+                    const int part = xs / nrow, x = xs - part * nrow;
+                    const int dr = x / (qn * ncomb), y = x - dr * qn * ncomb, pi = y / ncomb, cmb = y - pi * ncomb;
+                    const int dg = b.dig[cmb];
+                    const int ia = dg & 3, ib = (dg >> 2) & 3, ic = (dg >> 4) & 3, id = dg >> 6;
+                    const int2 pq = b.qlist[q0 + pi];
+                    const double *eb = S.ecoef + Q.Ub.e_off + ((((long long)pq.x * nreal + dr) * (Q.lsA + 1) + ia) * (Q.lsB + 1) + ib) * TCE_ECO;
+                    const double *ek = S.ecoef + Q.Uk.e_off + ((((long long)pq.y * nreal + dr) * (Q.lsC + 1) + ic) * (Q.lsD + 1) + id) * TCE_ECO;
+                    double sm[2 * TCE_ECO - 1];
+#pragma unroll
+                    for (int m = 0; m < 2 * TCE_ECO - 1; ++m) sm[m] = 0.0;
+#pragma unroll
+                    for (int u = 0; u < TCE_ECO; ++u) {
+                        if (u > ia + ib) continue;
+                        const double e = (u & 1) ? -eb[u] : eb[u];
+#pragma unroll
+                        for (int v = 0; v < TCE_ECO; ++v)
+                            if (v <= ic + id) sm[u + v] = fma(e, ek[v], sm[u + v]);
+                    }
+                    const int mm = ia + ib + ic + id;
+                    const double2 *g = reinterpret_cast<const double2 *>(b.gt + (size_t)(dr * TCE_GT_ROWS + pi * (NN + 1)) * RS);
+                    double2 *o = reinterpret_cast<double2 *>(b.realb + (size_t)(dr * cstride + y) * RS);
+                    for (int k = part * kp; k < min((part + 1) * kp, kn >> 1); ++k) {
+                        double2 v = g[k];
+                        v.x *= sm[0];
+                        v.y *= sm[0];
+#pragma unroll
+                        for (int m = 1; m < 2 * TCE_ECO - 1; ++m)
+                            if (m <= mm) {
+                                const double2 z = g[m * (RS / 2) + k];
+                                v.x = fma(sm[m], z.x, v.x);
+                                v.y = fma(sm[m], z.y, v.y);
+                            }
+                        o[k] = v;
+                    }
+                }
+                __syncwarp();
             }
-            const double fac = b.qfac[p];
-            const double *rowp = b.rows + (size_t)p * R * RS;
-            const int i = pq.x / Q.Ub.np2, j = pq.x % Q.Ub.np2;
-            const int kp = pq.y / Q.Uk.np2, lp = pq.y % Q.Uk.np2;
-            // The component quartets: sum_k w_k I_x I_y I_z per component.  G lanes
-            // share one component and split its nodes (G = 32 / next power of two of
-            // the component count, at most NQ), so that the warp holds 32 / G
-            // components at once and each needs log2(G) shuffles instead of a full
-            // warp reduction; each component's block entry has one owning lane.
-            const int G = Q.cqg < NC ? Q.cqg : NC;
-            const int slots = 32 / G, slot = lane / G, sub = lane - slot * G;
-            for (int c0 = 0; c0 < Q.ncq; c0 += slots) {
-                const int cq = c0 + slot;
-                double vK = 0.0, vG = 0.0;
-                int ca = 0, cb = 0, cc = 0, cd = 0;
-                if (cq < Q.ncq) {
-                    ca = cq % Q.nA;
-                    const int r1 = cq / Q.nA;
-                    cb = r1 % Q.nB;
-                    const int r2 = r1 / Q.nB;
-                    cc = r2 % Q.nC;
-                    cd = r2 / Q.nC;
-                    const int *pa = S.fn_pw + 3 * (S.sh_first[Q.SI] + ca);
-                    const int *pb = S.fn_pw + 3 * (S.sh_first[Q.SJ] + cb);
-                    const int *pc = S.fn_pw + 3 * (S.sh_first[Q.SK] + cc);
-                    const int *pd = S.fn_pw + 3 * (S.sh_first[Q.SL] + cd);
-                    const double *rw[3];
-    #pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const int cm = pa[d] + (lsA + 1) * (pb[d] + (lsB + 1) * (pc[d] + (lsC + 1) * pd[d]));
-                        rw[d] = (d < ndp) ? rowp + ((size_t)d * ncomb + cm) * RS
-                                          : b.realb + ((size_t)(d - ndp) * cstride + cm) * RS;
+#pragma unroll 1
+          for (int p0 = q0; p0 < q0 + qn; p0 += PW) {
+            const int pn = q0 + qn - p0 < PW ? q0 + qn - p0 : PW;
+            if (!few) {   // the primitive quartet's coefficient products of bra and ket components
+                const short4 ix = b.qidx[p0];
+                const double fac = b.qfac[p0];
+                for (int x = lane; x < nAB + nCD; x += 32) {
+                    const int z = x - nAB;
+                    if (x < nAB) {
+                        const int ca = x % Q.nA, cb = x / Q.nA;
+                        b.cf[x] = fac * (coA[ca * npA + ix.x] * apow(Q.SI, ca)) * (coB[cb * npB + ix.y] * apow(Q.SJ, cb));
+                    } else {
+                        const int cc = z % Q.nC, cd = z / Q.nC;
+                        b.cf[36 + z] = (coC[cc * npC + ix.z] * apow(Q.SK, cc)) * (coD[cd * npD + ix.w] * apow(Q.SL, cd));
                     }
-                    // two partial sums per estimate: shorter dependent FMA chains
-                    double vK1 = 0.0, vG1 = 0.0;
-                    int k = sub;
-                    for (; k + G < kn; k += 2 * G) {
-                        const double p0 = rw[0][k] * rw[1][k] * rw[2][k];
-                        const double p1 = rw[0][k + G] * rw[1][k + G] * rw[2][k + G];
-                        vK = fma(Rv.wk[k0 + k], p0, vK);
-                        vK1 = fma(Rv.wk[k0 + k + G], p1, vK1);
-                        if (judge) {
-                            vG = fma(Rv.wg[k0 + k], p0, vG);
-                            vG1 = fma(Rv.wg[k0 + k + G], p1, vG1);
-                        }
-                    }
-                    if (k < kn) {
-                        const double p0 = rw[0][k] * rw[1][k] * rw[2][k];
-                        vK = fma(Rv.wk[k0 + k], p0, vK);
-                        if (judge) vG = fma(Rv.wg[k0 + k], p0, vG);
-                    }
-                    vK += vK1;
-                    vG += vG1;
                 }
-                for (int o = G >> 1; o > 0; o >>= 1) {
-                    vK += __shfl_xor_sync(0xffffffffu, vK, o);
-                    if (judge) vG += __shfl_xor_sync(0xffffffffu, vG, o);
+                __syncwarp();
+            }
+            // sum_k w_k I_x I_y I_z per component: one lane per component (and primitive
+            // quartet), two nodes per load
+            const int p = p0 + pl;
+            for (int c = cl; c < Q.ncq && pl < pn; c += 32) {
+                const unsigned cm = few ? cm0 : b.cmap[c];
+                const double2 *rw[3];
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const int x = (cm >> (8 * d)) & 255;
+                    rw[d] = reinterpret_cast<const double2 *>(d < ndp ? b.rows + (size_t)(d * per + p * ncomb + x) * RS
+                                                                      : b.realb + (size_t)((d - ndp) * cstride + (p - q0) * ncomb + x) * RS);
                 }
-                if (cq < Q.ncq && sub == 0) {
-                    const double cf = S.sh_coef[S.sh_coff[Q.SI] + ca * npA + i] * S.sh_coef[S.sh_coff[Q.SJ] + cb * npB + j] *
-                                      S.sh_coef[S.sh_coff[Q.SK] + cc * npC + kp] * S.sh_coef[S.sh_coff[Q.SL] + cd * npD + lp];
-                    b.blkK[cq] += fac * cf * vK;
-                    if (judge) b.blkG[cq] += fac * cf * vG;
+                const double2 *wk2 = reinterpret_cast<const double2 *>(b.wts), *wg2 = wk2 + 16;
+                double vK = 0.0, vG = 0.0, vK1 = 0.0, vG1 = 0.0;
+#pragma unroll 4
+                for (int k = 0; k < (kn >> 1); ++k) {
+                    const double2 x = rw[0][k], y = rw[1][k], z = rw[2][k], w = wk2[k];
+                    const double a0 = x.x * y.x * z.x, a1 = x.y * y.y * z.y;
+                    vK = fma(w.x, a0, vK);
+                    vK1 = fma(w.y, a1, vK1);
+                    if (judge) {
+                        const double2 g = wg2[k];
+                        vG = fma(g.x, a0, vG);
+                        vG1 = fma(g.y, a1, vG1);
+                    }
+                }
+                if (few) {
+                    const short4 ix = b.qidx[p];
+                    const double f = b.qfac[p] * f0 * (coA[ix.x] * coB[ix.y] * coC[ix.z] * coD[ix.w]);
+                    accK = fma(f, vK + vK1, accK);
+                    if (judge) accG = fma(f, vG + vG1, accG);
+                } else {
+                    const int cd = c / nAB;
+                    const double f = b.cf[c - cd * nAB] * b.cf[36 + cd];
+                    b.blkK[c] = fma(f, vK + vK1, b.blkK[c]);
+                    if (judge) b.blkG[c] = fma(f, vG + vG1, b.blkG[c]);
                 }
             }
             __syncwarp();
+          }
         }
     }
+    accK_ += accK;
+    accG_ += accG;
 }
 
 __device__ __forceinline__ void make_ctx(const DevSys &S, int4 q, QCtx &Q)
@@ -472,11 +678,8 @@ __device__ __forceinline__ void make_ctx(const DevSys &S, int4 q, QCtx &Q)
     Q.lsA = S.sh_l[Q.SI]; Q.lsB = S.sh_l[Q.SJ]; Q.lsC = S.sh_l[Q.SK]; Q.lsD = S.sh_l[Q.SL];
     Q.ncomb = (Q.lsA + 1) * (Q.lsB + 1) * (Q.lsC + 1) * (Q.lsD + 1);
     Q.ncq = Q.nA * Q.nB * Q.nC * Q.nD;
-    {
-        int p2 = 1;
-        while (p2 < Q.ncq) p2 <<= 1;
-        Q.cqg = p2 >= 32 ? 1 : 32 / p2;
-    }
+    Q.cqp = 1;
+    while (Q.cqp < Q.ncq && Q.cqp < 32) Q.cqp <<= 1;
     Q.NN = Q.lsA + Q.lsB + Q.lsC + Q.lsD;
     Q.R = Q.ncomb * S.ndp;
     const int cK = Q.SK / S.nshuc;
@@ -488,15 +691,30 @@ __device__ __forceinline__ void make_ctx(const DevSys &S, int4 q, QCtx &Q)
     for (int d = 0; d < 3; ++d) Q.Tsh[d] = S.sh_r[3 * Q.SK + d] - S.sh_r[3 * SK0 + d];
 }
 
-// The block of one shell quartet with rule Rv: screen and batch the primitive
+// The block of one shell quartet with its rule (Q.R_): screen and batch the primitive
 // quartets, accumulate into b.blkK (and b.blkG); both are zeroed first.
 template <int NQ, bool RO>
-__device__ void eval_block(const DevSys &S, const QuartetArgs &A, const RuleView &Rv, const QCtx &Q, const WarpBuf &b,
-                           int lane, int want)
+__device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A, int wofs, int lane, int want)
 {
+    const QCtx &Q = warp_ctx(wofs);
+    const WarpBuf b = warp_buf(wofs);
+    double accK = 0.0, accG = 0.0;
     for (int c = lane; c < Q.ncq; c += 32) {
         b.blkK[c] = 0.0;
         b.blkG[c] = 0.0;
+        // the power combination of each direction
+        const int ca = c % Q.nA, r1 = c / Q.nA, cb = r1 % Q.nB, r2 = r1 / Q.nB, cc = r2 % Q.nC, cd = r2 / Q.nC;
+        const int *pa = S.fn_pw + 3 * (S.sh_first[Q.SI] + ca), *pb = S.fn_pw + 3 * (S.sh_first[Q.SJ] + cb);
+        const int *pc = S.fn_pw + 3 * (S.sh_first[Q.SK] + cc), *pd = S.fn_pw + 3 * (S.sh_first[Q.SL] + cd);
+        unsigned cm = 0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d)
+            cm |= (unsigned)(pa[d] + (Q.lsA + 1) * (pb[d] + (Q.lsB + 1) * (pc[d] + (Q.lsC + 1) * pd[d]))) << (8 * d);
+        b.cmap[c] = cm;
+    }
+    for (int x = lane; x < Q.ncomb; x += 32) {
+        const int ia = x % (Q.lsA + 1), t1 = x / (Q.lsA + 1), ib = t1 % (Q.lsB + 1), t2 = t1 / (Q.lsB + 1);
+        b.dig[x] = (unsigned char)(ia | ib << 2 | (t2 % (Q.lsC + 1)) << 4 | (t2 / (Q.lsC + 1)) << 6);
     }
     __syncwarp();
     int B = A.rowcap / Q.R;
@@ -535,19 +753,31 @@ __device__ void eval_block(const DevSys &S, const QuartetArgs &A, const RuleView
             if (take > cnt - done) take = cnt - done;
             if (keep && pos >= done && pos < done + take) {
                 b.qlist[nb + pos - done] = make_int2(ipb, ipk);
+                const int i = ipb / Q.Ub.np2, k = ipk / Q.Uk.np2;
+                b.qidx[nb + pos - done] = make_short4((short)i, (short)(ipb - i * Q.Ub.np2), (short)k, (short)(ipk - k * Q.Uk.np2));
                 b.qfac[nb + pos - done] = fac;
             }
             nb += take;
             done += take;
             __syncwarp();
             if (nb == B) {
-                process_batch<NQ, RO>(S, Rv, Q, nb, b, lane, A.cstride, A.use_tc != 0);
+                process_batch<NQ, RO>(wofs, nb, lane, A.cstride, A.use_tc != 0, accK, accG);
                 nb = 0;
                 __syncwarp();
             }
         }
     }
-    if (nb > 0) process_batch<NQ, RO>(S, Rv, Q, nb, b, lane, A.cstride, A.use_tc != 0);
+    if (nb > 0) process_batch<NQ, RO>(wofs, nb, lane, A.cstride, A.use_tc != 0, accK, accG);
+    if (Q.ncq <= 32) {
+        for (int o = Q.cqp; o < 32; o <<= 1) {
+            accK += __shfl_xor_sync(0xffffffffu, accK, o);
+            accG += __shfl_xor_sync(0xffffffffu, accG, o);
+        }
+        if (lane < Q.ncq) {
+            b.blkK[lane] = accK;
+            b.blkG[lane] = accG;
+        }
+    }
     __syncwarp();
 }
 
@@ -561,6 +791,7 @@ __device__ __forceinline__ RuleView dict_rule(const DevSys &S, const QuartetArgs
     R.wk = A.rule_wk + D.node_off;
     R.wg = judge ? A.rule_wg + D.node_off : nullptr;
     R.gmax = D.gmax;
+    R.t2 = D.t2;
     return R;
 }
 
@@ -648,22 +879,28 @@ __device__ __forceinline__ int item_count(const QuartetArgs &A)
 // method 0: one fixed rule for every item (the system's rule, or dictionary rule
 // rule_override, judged when blk_out2 is set); method 1: the learned grid.
 template <int NQ>
-__global__ void __launch_bounds__(256) k_quartets(DevSys S, QuartetArgs A)
+__global__ void __launch_bounds__(256, 2) k_quartets(DevSys S, QuartetArgs A)
 {
-    extern __shared__ double smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const WarpBuf b = warp_buf(A, smem + (size_t)wib * A.warp_smem_doubles, 3 - S.ndp, (NQ < 32 ? NQ : 32) + 1);
+    blk_header(S, A.lay);
+    const int wofs = TCE_HDR_DOUBLES + wib * A.warp_smem_doubles;
+    const WarpBuf b = warp_buf(wofs);
+    QCtx &Q = warp_ctx(wofs);
     const bool lg = (A.method == TCE_METHOD_LEARNED);
-    RuleView Rfix;
-    if (A.rule_override >= 0) {
-        Rfix = dict_rule(S, A, A.rule_override, A.blk_out2 != nullptr);
-    } else {
-        Rfix.T = S.Tt;
-        Rfix.strideD = (long long)(S.ncap + 1) * S.nq;
-        Rfix.t = S.tnode;
-        Rfix.wk = S.tweight;
-        Rfix.wg = nullptr;
-        Rfix.gmax = A.fixed_gmax;
+    if (lane == 0 && !lg) {
+        if (A.rule_override >= 0) {
+            Q.R_ = dict_rule(S, A, A.rule_override, A.blk_out2 != nullptr);
+        } else {
+            RuleView R;
+            R.T = S.Tt;
+            R.strideD = (long long)(S.ncap + 1) * S.nq;
+            R.t = S.tnode;
+            R.wk = S.tweight;
+            R.wg = nullptr;
+            R.gmax = A.fixed_gmax;
+            R.t2 = S.rule_t2;
+            Q.R_ = R;
+        }
     }
     const int nitems = item_count(A);
     while (true) {
@@ -671,13 +908,15 @@ __global__ void __launch_bounds__(256) k_quartets(DevSys S, QuartetArgs A)
         if (lane == 0) it = (int)atomicAdd(A.next, 1u);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= nitems) break;
-        QCtx Q;
-        make_ctx(S, A.items[it], Q);
+        if (lane == 0) {
+            make_ctx(S, A.items[it], Q);
+            if (lg) Q.R_ = dict_rule(S, A, A.item_rule[it], true);
+        }
+        __syncwarp();
         int want = -1;
         if (A.mode == TCE_MODE_PRIMTAB) want = A.prim_sel[2 * it] * Q.Ub.np2 + A.prim_sel[2 * it + 1];
+        eval_block<NQ, true>(S, A, wofs, lane, want);
         if (lg) {
-            const RuleView R = dict_rule(S, A, A.item_rule[it], true);
-            eval_block<NQ, true>(S, A, R, Q, b, lane, want);
             const double e = block_judge(b.blkK, b.blkG, Q.ncq, lane);
             if (!(e <= A.judge_tol)) {      // the judge rejects the predicted rule
                 if (lane == 0) {
@@ -688,8 +927,6 @@ __global__ void __launch_bounds__(256) k_quartets(DevSys S, QuartetArgs A)
                 __syncwarp();
                 continue;
             }
-        } else {
-            eval_block<NQ, true>(S, A, Rfix, Q, b, lane, want);
         }
         consume(S, A, Q, b, it, lane, want);
         __syncwarp();
@@ -733,7 +970,7 @@ __device__ __forceinline__ double tce_ive_debye(double nu, double x)
 }
 
 __device__ void plain_columns(const DevSys &S, const QuartetArgs &A, double *T, int nneed, double a, double bnd,
-                              double *tn, double *wk, double *wg, int *gmax, int lane)
+                              double *tn, double *wk, double *wg, int *gmax, float2 *t2, int lane)
 {
     double t = 0.0, w1 = 0.0, w2 = 0.0;
     if (lane < 15) {
@@ -747,6 +984,15 @@ __device__ void plain_columns(const DevSys &S, const QuartetArgs &A, double *T, 
         tn[lane] = t;
         wk[lane] = w1;
         wg[lane] = w2;
+    }
+    {   // t^2 range of the two node groups (the 16th node is padding)
+        float lo = lane < 15 ? (float)(t * t) : __int_as_float(0x7f800000), hi = lane < 15 ? lo : -lo;
+#pragma unroll
+        for (int o = 4; o > 0; o >>= 1) {
+            lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+            hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+        }
+        if (lane < 16 && (lane & 7) == 0) t2[lane >> 3] = make_float2(lo * 0.999999f, hi * 1.000001f);
     }
     for (int d = 0; d < S.ndp; ++d) {
         double *Td = T + (size_t)d * (nneed + 1) * 16;
@@ -817,15 +1063,18 @@ __device__ void plain_columns(const DevSys &S, const QuartetArgs &A, double *T, 
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(128) k_plain(DevSys S, QuartetArgs A)
+__global__ void __launch_bounds__(128, 4) k_plain(DevSys S, QuartetArgs A)
 {
-    extern __shared__ double smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    const WarpBuf b = warp_buf(A, smem + (size_t)wib * A.warp_smem_doubles, 3 - S.ndp, 17);
+    blk_header(S, A.lay);
+    const int wofs = TCE_HDR_DOUBLES + wib * A.warp_smem_doubles;
+    const WarpBuf b = warp_buf(wofs);
+    QCtx &Q = warp_ctx(wofs);
     // extra: panel bounds and errors, the panel's nodes and weights, gmax
     double *pa = b.extra, *pb = pa + PLAIN_PMAX, *perr = pb + PLAIN_PMAX;
     double *tn = perr + PLAIN_PMAX, *wk = tn + 16, *wg = wk + 16;
     int *gmax = reinterpret_cast<int *>(wg + 16);
+    float2 *t2 = reinterpret_cast<float2 *>(gmax + 3 * TCE_MAXG);
     const long long gw = (long long)blockIdx.x * (blockDim.x >> 5) + wib;
     double *T = A.scratch + gw * A.scratch_per_warp;
     double *pblk = T + A.T_doubles;      // [PLAIN_PMAX][blkcap]
@@ -838,8 +1087,8 @@ __global__ void __launch_bounds__(128) k_plain(DevSys S, QuartetArgs A)
         if (lane == 0) it = (int)atomicAdd(A.next, 1u);
         it = __shfl_sync(0xffffffffu, it, 0);
         if (it >= nitems) break;
-        QCtx Q;
-        make_ctx(S, A.items[it], Q);
+        if (lane == 0) make_ctx(S, A.items[it], Q);
+        __syncwarp();
         int nneed = 0;
         {   // largest truncation order among the bra's pair primitives (bounds min(N_bra, N_ket))
             int m = 0;
@@ -850,16 +1099,21 @@ __global__ void __launch_bounds__(128) k_plain(DevSys S, QuartetArgs A)
             nneed = m;
         }
         unsigned long long evals = 0;
-        RuleView R;
-        R.T = T;
-        R.strideD = (long long)(nneed + 1) * 16;
-        R.t = tn;
-        R.wk = wk;
-        R.wg = wg;
-        R.gmax = gmax;
+        if (lane == 0) {
+            RuleView R;
+            R.T = T;
+            R.strideD = (long long)(nneed + 1) * 16;
+            R.t = tn;
+            R.wk = wk;
+            R.wg = wg;
+            R.gmax = gmax;
+            R.t2 = t2;
+            Q.R_ = R;
+        }
+        __syncwarp();
         auto eval_panel = [&](int slot, double a, double bnd) {
-            plain_columns(S, A, T, nneed, a, bnd, tn, wk, wg, gmax, lane);
-            eval_block<16, false>(S, A, R, Q, b, lane, -1);
+            plain_columns(S, A, T, nneed, a, bnd, tn, wk, wg, gmax, t2, lane);
+            eval_block<16, false>(S, A, wofs, lane, -1);
             const double e = block_judge(b.blkK, b.blkG, Q.ncq, lane);
             for (int c = lane; c < Q.ncq; c += 32) pblk[(size_t)slot * A.blkcap + c] = b.blkK[c];
             if (lane == 0) {
@@ -917,8 +1171,8 @@ static int2 quartet_shape(size_t wbytes)
     if (it != known.end()) return it->second;
     int2 best = make_int2(0, 0);   // (warps, blocks per SM)
     for (int w = 8; w >= 1; --w) {
-        const size_t smem = wbytes * (size_t)w;
-        if (smem > 220 * 1024) continue;
+        const size_t smem = TCE_HDR_DOUBLES * 8 + wbytes * (size_t)w;
+        if (smem > 226 * 1024) continue;
         cudaFuncSetAttribute(k_quartets<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_quartets<NQ>, 32 * w, smem) != cudaSuccess) per = 0;
@@ -933,7 +1187,7 @@ static cudaError_t launch_nq(const DevSys &S, const QuartetArgs &A, size_t wbyte
 {
     const int2 sh = quartet_shape<NQ>(wbytes);
     if (sh.x < 1 || sh.y < 1) return cudaErrorInvalidConfiguration;
-    const size_t smem = wbytes * (size_t)sh.x;
+    const size_t smem = TCE_HDR_DOUBLES * 8 + wbytes * (size_t)sh.x;
     cudaFuncSetAttribute(k_quartets<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     k_quartets<NQ><<<nsm * sh.y, 32 * sh.x, smem, st>>>(S, A);
     return cudaGetLastError();
@@ -1032,22 +1286,24 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
     if (!plain && !dict && !h.fixed_gmax) return TCE_ERR_ARG;
     const int nq = plain ? 16 : (dict ? h.dict_nq : S.nq);
     const int R = h.max_ncomb * S.ndp;
-    const int rowcap = R > 32 ? R : 32;
-    const int RS = (nq < 32 ? nq : 32) + 1;   // rows of one chunk of at most 32 nodes
+    const int rowcap = std::max(R, 16 * S.ndp);   // at least a tile of rows per periodic direction
+    const int RS = (nq < TCE_NC ? nq : TCE_NC) + 2;   // rows of one chunk of at most 32 nodes
     const int nreal = 3 - S.ndp;
     const int blkcap = (h.max_ncq + 3) / 4 * 4;
-    long long wdoubles = 2LL * rowcap + (long long)rowcap * RS + (long long)nreal * h.max_ncomb * RS + 2LL * blkcap + 8;
-    if (plain) wdoubles += 3 * PLAIN_PMAX + 48 + 3 * TCE_MAXG;
+    const int cstride = h.max_ncomb > 16 ? h.max_ncomb : 16;   // real-direction rows: of one primitive quartet, or 32 / cqp small ones
+    A.lay = tce_warp_layout(rowcap, RS, nreal, cstride, blkcap, (nq + 15) / 16);
+    long long wdoubles = A.lay.extra;
+    if (plain) wdoubles += 3 * PLAIN_PMAX + 48 + 3 * TCE_MAXG / 2 + 4;
     wdoubles = (wdoubles + 31) / 32 * 32;
     A.rowcap = rowcap;
-    A.cstride = h.max_ncomb;
+    A.cstride = cstride;
     A.blkcap = blkcap;
     A.warp_smem_doubles = (int)wdoubles;
     const size_t wbytes = (size_t)wdoubles * sizeof(double);
     int warps = 4;
     while (warps > 1 && wbytes * warps > 220 * 1024) --warps;
     if (wbytes > 220 * 1024) return TCE_ERR_UNSUPPORTED;
-    const size_t smem = wbytes * warps;
+    const size_t smem = TCE_HDR_DOUBLES * 8 + wbytes * warps;
     if (cudaMemsetAsync(h.next, 0, sizeof(unsigned int), st) != cudaSuccess) return TCE_ERR_CUDA;
     const int nsm = h.num_sms > 0 ? h.num_sms : 148;
     cudaError_t e;
