@@ -80,3 +80,25 @@ def test_shells_of_one_d_component(nquad):
         J, K = eng.direct_JK(P)
     scale = np.abs(P).sum()
     assert np.abs(J - J0).max() <= 1e-12 * scale and np.abs(K - K0).max() <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("nquad", [32, 40, 64])
+@pytest.mark.parametrize("shells", ["sp", "spd"])
+def test_nuclear_attraction_few_orders(shells, nquad):
+    """One periodic direction, atoms off the axis, s to d shells: every element
+    within 1e-12 of the sum of charges times the largest s element's scale (1)."""
+    import pyoracle
+    from william_ci_b200 import system as S
+    from william_ci_b200.engine import Engine
+    cell, basis = S.workload("h_chain64")
+    if shells == "spd":
+        basis = S.workload("h2_sheet")[1]
+    cell = dataclasses.replace(cell, atoms=cell.atoms + [("H", (0.7, 0.9, -0.4))])
+    s = S.build_system(S.scaled_down(cell, (5, 1, 1)), basis)
+    pyoracle.normalize(s)
+    t, w = pyoracle.fast_quad(nquad)
+    V0 = pyoracle.Oracle(s, t_nodes=t, t_weights=w).one_electron()[2]
+    with Engine(s, t_nodes=t, t_weights=w) as eng:
+        V = eng.nuclear_attraction()
+    assert np.abs(V0).max() > 0.1
+    assert np.abs(V - V0).max() <= 1e-12 * max(1.0, np.abs(V0).max()) * len(s.charges), np.abs(V - V0).max()

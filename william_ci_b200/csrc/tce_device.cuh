@@ -205,6 +205,73 @@ __device__ __forceinline__ void tce_fourier_sin(int i, int l, double phA, double
     }
 }
 
+// Fourier coefficients of w(u) sin^i(u + phA) sin^l(u + phB), w = sum_n I~_n(A) e^{inu},
+// without the cancellation of sum_k d_k I~_{n-k}: with p = sin u, c = cos u and
+// c^2 = 1 - p^2 the factor is sum_k (a_k + b_k c) p^k, and integrating by parts
+//     <p^k>_n = (-i)^k R_k(n),  R_k(n) = (n R_{k-1}(n) - (k - 1) (R_{k-2}(n-1) + R_{k-2}(n+1)) / 2) / A,
+//     R_0(n) = I~_n(A),         <c p^k>_n = (-i)^k (R_k(n-1) + R_k(n+1)) / 2.
+// The d_k sum leaves a rounding error of eps I~_0 where the coefficient is of the
+// order A^{-(i+l)/2} I~_0 (at A = 1000 and i + l = 2, three digits); a sum over
+// every h-th order, times h (tce_orders.cuh), averages that error less well
+// than one over every order, so the vectors are built to full precision.
+struct PowerSeries {
+    int M;
+    double a[2 * TCE_LMAX + 1], b[2 * TCE_LMAX + 1];
+};
+__device__ __forceinline__ void tce_power_series(int i, int l, double phA, double phB, PowerSeries &ps)
+{
+    const int MM = 2 * TCE_LMAX;
+    const int M = i + l;
+    ps.M = M;
+    double e[MM + 1];   // coefficient of p^x c^(m - x) after m factors
+    for (int x = 0; x <= MM; ++x) e[x] = ps.a[x] = ps.b[x] = 0.0;
+    e[0] = 1.0;
+    for (int m = 1; m <= M; ++m) {
+        double sn, cs;
+        sincos(m <= i ? phA : phB, &sn, &cs);
+        for (int x = m; x >= 0; --x) e[x] = (x < m ? sn * e[x] : 0.0) + (x > 0 ? cs * e[x - 1] : 0.0);
+    }
+    for (int x = 0; x <= M; ++x) {   // p^x c^(M - x), c^2 = 1 - p^2
+        const int h = (M - x) / 2;
+        double *t = ((M - x) & 1) ? ps.b : ps.a;
+        const double v = e[x];
+        t[x] += v;
+        if (h == 1) {
+            t[x + 2] -= v;
+        } else if (h == 2) {
+            t[x + 2] -= 2.0 * v;
+            t[x + 4] += v;
+        }
+    }
+}
+// <w x series>_n for n of either sign; Iv: I~_0.., inv_A = 1 / A
+__device__ __forceinline__ double2 tce_power_coef(const PowerSeries &ps, const double *Iv, int n, double inv_A)
+{
+    const int MM = 2 * TCE_LMAX;
+    double R[MM + 1][2 * MM + 3];   // R_k(n + x - MM - 1) at [k][x]
+    const int M = ps.M, C = MM + 1;
+    for (int x = -M; x <= M; ++x) {
+        const int m = n + x;
+        R[0][C + x] = Iv[m < 0 ? -m : m];
+    }
+    for (int k = 1; k <= M; ++k)
+        for (int x = -(M - k); x <= M - k; ++x) {
+            const double c = k > 1 ? 0.5 * (double)(k - 1) * (R[k > 1 ? k - 2 : 0][C + x - 1] + R[k > 1 ? k - 2 : 0][C + x + 1]) : 0.0;
+            R[k][C + x] = ((double)(n + x) * R[k - 1][C + x] - c) * inv_A;
+        }
+    double re = 0.0, im = 0.0;
+    for (int k = 0; k <= M; ++k) {
+        double v = ps.a[k] * R[k][C];
+        if (k < M) v += ps.b[k] * 0.5 * (R[k][C - 1] + R[k][C + 1]);
+        const int r = k & 3;   // (-i)^k
+        if (r == 0) re += v;
+        else if (r == 1) im -= v;
+        else if (r == 2) re -= v;
+        else im += v;
+    }
+    return make_double2(re, im);
+}
+
 __device__ __forceinline__ double tce_warp_sum(double v)
 {
 #pragma unroll

@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "tce_handle.h"
+#include "tce_orders.cuh"
 
 namespace {
 
@@ -33,24 +34,23 @@ constexpr double PI_D = 3.14159265358979323846;
 constexpr int NA_WARPS_MAX = 8;
 constexpr int NA_MEXTRA = 4 * TCE_LMAX + 4;   // Bessel orders past N for the Fourier product
 
-// 1D overlap of x^j e^{-p (x - PA')...}: sum_k sum_q C(j,k) C(m,q) pa^{j-k} pb^{m-q}
-// <x^{k+q}>, moments (n-1)!! / (2p)^{n/2} sqrt(pi/p) (overlap_1D_real, :336-361)
-__device__ double na_overlap_1d(int j, int m, double p, double pa, double pb)
+// 1D overlap of (x + pa)^j (x + pb)^m with e^{-p x^2}, over sqrt(pi / p): the
+// polynomial's even coefficients times the moments (n-1)!! / (2p)^{n/2}
+// (overlap_1D_real, :336-361); inv = 1 / p
+__device__ __forceinline__ double na_overlap_1d(int j, int m, double inv, double pa, double pb)
 {
-    double mom[2 * TCE_LMAX + 1];
-    mom[0] = sqrt(PI_D / p);
-    if (j + m >= 1) mom[1] = 0.0;
-    for (int n = 2; n <= j + m; ++n) mom[n] = (n & 1) ? 0.0 : mom[n - 2] * (double)(n - 1) / (2.0 * p);
-    double acc = 0.0, bj = 1.0;
-    for (int k = 0; k <= j; ++k) {
-        double bm = 1.0;
-        for (int q = 0; q <= m; ++q) {
-            if (((k + q) & 1) == 0) acc += bj * bm * pow(pa, (double)(j - k)) * pow(pb, (double)(m - q)) * mom[k + q];
-            bm = bm * (double)(m - q) / (double)(q + 1);
-        }
-        bj = bj * (double)(j - k) / (double)(k + 1);
+    if (j + m == 0) return 1.0;
+    double c[2 * TCE_LMAX + 1];
+    c[0] = 1.0;
+#pragma unroll
+    for (int x = 1; x <= 2 * TCE_LMAX; ++x) c[x] = 0.0;
+    for (int f = 0; f < j + m; ++f) {
+        const double r = f < j ? pa : pb;
+#pragma unroll
+        for (int x = 2 * TCE_LMAX; x > 0; --x) c[x] = fma(r, c[x], c[x - 1]);
+        c[0] *= r;
     }
-    return acc;
+    return fma(0.75 * inv * inv, c[4], fma(0.5 * inv, c[2], c[0]));
 }
 
 struct NaArgs {
@@ -62,6 +62,7 @@ struct NaArgs {
     const int *Z;
     double *V;           // rows of the unit cell V[i + nfuc * j], or V[p] for a pair list
     int wdoubles;        // shared doubles per warp
+    double zsum;         // sum of |Z|
 };
 
 __global__ void __launch_bounds__(NA_WARPS_MAX * 32) k_nuclear(DevSys S, NaArgs A)
@@ -187,8 +188,8 @@ __global__ void __launch_bounds__(NA_WARPS_MAX * 32) k_nuclear(DevSys S, NaArgs 
                         } else {
                             const double ppt = es + t2, eta = t2 / ppt, pc = cen[d] - Cc[d];
                             const double ed = exp(-es * eta * pc * pc);
-                            prod *= ed * na_overlap_1d(l1[d], l2[d], ppt, (cen[d] - r1[d]) - eta * pc,
-                                                        (cen[d] - r2[d]) - eta * pc);
+                            prod *= ed * sqrt(PI_D / ppt) * na_overlap_1d(l1[d], l2[d], 1.0 / ppt, (cen[d] - r1[d]) - eta * pc,
+                                                                          (cen[d] - r2[d]) - eta * pc);
                         }
                     }
                     res = fma(S.tweight[k], prod, res);
@@ -208,182 +209,242 @@ __device__ __forceinline__ void na_dmma(double &d0, double &d1, double a, double
                  : "d"(a), "d"(b));
 }
 
-// One periodic direction, 32- or 64-node rule: per primitive pair the node
-// sums of every atom, X(atom, k) = sum_n F_n(atom) T[n][k], are an
-// (atoms x orders) x (orders x nodes) product done as FP64 mma.sync.m8n8k4
-// tiles: 16 atoms x 32 nodes per pass, lane l owns atom rows 8 m + l/4 and
-// order 4 s + l%4, cos / sin(n phi_atom) by the three-term recurrence in
-// steps of four (re-seeded every 32 orders), B fragments T[4 s + l%4][8 g + l/4].
-// The epilogue multiplies each (atom, node) by its real-direction factors,
-// weight and charge.  G vectors, prefactor and the rest as k_nuclear.
-template <int NQ>
-__global__ void __launch_bounds__(NA_WARPS_MAX * 32, 1) k_nuclear_tc(DevSys S, NaArgs A)
+// One periodic direction: a block per function pair, its warps over the
+// primitive pairs.  Per primitive pair the node sums of every atom,
+//     X(atom, k) = h sum_j F_{h j}(atom) T[h j][k],
+// run over the orders of tce_order_plan (tce_orders.cuh: two densities here, A of
+// the pair and C of the node) as (atoms x orders) x (orders x nodes) products,
+// FP64 mma.sync.m8n8k4 tiles of 16 atoms x 16 nodes: lane l owns atom rows
+// 8 m + l/4 and orders h (4 s + l%4), e^{i n phi_atom} by rotation; B fragments
+// T[n][8 g + l/4].  Atoms whose distance makes the 16 nodes' sums negligible
+// are skipped by the plan.
+// What bounds it: with every order (about 250) and powers by pow() it was the
+// epilogue, then the order loop, and 576 of 2304 warps had a 16-fold share.
+// 1 / (p + t^2) is found once per node and primitive pair, the powers are
+// multiplied out.  64-cell chain, 32 nodes: 15.5 -> 3.0 ms per call.
+// A primitive pair whose prefactor leaves nothing above 1e-28 (elements below
+// 1e-14 are set to zero) is skipped.
+constexpr int NA_TC_WARPS = 4;
+__global__ void __launch_bounds__(NA_TC_WARPS * 32) k_nuclear_tc(DevSys S, NaArgs A)
 {
+    constexpr int MT = 2;
     extern __shared__ double smem[];
+    __shared__ double vpart[NA_TC_WARPS];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int rq = lane >> 2, cq = lane & 3;
-    const long long pair = (long long)blockIdx.x * (blockDim.x >> 5) + wib;
-    if (pair >= A.npairs) return;
+    const long long pair = blockIdx.x;
     const int fi = A.plist ? A.plist[pair].x : (int)(pair % S.nfuc);
     const int fj = A.plist ? A.plist[pair].y : (int)(pair / S.nfuc);
-    const int NW = S.ncap + 1;
-    double *Iv = smem + (size_t)wib * A.wdoubles;
-    double *Gre = Iv + NW + NA_MEXTRA;
-    double *Gim = Gre + NW;
+    const int NW = S.ncap + 1, nq = S.nq, nhalf = (nq + 15) / 16;
+    double *Iv = smem + (size_t)wib * A.wdoubles;            // NW + NA_MEXTRA
+    double2 *G = reinterpret_cast<double2 *>(Iv + ((NW + NA_MEXTRA + 1) & ~1));   // [NW]
+    double2 *nd = G + NW;                                    // [nq]: 1 / (p + t^2), w pi / (p + t^2)
     const int2 a1 = A.fsh[fi], a2 = A.fsh[fj];
     const int S1 = a1.x, S2 = a2.x;
-    int l1[3], l2[3], M[3];
+    int l1[3], l2[3];
     for (int d = 0; d < 3; ++d) {
         l1[d] = S.fn_pw[3 * fi + d];
         l2[d] = S.fn_pw[3 * fj + d];
-        M[d] = l1[d] + l2[d];
     }
+    const int M = l1[0] + l2[0];
+    const bool powers = l1[1] + l2[1] + l1[2] + l2[2] > 0;
     const double *r1 = S.sh_r + 3 * S1, *r2 = S.sh_r + 3 * S2;
     const int n1 = S.sh_np[S1], n2 = S.sh_np[S2];
     const double a = S.a[0];
-    double V = 0.0;
-    for (int pi = 0; pi < n1; ++pi)
-        for (int pj = 0; pj < n2; ++pj) {
-            const double al = S.sh_exp[S.sh_eoff[S1] + pi], be = S.sh_exp[S.sh_eoff[S2] + pj];
-            const double es = al + be, mu = al * be / es;
-            double pref = S.sh_coef[S.sh_coff[S1] + a1.y * n1 + pi] * S.sh_coef[S.sh_coff[S2] + a2.y * n2 + pj] * 2.0 /
-                          sqrt(PI_D);
-            double cen[3], pe;
-            tce_bary(al, be, r1[0], r2[0], S.L[0], a, pe, cen[0]);
-            const double Aa = 2.0 * pe / (a * a);
-            pref *= exp(-2.0 * (es - pe) / (a * a)) * S.L[0] / pow(a, (double)M[0]);
-            const int est = tce_nmax_estimate(Aa);
-            const int Np = est < S.ncap ? est : S.ncap;
-            const int N = Np + M[0];
-            for (int d = 1; d < 3; ++d) {
-                cen[d] = (al * r1[d] + be * r2[d]) / es;
-                pref *= exp(-mu * (r1[d] - r2[d]) * (r1[d] - r2[d]));
+    const float E = tce_order_exponent(M);
+    // half `lane`: 1/C range and last stored order
+    float vmin, vmax;
+    int glast = -1;
+    {
+        float lo = __int_as_float(0x7f800000), hi = -lo;
+        for (int t = 0; t < 2; ++t) {
+            const int g = 2 * lane + t;
+            if (g < nq / 8) {
+                const float2 w = S.rule_t2[g];
+                lo = fminf(lo, w.x);
+                hi = fmaxf(hi, w.y);
+                glast = max(glast, S.rule_gmax[g]);
             }
-            if (lane == 0) {   // e^{-A} I_n(A), n = 0..N
-                if (Aa < 1e-10) {
-                    for (int k = 0; k <= N; ++k) Iv[k] = 0.0;
-                    Iv[0] = 1.0;
-                } else if (N < 2) {
-                    for (int k = 0; k <= N; ++k) Iv[k] = 0.0;
-                    Iv[0] = tce_iv0_scaled(Aa);
-                } else {
-                    const double inv_A2 = 2.0 / Aa;
-                    Iv[N] = 1e-280;
-                    Iv[N - 1] = Iv[N] * (double)N * inv_A2;
-                    for (int k = N - 1; k >= 1; --k) {
-                        Iv[k - 1] = Iv[k + 1] + (double)k * inv_A2 * Iv[k];
-                        if (Iv[k - 1] > 1e250)
-                            for (int m = k - 1; m <= N; ++m) Iv[m] *= 1e-250;
+        }
+        const float h2 = 0.5f * (float)(a * a);
+        vmin = h2 / hi;
+        vmax = h2 / lo;
+    }
+    double V = 0.0;
+    for (int pp = wib; pp < n1 * n2; pp += NA_TC_WARPS) {
+        const int pi = pp / n2, pj = pp - pi * n2;
+        const double al = S.sh_exp[S.sh_eoff[S1] + pi], be = S.sh_exp[S.sh_eoff[S2] + pj];
+        const double es = al + be, mu = al * be / es;
+        double pref = S.sh_coef[S.sh_coff[S1] + a1.y * n1 + pi] * S.sh_coef[S.sh_coff[S2] + a2.y * n2 + pj] * 2.0 /
+                      sqrt(PI_D);
+        double cen[3], pe;
+        tce_bary(al, be, r1[0], r2[0], S.L[0], a, pe, cen[0]);
+        const double Aa = 2.0 * pe / (a * a);
+        pref *= exp(-2.0 * (es - pe) / (a * a)) * S.L[0];
+        for (int i = 0; i < M; ++i) pref /= a;
+        const int est = tce_nmax_estimate(Aa);
+        const int Np = est < S.ncap ? est : S.ncap;
+        const int N = Np + M;
+        for (int d = 1; d < 3; ++d) {
+            cen[d] = (al * r1[d] + be * r2[d]) / es;
+            pref *= exp(-mu * (r1[d] - r2[d]) * (r1[d] - r2[d]));
+        }
+        if (fabs(pref) * A.zsum < 1e-36) continue;   // |P - A|, |P - C| to the fourth stay below 1e8
+        __syncwarp();
+        if (lane == 0) {   // e^{-A} I_n(A), n = 0..N
+            if (Aa < 1e-10) {
+                for (int k = 0; k <= N; ++k) Iv[k] = 0.0;
+                Iv[0] = 1.0;
+            } else if (N < 2) {
+                for (int k = 0; k <= N; ++k) Iv[k] = 0.0;
+                Iv[0] = tce_iv0_scaled(Aa);
+            } else {
+                const double inv_A2 = 2.0 / Aa;
+                double hi = 1e-280, lo = hi * (double)N * inv_A2;
+                Iv[N] = hi;
+                Iv[N - 1] = lo;
+                for (int k = N - 1; k >= 1; --k) {
+                    const double nx = hi + (double)k * inv_A2 * lo;
+                    hi = lo;
+                    lo = nx;
+                    Iv[k - 1] = nx;
+                    if (nx > 1e250) {
+                        for (int m = k - 1; m <= N; ++m) Iv[m] *= 1e-250;
+                        hi *= 1e-250;
+                        lo *= 1e-250;
                     }
-                    const double sc = tce_iv0_scaled(Aa) / Iv[0];
-                    for (int k = 0; k <= N; ++k) Iv[k] *= sc;
                 }
             }
-            __syncwarp();
+        }
+        __syncwarp();
+        const double sc = Aa < 1e-10 || N < 2 ? 1.0 : tce_iv0_scaled(Aa) / Iv[0];
+        __syncwarp();
+        for (int k = lane; k <= N; k += 32) Iv[k] *= sc;
+        for (int k = lane; k < nq; k += 32) {
+            const double t = S.tnode[k], inv = 1.0 / fma(t, t, es);
+            nd[k] = make_double2(inv, S.tweight[k] * PI_D * inv);
+        }
+        __syncwarp();
+        if (M == 0) {
+            for (int n = lane; n <= Np; n += 32) G[n] = make_double2(Iv[n], 0.0);
+        } else if (Aa >= 4.0) {
+            PowerSeries ps;   // the vectors sum_k d_k I_{n+k} are the ones of sign -1
+            tce_power_series(l1[0], l2[0], a * (cen[0] - r1[0]), a * (cen[0] - r2[0]), ps);
+            const double inv_A = 1.0 / Aa;
+            for (int n = lane; n <= Np; n += 32) G[n] = tce_power_coef(ps, Iv, -n, inv_A);
+        } else {
             double dre[4 * TCE_LMAX + 1], dim[4 * TCE_LMAX + 1];
-            if (M[0] > 0) tce_fourier_sin(l1[0], l2[0], a * (cen[0] - r1[0]), a * (cen[0] - r2[0]), dre, dim);
+            tce_fourier_sin(l1[0], l2[0], a * (cen[0] - r1[0]), a * (cen[0] - r2[0]), dre, dim);
             for (int n = lane; n <= Np; n += 32) {
                 double gr = 0.0, gi = 0.0;
-                if (M[0] == 0) {
-                    gr = Iv[n];
-                } else {
-                    for (int kk = -M[0]; kk <= M[0]; ++kk) {
-                        const int idx = n + kk;
-                        const double bv = Iv[idx < 0 ? -idx : idx];
-                        gr += dre[kk + M[0]] * bv;
-                        gi += dim[kk + M[0]] * bv;
-                    }
+                for (int kk = -M; kk <= M; ++kk) {
+                    const int idx = n + kk;
+                    const double bv = Iv[idx < 0 ? -idx : idx];
+                    gr += dre[kk + M] * bv;
+                    gi += dim[kk + M] * bv;
                 }
-                Gre[n] = gr;
-                Gim[n] = gi;
+                G[n] = make_double2(gr, gi);
             }
-            __syncwarp();
-            double vsum = 0.0;
-            for (int at0 = 0; at0 < A.natoms; at0 += 16) {
-                double phr[2];
-                bool valid[2];
-#pragma unroll
-                for (int m = 0; m < 2; ++m) {
-                    const int at = at0 + 8 * m + rq;
-                    valid[m] = at < A.natoms;
-                    phr[m] = valid[m] ? a * (cen[0] - A.geo[at]) : 0.0;
-                }
-#pragma unroll 1
-                for (int g0 = 0; g0 < NQ / 8; g0 += 4) {
-                    double acc[16];
-#pragma unroll
-                    for (int x = 0; x < 16; ++x) acc[x] = 0.0;
-                    double cc[2], cp[2], sc[2], sp[2], c4[2];
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        sincos((double)cq * phr[m], &sc[m], &cc[m]);
-                        sincos((double)(cq - 4) * phr[m], &sp[m], &cp[m]);
-                        c4[m] = 2.0 * cos(4.0 * phr[m]);
-                    }
-                    for (int s4 = 0; s4 <= Np; s4 += 4) {
-                        const int n = s4 + cq, n1 = n + 4;
-                        const bool inr = n <= Np;
-                        const double gr = inr ? Gre[n] : 0.0, gi = inr ? Gim[n] : 0.0;
-                        double F[2];
-#pragma unroll
-                        for (int m = 0; m < 2; ++m) F[m] = valid[m] ? gr * cc[m] - gi * sc[m] : 0.0;
-                        double Tb[4];
-#pragma unroll
-                        for (int t = 0; t < 4; ++t)
-                            Tb[t] = (n <= S.ncap) ? __ldg(S.Tt + (size_t)n * S.nq + 8 * (g0 + t) + rq) : 0.0;
-                        if (((s4 + 4) & 31) == 0) {
-#pragma unroll
-                            for (int m = 0; m < 2; ++m) {
-                                sincos((double)n * phr[m], &sp[m], &cp[m]);
-                                sincos((double)n1 * phr[m], &sc[m], &cc[m]);
-                            }
-                        } else {
-#pragma unroll
-                            for (int m = 0; m < 2; ++m) {
-                                const double tc_ = c4[m] * cc[m] - cp[m], ts_ = c4[m] * sc[m] - sp[m];
-                                cp[m] = cc[m];
-                                cc[m] = tc_;
-                                sp[m] = sc[m];
-                                sc[m] = ts_;
-                            }
-                        }
-#pragma unroll
-                        for (int t = 0; t < 4; ++t)
-#pragma unroll
-                            for (int m = 0; m < 2; ++m) na_dmma(acc[(m * 4 + t) * 2], acc[(m * 4 + t) * 2 + 1], F[m], Tb[t]);
-                    }
-                    // epilogue: acc[(m 4 + t) 2 + i] = X(atom 8 m + rq, node 8 (g0 + t) + 2 cq + i)
-#pragma unroll
-                    for (int m = 0; m < 2; ++m) {
-                        if (!valid[m]) continue;
-                        const int at = at0 + 8 * m + rq;
-                        double Cc[3];
-                        for (int d = 1; d < 3; ++d) Cc[d] = A.geo[at + (size_t)A.natoms * d];
-                        double part = 0.0;
-#pragma unroll
-                        for (int t = 0; t < 4; ++t)
-#pragma unroll
-                            for (int i = 0; i < 2; ++i) {
-                                const int k = 8 * (g0 + t) + 2 * cq + i;
-                                const double t2 = S.tnode[k] * S.tnode[k];
-                                double prod = acc[(m * 4 + t) * 2 + i];
-                                for (int d = 1; d < 3; ++d) {
-                                    const double ppt = es + t2, eta = t2 / ppt, pc = cen[d] - Cc[d];
-                                    const double ed = exp(-es * eta * pc * pc);
-                                    prod *= ed * na_overlap_1d(l1[d], l2[d], ppt, (cen[d] - r1[d]) - eta * pc,
-                                                                (cen[d] - r2[d]) - eta * pc);
-                                }
-                                part = fma(S.tweight[k], prod, part);
-                            }
-                        vsum = fma((double)A.Z[at], part, vsum);
-                    }
-                }
-            }
-            vsum = tce_warp_sum(vsum);
-            V -= pref * vsum;
-            __syncwarp();
         }
-    if (lane == 0) A.V[A.plist ? pair : fi + (long long)S.nfuc * fj] = fabs(V) < 1e-14 ? 0.0 : V;
+        __syncwarp();
+        const float u = 1.0f / (float)Aa;
+        double vsum = 0.0;
+        for (int at0 = 0; at0 < A.natoms; at0 += 8 * MT) {
+            double phr[MT], cy[MT], cz[MT], zc[MT];
+            float pmin = 0.0f, pmax = 0.0f;
+#pragma unroll
+            for (int m = 0; m < MT; ++m) {
+                const int at = at0 + 8 * m + rq, ar = at < A.natoms ? at : A.natoms - 1;
+                zc[m] = at < A.natoms ? (double)A.Z[ar] : 0.0;
+                phr[m] = a * (cen[0] - A.geo[ar]);
+                cy[m] = cen[1] - A.geo[ar + (size_t)A.natoms];
+                cz[m] = cen[2] - A.geo[ar + (size_t)A.natoms * 2];
+                const float ap = tce_fold_phase(phr[m]);
+                pmin = m == 0 ? ap : fminf(pmin, ap);
+                pmax = m == 0 ? ap : fmaxf(pmax, ap);
+            }
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) {
+                pmin = fminf(pmin, __shfl_xor_sync(0xffffffffu, pmin, o));
+                pmax = fmaxf(pmax, __shfl_xor_sync(0xffffffffu, pmax, o));
+            }
+            OrderPlan plan = tce_order_plan(E, M, u, u, pmin, pmax, vmin, vmax, min(glast, Np));
+            if (glast < 0) plan.h = 0;
+            double cs = 1.0, sn = 0.0;
+#pragma unroll 1
+            for (int hf = 0; hf < nhalf; ++hf) {
+                if ((hf & 1) == 0)   // lane column cq: row 8 (cq / 2) + rq, half hf + cq % 2
+                    sincos((double)__shfl_sync(0xffffffffu, plan.h, hf + (cq & 1)) * ((cq >> 1) ? phr[1] : phr[0]), &sn, &cs);
+                const int h = __shfl_sync(0xffffffffu, plan.h, hf), last = __shfl_sync(0xffffffffu, plan.last, hf);
+                if (h == 0) continue;
+                const int ntile = nq / 8 - 2 * hf > 1 ? 2 : 1;
+                double acc[2][MT][2];
+#pragma unroll
+                for (int t = 0; t < 2; ++t)
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) acc[t][m][0] = acc[t][m][1] = 0.0;
+                double cc[MT], ss[MT], c4[MT], s4[MT];
+#pragma unroll
+                for (int m = 0; m < MT; ++m) {
+                    const int src = (lane & ~3) | (2 * m + (hf & 1));
+                    const double c = __shfl_sync(0xffffffffu, cs, src), s = __shfl_sync(0xffffffffu, sn, src);
+                    const double c2 = fma(-2.0 * s, s, 1.0), s2 = 2.0 * s * c;
+                    cc[m] = cq == 0 ? 1.0 : cq == 1 ? c : cq == 2 ? c2 : fma(c2, c, -s2 * s);
+                    ss[m] = cq == 0 ? 0.0 : cq == 1 ? s : cq == 2 ? s2 : fma(s2, c, c2 * s);
+                    c4[m] = fma(-2.0 * s2, s2, 1.0);
+                    s4[m] = 2.0 * s2 * c2;
+                }
+                const double *T = S.Tt + 16 * hf + rq;
+                const int t1 = ntile > 1 ? 8 : 0;
+#pragma unroll 2
+                for (int n0 = 0; n0 <= last; n0 += 4 * h) {
+                    const int n = n0 + h * cq, nn = min(n, last);
+                    double2 g = G[nn];
+                    if (n > last) g = make_double2(0.0, 0.0);
+                    const double T0 = __ldg(T + (size_t)nn * nq), T1 = __ldg(T + (size_t)nn * nq + t1);
+#pragma unroll
+                    for (int m = 0; m < MT; ++m) {
+                        const double F = g.x * cc[m] - g.y * ss[m];
+                        const double t = cc[m];
+                        cc[m] = fma(t, c4[m], -ss[m] * s4[m]);
+                        ss[m] = fma(ss[m], c4[m], t * s4[m]);
+                        na_dmma(acc[0][m][0], acc[0][m][1], F, T0);
+                        na_dmma(acc[1][m][0], acc[1][m][1], F, T1);
+                    }
+                }
+                // epilogue: acc[t][m][i] = X(atom 8 m + rq, node 16 hf + 8 t + 2 cq + i) / h
+#pragma unroll
+                for (int t = 0; t < 2; ++t) {
+                    if (t >= ntile) continue;
+#pragma unroll
+                    for (int i = 0; i < 2; ++i) {
+                        const int k = 16 * hf + 8 * t + 2 * cq + i;
+                        const double2 w = nd[k];
+                        const double tk = __ldg(S.tnode + k), eta = tk * tk * w.x;   // t^2 / (p + t^2)
+#pragma unroll
+                        for (int m = 0; m < MT; ++m) {
+                            const double R2 = cy[m] * cy[m] + cz[m] * cz[m];
+                            double v = acc[t][m][i] * w.y;
+                            if (R2 != 0.0) v *= exp(-es * eta * R2);
+                            if (powers)
+                                v *= na_overlap_1d(l1[1], l2[1], w.x, (cen[1] - r1[1]) - eta * cy[m], (cen[1] - r2[1]) - eta * cy[m]) *
+                                     na_overlap_1d(l1[2], l2[2], w.x, (cen[2] - r1[2]) - eta * cz[m], (cen[2] - r2[2]) - eta * cz[m]);
+                            vsum = fma(zc[m] * (double)h, v, vsum);
+                        }
+                    }
+                }
+            }
+        }
+        vsum = tce_warp_sum(vsum);
+        V -= pref * vsum;
+    }
+    if (lane == 0) vpart[wib] = V;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        V = 0.0;
+        for (int w = 0; w < NA_TC_WARPS; ++w) V += vpart[w];
+        A.V[A.plist ? pair : fi + (long long)S.nfuc * fj] = fabs(V) < 1e-14 ? 0.0 : V;
+    }
 }
 
 }  // namespace
@@ -430,23 +491,26 @@ static int nuclear_elements(Handle *h, int natoms, const double *geo, const int3
     A.geo = d_geo;
     A.Z = d_Z;
     A.V = d_V;
+    A.zsum = 1.0;
+    for (int x : z) A.zsum += std::abs((double)x);
     const int NW = h->ncap + 1;
-    A.wdoubles = (NW + NA_MEXTRA + 3 * h->ndp * NW + 31) / 32 * 32;
-    const size_t wbytes = (size_t)A.wdoubles * sizeof(double);
-    int warps = NA_WARPS_MAX;
-    while (warps > 1 && wbytes * warps > 200 * 1024) --warps;
-    if (wbytes > 200 * 1024) {
-        cleanup();
-        return fail(h, TCE_ERR_UNSUPPORTED, "truncation order too large for the nuclear-attraction kernel");
-    }
-    const size_t smem = wbytes * (size_t)warps;
-    // one periodic direction with a 32- or 64-node rule: the tensor-core form
-    const unsigned grid = (unsigned)((npairs + warps - 1) / warps);
-    if (h->use_tc && h->ndp == 1 && (h->nq == 32 || h->nq == 64)) {
-        auto kern = h->nq == 32 ? k_nuclear_tc<32> : k_nuclear_tc<64>;
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kern<<<grid, 32 * warps, smem, h->st>>>(h->S, A);
+    // one periodic direction: the tensor-core form, where its buffers fit
+    A.wdoubles = ((NW + NA_MEXTRA + 1) & ~1) + 2 * NW + 2 * h->nq;
+    const size_t tbytes = (size_t)A.wdoubles * sizeof(double) * NA_TC_WARPS;
+    if (h->use_tc && h->ndp == 1 && tbytes <= 200 * 1024 && npairs < 0x7fffffffLL) {
+        cudaFuncSetAttribute(k_nuclear_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tbytes);
+        k_nuclear_tc<<<(unsigned)npairs, 32 * NA_TC_WARPS, tbytes, h->st>>>(h->S, A);
     } else {
+        A.wdoubles = (NW + NA_MEXTRA + 3 * h->ndp * NW + 31) / 32 * 32;
+        const size_t wbytes = (size_t)A.wdoubles * sizeof(double);
+        int warps = NA_WARPS_MAX;
+        while (warps > 1 && wbytes * warps > 200 * 1024) --warps;
+        if (wbytes > 200 * 1024) {
+            cleanup();
+            return fail(h, TCE_ERR_UNSUPPORTED, "truncation order too large for the nuclear-attraction kernel");
+        }
+        const size_t smem = wbytes * (size_t)warps;
+        const unsigned grid = (unsigned)((npairs + warps - 1) / warps);
         cudaFuncSetAttribute(k_nuclear, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_nuclear<<<grid, 32 * warps, smem, h->st>>>(h->S, A);
     }
