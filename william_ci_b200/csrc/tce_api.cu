@@ -669,26 +669,27 @@ int build(Handle *h, const tce_system *sys)
     return TCE_OK;
 }
 
-// the launches of one J/K pass (zeroing of J and K included)
-static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStream_t st)
+// Every work list of the handle with the system's rule: J and K added up
+// (TCE_MODE_JK) or the integrals stored (TCE_MODE_STORE: dJ the array).
+static int fixed_lists(Handle *h, int mode, const double *dP, double *dJ, double *dK, cudaStream_t st)
 {
-    CK(h, cudaMemsetAsync(dJ, 0, sizeof(double) * h->nfuc * h->nbas, st));
-    CK(h, cudaMemsetAsync(dK, 0, sizeof(double) * h->nfuc * h->nbas, st));
-    if (h->method != TCE_METHOD_FIXED) return lg_jk_passes(h, dP, dJ, dK, st);
     for (const auto &w : h->lists) {
         if (w.n == 0) continue;
-        // the CUDA-core kernels of the all-s and one-p classes are built for 32 nodes (all-s: and 40)
-        const bool core = w.kind == 1 ? (h->nq == 32 || h->nq == 40) : tce_r1_supported(h->ndp, h->nq, w.cls);
+        // the CUDA-core kernels of the all-s and one-p classes are built for 32 nodes (all-s: and 40) and J/K
+        const bool core = mode == TCE_MODE_JK && (w.kind == 1 ? (h->nq == 32 || h->nq == 40) : tce_r1_supported(h->ndp, h->nq, w.cls));
         if (w.kind == 0 || (!h->use_tc && !core)) {   // every other class: generic kernel
             QuartetHostArgs a;
             a.items = w.d;
             a.nitems = (int)w.n;
-            a.mode = TCE_MODE_JK;
+            a.mode = mode;
             a.prim_screen = h->prim_screen;
             a.next = h->d_next;
             a.P = dP;
             a.J = dJ;
             a.K = dK;
+            a.eri = dJ;
+            a.eri_size = h->eri_size;
+            a.physicist = h->physicist;
             a.max_ncomb = w.max_ncomb;
             a.max_ncq = w.max_ncq;
             a.fixed_gmax = h->d_gmax;
@@ -704,6 +705,9 @@ static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStre
             b.P = dP;
             b.J = dJ;
             b.K = dK;
+            b.eri = mode == TCE_MODE_STORE ? dJ : nullptr;
+            b.eri_size = h->eri_size;
+            b.physicist = h->physicist;
             b.num_sms = h->num_sms;
             if (h->use_tc) {
                 if (w.kind == 1) CKS(h, tce_launch_quartets_s_tc(h->S, b, h->nq, 1, st));
@@ -715,6 +719,15 @@ static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStre
         }
     }
     return TCE_OK;
+}
+
+// the launches of one J/K pass (zeroing of J and K included)
+static int jk_body(Handle *h, const double *dP, double *dJ, double *dK, cudaStream_t st)
+{
+    CK(h, cudaMemsetAsync(dJ, 0, sizeof(double) * h->nfuc * h->nbas, st));
+    CK(h, cudaMemsetAsync(dK, 0, sizeof(double) * h->nfuc * h->nbas, st));
+    if (h->method != TCE_METHOD_FIXED) return lg_jk_passes(h, dP, dJ, dK, st);
+    return fixed_lists(h, TCE_MODE_JK, dP, dJ, dK, st);
 }
 
 // streams, events and pinned host memory of a handle
@@ -1274,7 +1287,11 @@ int tce_eri_stored(void *handle, int64_t eri_size, double *eri)
     }
     h->eri_size = esz;
     CK(h, cudaMemsetAsync(h->d_eri, 0, sizeof(double) * elems, h->st));
-    if (h->nitems > 0) {
+    if (h->nitems > 0 && h->nitems_shard == h->nitems) {
+        // the classes' own kernels over their lists, as a J/K pass
+        int s = fixed_lists(h, TCE_MODE_STORE, nullptr, h->d_eri, nullptr, h->st);
+        if (s) return s;
+    } else if (h->nitems > 0) {   // a shard's lists hold its quartets only: every quartet through the generic kernel
         QuartetHostArgs a;
         a.items = h->d_items;
         a.nitems = (int)h->nitems;

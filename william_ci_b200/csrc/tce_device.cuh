@@ -305,6 +305,26 @@ __device__ __forceinline__ int tce_shift_fn(const DevSys &S, int f, int rx, int 
     return (cx + S.ncl[0] * (cy + S.ncl[1] * cz)) * S.nfuc + c.w;
 }
 
+// One function quartet of the stored integrals: val at the quartet's eight
+// permutations moved to the unit cell (ERI_toroidal.f90:416-454).
+__device__ __forceinline__ void tce_store_eri(const DevSys &S, double *eri, int eri_size, int physicist, const int f[4],
+                                              double val)
+{
+    const int perm[8][4] = {{0,1,2,3},{1,0,2,3},{0,1,3,2},{1,0,3,2},{2,3,0,1},{3,2,0,1},{2,3,1,0},{3,2,1,0}};
+    for (int ip = 0; ip < 8; ++ip) {
+        int g[4];
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii) g[ii] = f[perm[ip][ii]];
+        const int4 rc = __ldg(S.fn_cell + g[0]);
+#pragma unroll
+        for (int ii = 0; ii < 4; ++ii) g[ii] = tce_shift_fn(S, g[ii], rc.x, rc.y, rc.z);
+        const long long n = S.nbas;
+        const long long e = physicist ? g[0] + (long long)eri_size * (g[2] + n * (g[1] + n * g[3]))
+                                      : g[0] + (long long)eri_size * (g[1] + n * (g[2] + n * g[3]));
+        eri[e] = val;
+    }
+}
+
 // J/K contributions of one function quartet f = (i,j|k,l) of the block of
 // shell quartet (fI..|..), every stored element (p1 in the unit cell) once:
 // J(p1,p2) += E P(p3,p4), K(p1,p4) += -1/2 E P(p2,p3) (eri_direct.f90:331-357).

@@ -70,6 +70,8 @@ struct SArgsHost {
     unsigned int *next = nullptr;
     const double *P = nullptr;
     double *J = nullptr, *K = nullptr;
+    double *eri = nullptr;           // stored-integral scatter instead of J/K (system rule, tensor-core kernels)
+    int eri_size = 0, physicist = 0;
     int num_sms = 148;
     // learned grid (the _lg launchers): per-item rules, judge, fallback queue
     const int *item_rule = nullptr;

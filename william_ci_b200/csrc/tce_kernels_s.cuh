@@ -51,6 +51,8 @@ struct SArgs {
     unsigned int *next;
     const double *P;
     double *J, *K;
+    double *eri;              // stored-integral scatter instead of J/K when set (tensor-core kernels)
+    int eri_size, physicist;
     int tsoff[3][TCE_MAXG];   // doubles from the start of the T buffer
     int ts_doubles;           // size of the T buffer
     int t_smem;               // 1: T copied to shared memory, 0: read from global

@@ -306,8 +306,12 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
         if (lane == 0) {
             const int fI = S.sh_first[q.x], fJ = S.sh_first[q.y], fK = S.sh_first[q.z], fL = S.sh_first[q.w];
             const int f[4] = {fI, fJ, fK, fL};
-            if (S.Q[fI + (long long)S.nbas * fJ] * S.Q[fK + (long long)S.nbas * fL] >= S.thr)
-                tce_scatter_jk(S, A.P, A.J, A.K, f, blk, fI, 1, fJ, 1, fK, 1, fL, 1);
+            if (S.Q[fI + (long long)S.nbas * fJ] * S.Q[fK + (long long)S.nbas * fL] >= S.thr) {
+                if (!LG && A.eri)
+                    tce_store_eri(S, A.eri, A.eri_size, A.physicist, f, blk);
+                else
+                    tce_scatter_jk(S, A.P, A.J, A.K, f, blk, fI, 1, fJ, 1, fK, 1, fL, 1);
+            }
         }
         __syncwarp();
     }

@@ -152,6 +152,9 @@ static inline void tc_args(SArgs &A, const SArgsHost &h)
     A.P = h.P;
     A.J = h.J;
     A.K = h.K;
+    A.eri = h.eri;
+    A.eri_size = h.eri_size;
+    A.physicist = h.physicist;
     A.item_rule = h.item_rule;
     A.rules = h.rules;
     A.rule_T = h.rule_T;
@@ -594,7 +597,10 @@ __global__ void __launch_bounds__(256, LA + LB + LC + LD == 1 ? 2 : 1) k_quartet
             if (lane == (c & 31)) {
                 const int ca = c % NA, cb = (c / NA) % NB, cc_ = (c / (NA * NB)) % NC, cd = c / (NA * NB * NC);
                 const int f[4] = {fI + ca, fJ + cb, fK + cc_, fL + cd};
-                if (S.Q[f[0] + (long long)S.nbas * f[1]] * S.Q[f[2] + (long long)S.nbas * f[3]] >= S.thr)
+                if (S.Q[f[0] + (long long)S.nbas * f[1]] * S.Q[f[2] + (long long)S.nbas * f[3]] < S.thr) continue;
+                if (!LG && A.eri)
+                    tce_store_eri(S, A.eri, A.eri_size, A.physicist, f, v);
+                else
                     tce_scatter_jk(S, A.P, A.J, A.K, f, v, fI, NA, fJ, NB, fK, NC, fL, ND);
             }
         }

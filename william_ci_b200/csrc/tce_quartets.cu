@@ -828,21 +828,7 @@ __device__ void consume(const DevSys &S, const QuartetArgs &A, const QCtx &Q, co
             if (S.Q[f[0] + (long long)S.nbas * f[1]] * S.Q[f[2] + (long long)S.nbas * f[3]] < S.thr) continue;
             const double val = blk[cq];
             if (A.mode == TCE_MODE_STORE) {
-                const int perm[8][4] = {{0,1,2,3},{1,0,2,3},{0,1,3,2},{1,0,3,2},{2,3,0,1},{3,2,0,1},{2,3,1,0},{3,2,1,0}};
-                for (int ip = 0; ip < 8; ++ip) {
-                    int g[4];
-#pragma unroll
-                    for (int ii = 0; ii < 4; ++ii) g[ii] = f[perm[ip][ii]];
-                    const int4 rc = __ldg(S.fn_cell + g[0]);
-#pragma unroll
-                    for (int ii = 0; ii < 4; ++ii) g[ii] = tce_shift_fn(S, g[ii], rc.x, rc.y, rc.z);
-                    long long e;
-                    if (A.physicist)
-                        e = g[0] + (long long)A.eri_size * (g[2] + (long long)S.nbas * (g[1] + (long long)S.nbas * g[3]));
-                    else
-                        e = g[0] + (long long)A.eri_size * (g[1] + (long long)S.nbas * (g[2] + (long long)S.nbas * g[3]));
-                    A.eri[e] = val;
-                }
+                tce_store_eri(S, A.eri, A.eri_size, A.physicist, f, val);
                 continue;
             }
             tce_scatter_jk(S, A.P, A.J, A.K, f, val, fI, nA, fJ, nB, fK, nC, fL, nD);
