@@ -28,7 +28,8 @@ def _case(ncl, no, nv, nau, seed, degenerate=False):
     return L, eo, oo, ev, ovv
 
 
-@pytest.mark.parametrize("ncl,no,nv,nau", [((4, 1, 1), 2, 4, 16), ((2, 2, 2), 1, 6, 16), ((3, 1, 1), 2, 3, 12)])
+@pytest.mark.parametrize("ncl,no,nv,nau", [((4, 1, 1), 2, 4, 16), ((2, 2, 2), 1, 6, 16), ((3, 1, 1), 2, 3, 12),
+                                           ((5, 1, 1), 1, 1, 7), ((3, 1, 1), 4, 8, 33)])   # smallest; tiles past shared memory
 def test_dfmp2_energy_vs_oracle(ncl, no, nv, nau):
     from william_ci_b200.engine import dfmp2_energy
     L, eo, oo, ev, ovv = _case(ncl, no, nv, nau, seed=no * 7 + nv)

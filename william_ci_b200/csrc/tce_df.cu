@@ -20,9 +20,8 @@
 //     e^{-i kap.s} e^{i k2.R}] C_k2(b, q), kap = k2 - k1 (df_L_kap), then the
 //     (ov|ov) contraction and the energy of tce_dfmp2_energy.
 //
-// Each transform is a sum over cells run as one thread per output element
-// against a table of the N x N phases; with N = 128 cells, nf = 6, nau = 16 it
-// is about 1e9 complex multiply-adds per step, a few milliseconds.
+// Each transform is a sum over cells against a table of the N x N phases; with
+// N = 128 cells, nf = 6, nau = 16 it is about 1e9 complex multiply-adds per step.
 #include <algorithm>
 #include <cmath>
 #include <complex>
@@ -32,6 +31,11 @@
 #include "tce_handle.h"
 
 using namespace tcehost;
+
+// tce_mp2.cu
+int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord, int32_t no, int32_t nv, int32_t nau,
+                      const double *L, bool l_dev, const double *eps_o, const int32_t *occ_o, const double *eps_v,
+                      const int32_t *occ_v, int32_t mode, double *e2d, double *e2x, int64_t *nzero, double *gzero, double *ms);
 
 namespace {
 
@@ -45,6 +49,8 @@ struct DfHandle {
     int *d_crd = nullptr;     // [3 k + d] cell coordinates
     double *d_Vm = nullptr, *d_T3 = nullptr, *d_B = nullptr;
     double2 *d_W = nullptr;   // W(k)(x, q) = [sum_R T3(R) e^{ikR}] f(k), x = mu + nf nu
+    double2 *d_ws1 = nullptr, *d_wsF = nullptr, *d_wsC = nullptr;   // tce_dfmp2's workspaces
+    size_t n_ws1 = 0;
     std::vector<void *> mem;
 };
 
@@ -198,47 +204,74 @@ __global__ void k_df_bh(const double2 *__restrict__ W, const double2 *__restrict
     Bh[t] = make_double2(re, im);
 }
 
-// G1(kap)(x, q) = sum_s B(x, s nau + q) conj e^{i kap s}
+// The two cell sums of df_L_kap: DF_KT k values per thread, so that an element of
+// B or G1 is read once for DF_KT phases (shared memory, read as broadcasts) instead
+// of once per k: the one-output-per-thread form read each of them N times from the
+// L2.  96 cells: G1 413 and F 976 us before.
+constexpr int DF_KT = 8;
+// ph[k0 + j][R] of the block's DF_KT values of k into shared memory (zero past N)
+__device__ __forceinline__ void df_phases(const double2 *__restrict__ ph, int k0, int N, double2 *sp)
+{
+    for (int x = threadIdx.x; x < DF_KT * N; x += blockDim.x) {
+        const int j = x % DF_KT, R = x / DF_KT;
+        sp[x] = k0 + j < N ? ph[(long long)(k0 + j) * N + R] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+}
+
+// G1(kap)(x, q) = sum_s B(x, s nau + q) conj e^{i kap s}; blockIdx.y = kap tile
 __global__ void k_df_g1(const double *__restrict__ B, const double2 *__restrict__ ph, long long X, int N, int nau,
                         double2 *G1)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= X * nau * N) return;
-    const long long x = t % X;
-    const long long c = t / X;
-    const int q = (int)(c % nau), kap = (int)(c / nau);
-    double re = 0.0, im = 0.0;
+    extern __shared__ double2 sp[];
+    const int k0 = blockIdx.y * DF_KT;
+    df_phases(ph, k0, N, sp);
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // x + X q
+    if (t >= X * nau) return;
+    double re[DF_KT], im[DF_KT];
+#pragma unroll
+    for (int j = 0; j < DF_KT; ++j) re[j] = im[j] = 0.0;
     for (int s = 0; s < N; ++s) {
-        const double b = B[x + X * ((long long)s * nau + q)];
-        const double2 e = ph[(long long)kap * N + s];
-        re = fma(b, e.x, re);
-        im = fma(-b, e.y, im);
+        const double b = B[t + X * nau * s];
+#pragma unroll
+        for (int j = 0; j < DF_KT; ++j) {
+            const double2 e = sp[s * DF_KT + j];
+            re[j] = fma(b, e.x, re[j]);
+            im[j] = fma(-b, e.y, im[j]);
+        }
     }
-    G1[t] = make_double2(re, im);
+#pragma unroll
+    for (int j = 0; j < DF_KT; ++j)
+        if (k0 + j < N) G1[t + X * nau * (k0 + j)] = make_double2(re[j], im[j]);
 }
 
-// F(a, b, q, kap, k2) = sum_R G1(kap)(a + nf (R nf + b), q) e^{i k2 R}
+// F(a, b, q, kap, k2) = sum_R G1(kap)(a + nf (R nf + b), q) e^{i k2 R}; blockIdx.y = k2 tile
 __global__ void k_df_f(const double2 *__restrict__ G1, const double2 *__restrict__ ph, long long X, int N, int nf,
                        int nau, double2 *F)
 {
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long tot = (long long)nf * nf * nau * N * N;
+    extern __shared__ double2 sp[];
+    const int k0 = blockIdx.y * DF_KT;
+    df_phases(ph, k0, N, sp);
+    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // a + nf (b + nf (q + nau kap))
+    const long long tot = (long long)nf * nf * nau * N;
     if (t >= tot) return;
-    long long r = t;
-    const int a = (int)(r % nf); r /= nf;
-    const int b = (int)(r % nf); r /= nf;
-    const int q = (int)(r % nau); r /= nau;
-    const int kap = (int)(r % N);
-    const int k2 = (int)(r / N);
-    double re = 0.0, im = 0.0;
-    const double2 *g = G1 + ((long long)kap * nau + q) * X;
+    const int nf2 = nf * nf, ab = (int)(t % nf2);
+    const double2 *g = G1 + (t / nf2) * X + ab;          // (kap nau + q) X + a + nf b, + nf^2 R
+    double re[DF_KT], im[DF_KT];
+#pragma unroll
+    for (int j = 0; j < DF_KT; ++j) re[j] = im[j] = 0.0;
     for (int R = 0; R < N; ++R) {
-        const double2 v = g[a + (long long)nf * ((long long)R * nf + b)];
-        const double2 e = ph[(long long)k2 * N + R];
-        re += v.x * e.x - v.y * e.y;
-        im += v.x * e.y + v.y * e.x;
+        const double2 v = g[(long long)nf2 * R];
+#pragma unroll
+        for (int j = 0; j < DF_KT; ++j) {
+            const double2 e = sp[R * DF_KT + j];
+            re[j] = fma(v.x, e.x, fma(-v.y, e.y, re[j]));
+            im[j] = fma(v.x, e.y, fma(v.y, e.x, im[j]));
+        }
     }
-    F[t] = make_double2(re, im);
+#pragma unroll
+    for (int j = 0; j < DF_KT; ++j)
+        if (k0 + j < N) F[t + tot * (k0 + j)] = make_double2(re[j], im[j]);
 }
 
 // L(p, v, q, k1, k2) = sum_ab conj C_k1(a, p0 + p) F(a, b, q, kap, k2) C_k2(b, v0 + v),
@@ -735,29 +768,35 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     const int no = ohi, nv = nf - vlo;
     if (no < 1 || nv < 1) return df_fail(d, TCE_ERR_ARG, "no occupied or no virtual bands");
     int s;
-    double2 *d_G1 = nullptr, *d_F = nullptr, *d_C = nullptr, *d_L = nullptr;
-    if ((s = df_alloc(d, &d_G1, (size_t)X * nau * N))) return s;
-    k_df_g1<<<nblk(X * nau * N, 256), 256, 0, d->st>>>(d->d_B, d->d_ph, X, N, nau, d_G1);
-    DCK(d, cudaGetLastError());
-    const long long nF = (long long)nf * nf * nau * N * N;
-    if ((s = df_alloc(d, &d_F, (size_t)nF))) return s;
-    k_df_f<<<nblk(nF, 256), 256, 0, d->st>>>(d_G1, d->d_ph, X, N, nf, nau, d_F);
-    DCK(d, cudaGetLastError());
-    DCK(d, cudaStreamSynchronize(d->st));
-    df_free(d, d_G1);
-    if ((s = df_alloc(d, &d_C, (size_t)nbas * nbas))) return s;
+    // workspaces kept with the handle: G1 and the L vectors share one buffer (L after G1 is read)
+    const long long nG1 = X * nau * N, nF = (long long)nf * nf * nau * N * N, nL = (long long)no * nv * nau * N * N;
+    const size_t need1 = (size_t)std::max(nG1, nL);
+    if (d->n_ws1 < need1) {
+        df_free(d, d->d_ws1);
+        d->n_ws1 = 0;
+        d->d_ws1 = nullptr;
+        if ((s = df_alloc(d, &d->d_ws1, need1))) return s;
+        d->n_ws1 = need1;
+    }
+    if (!d->d_wsF && (s = df_alloc(d, &d->d_wsF, (size_t)nF))) return s;
+    if (!d->d_wsC && (s = df_alloc(d, &d->d_wsC, (size_t)nbas * nbas))) return s;
+    double2 *d_G1 = d->d_ws1, *d_F = d->d_wsF, *d_C = d->d_wsC, *d_L = d->d_ws1;
+    const dim3 tiles(1, (unsigned)((N + DF_KT - 1) / DF_KT));
+    const size_t psm = sizeof(double2) * DF_KT * (size_t)N;
+    if (psm > 200 * 1024) return df_fail(d, TCE_ERR_UNSUPPORTED, "too many cells for the phase tiles");
+    if (psm > 48 * 1024) {
+        DCK(d, cudaFuncSetAttribute(k_df_g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+        DCK(d, cudaFuncSetAttribute(k_df_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+    }
     DCK(d, cudaMemcpyAsync(d_C, coeff, sizeof(double2) * nbas * nbas, cudaMemcpyHostToDevice, d->st));
-    const long long nL = (long long)no * nv * nau * N * N;
-    if ((s = df_alloc(d, &d_L, (size_t)nL))) return s;
+    k_df_g1<<<dim3(nblk(X * nau, 128), tiles.y), 128, psm, d->st>>>(d->d_B, d->d_ph, X, N, nau, d_G1);
+    DCK(d, cudaGetLastError());
+    k_df_f<<<dim3(nblk((long long)nf * nf * nau * N, 128), tiles.y), 128, psm, d->st>>>(d_G1, d->d_ph, X, N, nf, nau, d_F);
+    DCK(d, cudaGetLastError());
     k_df_l<<<nblk(nL, 256), 256, 0, d->st>>>(d_F, d_C, d->d_crd, d->ncl[0], d->ncl[1], d->ncl[2], N, nf, nau, 0, no,
                                              vlo, nv, d_L);
     DCK(d, cudaGetLastError());
-    std::vector<double> L(2 * (size_t)nL);
-    DCK(d, cudaMemcpyAsync(L.data(), d_L, sizeof(double2) * nL, cudaMemcpyDeviceToHost, d->st));
     DCK(d, cudaStreamSynchronize(d->st));
-    df_free(d, d_F);
-    df_free(d, d_C);
-    df_free(d, d_L);
     std::vector<int32_t> crd(3 * (size_t)N), oo((size_t)N * no), ov((size_t)N * nv);
     std::vector<double> eo((size_t)N * no), ev((size_t)N * nv);
     for (int k = 0; k < N; ++k) {
@@ -776,7 +815,7 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     double a2d = 0.0, a2x = 0.0;
     int64_t nz = 0;
     double gz = 0.0, ms = 0.0;
-    s = tce_dfmp2_energy(N, d->ncl, crd.data(), no, nv, nau, L.data(), eo.data(), oo.data(), ev.data(), ov.data(),
+    s = tce_mp2_energy_on(N, d->ncl, crd.data(), no, nv, nau, reinterpret_cast<const double *>(d_L), true, eo.data(), oo.data(), ev.data(), ov.data(),
                          mode, &a2d, &a2x, &nz, &gz, &ms);
     if (s) return df_fail(d, s, std::string("contraction: ") + tce_mp2_last_error());
     *e_mp2 = 2.0 * a2d - a2x;

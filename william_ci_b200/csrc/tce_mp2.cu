@@ -25,6 +25,10 @@
 
 using namespace nvcuda;
 
+int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord, int32_t no, int32_t nv, int32_t nau,
+                      const double *L, bool l_dev, const double *eps_o, const int32_t *occ_o, const double *eps_v,
+                      const int32_t *occ_v, int32_t mode, double *e2d, double *e2x, int64_t *nzero, double *gzero, double *ms);
+
 namespace {
 
 thread_local std::string g_mp2_err;
@@ -91,6 +95,100 @@ __global__ void k_ovov_fp64(Mp2Dims D, const int *crd, const double2 *L, double2
             im = fma(x.x, y.y, fma(x.y, y.x, im));
         }
         G[gidx(D, ia, jb, k1, k2, k3)] = make_double2(re * invN, im * invN);
+    }
+}
+
+// FP64 contraction and energy in one kernel, no G array: the exchange partner of
+// triple (ki, ka, kj) is the direct block of (ki, kb, kj), kb = ki - ka + kj, whose
+// own partner is ka.  A block takes one (ki, kj); its warps take the pairs
+// {ka, kb}: the four L tiles of a pair go to shared memory, both direct blocks
+// G(ka), G(kb) are formed there and both triples' energies follow.
+// G through memory cost 354 MB written and read (and allocated) per call on 96
+// cells with 5 bands; L (12 MB) stays in the L2.
+constexpr int MP2_FW = 4;   // warps per block
+__global__ void __launch_bounds__(32 * MP2_FW) k_mp2_fused(Mp2Dims D, const int *crd, const double2 *__restrict__ L, const double *eo,
+                                                           const int *oo, const double *ev, const int *ov_,
+                                                           double *acc /* e2d, e2x, gzero */, unsigned long long *nzero)
+{
+    extern __shared__ double2 sm2[];
+    __shared__ double red[4][MP2_FW];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int tl = D.ov * D.nau, o2 = D.ov * D.ov;
+    double2 *La = sm2 + (size_t)w * (4 * tl + 2 * o2);   // L(., ki, ka), L(., kj, kb), L(., ki, kb), L(., kj, ka)
+    double2 *G0 = La + 4 * tl, *G1 = G0 + o2;
+    const double invN = 1.0 / D.N;
+    double e2d = 0.0, e2x = 0.0, gz = 0.0;
+    unsigned long long nz = 0;
+    for (long long kk = blockIdx.x; kk < (long long)D.N * D.N; kk += gridDim.x) {
+        const int ki = (int)(kk % D.N), kj = (int)(kk / D.N);
+        for (int ka = w; ka < D.N; ka += MP2_FW) {
+            const int kb = k4_of(D, crd, ki, ka, kj);
+            if (kb < ka) continue;                       // the pair is taken at its smaller member
+            const bool two = kb != ka;
+            __syncwarp();
+            for (int x = lane; x < (two ? 4 : 2) * tl; x += 32) {
+                const int b = x / tl, e = x - b * tl;
+                const int k1 = (b & 1) ? kj : ki, k2 = (b == 0 || b == 3) ? ka : kb;
+                La[x] = L[lidx(D, e % D.ov, e / D.ov, k1, k2)];
+            }
+            __syncwarp();
+            for (int x = lane; x < (two ? 2 : 1) * o2; x += 32) {
+                const int b = x / o2, e = x - b * o2, ia = e % D.ov, jb = e / D.ov;
+                const double2 *X = La + 2 * b * tl + ia, *Y = La + (2 * b + 1) * tl + jb;
+                double re = 0.0, im = 0.0;
+                for (int Q = 0; Q < D.nau; ++Q) {
+                    const double2 u = X[Q * D.ov], v = Y[Q * D.ov];
+                    re = fma(u.x, v.x, fma(-u.y, v.y, re));
+                    im = fma(u.x, v.y, fma(u.y, v.x, im));
+                }
+                G0[x] = make_double2(re * invN, im * invN);
+            }
+            __syncwarp();
+            for (int x = lane; x < (two ? 2 : 1) * o2; x += 32) {
+                const int t = x / o2, e = x - t * o2, ia = e % D.ov, jb = e / D.ov;
+                const int i = ia % D.no, a = ia / D.no, j = jb % D.no, b = jb / D.no;
+                const int qa = t ? kb : ka, qb = t ? ka : kb;
+                if (oo[ki * D.no + i] != 2 || oo[kj * D.no + j] != 2 || ov_[qa * D.nv + a] != 0 || ov_[qb * D.nv + b] != 0) continue;
+                const double Dn = ev[qa * D.nv + a] + ev[qb * D.nv + b] - eo[ki * D.no + i] - eo[kj * D.no + j];
+                const double2 gd = G0[x];
+                if (fabs(Dn) < 1e-8) {
+                    ++nz;
+                    gz = fmax(gz, sqrt(gd.x * gd.x + gd.y * gd.y));
+                    continue;
+                }
+                const double2 gx = (two && !t ? G1 : G0)[(i + D.no * b) + D.ov * (j + D.no * a)];
+                e2d -= (gd.x * gd.x + gd.y * gd.y) / Dn;
+                e2x -= (gd.x * gx.x + gd.y * gx.y) / Dn;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        e2d += __shfl_xor_sync(0xffffffffu, e2d, o);
+        e2x += __shfl_xor_sync(0xffffffffu, e2x, o);
+        gz = fmax(gz, __shfl_xor_sync(0xffffffffu, gz, o));
+        nz += __shfl_xor_sync(0xffffffffu, nz, o);
+    }
+    if (lane == 0) {
+        red[0][w] = e2d;
+        red[1][w] = e2x;
+        red[2][w] = gz;
+        red[3][w] = (double)nz;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int x = 1; x < MP2_FW; ++x) {
+            red[0][0] += red[0][x];
+            red[1][0] += red[1][x];
+            red[2][0] = fmax(red[2][0], red[2][x]);
+            red[3][0] += red[3][x];
+        }
+        atomicAdd(acc, red[0][0]);
+        atomicAdd(acc + 1, red[1][0]);
+        if (red[3][0] > 0.0) {
+            atomicAdd(nzero, (unsigned long long)red[3][0]);
+            atomicMax(reinterpret_cast<unsigned long long *>(acc + 2), (unsigned long long)__double_as_longlong(red[2][0]));
+        }
     }
 }
 
@@ -274,6 +372,16 @@ int tce_dfmp2_energy(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord,
                      const int32_t *occ_v, int32_t mode, double *e2d, double *e2x, int64_t *nzero, double *gzero,
                      double *ms)
 {
+    return tce_mp2_energy_on(ncell, ncl, kcoord, no, nv, nau, L, false, eps_o, occ_o, eps_v, occ_v, mode, e2d, e2x, nzero, gzero, ms);
+}
+
+}  // extern "C"
+
+// The same with L on the host or, l_dev, on the device already (tce_dfmp2)
+int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord, int32_t no, int32_t nv, int32_t nau,
+                      const double *L, bool l_dev, const double *eps_o, const int32_t *occ_o, const double *eps_v,
+                      const int32_t *occ_v, int32_t mode, double *e2d, double *e2x, int64_t *nzero, double *gzero, double *ms)
+{
     if (ncell < 1 || !ncl || !kcoord || no < 1 || nv < 1 || nau < 1 || !L || !eps_o || !occ_o || !eps_v ||
         !occ_v || !e2d || !e2x)
         return mp2_fail(TCE_ERR_ARG, "bad argument");
@@ -296,8 +404,12 @@ int tce_dfmp2_energy(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord,
     if (!s) s = dmalloc(&d_crd, 3 * (size_t)ncell, keep);
     if (!s) s = dmalloc(&d_oo, (size_t)ncell * no, keep);
     if (!s) s = dmalloc(&d_ov, (size_t)ncell * nv, keep);
-    if (!s) s = dmalloc(&d_L, nL, keep);
-    if (!s) s = dmalloc(&d_G, nG, keep);
+    // the fused FP64 kernel where its tiles fit a block's shared memory, else G in memory
+    const size_t fsmem = sizeof(double2) * MP2_FW * ((size_t)4 * ov * nau + (size_t)2 * ov * ov);
+    const bool fused = mode == 0 && fsmem <= 200 * 1024;
+    if (l_dev) d_L = reinterpret_cast<double2 *>(const_cast<double *>(L));
+    else if (!s) s = dmalloc(&d_L, nL, keep);
+    if (!s && !fused) s = dmalloc(&d_G, nG, keep);
     if (!s) s = dmalloc(&d_eo, (size_t)ncell * no, keep);
     if (!s) s = dmalloc(&d_ev, (size_t)ncell * nv, keep);
     if (!s) s = dmalloc(&d_acc, 3, keep);
@@ -312,13 +424,19 @@ int tce_dfmp2_energy(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord,
     cudaMemcpy(d_crd, kcoord, sizeof(int) * 3 * ncell, cudaMemcpyHostToDevice);
     cudaMemcpy(d_oo, occ_o, sizeof(int) * ncell * no, cudaMemcpyHostToDevice);
     cudaMemcpy(d_ov, occ_v, sizeof(int) * ncell * nv, cudaMemcpyHostToDevice);
-    cudaMemcpy(d_L, L, sizeof(double2) * nL, cudaMemcpyHostToDevice);
+    if (!l_dev) cudaMemcpy(d_L, L, sizeof(double2) * nL, cudaMemcpyHostToDevice);
     cudaMemcpy(d_eo, eps_o, sizeof(double) * ncell * no, cudaMemcpyHostToDevice);
     cudaMemcpy(d_ev, eps_v, sizeof(double) * ncell * nv, cudaMemcpyHostToDevice);
     cudaMemset(d_acc, 0, sizeof(double) * 3);
     cudaMemset(d_nz, 0, sizeof(unsigned long long));
     cudaEventRecord(e0);
-    if (mode == 0) {
+    if (fused) {
+        cudaFuncSetAttribute(k_mp2_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
+        int per = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mp2_fused, 32 * MP2_FW, fsmem);
+        const long long blocks = std::min<long long>((long long)ncell * ncell, 148LL * std::max(per, 1));
+        k_mp2_fused<<<(unsigned)blocks, 32 * MP2_FW, fsmem>>>(D, d_crd, d_L, d_eo, d_oo, d_ev, d_ov, d_acc, d_nz);
+    } else if (mode == 0) {
         k_ovov_fp64<<<148 * 16, 256>>>(D, d_crd, d_L, d_G);
     } else {
         const int MP = (ov + 15) / 16 * 16, KP = (2 * nau + 15) / 16 * 16;
@@ -336,7 +454,7 @@ int tce_dfmp2_energy(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord,
     }
     const long long ntrip = (long long)ncell * ncell * ncell;
     const int eblocks = (int)std::min<long long>((ntrip + 255) / 256, 148 * 8);
-    k_mp2_energy<<<eblocks, 256>>>(D, d_crd, d_G, d_eo, d_oo, d_ev, d_ov, d_acc, d_nz);
+    if (!fused) k_mp2_energy<<<eblocks, 256>>>(D, d_crd, d_G, d_eo, d_oo, d_ev, d_ov, d_acc, d_nz);
     cudaEventRecord(e1);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
@@ -361,5 +479,3 @@ int tce_dfmp2_energy(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord,
     cudaEventDestroy(e1);
     return TCE_OK;
 }
-
-}  // extern "C"
