@@ -486,7 +486,7 @@ int build(Handle *h, const tce_system *sys)
     std::vector<PairPrim> hpp((size_t)npp_tot);
     CK(h, cudaMemcpyAsync(hpp.data(), h->d_pp, npp_tot * sizeof(PairPrim), cudaMemcpyDeviceToHost, h->st));
     CK(h, cudaStreamSynchronize(h->st));
-    long long v_tot = 0;
+    long long v_tot = 0, r_tot = 0;
     for (auto &U : h->up) {
         int nmax = 0;
         double km = 0.0;
@@ -498,17 +498,22 @@ int build(Handle *h, const tce_system *sys)
         U.Nlen = nmax + 1;
         U.ket_max = km;
         U.vec_off = v_tot;
+        U.r_off = r_tot;
+        r_tot += (long long)h->ndp * U.Nlen * U.npp;
         v_tot += (long long)h->ndp * (U.l1 + 1) * (U.l2 + 1) * 2 * U.Nlen * U.npp;
     }
     CK(h, cudaMemcpyAsync(d_up, h->up.data(), h->up.size() * sizeof(UnitPair), cudaMemcpyHostToDevice, h->st));
     double2 *d_vec = nullptr;
     if ((s = dalloc(h, &d_vec, (size_t)v_tot))) return s;
     S.vec = d_vec;
+    double *d_rvec = nullptr;
+    if ((s = dalloc(h, &d_rvec, (size_t)r_tot))) return s;
+    S.rvec = d_rvec;
     {
         int stride = h->ncap + 2 * TCE_LMAX + 2;
         double *scr = nullptr;
         if ((s = dalloc(h, &scr, (size_t)npp_tot * h->ndp * stride))) return s;
-        CKS(h, tce_launch_pair_vectors(S, npp_tot, d_ppu, h->d_pp, stride, scr, d_vec, h->st));
+        CKS(h, tce_launch_pair_vectors(S, npp_tot, d_ppu, h->d_pp, stride, scr, d_vec, d_rvec, h->st));
         CK(h, cudaStreamSynchronize(h->st));
         dfree(h, scr);
     }
@@ -710,8 +715,8 @@ static int fixed_lists(Handle *h, int mode, const double *dP, double *dJ, double
             b.physicist = h->physicist;
             b.num_sms = h->num_sms;
             if (h->use_tc) {
-                if (w.kind == 1) CKS(h, tce_launch_quartets_s_tc(h->S, b, h->nq, 1, st));
-                else CKS(h, tce_launch_quartets_sp_tc(h->S, w.cls, b, h->nq, 1, st));
+                if (w.kind == 1) CKS(h, tce_launch_quartets_s_tc(h->S, b, h->nq, tce_tc_shape_s(h->S), st));
+                else CKS(h, tce_launch_quartets_sp_tc(h->S, w.cls, b, h->nq, tce_tc_shape_sp(h->S), st));
             } else {
                 if (w.kind == 1) CKS(h, tce_launch_quartets_s(h->S, b, st));
                 else CKS(h, tce_launch_quartets_r1(h->S, w.cls, b, st));

@@ -31,6 +31,7 @@ struct UnitPair {
     int S1, S2, l1, l2, np1, np2, npp, Nlen;   // Nlen = padded vector length
     long long pp_off;    // first PairPrim
     long long vec_off;   // first double2 of the vector slabs
+    long long r_off;     // first double of the zero-power vectors, [d][n][primitive pair]
     long long e_off;     // first double of the Hermite E table
     double ket_max;      // max_pp |pfac| cmax1 cmax2 (the kernel's ket_max)
 };
@@ -63,6 +64,7 @@ struct DevSys {
     const UnitPair *up;
     const PairPrim *pp;
     const double2 *vec;
+    const double *rvec;      // zero-power vectors (real, equal for both signs): half the bytes of their slabs in vec
     const double *ecoef;
     // t tables
     const double *tnode, *tweight, *Tt;   // Tt[(d*(ncap+1)+n)*nq + k]

@@ -173,7 +173,7 @@ __global__ void k_pair_bessel(DevSys S, long long npp_tot, const int *pp_unit, c
 // one thread per (pp, d, ia, ib, sign): V_n = sum_k d_k I~_{|n - s k|}, n < Nlen
 // (zero beyond the pair's own N), written n-major into the unit pair's slab.
 __global__ void k_pair_vectors(DevSys S, long long npp_tot, const int *pp_unit, const PairPrim *pp, int stride,
-                               const double *scratch, double2 *vec)
+                               const double *scratch, double2 *vec, double *rvec)
 {
     const int NV = (TCE_LMAX + 1) * (TCE_LMAX + 1) * 2;
     long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -217,6 +217,7 @@ __global__ void k_pair_vectors(DevSys S, long long npp_tot, const int *pp_unit, 
                 }
         }
         out[(long long)n * U.npp + loc] = val;
+        if (M == 0 && s == 0) rvec[U.r_off + ((long long)d * U.Nlen + n) * U.npp + loc] = val.x;
     }
 }
 
@@ -488,14 +489,14 @@ int tce_launch_pair_scalars(const DevSys &S, long long npp_tot, const int *pp_un
 }
 
 int tce_launch_pair_vectors(const DevSys &S, long long npp_tot, const int *pp_unit, const PairPrim *pp, int stride,
-                            double *scratch, double2 *vec, cudaStream_t st)
+                            double *scratch, double2 *vec, double *rvec, cudaStream_t st)
 {
     if (npp_tot == 0) return TCE_OK;
     long long n1 = npp_tot * S.ndp;
     k_pair_bessel<<<(unsigned)((n1 + 127) / 128), 128, 0, st>>>(S, npp_tot, pp_unit, pp, stride, scratch);
     const int NV = (TCE_LMAX + 1) * (TCE_LMAX + 1) * 2;
     long long n2 = npp_tot * S.ndp * NV;
-    k_pair_vectors<<<(unsigned)((n2 + 127) / 128), 128, 0, st>>>(S, npp_tot, pp_unit, pp, stride, scratch, vec);
+    k_pair_vectors<<<(unsigned)((n2 + 127) / 128), 128, 0, st>>>(S, npp_tot, pp_unit, pp, stride, scratch, vec, rvec);
     return cudaGetLastError() == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }
 

@@ -99,6 +99,13 @@ int tce_tc_shapes_s(int nq);
 // 1..tce_tc_shapes_sp(nq); cls: bit i set when shell i of (A, B | C, D) is p
 int tce_launch_quartets_sp_tc(const DevSys &S, int cls, const SArgsHost &h, int nq, int shape, cudaStream_t st);
 int tce_tc_shapes_sp(int nq);
+// Default tile shapes by the torus' length (in orders, ncap): on long ones the
+// strides differ much from node to node, and passes of 8 nodes need fewer orders
+// than passes of 16, which build fewer fragments.  Measured (ms, 8 against 16
+// nodes per pass): 64 cells (ncap 592) all-s 64-node list 6.4 / 7.4, one-p lists
+// 1.3 / 1.5; 16 cells (ncap 166) 1.45 / 1.30 and 0.36 / 0.32.
+inline int tce_tc_shape_s(const DevSys &S) { return S.ndp > 1 || S.ncap >= 300 ? 1 : 2; }
+inline int tce_tc_shape_sp(const DevSys &S) { return S.ncap >= 300 ? 2 : 1; }
 inline bool tce_r1_supported(int ndp, int nq, int cls)
 {
     return ndp == 1 && nq == 32 && cls >= 0 && cls < 16 && __builtin_popcount(cls) == 1;
@@ -108,7 +115,7 @@ int tce_launch_t_tables(int nq, int ndp, int ncap, const double *tnode, const do
 int tce_launch_pair_scalars(const DevSys &S, long long npp_tot, const int *pp_unit, PairPrim *pp, UnitPair *up,
                             double *ecoef, cudaStream_t st);
 int tce_launch_pair_vectors(const DevSys &S, long long npp_tot, const int *pp_unit, const PairPrim *pp, int stride,
-                            double *scratch, double2 *vec, cudaStream_t st);
+                            double *scratch, double2 *vec, double *rvec, cudaStream_t st);
 int tce_launch_enumerate(const DevSys &S, const double *Qsh, double Qmax, int4 *items, unsigned long long *count,
                          unsigned long long cap, unsigned long long *nfunc, cudaStream_t st);
 int tce_launch_stored_jk(int n1, int nbas, int physicist, const double *P, const double *eri, double *J, double *K,

@@ -21,6 +21,6 @@ static int sp2_launch(const DevSys &S, int cls, const SArgs &A, int nsm, cudaStr
 
 int tce_sp2_launch(const DevSys &S, int cls, const SArgs &A, int shape, int nsm, cudaStream_t st)
 {
-    if (!A.item_rule) return sp2_launch<2, false>(S, cls, A, nsm, st);
+    if (!A.item_rule) return shape == 1 ? sp2_launch<2, false>(S, cls, A, nsm, st) : sp2_launch<1, false>(S, cls, A, nsm, st);
     return shape == 1 ? sp2_launch<2, true>(S, cls, A, nsm, st) : sp2_launch<1, true>(S, cls, A, nsm, st);
 }

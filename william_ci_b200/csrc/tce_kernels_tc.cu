@@ -10,18 +10,18 @@
 // a pass of NT node tiles of 8 (T[n][k] = c_n e^{-C_k} I_n(C_k)): an (8 MT x J)
 // x (J x 8 NT) product per pass, mma.sync.m8n8k4 (FP64) per 8 x 8 tile and step
 // of four orders.  Lane l builds the A fragments (F) of rows 8 m + l/4 at order
-// h (4 s + l%4), cos(n phi) from the three-term recurrence in steps of 4 h
-// (re-seeded every eight steps); the B fragments are T[h (4 s + l%4)][8 g + l/4].
-// The next step's G, H and T are loaded before the current step's mma.
+// h (4 s + l%4), e^{i n phi} by rotation; the B fragments are T[h (4 s + l%4)][8 g + l/4].
+// The G, H and T of four steps are loaded together before their mma.
 //
 // What bounds it: with every order summed (about 170 per node on the 64-cell
 // chain) the mma instructions did; with 13 to 27 orders per tile the epilogue
 // (one reciprocal per two nodes), the plans and the loads' latency weigh as
-// much.  Passes of 16 nodes share one plan: 8-node passes need as many tile
-// products and twice the fragments, 32-node passes twice the tile products,
-// because the node with the smallest C sets the stride.
-// 64-cell chain, all-s 64-node list 16.4 -> 8.2 ms, 32-node list 6.5 -> 4.8 ms;
-// fixed 32-node rule, whole pass 72.7 -> 16.7 ms.
+// much.  The node with the smallest C sets a pass's stride, the largest its last
+// order: passes of 8 nodes need half the tile products of passes of 16 on the
+// 64-cell chain, 32-node passes twice as many (tce_tc_shape_s).
+// 64-cell chain: all-s 64-node list 16.4 -> 6.4 ms, 32-node list 6.5 -> 2.9 ms;
+// fixed 32-node rule, whole pass 72.7 -> 14.4 ms.  (With one step's loads ahead
+// and 16-node passes it was 8.2, 4.8 and 16.7 ms.)
 //
 // Also here: the launch of the s/p tensor-core kernel (k_quartets_sp_tc,
 // tce_kernels_tc.cuh) for the classes with one p shell; those with two are
@@ -34,12 +34,15 @@
 template <int NDP, int MT, int NT, bool LG>
 __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
 {
-    constexpr int BT = 8 * MT;
+    constexpr int BT = 8 * MT, US = 4, RW = 3 + NDP;
+    static_assert(MT <= 2, "the epilogue's shared reciprocal takes two row tiles");
     constexpr float E = tce_order_exponent(0);
     extern __shared__ double smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     const int rq = lane >> 2, cq = lane & 3;   // fragment row in an 8-row tile, fragment column
     const PrimPool Pool = tce_pool(smem, wib);
+    // per row of the batch: pq, p + q, R^2, phi per periodic direction
+    double *Rows = reinterpret_cast<double *>(reinterpret_cast<char *>(smem) + 8 * (size_t)TCE_POOL_BYTES) + (size_t)wib * BT * RW;
 
     while (true) {
         int it = 0;
@@ -95,41 +98,42 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
                 // this lane's fragment rows (primitive quartets 8 m + rq of the batch; past
                 // its end the first one, with factor zero)
                 const double *Gp[NDP][MT], *Hp[NDP][MT];
-                double f[MT], pq_[MT], ps[MT], R2[MT], c1[NDP][MT], s1[NDP][MT];
-                double phi[NDP][MT];
+                double c1[NDP][MT], s1[NDP][MT];
                 float umin[NDP], umax[NDP], pmin[NDP], pmax[NDP];
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
                     const int r = b0 + 8 * m + rq;
-                    const int e = Pool.key[r < np ? r : b0];
-                    const int2 pq = Pool.pq[e];
-                    f[m] = r < np ? Pool.fac[e] : 0.0;
+                    const int2 pq = Pool.pq[Pool.key[r < np ? r : b0]];
                     const PairPrim &Pb = S.pp[Ub.pp_off + pq.x];
                     const PairPrim &Pk = S.pp[Uk.pp_off + pq.y];
-                    pq_[m] = Pb.esum * Pk.esum;
-                    ps[m] = Pb.esum + Pk.esum;
-                    R2[m] = 0.0;
+                    double *row = Rows + (8 * m + rq) * RW;
+                    double R2 = 0.0;
 #pragma unroll
                     for (int d = 0; d < 3; ++d) {
                         const double x = Pb.cen[d] - (Pk.cen[d] + Tsh[d]);
                         if (d < NDP) {
-                            phi[d < NDP ? d : 0][m] = S.a[d] * x;
-                            const float u = 1.0f / (float)Pb.A[d] + 1.0f / (float)Pk.A[d], ap = tce_fold_phase(S.a[d] * x);
+                            const double phi = S.a[d] * x;
+                            row[3 + (d < NDP ? d : 0)] = phi;
+                            const float u = 1.0f / (float)Pb.A[d] + 1.0f / (float)Pk.A[d], ap = tce_fold_phase(phi);
                             umin[d < NDP ? d : 0] = m == 0 ? u : fminf(umin[d < NDP ? d : 0], u);
                             umax[d < NDP ? d : 0] = m == 0 ? u : fmaxf(umax[d < NDP ? d : 0], u);
                             pmin[d < NDP ? d : 0] = m == 0 ? ap : fminf(pmin[d < NDP ? d : 0], ap);
                             pmax[d < NDP ? d : 0] = m == 0 ? ap : fmaxf(pmax[d < NDP ? d : 0], ap);
                         } else {
-                            R2[m] += x * x;
+                            R2 += x * x;
                         }
                     }
+                    row[0] = Pb.esum * Pk.esum;
+                    row[1] = Pb.esum + Pk.esum;
+                    row[2] = R2;
 #pragma unroll
                     for (int d = 0; d < NDP; ++d) {
-                        Gp[d][m] = reinterpret_cast<const double *>(S.vec + Ub.vec_off + (long long)(2 * d) * Ub.Nlen * nppb + pq.x);
-                        Hp[d][m] = reinterpret_cast<const double *>(S.vec + Uk.vec_off + (long long)(2 * d + 1) * Uk.Nlen * nppk + pq.y);
+                        Gp[d][m] = S.rvec + Ub.r_off + (long long)d * Ub.Nlen * nppb + pq.x;
+                        Hp[d][m] = S.rvec + Uk.r_off + (long long)d * Uk.Nlen * nppk + pq.y;
                     }
                 }
-                OrderPlan plan[NDP];   // of pass `lane`
+                OrderPlan plan[NDP];   // of pass `lane`; last: with the number of steps in pstep
+                int pstep[NDP];
 #pragma unroll
                 for (int d = 0; d < NDP; ++d) {
 #pragma unroll
@@ -141,8 +145,10 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
                     }
                     const int nlast = min(glast[d], min(Ub.Nlen, Uk.Nlen) - 1);
                     plan[d] = tce_order_plan(E, 0, umin[d], umax[d], pmin[d], pmax[d], vmin[d], vmax[d], nlast);
+                    pstep[d] = plan[d].h > 0 ? plan[d].last / (4 * plan[d].h) + 1 : 0;
                     if (glast[d] < 0) plan[d].h = 0;
                 }
+                __syncwarp();
                 double vK[MT], vG[MT];
 #pragma unroll
                 for (int m = 0; m < MT; ++m) vK[m] = vG[m] = 0.0;
@@ -154,17 +160,18 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
                         for (int d = 0; d < NDP; ++d) {
                             const double hd = (double)__shfl_sync(0xffffffffu, plan[d].h, c + cq);
 #pragma unroll
-                            for (int m = 0; m < MT; ++m) sincos(hd * phi[d][m], &s1[d][m], &c1[d][m]);
+                            for (int m = 0; m < MT; ++m) sincos(hd * Rows[(8 * m + rq) * RW + 3 + d], &s1[d][m], &c1[d][m]);
                         }
                     }
                     double pr[2 * MT * NT];
                     bool none = false;
                     double hw = 1.0;
-                    int h[NDP], last[NDP];
+                    int h[NDP], last[NDP], steps[NDP];
 #pragma unroll
                     for (int d = 0; d < NDP; ++d) {
                         h[d] = __shfl_sync(0xffffffffu, plan[d].h, c);
                         last[d] = __shfl_sync(0xffffffffu, plan[d].last, c);
+                        steps[d] = __shfl_sync(0xffffffffu, pstep[d], c);
                         none = none || h[d] == 0;
                         hw *= (double)h[d];
                     }
@@ -174,63 +181,51 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
                     for (int t = 0; t < NT; ++t) col[t] = 8 * min(c * NT + t, ng - 1) + rq;
 #pragma unroll
                     for (int d = 0; d < NDP; ++d) {
+                        const double *Tg = R.T + d * R.strideD;
+                        const int h4 = 4 * h[d];
+                        int n = h[d] * cq;
                         double acc[2 * MT * NT];
 #pragma unroll
                         for (int x = 0; x < 2 * MT * NT; ++x) acc[x] = 0.0;
-                        double cc[MT], cp[MT], c4[MT];   // cos(n phi), cos((n - 4 h) phi), 2 cos(4 h phi)
+                        double cc[MT], sc[MT], c4[MT], s4[MT];   // e^{i n phi}, e^{4 i h phi}
+                        // US steps of loads at once: a step's mma take far less than the L2's latency
+#pragma unroll 1
+                        for (int s = 0; s < steps[d]; s += US) {
+                            double gN[US][MT], hN[US][MT], tN[US][NT];
 #pragma unroll
-                        for (int m = 0; m < MT; ++m) {
-                            const int src = (lane & ~3) | (c & 3);
-                            const double cb = __shfl_sync(0xffffffffu, c1[d][m], src);
-                            const double sb = __shfl_sync(0xffffffffu, s1[d][m], src);
-                            double u0, u1;
-                            tce_phase_start(cb, sb, cq, cc[m], u0, cp[m], u1, c4[m]);
-                        }
-                        const double *Tg = R.T + d * R.strideD;
-                        const int steps = last[d] / (4 * h[d]) + 1, h4 = 4 * h[d];
-                        int n = h[d] * cq;
-                        double gN[MT], hN[MT], tN[NT];
-                        auto load = [&]() {   // the values of order n (past the last order: T = 0)
-                            const int nn = min(n, last[d]);
-#pragma unroll
-                            for (int m = 0; m < MT; ++m) {
-                                gN[m] = __ldg(Gp[d][m] + (long long)nn * (2 * nppb));
-                                hN[m] = __ldg(Hp[d][m] + (long long)nn * (2 * nppk));
-                            }
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) {
-                                const double tv = __ldg(Tg + ((long long)nn * nq + col[t]));
-                                tN[t] = n <= last[d] ? tv : 0.0;
-                            }
-                            n += h4;
-                        };
-                        load();
-#pragma unroll 2
-                        for (int s = 0; s < steps; ++s) {
-                            double F[MT], Tb[NT];
-#pragma unroll
-                            for (int m = 0; m < MT; ++m) F[m] = gN[m] * hN[m] * cc[m];
-#pragma unroll
-                            for (int t = 0; t < NT; ++t) Tb[t] = tN[t];
-                            load();
-                            if ((s & 7) == 7) {   // re-seed the recurrence
+                            for (int u = 0; u < US; ++u) {
+                                const int nn = min(n + u * h4, last[d]);
 #pragma unroll
                                 for (int m = 0; m < MT; ++m) {
-                                    cp[m] = cos((double)(n - 2 * h4) * phi[d][m]);
-                                    cc[m] = cos((double)(n - h4) * phi[d][m]);
+                                    gN[u][m] = __ldg(Gp[d][m] + (long long)nn * nppb);
+                                    hN[u][m] = __ldg(Hp[d][m] + (long long)nn * nppk);
                                 }
-                            } else {
+#pragma unroll
+                                for (int t = 0; t < NT; ++t) tN[u][t] = __ldg(Tg + ((long long)nn * nq + col[t]));
+                            }
+                            if (s == 0) {
 #pragma unroll
                                 for (int m = 0; m < MT; ++m) {
-                                    const double t = c4[m] * cc[m] - cp[m];
-                                    cp[m] = cc[m];
-                                    cc[m] = t;
+                                    const int src = (lane & ~3) | (c & 3);
+                                    tce_phase_start(__shfl_sync(0xffffffffu, c1[d][m], src), __shfl_sync(0xffffffffu, s1[d][m], src),
+                                                    cq, cc[m], sc[m], c4[m], s4[m]);
                                 }
                             }
 #pragma unroll
-                            for (int t = 0; t < NT; ++t)
+                            for (int u = 0; u < US; ++u) {
+                                if (s + u >= steps[d]) break;
+                                double F[MT];
 #pragma unroll
-                                for (int m = 0; m < MT; ++m) tce_dmma(acc[(m * NT + t) * 2], acc[(m * NT + t) * 2 + 1], F[m], Tb[t]);
+                                for (int m = 0; m < MT; ++m) {
+                                    F[m] = n <= last[d] ? gN[u][m] * hN[u][m] * cc[m] : 0.0;
+                                    tce_phase_step(cc[m], sc[m], c4[m], s4[m]);
+                                }
+                                n += h4;
+#pragma unroll
+                                for (int t = 0; t < NT; ++t)
+#pragma unroll
+                                    for (int m = 0; m < MT; ++m) tce_dmma(acc[(m * NT + t) * 2], acc[(m * NT + t) * 2 + 1], F[m], tN[u][t]);
+                            }
                         }
 #pragma unroll
                         for (int x = 0; x < 2 * MT * NT; ++x) pr[x] = d == 0 ? acc[x] : pr[x] * acc[x];
@@ -249,46 +244,61 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
                         }
                         wk.x *= hw;
                         wk.y *= hw;
-                        const double t20 = tn.x * tn.x, t21 = tn.y * tn.y;
+                        const double t2[2] = {tn.x * tn.x, tn.y * tn.y};
+                        double D[MT][2];   // 1 / (pq + (p + q) t^2), for NDP = 2 its square root
+                        if (NDP < 3) {
+#pragma unroll
+                            for (int m = 0; m < MT; ++m)
+#pragma unroll
+                                for (int i = 0; i < 2; ++i) D[m][i] = fma(Rows[(8 * m + rq) * RW + 1], t2[i], Rows[(8 * m + rq) * RW]);
+                            if (NDP == 1) {   // one reciprocal for all of them
+                                double q0 = D[0][0] * D[0][1], q1 = MT > 1 ? D[MT - 1][0] * D[MT - 1][1] : 1.0;
+                                const double ri = 1.0 / (q0 * q1), x = q0;
+                                q0 = ri * q1;
+                                q1 = ri * x;
+#pragma unroll
+                                for (int m = 0; m < MT; ++m) {
+                                    const double qm = m == 0 ? q0 : q1, y = D[m][0];
+                                    D[m][0] = qm * D[m][1];
+                                    D[m][1] = qm * y;
+                                }
+                            } else {
+#pragma unroll
+                                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                                    for (int i = 0; i < 2; ++i) D[m][i] = rsqrt(D[m][i]);
+                            }
+                        }
 #pragma unroll
                         for (int m = 0; m < MT; ++m) {
-                            double b0_ = pr[(m * NT + t) * 2], b1_ = pr[(m * NT + t) * 2 + 1];
+                            double b[2] = {pr[(m * NT + t) * 2], pr[(m * NT + t) * 2 + 1]};
                             if (NDP < 3) {
-                                const double d0 = fma(ps[m], t20, pq_[m]), d1 = fma(ps[m], t21, pq_[m]);
-                                double D0, D1;   // 1 / d0 and 1 / d1
-                                if (NDP == 1) {
-                                    const double ri = 1.0 / (d0 * d1);
-                                    D0 = ri * d1;
-                                    D1 = ri * d0;
-                                    b0_ *= D0;
-                                    b1_ *= D1;
-                                } else {
-                                    const double r0 = rsqrt(d0), r1 = rsqrt(d1);
-                                    D0 = r0 * r0;
-                                    D1 = r1 * r1;
-                                    b0_ *= r0;
-                                    b1_ *= r1;
-                                }
-                                if (R2[m] != 0.0) {
-                                    const double w = -pq_[m] * R2[m];
-                                    b0_ *= exp(w * t20 * D0);
-                                    b1_ *= exp(w * t21 * D1);
+                                b[0] *= D[m][0];
+                                b[1] *= D[m][1];
+                                const double R2 = Rows[(8 * m + rq) * RW + 2];
+                                if (R2 != 0.0) {
+                                    const double w = -Rows[(8 * m + rq) * RW] * R2;
+#pragma unroll
+                                    for (int i = 0; i < 2; ++i) b[i] *= exp(w * t2[i] * (NDP == 1 ? D[m][i] : D[m][i] * D[m][i]));
                                 }
                             }
-                            vK[m] = fma(b0_, wk.x, vK[m]);
-                            vK[m] = fma(b1_, wk.y, vK[m]);
+                            vK[m] = fma(b[0], wk.x, vK[m]);
+                            vK[m] = fma(b[1], wk.y, vK[m]);
                             if (LG) {
-                                vG[m] = fma(b0_, wg.x, vG[m]);
-                                vG[m] = fma(b1_, wg.y, vG[m]);
+                                vG[m] = fma(b[0], wg.x, vG[m]);
+                                vG[m] = fma(b[1], wg.y, vG[m]);
                             }
                         }
                     }
                 }
 #pragma unroll
                 for (int m = 0; m < MT; ++m) {
-                    blk = fma(f[m], vK[m], blk);
-                    if (LG) blkG = fma(f[m], vG[m], blkG);
+                    const int r = b0 + 8 * m + rq;
+                    const double f = r < np ? Pool.fac[Pool.key[r]] : 0.0;
+                    blk = fma(f, vK[m], blk);
+                    if (LG) blkG = fma(f, vG[m], blkG);
                 }
+                __syncwarp();
             }
             __syncwarp();
             np = 0;
@@ -322,7 +332,7 @@ int tce_tc_shapes_sp(int nq)
     return nq == 64 ? 3 : nq == 32 ? 2 : 0;
 }
 
-// one p shell.  shape 1: 8 rows x 16 nodes per pass, 2: 16 x 16, 3: 8 x 8
+// one p shell.  shape 1: 8 rows x 16 nodes per pass, 2 and 3: 8 x 8
 template <bool LG>
 static int sp1_launch(const DevSys &S, int cls, const SArgs &A, int shape, int nsm, cudaStream_t st)
 {
@@ -334,11 +344,7 @@ static int sp1_launch(const DevSys &S, int cls, const SArgs &A, int shape, int n
     case 8: sp_tc_launch<0, 0, 0, 1, MTv, NTv, LG>(S, A, nsm, st); break;              \
     default: return TCE_ERR_UNSUPPORTED;                                               \
     }
-    if constexpr (!LG) {
-        TCE_SP1(1, 2)
-    } else {
-        if (shape == 1) { TCE_SP1(1, 2) } else if (shape == 2) { TCE_SP1(2, 2) } else { TCE_SP1(1, 1) }
-    }
+    if (shape == 1) { TCE_SP1(1, 2) } else { TCE_SP1(1, 1) }
 #undef TCE_SP1
     return TCE_OK;
 }
@@ -358,7 +364,7 @@ int tce_launch_quartets_sp_tc(const DevSys &S, int cls, const SArgsHost &h, int 
     const int nsm = h.num_sms > 0 ? h.num_sms : 148;
     const int s = np == 2 ? tce_sp2_launch(S, cls, A, shape, nsm, st)
                   : lg    ? sp1_launch<true>(S, cls, A, shape, nsm, st)
-                          : sp1_launch<false>(S, cls, A, 1, nsm, st);
+                          : sp1_launch<false>(S, cls, A, shape, nsm, st);
     if (s != TCE_OK) return s;
     return cudaGetLastError() == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }
@@ -368,8 +374,7 @@ int tce_tc_shapes_s(int nq)
     return (nq == 32 || nq == 64) ? 5 : 0;
 }
 
-// shape 1: 16 rows x 16 nodes per pass (the default), 2: 8 x 16, 3: 16 x 8,
-// 4: 8 x 8, 5: 16 x 32
+// shape 1: 16 rows x 8 nodes per pass, 2 and 5: 16 x 16, 3: 8 x 8, 4: 8 x 16
 int tce_launch_quartets_s_tc(const DevSys &S, const SArgsHost &h, int nq, int shape, cudaStream_t st)
 {
     const bool lg = h.item_rule != nullptr;
@@ -380,22 +385,25 @@ int tce_launch_quartets_s_tc(const DevSys &S, const SArgsHost &h, int nq, int sh
     tc_args(A, h);
     if (cudaMemsetAsync(h.next, 0, sizeof(unsigned int), st) != cudaSuccess) return TCE_ERR_CUDA;
     const int nsm = h.num_sms > 0 ? h.num_sms : 148;
+#define TCE_S_TC(NDPv, MTv, NTv, LGv) \
+    tc_launch(k_quartets_s_tc<NDPv, MTv, NTv, LGv>, S, A, nsm, st, 8 * 8 * sizeof(double) * MTv * (3 + NDPv))
     if (!lg) {
-        if (S.ndp == 1) tc_launch(k_quartets_s_tc<1, 2, 2, false>, S, A, nsm, st);
-        else if (S.ndp == 2) tc_launch(k_quartets_s_tc<2, 1, 2, false>, S, A, nsm, st);
-        else tc_launch(k_quartets_s_tc<3, 1, 2, false>, S, A, nsm, st);
+        if (S.ndp == 2) TCE_S_TC(2, 1, 2, false);
+        else if (S.ndp == 3) TCE_S_TC(3, 1, 2, false);
+        else if (shape == 1) TCE_S_TC(1, 2, 1, false);
+        else TCE_S_TC(1, 2, 2, false);
     } else if (S.ndp == 2) {
-        tc_launch(k_quartets_s_tc<2, 1, 2, true>, S, A, nsm, st);
+        TCE_S_TC(2, 1, 2, true);
     } else if (S.ndp == 3) {
-        tc_launch(k_quartets_s_tc<3, 1, 2, true>, S, A, nsm, st);
+        TCE_S_TC(3, 1, 2, true);
     } else {
         switch (shape) {
-        case 1: tc_launch(k_quartets_s_tc<1, 2, 2, true>, S, A, nsm, st); break;
-        case 2: tc_launch(k_quartets_s_tc<1, 1, 2, true>, S, A, nsm, st); break;
-        case 3: tc_launch(k_quartets_s_tc<1, 2, 1, true>, S, A, nsm, st); break;
-        case 4: tc_launch(k_quartets_s_tc<1, 1, 1, true>, S, A, nsm, st); break;
-        default: tc_launch(k_quartets_s_tc<1, 2, 4, true>, S, A, nsm, st); break;
+        case 1: TCE_S_TC(1, 2, 1, true); break;
+        case 3: TCE_S_TC(1, 1, 1, true); break;
+        case 4: TCE_S_TC(1, 1, 2, true); break;
+        default: TCE_S_TC(1, 2, 2, true); break;
         }
     }
+#undef TCE_S_TC
     return cudaGetLastError() == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }

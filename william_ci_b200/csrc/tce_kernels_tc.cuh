@@ -167,12 +167,11 @@ static inline void tc_args(SArgs &A, const SArgsHost &h)
 }
 
 // persistent launch: as many 256-thread blocks as fit on every SM; shared
-// memory = the eight warps' pools plus, for ncq components, their per-lane
-// Kronrod and Gauss block accumulators
+// memory = the eight warps' pools and `extra` bytes
 template <class Kern>
-static void tc_launch(Kern kern, const DevSys &S, const SArgs &A, int nsm, cudaStream_t st, int ncq = 0)
+static void tc_launch(Kern kern, const DevSys &S, const SArgs &A, int nsm, cudaStream_t st, size_t extra)
 {
-    const size_t smem = 8 * ((size_t)TCE_POOL_BYTES + 2 * (size_t)ncq * 32 * sizeof(double));
+    const size_t smem = 8 * (size_t)TCE_POOL_BYTES + extra;
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     int per = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, smem);
@@ -191,8 +190,7 @@ static void tc_launch(Kern kern, const DevSys &S, const SArgs &A, int nsm, cudaS
 //     I_cmb[pq][k] = sum_n Re[G^(ia,ib)_n H^(ic,id)_n e^{i n phi}] T[n][k],
 // all of them in the same step loop over the orders of tce_order_plan: the
 // zero-power vectors G^(0,0), H^(0,0) are real and loaded once for every
-// combination, and cos(n phi), sin(n phi) come from one three-term recurrence
-// in steps of four strides (re-seeded every eight steps).  The A fragments are F = Re(G H) cos(n phi) - Im(G H) sin(n phi)
+// combination, and e^{i n phi} advances by one rotation per step of four strides.  The A fragments are F = Re(G H) cos(n phi) - Im(G H) sin(n phi)
 // with the products of real factors left out.
 //
 // Epilogue by moments.  The real directions add, per node k and component c
@@ -228,6 +226,7 @@ __global__ void __launch_bounds__(256, LA + LB + LC + LD == 1 ? 2 : 1) k_quartet
     constexpr int NN = NP;                                // largest y + z power of a component
     constexpr int EB = tce_ecount(LA, LB), EK = tce_ecount(LC, LD);
     constexpr int AT = 2 * MT * NT;                       // accumulators per combination and lane
+    constexpr int US = NP == 1 ? 3 : 2;                   // steps loaded together
     constexpr int NW = LG ? 2 : 1;                        // Kronrod sums, and Gauss sums with the judge
     extern __shared__ double smem[];
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -284,6 +283,7 @@ __global__ void __launch_bounds__(256, LA + LB + LC + LD == 1 ? 2 : 1) k_quartet
         // of the bra is the slab ia (LB + 1) + ib, at Gv + 2 slab gl; the ket alike
         const long long gl = (long long)Ub.Nlen * nppb, hl = (long long)Uk.Nlen * nppk;
         const double2 *Gv = S.vec + Ub.vec_off, *Hv = S.vec + Uk.vec_off + hl;
+        const double *G0 = S.rvec + Ub.r_off, *H0 = S.rvec + Uk.r_off;   // the zero powers, real
 #pragma unroll
         for (int c = 0; c < NW * NCQ; ++c) bacc[c * 32 + lane] = 0.0;
         int np = 0;
@@ -324,6 +324,7 @@ __global__ void __launch_bounds__(256, LA + LB + LC + LD == 1 ? 2 : 1) k_quartet
                 }
                 OrderPlan plan = tce_order_plan(E, SHIFT, umin, umax, pmin, pmax, vmin, vmax,
                                                 min(glast, min(Ub.Nlen, Uk.Nlen) - 1));   // of pass `lane`
+                const int pstep = plan.h > 0 ? plan.last / (4 * plan.h) + 1 : 0;
                 if (glast < 0) plan.h = 0;
                 // moments [m][cmb][j][Kronrod, Gauss], j <= NN - xsum(cmb)
                 double Mo[MT][NCOMB][NN + 1][NW];
@@ -353,90 +354,77 @@ __global__ void __launch_bounds__(256, LA + LB + LC + LD == 1 ? 2 : 1) k_quartet
                     for (int cmb = 0; cmb < NCOMB; ++cmb)
 #pragma unroll
                         for (int x = 0; x < AT; ++x) acc[cmb][x] = 0.0;
-                    // cos / sin of n phi and (n - 4 h) phi, 2 cos(4 h phi)
-                    double cc[MT], cp[MT], sc[MT], sp[MT], c4[MT];
-#pragma unroll
-                    for (int m = 0; m < MT; ++m) {
-                        const int src = (lane & ~3) | (c & 3);
-                        const double cb = __shfl_sync(0xffffffffu, c1[m], src);
-                        const double sb = __shfl_sync(0xffffffffu, s1[m], src);
-                        tce_phase_start(cb, sb, cq, cc[m], sc[m], cp[m], sp[m], c4[m]);
-                    }
-                    const int steps = last / (4 * h) + 1, h4 = 4 * h;
+                    double cc[MT], sc[MT], c4[MT], s4[MT];   // e^{i n phi}, e^{4 i h phi}
+                    const int steps = __shfl_sync(0xffffffffu, pstep, c), h4 = 4 * h;
                     int n = h * cq;
-                    double g0N[MT], h0N[MT], tN[NT];
-                    double2 gN[NGV - 1 > 0 ? NGV - 1 : 1][MT], hN[NHV - 1 > 0 ? NHV - 1 : 1][MT];
-                    auto load = [&]() {   // the values of order n (past the last order: T = 0)
-                        const int nn = min(n, last);
+                    // US steps of loads at once: a step's mma take far less than the L2's latency
+#pragma unroll 1
+                    for (int s = 0; s < steps; s += US) {
+                        double g0N[US][MT], h0N[US][MT], tN[US][NT];
+                        double2 gN[US][NGV - 1 > 0 ? NGV - 1 : 1][MT], hN[US][NHV - 1 > 0 ? NHV - 1 : 1][MT];
 #pragma unroll
-                        for (int m = 0; m < MT; ++m) {
-                            const double2 *gp = Gv + ((long long)nn * nppb + go[m]), *hp = Hv + ((long long)nn * nppk + ho[m]);
-                            g0N[m] = __ldg(reinterpret_cast<const double *>(gp));
-                            h0N[m] = __ldg(reinterpret_cast<const double *>(hp));
-#pragma unroll
-                            for (int g = 1; g < NGV; ++g) gN[g - 1][m] = __ldg(gp + 2 * (g % (LA + 1) * (LB + 1) + g / (LA + 1)) * gl);
-#pragma unroll
-                            for (int x = 1; x < NHV; ++x) hN[x - 1][m] = __ldg(hp + 2 * (x % (LC + 1) * (LD + 1) + x / (LC + 1)) * hl);
-                        }
-#pragma unroll
-                        for (int t = 0; t < NT; ++t) {
-                            const double tv = __ldg(R.T + ((long long)nn * nq + col[t]));
-                            tN[t] = n <= last ? tv : 0.0;
-                        }
-                        n += h4;
-                    };
-                    load();
-#pragma unroll 2
-                    for (int s = 0; s < steps; ++s) {
-                        double F[NCOMB][MT], Tb[NT];
-#pragma unroll
-                        for (int m = 0; m < MT; ++m) {
-#pragma unroll
-                            for (int cmb = 0; cmb < NCOMB; ++cmb) {
-                                const int gi = cmb % NGV, hi = cmb / NGV;
-                                if (gi == 0 && hi == 0) {
-                                    F[cmb][m] = g0N[m] * h0N[m] * cc[m];
-                                } else if (gi == 0) {
-                                    const double2 hv = hN[hi > 0 ? hi - 1 : 0][m];
-                                    F[cmb][m] = g0N[m] * (hv.x * cc[m] - hv.y * sc[m]);
-                                } else if (hi == 0) {
-                                    const double2 gv = gN[gi > 0 ? gi - 1 : 0][m];
-                                    F[cmb][m] = h0N[m] * (gv.x * cc[m] - gv.y * sc[m]);
-                                } else {
-                                    const double2 gv = gN[gi - 1][m], hv = hN[hi - 1][m];
-                                    const double ar = gv.x * hv.x - gv.y * hv.y, ai = gv.x * hv.y + gv.y * hv.x;
-                                    F[cmb][m] = ar * cc[m] - ai * sc[m];
-                                }
-                            }
-                        }
-#pragma unroll
-                        for (int t = 0; t < NT; ++t) Tb[t] = tN[t];
-                        load();
-                        if ((s & 7) == 7) {   // re-seed the recurrences
+                        for (int u = 0; u < US; ++u) {
+                            const int nn = min(n + u * h4, last);
 #pragma unroll
                             for (int m = 0; m < MT; ++m) {
-                                sincos((double)(n - 2 * h4) * phi[m], &sp[m], &cp[m]);
-                                sincos((double)(n - h4) * phi[m], &sc[m], &cc[m]);
+                                const double2 *gp = Gv + ((long long)nn * nppb + go[m]), *hp = Hv + ((long long)nn * nppk + ho[m]);
+                                g0N[u][m] = __ldg(G0 + ((long long)nn * nppb + go[m]));
+                                h0N[u][m] = __ldg(H0 + ((long long)nn * nppk + ho[m]));
+#pragma unroll
+                                for (int g = 1; g < NGV; ++g) gN[u][g - 1][m] = __ldg(gp + 2 * (g % (LA + 1) * (LB + 1) + g / (LA + 1)) * gl);
+#pragma unroll
+                                for (int x = 1; x < NHV; ++x) hN[u][x - 1][m] = __ldg(hp + 2 * (x % (LC + 1) * (LD + 1) + x / (LC + 1)) * hl);
                             }
-                        } else {
+#pragma unroll
+                            for (int t = 0; t < NT; ++t) tN[u][t] = __ldg(R.T + ((long long)nn * nq + col[t]));
+                        }
+                        if (s == 0) {
 #pragma unroll
                             for (int m = 0; m < MT; ++m) {
-                                const double tc_ = c4[m] * cc[m] - cp[m], ts_ = c4[m] * sc[m] - sp[m];
-                                cp[m] = cc[m];
-                                cc[m] = tc_;
-                                sp[m] = sc[m];
-                                sc[m] = ts_;
+                                const int src = (lane & ~3) | (c & 3);
+                                tce_phase_start(__shfl_sync(0xffffffffu, c1[m], src), __shfl_sync(0xffffffffu, s1[m], src), cq, cc[m],
+                                                sc[m], c4[m], s4[m]);
                             }
                         }
 #pragma unroll
-                        for (int t = 0; t < NT; ++t)
+                        for (int u = 0; u < US; ++u) {
+                            if (s + u >= steps) break;
+                            double F[NCOMB][MT];
 #pragma unroll
-                            for (int m = 0; m < MT; ++m)
+                            for (int m = 0; m < MT; ++m) {
+                                const bool in = n <= last;
 #pragma unroll
                                 for (int cmb = 0; cmb < NCOMB; ++cmb) {
-                                    const int x = (m * NT + t) * 2;
-                                    tce_dmma(acc[cmb][x], acc[cmb][x + 1], F[cmb][m], Tb[t]);
+                                    const int gi = cmb % NGV, hi = cmb / NGV;
+                                    double v;
+                                    if (gi == 0 && hi == 0) {
+                                        v = g0N[u][m] * h0N[u][m] * cc[m];
+                                    } else if (gi == 0) {
+                                        const double2 hv = hN[u][hi > 0 ? hi - 1 : 0][m];
+                                        v = g0N[u][m] * (hv.x * cc[m] - hv.y * sc[m]);
+                                    } else if (hi == 0) {
+                                        const double2 gv = gN[u][gi > 0 ? gi - 1 : 0][m];
+                                        v = h0N[u][m] * (gv.x * cc[m] - gv.y * sc[m]);
+                                    } else {
+                                        const double2 gv = gN[u][gi - 1][m], hv = hN[u][hi - 1][m];
+                                        const double ar = gv.x * hv.x - gv.y * hv.y, ai = gv.x * hv.y + gv.y * hv.x;
+                                        v = ar * cc[m] - ai * sc[m];
+                                    }
+                                    F[cmb][m] = in ? v : 0.0;
                                 }
+                                tce_phase_step(cc[m], sc[m], c4[m], s4[m]);
+                            }
+                            n += h4;
+#pragma unroll
+                            for (int t = 0; t < NT; ++t)
+#pragma unroll
+                                for (int m = 0; m < MT; ++m)
+#pragma unroll
+                                    for (int cmb = 0; cmb < NCOMB; ++cmb) {
+                                        const int x = (m * NT + t) * 2;
+                                        tce_dmma(acc[cmb][x], acc[cmb][x + 1], F[cmb][m], tN[u][t]);
+                                    }
+                        }
                     }
                     // epilogue: acc[cmb][2 (m NT + t) + i] = I_cmb[8 m + rq][8 (c NT + t) + 2 cq + i] / h
                     const double hw = (double)h;
@@ -613,7 +601,7 @@ template <int LA, int LB, int LC, int LD, int MT, int NT, bool LG>
 static void sp_tc_launch(const DevSys &S, const SArgs &A, int nsm, cudaStream_t st)
 {
     constexpr int ncq = (LA ? 3 : 1) * (LB ? 3 : 1) * (LC ? 3 : 1) * (LD ? 3 : 1);
-    tc_launch(k_quartets_sp_tc<LA, LB, LC, LD, MT, NT, LG>, S, A, nsm, st, ncq);
+    tc_launch(k_quartets_sp_tc<LA, LB, LC, LD, MT, NT, LG>, S, A, nsm, st, 8 * 2 * (size_t)ncq * 32 * sizeof(double));
 }
 
 // the classes with two p shells (tce_kernels_sp2.cu), as sp1_launch in tce_kernels_tc.cu

@@ -550,7 +550,8 @@ static bool lg_tc_available(const Handle *h, const Handle::LgList &w) { return l
 
 static int lg_tc_default(const Handle *h, const Handle::LgList &w)
 {
-    return lg_tc_available(h, w) ? 1 : 0;
+    if (!lg_tc_available(h, w)) return 0;
+    return w.kind == 1 ? tce_tc_shape_s(h->S) : w.kind == 2 ? tce_tc_shape_sp(h->S) : 1;
 }
 
 static int lg_tc(const Handle *h, const Handle::LgList &w)

@@ -82,17 +82,22 @@ __device__ __forceinline__ float tce_fold_phase(double phi)
     return fabsf((float)(t - rint(t))) * 6.2831853f;
 }
 
-// cos and sin of q phi and (4 - q) phi, q = 0..3, and 2 cos(4 phi), from
-// (c, s) = (cos phi, sin phi): the start of the three-term recurrence in steps of four
-__device__ __forceinline__ void tce_phase_start(double c, double s, int q, double &cc, double &sc, double &cm, double &sm,
-                                                double &c4)
+// e^{i q phi} (q = 0..3: a lane's first order) and e^{4 i phi} (the rotation per
+// step of four orders) from (c, s) = e^{i phi}, phi the stride's phase; cosines of
+// doubled angles by 1 - 2 sin^2
+__device__ __forceinline__ void tce_phase_start(double c, double s, int q, double &cc, double &sc, double &c4, double &s4)
 {
     const double c2 = fma(-2.0 * s, s, 1.0), s2 = 2.0 * s * c;
-    const double c3 = fma(c2, c, -s2 * s), s3 = fma(s2, c, c2 * s);
-    const double k4 = fma(-2.0 * s2, s2, 1.0), z4 = 2.0 * s2 * c2;
-    cc = q == 0 ? 1.0 : q == 1 ? c : q == 2 ? c2 : c3;
-    sc = q == 0 ? 0.0 : q == 1 ? s : q == 2 ? s2 : s3;
-    cm = q == 0 ? k4 : q == 1 ? c3 : q == 2 ? c2 : c;
-    sm = -(q == 0 ? z4 : q == 1 ? s3 : q == 2 ? s2 : s);
-    c4 = 2.0 * k4;
+    cc = q == 0 ? 1.0 : q == 1 ? c : q == 2 ? c2 : fma(c2, c, -s2 * s);
+    sc = q == 0 ? 0.0 : q == 1 ? s : q == 2 ? s2 : fma(s2, c, c2 * s);
+    c4 = fma(-2.0 * s2, s2, 1.0);
+    s4 = 2.0 * s2 * c2;
+}
+
+// the next step: one rounding per step, so errors grow linearly with the few steps taken
+__device__ __forceinline__ void tce_phase_step(double &cc, double &sc, double c4, double s4)
+{
+    const double t = cc;
+    cc = fma(t, c4, -sc * s4);
+    sc = fma(sc, c4, t * s4);
 }
