@@ -32,3 +32,24 @@ def test_ao_to_kmo_vs_restatement():
             assert got.shape == ref.shape
             assert np.abs(got - ref).max() <= 1e-10, np.abs(got - ref).max()
             assert np.abs(ref).max() > 1e-2
+
+
+@pytest.mark.parametrize("name,ncell,pr,qr", [("h2_ring", (9, 1, 1), (0, 1), (0, 1)), ("h_chain64", (5, 1, 1), (0, 2), (1, 6)),
+                                              ("li_cube", (2, 2, 1), (0, 1), (1, 3))])
+def test_ao_to_kmo_ragged_cells(systems, name, ncell, pr, qr):
+    """Cell counts that are no multiple of the kernels' k tiles, and more than
+    one periodic direction: 1e-12 of the largest element times the cells."""
+    from william_ci_b200.engine import Engine
+    ao = systems(name, ncell)
+    nf, N = ao.nfuc, int(np.prod(ncell))
+    rng = np.random.default_rng(11)
+    C = np.linalg.qr(rng.standard_normal((N, nf, nf)) + 1j * rng.standard_normal((N, nf, nf)))[0]
+    coeff = np.zeros((ao.nbas, ao.nbas), dtype=np.complex128)
+    for k in range(N):
+        coeff[k * nf:(k + 1) * nf, k * nf:(k + 1) * nf] = C[k]
+    with Engine(ao) as eng:
+        eri = eng.ERI_integral_toroidal()
+        for _ in range(2):      # the second call on the kept workspaces
+            got = eng.ao_to_kmo(C, pr, qr)
+            ref = kmo_ref.ao_to_kmo(eri, coeff, tuple(ncell), nf, pr[0] + 1, pr[1], qr[0] + 1, qr[1])
+            assert np.abs(got - ref).max() <= 1e-12 * N * max(1.0, np.abs(ref).max())

@@ -62,6 +62,8 @@ struct Handle {
     double *d_eri = nullptr;
     long long eri_elems = 0;
     int eri_size = 0;
+    double2 *d_kmo[5] = {};              // tce_ao_to_kmo: phases, coefficients, X1 / S, X2, output
+    size_t n_kmo[5] = {};
     double *d_blk = nullptr;
     long long *d_blkoff = nullptr;
     int4 *d_one = nullptr;

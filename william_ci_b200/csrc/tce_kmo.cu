@@ -3,13 +3,17 @@
 //   ERI_out(p, q, r, s, k1, k2, k3) = (p k1, q k2 | r k3, s k4),
 //   k4 = k1 - k2 + k3, p, r in p_lo..p_hi, q, s in q_lo..q_hi.
 // The handle's stored integrals ERI(a, j2, j3, j4) (tce_eri_stored with
-// eri_size = nfuc, chemist order) stay on the device; per k4:
+// eri_size = nfuc, chemist order) stay on the device; per group of up to KMO_G k4:
 //   k_kmo_x1: X1(a, j2, j3, d)    = sum_R4 ERI(a, j2, j3, d R4) e^{+i k4 R4}
 //   k_kmo_x2: X2(a, j2, c, d, k3) = sum_R3 X1(a, j2, c R3, d) e^{-i k3 R3}
-//   k_kmo_q : one block per (k1, k2), k3 = k4 - k1 + k2:
-//             S(a, b, c, d) = 1/N sum_R2 X2(a, b R2, c, d, k3) e^{+i k2 R2}
-//             and the four quarter transforms with the k-block coefficients
+//   k_kmo_x3: S(a, b, c, d, k2, k3) = 1/N sum_R2 X2(a, b R2, c, d, k3) e^{+i k2 R2}
+//   k_kmo_q : one block per (k1, k2), k3 = k4 - k1 + k2: the four quarter
+//             transforms with the k-block coefficients
 //             C_k(a, p) = coeff_SAO(k nfuc + a, k nfuc + p), in shared memory.
+// The three sums over cells read every input once per KMO_T (x1: KMO_G) values of
+// k, phases as shared-memory broadcasts; reading it once per k they moved N
+// times the stored integrals, X1 and X2.  The groups follow each other on one
+// stream without waiting for the host, and the workspaces stay with the handle.
 #include <vector>
 
 #include "tce_handle.h"
@@ -24,77 +28,137 @@ __device__ __forceinline__ void kadd(double2 &s, double2 v)
     s.y += v.y;
 }
 
-__global__ void k_kmo_x1(int nf, int nbas, int N, int k4, const double *eri, const double2 *ph, double2 *X1)
+constexpr int KMO_G = 4;    // k4 values per group
+constexpr int KMO_T = 8;    // k values per thread of the other two sums
+
+constexpr int KMO_R = 128;  // cells per shared-memory tile of phases
+
+// ph[k0 + j][r0 + R], j < T, R < KMO_R, into shared memory (zero past N)
+template <int T>
+__device__ __forceinline__ void kmo_phases(const double2 *__restrict__ ph, int k0, int r0, int N, double2 *sp)
 {
-    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // a + nf (j2 + nbas (j3 + nbas d))
-    const long long n = (long long)nf * nbas * nbas * nf;
-    if (id >= n) return;
-    const long long abc = id % ((long long)nf * nbas * nbas);
-    const int d = (int)(id / ((long long)nf * nbas * nbas));
-    const long long slab = (long long)nf * nbas * nbas;
-    double2 s = make_double2(0.0, 0.0);
-    for (int r = 0; r < N; ++r) {
-        const double v = eri[(size_t)abc + (size_t)slab * (d + (size_t)r * nf)];
-        const double2 e = ph[(size_t)k4 * N + r];
-        s.x += v * e.x;
-        s.y += v * e.y;
+    __syncthreads();
+    for (int x = threadIdx.x; x < T * KMO_R; x += blockDim.x) {
+        const int j = x % T, R = r0 + x / T;
+        sp[x] = k0 + j < N && R < N ? ph[(size_t)(k0 + j) * N + R] : make_double2(0.0, 0.0);
     }
-    X1[id] = s;
+    __syncthreads();
 }
 
-__global__ void k_kmo_x2(int nf, int nbas, int N, const double2 *ph, const double2 *X1, double2 *X2)
+__global__ void k_kmo_x1(int nf, int nbas, int N, int k4, int ng, const double *__restrict__ eri, const double2 *__restrict__ ph,
+                         double2 *X1)
 {
+    __shared__ double2 sq[KMO_G * KMO_R];
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // a + nf (j2 + nbas (j3 + nbas d))
+    const long long slab = (long long)nf * nbas * nbas, n = slab * nf;
+    const long long abc = id % slab;
+    const int d = (int)(id / slab);
+    double2 s[KMO_G];
+#pragma unroll
+    for (int j = 0; j < KMO_G; ++j) s[j] = make_double2(0.0, 0.0);
+    for (int r0 = 0; r0 < N; r0 += KMO_R) {
+        kmo_phases<KMO_G>(ph, k4, r0, N, sq);
+        for (int r = r0; id < n && r < min(N, r0 + KMO_R); ++r) {
+            const double v = eri[(size_t)abc + (size_t)slab * (d + (size_t)r * nf)];
+#pragma unroll
+            for (int j = 0; j < KMO_G; ++j) {
+                const double2 e = sq[(r - r0) * KMO_G + j];
+                s[j].x = fma(v, e.x, s[j].x);
+                s[j].y = fma(v, e.y, s[j].y);
+            }
+        }
+    }
+    if (id >= n) return;
+#pragma unroll
+    for (int j = 0; j < KMO_G; ++j)
+        if (j < ng) X1[(size_t)n * j + id] = s[j];
+}
+
+// blockIdx.y: k3 tile, blockIdx.z: k4 of the group
+__global__ void k_kmo_x2(int nf, int nbas, int N, const double2 *__restrict__ ph, const double2 *__restrict__ X1, double2 *X2)
+{
+    __shared__ double2 sq[KMO_T * KMO_R];
+    const int k0 = blockIdx.y * KMO_T;
     // X2 index: a + nf (j2 + nbas (c + nf (d + nf k3)))
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    const long long aj = (long long)nf * nbas;
-    const long long n = aj * nf * nf * N;
-    if (id >= n) return;
-    const long long a2 = id % aj;
-    long long rest = id / aj;
-    const int c = (int)(rest % nf);
-    rest /= nf;
-    const int d = (int)(rest % nf);
-    const int k3 = (int)(rest / nf);
-    double2 s = make_double2(0.0, 0.0);
-    for (int r = 0; r < N; ++r) {
-        const double2 x = X1[(size_t)a2 + (size_t)aj * ((c + (size_t)r * nf) + (size_t)nbas * d)];
-        kadd(s, kmul(x, kconj(ph[(size_t)k3 * N + r])));
+    const long long aj = (long long)nf * nbas, n = aj * nf * nf;
+    X1 += (size_t)aj * nbas * nf * blockIdx.z;
+    X2 += (size_t)n * N * blockIdx.z;
+    const long long a2 = id % aj, cd = id / aj;
+    const int c = (int)(cd % nf), d = (int)(cd / nf);
+    double2 s[KMO_T];
+#pragma unroll
+    for (int j = 0; j < KMO_T; ++j) s[j] = make_double2(0.0, 0.0);
+    for (int r0 = 0; r0 < N; r0 += KMO_R) {
+        kmo_phases<KMO_T>(ph, k0, r0, N, sq);
+        for (int r = r0; id < n && r < min(N, r0 + KMO_R); ++r) {
+            const double2 x = X1[(size_t)a2 + (size_t)aj * ((c + (size_t)r * nf) + (size_t)nbas * d)];
+#pragma unroll
+            for (int j = 0; j < KMO_T; ++j) kadd(s[j], kmul(x, kconj(sq[(r - r0) * KMO_T + j])));
+        }
     }
-    X2[id] = s;
+    if (id >= n) return;
+#pragma unroll
+    for (int j = 0; j < KMO_T; ++j)
+        if (k0 + j < N) X2[(size_t)id + (size_t)n * (k0 + j)] = s[j];
+}
+
+// S(a, b, c, d; k2, k3), (a, b, c, d) fastest; blockIdx.y: k2 tile, blockIdx.z: k4 of the group
+__global__ void k_kmo_x3(int nf, int nbas, int N, const double2 *__restrict__ ph, const double2 *__restrict__ X2, double2 *Sk)
+{
+    __shared__ double2 sq[KMO_T * KMO_R];
+    const int k0 = blockIdx.y * KMO_T;
+    const long long aj = (long long)nf * nbas, n = (long long)nf * nf * nf * nf;   // per (k2, k3)
+    const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;         // (a, b, c, d) + n k3
+    X2 += (size_t)aj * nf * nf * N * blockIdx.z;
+    Sk += (size_t)n * N * N * blockIdx.z;
+    const int ab = (int)(id % (nf * nf));
+    const long long cdk = id / (nf * nf);                                          // c + nf (d + nf k3)
+    const double2 *x2 = X2 + ab + (size_t)aj * cdk;
+    double2 s[KMO_T];
+#pragma unroll
+    for (int j = 0; j < KMO_T; ++j) s[j] = make_double2(0.0, 0.0);
+    for (int r0 = 0; r0 < N; r0 += KMO_R) {
+        kmo_phases<KMO_T>(ph, k0, r0, N, sq);
+        for (int r = r0; id < n * N && r < min(N, r0 + KMO_R); ++r) {
+            const double2 x = x2[(size_t)nf * nf * r];
+#pragma unroll
+            for (int j = 0; j < KMO_T; ++j) kadd(s[j], kmul(x, sq[(r - r0) * KMO_T + j]));
+        }
+    }
+    if (id >= n * N) return;
+    const double invN = 1.0 / (double)N;
+    const long long abcd = id % n, k3 = id / n;
+#pragma unroll
+    for (int j = 0; j < KMO_T; ++j)
+        if (k0 + j < N) Sk[(size_t)abcd + (size_t)n * ((k0 + j) + (size_t)N * k3)] = make_double2(s[j].x * invN, s[j].y * invN);
 }
 
 struct KmoArgs {
-    int nf, nbas, N, no, nv, p0, q0, k4;
-    const int *k3of;        // [k1 N + k2]
-    const double2 *ph, *X2, *C;   // C: coeff_SAO (nbas x nbas), column-major
+    int nf, nbas, N, no, nv, p0, q0, k4, n0, n1, n2;
+    const double2 *Sk, *C;   // C: coeff_SAO (nbas x nbas), column-major
     double2 *out;           // (no, nv, no, nv, N, N, N)
 };
 
+// blockIdx.y: k4 of the group
 __global__ void k_kmo_q(KmoArgs A)
 {
     extern __shared__ double2 sq[];
     const int nf = A.nf, N = A.N, no = A.no, nv = A.nv, nbas = A.nbas;
-    const int k1 = blockIdx.x / N, k2 = blockIdx.x % N, k4 = A.k4;
-    const int k3 = A.k3of[k1 * N + k2];
+    const int k1 = blockIdx.x / N, k2 = blockIdx.x % N, k4 = A.k4 + blockIdx.y;
+    auto wrap = [](int c, int n) { return (c % n + n) % n; };
+    const int k3 = wrap(k4 % A.n0 - k1 % A.n0 + k2 % A.n0, A.n0) +
+                   A.n0 * (wrap((k4 / A.n0) % A.n1 - (k1 / A.n0) % A.n1 + (k2 / A.n0) % A.n1, A.n1) +
+                           A.n1 * wrap(k4 / (A.n0 * A.n1) - k1 / (A.n0 * A.n1) + k2 / (A.n0 * A.n1), A.n2));
     const int f2 = nf * nf, f3 = f2 * nf, f4 = f3 * nf;
     double2 *S = sq;                    // (a, b, c, d)
     double2 *T4 = S + f4;               // (a, b, c, s)
     double2 *T3 = T4 + f3 * nv;         // (a, b, r, s)
     double2 *T2 = T3 + f2 * no * nv;    // (a, q, r, s)
     const int t = threadIdx.x, nt = blockDim.x;
-    const double invN = 1.0 / (double)N;
-    const long long aj = (long long)nf * nbas;
     auto C = [&](int k, int a, int p) { return A.C[(size_t)(k * nf + a) + (size_t)nbas * (k * nf + p)]; };
-    for (int x = t; x < f4; x += nt) {   // x = a + nf (b + nf (c + nf d))
-        const int a = x % nf, b = (x / nf) % nf, c = (x / f2) % nf, d = x / f3;
-        double2 s = make_double2(0.0, 0.0);
-        for (int r = 0; r < N; ++r) {
-            const double2 v = A.X2[(size_t)(a + (long long)nf * (b + (long long)r * nf)) +
-                                   (size_t)aj * (c + (size_t)nf * (d + (size_t)nf * k3))];
-            kadd(s, kmul(v, A.ph[(size_t)k2 * N + r]));
-        }
-        S[x] = make_double2(s.x * invN, s.y * invN);
-    }
+    const double2 *Sg = A.Sk + (size_t)f4 * (k2 + (size_t)N * (k3 + (size_t)N * blockIdx.y));
+    for (int x = t; x < f4; x += nt) S[x] = Sg[x];
     __syncthreads();
     for (int x = t; x < f3 * nv; x += nt) {   // 4th index d -> s
         const int abc = x % f3, s = x / f3;
@@ -145,7 +209,7 @@ extern "C" int tce_ao_to_kmo(void *handle, const double *coeff, int32_t p_lo, in
     const size_t smem = sizeof(double2) * ((size_t)nf * nf * nf * nf + (size_t)nf * nf * nf * nv +
                                            (size_t)nf * nf * no * nv + (size_t)nf * nv * no * nv);
     if (smem > 200 * 1024) return fail(h, TCE_ERR_UNSUPPORTED, "nfuc too large for the quarter-transform kernel");
-    // cell coordinates (x fastest), phases, k3 = k4 - k1 + k2 per k4
+    // phases (cells x fastest)
     std::vector<int> cx(N), cy(N), cz(N);
     for (int k = 0; k < N; ++k) {
         cx[k] = k % h->ncl[0];
@@ -159,52 +223,52 @@ extern "C" int tce_ao_to_kmo(void *handle, const double *coeff, int32_t p_lo, in
                                           (double)cz[k] * cz[r] / h->ncl[2]);
             ph[(size_t)k * N + r] = make_double2(std::cos(th), std::sin(th));
         }
-    auto cell = [&](int x, int y, int z) {
-        x = ((x % h->ncl[0]) + h->ncl[0]) % h->ncl[0];
-        y = ((y % h->ncl[1]) + h->ncl[1]) % h->ncl[1];
-        z = ((z % h->ncl[2]) + h->ncl[2]) % h->ncl[2];
-        return x + h->ncl[0] * (y + h->ncl[1] * z);
+    const size_t f4 = (size_t)nf * nf * nf * nf;
+    const size_t n1 = (size_t)nf * nbas * nbas * nf, n2 = (size_t)nf * nbas * nf * nf * N, n3 = f4 * N * N;
+    const size_t nout = (size_t)no * nv * no * nv * N * N * N, nC = (size_t)nbas * nbas, nph = (size_t)N * N;
+    // k4 per group: what a gigabyte of buffers takes (S shares X1's), at least one;
+    // one at a time also where the device has no room for more
+    const double keep = 1e9;
+    int G = std::min(KMO_G, N), s = TCE_OK;
+    while (G > 1 && (double)G * (std::max(n1, n3) + n2) * sizeof(double2) > keep) --G;
+    auto release = [&]() {
+        for (int i = 0; i < 5; ++i) {
+            dfree(h, h->d_kmo[i]);
+            h->d_kmo[i] = nullptr;
+            h->n_kmo[i] = 0;
+        }
     };
-    std::vector<double2> Ch((size_t)nbas * nbas);
-    for (size_t i = 0; i < Ch.size(); ++i) Ch[i] = make_double2(coeff[2 * i], coeff[2 * i + 1]);
-    const size_t n1 = (size_t)nf * nbas * nbas * nf, n2 = (size_t)nf * nbas * nf * nf * N;
-    const size_t nout = (size_t)no * nv * no * nv * N * N * N;
-    double2 *d_ph = nullptr, *d_C = nullptr, *d_X1 = nullptr, *d_X2 = nullptr, *d_out = nullptr;
-    int *d_k3 = nullptr;
-    int s;
-    auto cleanup = [&]() {
-        dfree(h, d_ph);
-        dfree(h, d_C);
-        dfree(h, d_X1);
-        dfree(h, d_X2);
-        dfree(h, d_out);
-        dfree(h, d_k3);
-    };
-    if ((s = upload(h, &d_ph, ph)) || (s = upload(h, &d_C, Ch)) || (s = dalloc(h, &d_X1, n1)) ||
-        (s = dalloc(h, &d_X2, n2)) || (s = dalloc(h, &d_out, nout)) || (s = dalloc(h, &d_k3, (size_t)N * N))) {
-        cleanup();
-        return s;
+    for (;;) {
+        const size_t need[5] = {nph, nC, G * std::max(n1, n3), G * n2, nout};
+        s = TCE_OK;
+        for (int i = 0; i < 5 && s == TCE_OK; ++i) {   // workspaces grow with the largest call and stay with the handle
+            if (h->n_kmo[i] >= need[i]) continue;
+            dfree(h, h->d_kmo[i]);
+            h->d_kmo[i] = nullptr;
+            h->n_kmo[i] = 0;
+            if ((s = dalloc(h, &h->d_kmo[i], need[i])) == TCE_OK) h->n_kmo[i] = need[i];
+        }
+        if (s == TCE_OK) break;
+        release();
+        if (G == 1) return s;
+        G = 1;
     }
-    std::vector<int> k3of((size_t)N * N);
-    cudaFuncSetAttribute(k_kmo_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    cudaError_t e = cudaSuccess;
-    for (int k4 = 0; k4 < N && e == cudaSuccess; ++k4) {
-        for (int k1 = 0; k1 < N; ++k1)
-            for (int k2 = 0; k2 < N; ++k2)
-                k3of[(size_t)k1 * N + k2] = cell(cx[k4] - cx[k1] + cx[k2], cy[k4] - cy[k1] + cy[k2], cz[k4] - cz[k1] + cz[k2]);
-        e = cudaMemcpyAsync(d_k3, k3of.data(), sizeof(int) * k3of.size(), cudaMemcpyHostToDevice, h->st);
-        if (e != cudaSuccess) break;
-        k_kmo_x1<<<(unsigned)((n1 + 255) / 256), 256, 0, h->st>>>(nf, nbas, N, k4, h->d_eri, d_ph, d_X1);
-        k_kmo_x2<<<(unsigned)((n2 + 255) / 256), 256, 0, h->st>>>(nf, nbas, N, d_ph, d_X1, d_X2);
-        KmoArgs A{nf, nbas, N, no, nv, p_lo - 1, q_lo - 1, k4, d_k3, d_ph, d_X2, d_C, d_out};
-        k_kmo_q<<<(unsigned)(N * N), 256, smem, h->st>>>(A);
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);   // k3of is reused
+    double2 *d_ph = h->d_kmo[0], *d_C = h->d_kmo[1], *d_X1 = h->d_kmo[2], *d_X2 = h->d_kmo[3], *d_out = h->d_kmo[4];
+    CK(h, cudaMemcpyAsync(d_ph, ph.data(), sizeof(double2) * nph, cudaMemcpyHostToDevice, h->st));
+    CK(h, cudaMemcpyAsync(d_C, coeff, sizeof(double2) * nC, cudaMemcpyHostToDevice, h->st));
+    CK(h, cudaFuncSetAttribute(k_kmo_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const unsigned tiles = (unsigned)((N + KMO_T - 1) / KMO_T);
+    for (int k4 = 0; k4 < N; k4 += G) {
+        const int ng = std::min(G, N - k4);
+        k_kmo_x1<<<(unsigned)((n1 + 255) / 256), 256, 0, h->st>>>(nf, nbas, N, k4, ng, h->d_eri, d_ph, d_X1);
+        k_kmo_x2<<<dim3((unsigned)((n2 / N + 127) / 128), tiles, ng), 128, 0, h->st>>>(nf, nbas, N, d_ph, d_X1, d_X2);
+        k_kmo_x3<<<dim3((unsigned)((f4 * N + 127) / 128), tiles, ng), 128, 0, h->st>>>(nf, nbas, N, d_ph, d_X2, d_X1);
+        KmoArgs A{nf, nbas, N, no, nv, p_lo - 1, q_lo - 1, k4, h->ncl[0], h->ncl[1], h->ncl[2], d_X1, d_C, d_out};
+        k_kmo_q<<<dim3((unsigned)(N * N), ng), 256, smem, h->st>>>(A);
+        CK(h, cudaGetLastError());
     }
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, d_out, sizeof(double2) * nout, cudaMemcpyDeviceToHost, h->st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-    cleanup();
-    if (e != cudaSuccess) return fail(h, TCE_ERR_CUDA, std::string("tce_ao_to_kmo: ") + cudaGetErrorString(e));
+    CK(h, cudaMemcpyAsync(out, d_out, sizeof(double2) * nout, cudaMemcpyDeviceToHost, h->st));
+    CK(h, cudaStreamSynchronize(h->st));
+    if ((double)(h->n_kmo[2] + h->n_kmo[3] + h->n_kmo[4]) * sizeof(double2) > keep) release();   // large ones are given back
     return TCE_OK;
 }

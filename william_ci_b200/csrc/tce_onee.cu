@@ -533,18 +533,14 @@ extern "C" int tce_nuclear_attraction(void *handle, int32_t natoms, const double
     if (s) return s;
     // rows of the unit cell, the rest by translation (fill_with_symmetry)
     const int nx = h->ncl[0], ny = h->ncl[1], nz = h->ncl[2];
-    for (int i = 0; i < nbas; ++i) {
-        const int Ri = i / nfuc, a = i % nfuc;
-        const int Rxi = Ri % nx, Ryi = (Ri / nx) % ny, Rzi = Ri / (nx * ny);
-        for (int j = 0; j < nbas; ++j) {
-            const int Rj = j / nfuc, b = j % nfuc;
-            const int Rxj = Rj % nx, Ryj = (Rj / nx) % ny, Rzj = Rj / (nx * ny);
-            const int dx = ((Rxj - Rxi) % nx + nx) % nx, dy = ((Ryj - Ryi) % ny + ny) % ny;
-            const int dz = ((Rzj - Rzi) % nz + nz) % nz;
-            const int src = (dz * ny + dy) * nx + dx;
-            V[i + (size_t)nbas * j] = rows[a + (size_t)nfuc * (b + (size_t)src * nfuc)];
+    for (int Rj = 0; Rj < nbas / nfuc; ++Rj)
+        for (int Ri = 0; Ri < nbas / nfuc; ++Ri) {   // one cell block at a time: its source cell is the same for all of it
+            const int dx = (Rj % nx - Ri % nx + nx) % nx, dy = ((Rj / nx) % ny - (Ri / nx) % ny + ny) % ny;
+            const int dz = (Rj / (nx * ny) - Ri / (nx * ny) + nz) % nz;
+            const double *src = rows.data() + (size_t)nfuc * nfuc * ((size_t)(dz * ny + dy) * nx + dx);
+            for (int b = 0; b < nfuc; ++b)
+                std::copy(src + (size_t)nfuc * b, src + (size_t)nfuc * (b + 1), V + (size_t)Ri * nfuc + (size_t)nbas * (Rj * nfuc + b));
         }
-    }
     return TCE_OK;
 }
 
