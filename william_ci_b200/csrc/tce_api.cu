@@ -221,6 +221,7 @@ int run_blocks(Handle *h, const std::vector<int4> &items, const std::vector<int>
     a.max_ncq = h->max_ncq;
     a.fixed_gmax = h->d_gmax;
     a.num_sms = h->num_sms;
+    a.use_tc = !h->blocks_only;
     CKS(h, tce_launch_quartets(h->S, a, h->st));
     if (blocks) {
         blocks->resize(off.back());
@@ -513,7 +514,7 @@ int build(Handle *h, const tce_system *sys)
         int stride = h->ncap + 2 * TCE_LMAX + 2;
         double *scr = nullptr;
         if ((s = dalloc(h, &scr, (size_t)npp_tot * h->ndp * stride))) return s;
-        CKS(h, tce_launch_pair_vectors(S, npp_tot, d_ppu, h->d_pp, stride, scr, d_vec, d_rvec, h->st));
+        CKS(h, tce_launch_pair_vectors(S, npp_tot, d_ppu, h->d_pp, stride, scr, d_vec, d_rvec, !h->blocks_only, h->st));
         CK(h, cudaStreamSynchronize(h->st));
         dfree(h, scr);
     }

@@ -209,12 +209,14 @@ __global__ void k_df_bh(const double2 *__restrict__ W, const double2 *__restrict
 // of once per k: the one-output-per-thread form read each of them N times from the
 // L2.  96 cells: G1 413 and F 976 us before.
 constexpr int DF_KT = 8;
-// ph[k0 + j][R] of the block's DF_KT values of k into shared memory (zero past N)
-__device__ __forceinline__ void df_phases(const double2 *__restrict__ ph, int k0, int N, double2 *sp)
+constexpr int DF_R = 128;   // cells per shared-memory tile of phases
+// ph[k0 + j][r0 + R], R < DF_R, of the block's DF_KT values of k into shared memory (zero past N)
+__device__ __forceinline__ void df_phases(const double2 *__restrict__ ph, int k0, int r0, int N, double2 *sp)
 {
-    for (int x = threadIdx.x; x < DF_KT * N; x += blockDim.x) {
-        const int j = x % DF_KT, R = x / DF_KT;
-        sp[x] = k0 + j < N ? ph[(long long)(k0 + j) * N + R] : make_double2(0.0, 0.0);
+    __syncthreads();
+    for (int x = threadIdx.x; x < DF_KT * DF_R; x += blockDim.x) {
+        const int j = x % DF_KT, R = r0 + x / DF_KT;
+        sp[x] = k0 + j < N && R < N ? ph[(long long)(k0 + j) * N + R] : make_double2(0.0, 0.0);
     }
     __syncthreads();
 }
@@ -223,23 +225,25 @@ __device__ __forceinline__ void df_phases(const double2 *__restrict__ ph, int k0
 __global__ void k_df_g1(const double *__restrict__ B, const double2 *__restrict__ ph, long long X, int N, int nau,
                         double2 *G1)
 {
-    extern __shared__ double2 sp[];
+    __shared__ double2 sp[DF_KT * DF_R];
     const int k0 = blockIdx.y * DF_KT;
-    df_phases(ph, k0, N, sp);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // x + X q
-    if (t >= X * nau) return;
     double re[DF_KT], im[DF_KT];
 #pragma unroll
     for (int j = 0; j < DF_KT; ++j) re[j] = im[j] = 0.0;
-    for (int s = 0; s < N; ++s) {
-        const double b = B[t + X * nau * s];
+    for (int r0 = 0; r0 < N; r0 += DF_R) {
+        df_phases(ph, k0, r0, N, sp);
+        for (int s = r0; t < X * nau && s < min(N, r0 + DF_R); ++s) {
+            const double b = B[t + X * nau * s];
 #pragma unroll
-        for (int j = 0; j < DF_KT; ++j) {
-            const double2 e = sp[s * DF_KT + j];
-            re[j] = fma(b, e.x, re[j]);
-            im[j] = fma(-b, e.y, im[j]);
+            for (int j = 0; j < DF_KT; ++j) {
+                const double2 e = sp[(s - r0) * DF_KT + j];
+                re[j] = fma(b, e.x, re[j]);
+                im[j] = fma(-b, e.y, im[j]);
+            }
         }
     }
+    if (t >= X * nau) return;
 #pragma unroll
     for (int j = 0; j < DF_KT; ++j)
         if (k0 + j < N) G1[t + X * nau * (k0 + j)] = make_double2(re[j], im[j]);
@@ -249,26 +253,28 @@ __global__ void k_df_g1(const double *__restrict__ B, const double2 *__restrict_
 __global__ void k_df_f(const double2 *__restrict__ G1, const double2 *__restrict__ ph, long long X, int N, int nf,
                        int nau, double2 *F)
 {
-    extern __shared__ double2 sp[];
+    __shared__ double2 sp[DF_KT * DF_R];
     const int k0 = blockIdx.y * DF_KT;
-    df_phases(ph, k0, N, sp);
     const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;   // a + nf (b + nf (q + nau kap))
     const long long tot = (long long)nf * nf * nau * N;
-    if (t >= tot) return;
     const int nf2 = nf * nf, ab = (int)(t % nf2);
     const double2 *g = G1 + (t / nf2) * X + ab;          // (kap nau + q) X + a + nf b, + nf^2 R
     double re[DF_KT], im[DF_KT];
 #pragma unroll
     for (int j = 0; j < DF_KT; ++j) re[j] = im[j] = 0.0;
-    for (int R = 0; R < N; ++R) {
-        const double2 v = g[(long long)nf2 * R];
+    for (int r0 = 0; r0 < N; r0 += DF_R) {
+        df_phases(ph, k0, r0, N, sp);
+        for (int R = r0; t < tot && R < min(N, r0 + DF_R); ++R) {
+            const double2 v = g[(long long)nf2 * R];
 #pragma unroll
-        for (int j = 0; j < DF_KT; ++j) {
-            const double2 e = sp[R * DF_KT + j];
-            re[j] = fma(v.x, e.x, fma(-v.y, e.y, re[j]));
-            im[j] = fma(v.x, e.y, fma(v.y, e.x, im[j]));
+            for (int j = 0; j < DF_KT; ++j) {
+                const double2 e = sp[(R - r0) * DF_KT + j];
+                re[j] = fma(v.x, e.x, fma(-v.y, e.y, re[j]));
+                im[j] = fma(v.x, e.y, fma(v.y, e.x, im[j]));
+            }
         }
     }
+    if (t >= tot) return;
 #pragma unroll
     for (int j = 0; j < DF_KT; ++j)
         if (k0 + j < N) F[t + tot * (k0 + j)] = make_double2(re[j], im[j]);
@@ -438,6 +444,10 @@ int device_blocks(DfHandle *d, Handle *h, const std::vector<int4> &items, double
     a.max_ncq = std::max(mq, 1);
     a.fixed_gmax = h->d_gmax;
     a.num_sms = h->num_sms;
+    // every order, on the vectors the d_k sums give (tce_create_blocks): the metric's
+    // factorisation magnifies a rounding of the integrals some 1e4 times, so that
+    // equally good integrals move the fitted energy by 1e-8
+    a.use_tc = 0;
     if (tce_launch_quartets(h->S, a, d->st) != TCE_OK)
         return df_fail(d, TCE_ERR_CUDA, std::string("fit integrals: ") + cudaGetErrorString(cudaGetLastError()));
     DCK(d, cudaStreamSynchronize(d->st));
@@ -768,7 +778,7 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     const int no = ohi, nv = nf - vlo;
     if (no < 1 || nv < 1) return df_fail(d, TCE_ERR_ARG, "no occupied or no virtual bands");
     int s;
-    // workspaces kept with the handle: G1 and the L vectors share one buffer (L after G1 is read)
+    // workspaces kept with the handle up to a gigabyte: G1 and the L vectors share one buffer (L after G1 is read)
     const long long nG1 = X * nau * N, nF = (long long)nf * nf * nau * N * N, nL = (long long)no * nv * nau * N * N;
     const size_t need1 = (size_t)std::max(nG1, nL);
     if (d->n_ws1 < need1) {
@@ -782,16 +792,10 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     if (!d->d_wsC && (s = df_alloc(d, &d->d_wsC, (size_t)nbas * nbas))) return s;
     double2 *d_G1 = d->d_ws1, *d_F = d->d_wsF, *d_C = d->d_wsC, *d_L = d->d_ws1;
     const dim3 tiles(1, (unsigned)((N + DF_KT - 1) / DF_KT));
-    const size_t psm = sizeof(double2) * DF_KT * (size_t)N;
-    if (psm > 200 * 1024) return df_fail(d, TCE_ERR_UNSUPPORTED, "too many cells for the phase tiles");
-    if (psm > 48 * 1024) {
-        DCK(d, cudaFuncSetAttribute(k_df_g1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-        DCK(d, cudaFuncSetAttribute(k_df_f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-    }
     DCK(d, cudaMemcpyAsync(d_C, coeff, sizeof(double2) * nbas * nbas, cudaMemcpyHostToDevice, d->st));
-    k_df_g1<<<dim3(nblk(X * nau, 128), tiles.y), 128, psm, d->st>>>(d->d_B, d->d_ph, X, N, nau, d_G1);
+    k_df_g1<<<dim3(nblk(X * nau, 128), tiles.y), 128, 0, d->st>>>(d->d_B, d->d_ph, X, N, nau, d_G1);
     DCK(d, cudaGetLastError());
-    k_df_f<<<dim3(nblk((long long)nf * nf * nau * N, 128), tiles.y), 128, psm, d->st>>>(d_G1, d->d_ph, X, N, nf, nau, d_F);
+    k_df_f<<<dim3(nblk((long long)nf * nf * nau * N, 128), tiles.y), 128, 0, d->st>>>(d_G1, d->d_ph, X, N, nf, nau, d_F);
     DCK(d, cudaGetLastError());
     k_df_l<<<nblk(nL, 256), 256, 0, d->st>>>(d_F, d_C, d->d_crd, d->ncl[0], d->ncl[1], d->ncl[2], N, nf, nau, 0, no,
                                              vlo, nv, d_L);
@@ -817,6 +821,12 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     double gz = 0.0, ms = 0.0;
     s = tce_mp2_energy_on(N, d->ncl, crd.data(), no, nv, nau, reinterpret_cast<const double *>(d_L), true, eo.data(), oo.data(), ev.data(), ov.data(),
                          mode, &a2d, &a2x, &nz, &gz, &ms);
+    if ((double)(d->n_ws1 + (size_t)nF) * sizeof(double2) > 1e9) {   // large ones are given back
+        df_free(d, d->d_ws1);
+        df_free(d, d->d_wsF);
+        d->d_ws1 = d->d_wsF = nullptr;
+        d->n_ws1 = 0;
+    }
     if (s) return df_fail(d, s, std::string("contraction: ") + tce_mp2_last_error());
     *e_mp2 = 2.0 * a2d - a2x;
     if (e2d) *e2d = a2d;

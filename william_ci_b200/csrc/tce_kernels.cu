@@ -173,7 +173,7 @@ __global__ void k_pair_bessel(DevSys S, long long npp_tot, const int *pp_unit, c
 // one thread per (pp, d, ia, ib, sign): V_n = sum_k d_k I~_{|n - s k|}, n < Nlen
 // (zero beyond the pair's own N), written n-major into the unit pair's slab.
 __global__ void k_pair_vectors(DevSys S, long long npp_tot, const int *pp_unit, const PairPrim *pp, int stride,
-                               const double *scratch, double2 *vec, double *rvec)
+                               const double *scratch, double2 *vec, double *rvec, bool by_parts)
 {
     const int NV = (TCE_LMAX + 1) * (TCE_LMAX + 1) * 2;
     long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -194,7 +194,7 @@ __global__ void k_pair_vectors(DevSys S, long long npp_tot, const int *pp_unit, 
                    ((((long long)d * (U.l1 + 1) + ia) * (U.l2 + 1) + ib) * 2 + s) * (long long)U.Nlen * U.npp;
     double dre[4 * TCE_LMAX + 1], dim[4 * TCE_LMAX + 1];
     PowerSeries ps;
-    const bool parts = M > 0 && P.A[d] >= 4.0;   // below, d_k sums lose at most 2^M
+    const bool parts = by_parts && M > 0 && P.A[d] >= 4.0;   // below, d_k sums lose at most 2^M
     if (M > 0) {
         const double *r1 = S.sh_r + 3 * U.S1, *r2 = S.sh_r + 3 * U.S2;
         const double phA = S.a[d] * (P.cen[d] - r1[d]), phB = S.a[d] * (P.cen[d] - r2[d]);
@@ -489,14 +489,14 @@ int tce_launch_pair_scalars(const DevSys &S, long long npp_tot, const int *pp_un
 }
 
 int tce_launch_pair_vectors(const DevSys &S, long long npp_tot, const int *pp_unit, const PairPrim *pp, int stride,
-                            double *scratch, double2 *vec, double *rvec, cudaStream_t st)
+                            double *scratch, double2 *vec, double *rvec, bool by_parts, cudaStream_t st)
 {
     if (npp_tot == 0) return TCE_OK;
     long long n1 = npp_tot * S.ndp;
     k_pair_bessel<<<(unsigned)((n1 + 127) / 128), 128, 0, st>>>(S, npp_tot, pp_unit, pp, stride, scratch);
     const int NV = (TCE_LMAX + 1) * (TCE_LMAX + 1) * 2;
     long long n2 = npp_tot * S.ndp * NV;
-    k_pair_vectors<<<(unsigned)((n2 + 127) / 128), 128, 0, st>>>(S, npp_tot, pp_unit, pp, stride, scratch, vec, rvec);
+    k_pair_vectors<<<(unsigned)((n2 + 127) / 128), 128, 0, st>>>(S, npp_tot, pp_unit, pp, stride, scratch, vec, rvec, by_parts);
     return cudaGetLastError() == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }
 

@@ -115,7 +115,7 @@ int tce_launch_t_tables(int nq, int ndp, int ncap, const double *tnode, const do
 int tce_launch_pair_scalars(const DevSys &S, long long npp_tot, const int *pp_unit, PairPrim *pp, UnitPair *up,
                             double *ecoef, cudaStream_t st);
 int tce_launch_pair_vectors(const DevSys &S, long long npp_tot, const int *pp_unit, const PairPrim *pp, int stride,
-                            double *scratch, double2 *vec, double *rvec, cudaStream_t st);
+                            double *scratch, double2 *vec, double *rvec, bool by_parts, cudaStream_t st);
 int tce_launch_enumerate(const DevSys &S, const double *Qsh, double Qmax, int4 *items, unsigned long long *count,
                          unsigned long long cap, unsigned long long *nfunc, cudaStream_t st);
 int tce_launch_stored_jk(int n1, int nbas, int physicist, const double *P, const double *eri, double *J, double *K,

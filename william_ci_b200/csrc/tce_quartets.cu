@@ -459,7 +459,7 @@ __device__ __noinline__ void tc_rows(int wofs, int nb, int lane, int g0c)
 // l / cqp + PW j; otherwise the lanes run over the components of one primitive
 // quartet after the other and accumulate into blkK (and blkG).
 template <int NQ, bool RO>
-__device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstride, bool tc, double &accK_, double &accG_)
+__device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstride, double &accK_, double &accG_)
 {
     const DevSys &S = blk_sys();
     const QCtx &Q = warp_ctx(wofs);
@@ -511,30 +511,11 @@ __device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstri
             b.pqm[4 * p + 1] = Pb.esum + Pk.esum;
             for (int dr = 0; dr < nreal; ++dr) b.pqm[4 * p + 2 + dr] = Pb.cen[ndp + dr] - (Pk.cen[ndp + dr] + Q.Tsh[ndp + dr]);
         }
-    if (tc) row_setup<NQ>(wofs, nb, lane);
+    row_setup<NQ>(wofs, nb, lane);
 #pragma unroll 1
     for (int k0 = 0; k0 < NQ; k0 += NC) {
         const int g0c = k0 / 8, kn = NQ - k0 < NC ? NQ - k0 : NC;
-        if (tc) {
-            tc_rows<NQ, RO, RS>(wofs, nb, lane, g0c);
-        } else {
-            const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
-            for (int r = lane; r < per * ndp; r += 32) {
-                const int d = r / per, rr = r - d * per, p = rr / ncomb;
-                const int dg = b.dig[rr - p * ncomb];
-                const int ia = dg & 3, ib = (dg >> 2) & 3, ic = (dg >> 4) & 3, id = dg >> 6;
-                int2 pq = b.qlist[p];
-                const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
-                const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
-                const double2 *G = S.vec + Q.Ub.vec_off +
-                                   ((((long long)d * (Q.lsA + 1) + ia) * (Q.lsB + 1) + ib) * 2 + 0) * (long long)Q.Ub.Nlen * nppb;
-                const double2 *H = S.vec + Q.Uk.vec_off +
-                                   ((((long long)d * (Q.lsC + 1) + ic) * (Q.lsD + 1) + id) * 2 + 1) * (long long)Q.Uk.Nlen * nppk;
-                int nm = Pb.N[d] < Pk.N[d] ? Pb.N[d] : Pk.N[d];
-                double phi = S.a[d] * (Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]));
-                row_dot<NQ, RO>(Rv, d, G, nppb, pq.x, H, nppk, pq.y, nm, phi, 1.0, g0c, b.rows + (size_t)r * RS);
-            }
-        }
+        tc_rows<NQ, RO, RS>(wofs, nb, lane, g0c);
         for (int k = lane; k < 2 * kn; k += 32) {   // the chunk's weights: Kronrod, then Gauss
             const int kk = k < kn ? k : k - kn;
             b.wts[(k < kn ? 0 : 32) + kk] = k < kn ? Rv.wk[k0 + kk] : (judge ? Rv.wg[k0 + kk] : 0.0);
@@ -671,6 +652,161 @@ __device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstri
     accG_ += accG;
 }
 
+// The same batch on the CUDA cores over every order of the reference's truncation
+// (tensor cores off, density-fitting blocks), accumulating into blkK (and blkG).
+// The fit's pivoted Cholesky follows the last bits of its integrals where
+// symmetric functions tie, so this form keeps its order of operations.
+template <int NQ, bool RO>
+__device__ __noinline__ void process_batch_every(int wofs, int nb, int lane, int cstride)
+{
+    const DevSys &S = blk_sys();
+    const QCtx &Q = warp_ctx(wofs);
+    const RuleView &Rv = Q.R_;
+    const WarpBuf b = warp_buf(wofs);
+    constexpr int NC = NQ < TCE_NC ? NQ : TCE_NC;
+    constexpr int RS = NC + 2;
+    const int ndp = S.ndp, nreal = 3 - ndp;
+    const int lsA = Q.lsA, lsB = Q.lsB, lsC = Q.lsC, lsD = Q.lsD, ncomb = Q.ncomb, R = Q.R;
+    const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
+    const int nrows = nb * R;
+    int cqg = 1;   // lanes per component: 32 / next power of two of the component count
+    while (cqg < Q.ncq && cqg < 32) cqg <<= 1;
+    cqg = 32 / cqg;
+    const int npA = S.sh_np[Q.SI], npB = S.sh_np[Q.SJ], npC = S.sh_np[Q.SK], npD = S.sh_np[Q.SL];
+    const bool judge = Rv.wg != nullptr;
+#pragma unroll 1
+    for (int k0 = 0; k0 < NQ; k0 += NC) {
+        const int g0c = k0 / 8, kn = NQ - k0 < NC ? NQ - k0 : NC;
+        for (int r = lane; r < nrows; r += 32) {
+            int p = r / R, rem = r - p * R;
+            int d = rem / ncomb, cmb = rem - d * ncomb;
+            int ia = cmb % (lsA + 1), t1 = cmb / (lsA + 1);
+            int ib = t1 % (lsB + 1), t2 = t1 / (lsB + 1);
+            int ic = t2 % (lsC + 1), id = t2 / (lsC + 1);
+            int2 pq = b.qlist[p];
+            const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
+            const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
+            const double2 *G = S.vec + Q.Ub.vec_off +
+                               ((((long long)d * (lsA + 1) + ia) * (lsB + 1) + ib) * 2 + 0) * (long long)Q.Ub.Nlen * nppb;
+            const double2 *H = S.vec + Q.Uk.vec_off +
+                               ((((long long)d * (lsC + 1) + ic) * (lsD + 1) + id) * 2 + 1) * (long long)Q.Uk.Nlen * nppk;
+            int nm = Pb.N[d] < Pk.N[d] ? Pb.N[d] : Pk.N[d];
+            double phi = S.a[d] * (Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]));
+            double sgn = pow(S.a[d], -(double)(ia + ib + ic + id));
+            row_dot<NQ, RO>(Rv, d, G, nppb, pq.x, H, nppk, pq.y, nm, phi, sgn, g0c, b.rows + (size_t)r * RS);
+        }
+        __syncwarp();
+        for (int p = 0; p < nb; ++p) {
+            int2 pq = b.qlist[p];
+            const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
+            const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
+            const double pp_ = Pb.esum, qq = Pk.esum;
+            if (nreal > 0) {
+                const double *Eb = S.ecoef + Q.Ub.e_off + (long long)pq.x * nreal * (lsA + 1) * (lsB + 1) * TCE_ECO;
+                const double *Ek = S.ecoef + Q.Uk.e_off + (long long)pq.y * nreal * (lsC + 1) * (lsD + 1) * TCE_ECO;
+                for (int k = lane; k < kn; k += 32) {
+                    double t = Rv.t[k0 + k], t2 = t * t;
+                    const double rr = rsqrt(pp_ * qq + (pp_ + qq) * t2), D2 = rr * rr;
+                    double w = pp_ * qq * t2 * D2, rs = PI_D * rr;
+                    for (int dr = 0; dr < nreal; ++dr) {
+                        int d = ndp + dr;
+                        double Rr = Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]);
+                        double gt[4 * TCE_LMAX + 2];
+                        gt[0] = (Rr == 0.0) ? rs : rs * exp(-w * Rr * Rr);
+                        double gm1 = 0.0, g0 = gt[0];
+                        for (int n = 0; n < Q.NN; ++n) {
+                            double gp1 = 2.0 * w * Rr * g0 - 2.0 * (double)n * w * gm1;
+                            gt[n + 1] = gp1;
+                            gm1 = g0;
+                            g0 = gp1;
+                        }
+                        for (int cmb = 0; cmb < ncomb; ++cmb) {
+                            int ia = cmb % (lsA + 1), u1 = cmb / (lsA + 1);
+                            int ib = u1 % (lsB + 1), u2 = u1 / (lsB + 1);
+                            int ic = u2 % (lsC + 1), id = u2 / (lsC + 1);
+                            const double *eb = Eb + ((dr * (lsA + 1) + ia) * (lsB + 1) + ib) * TCE_ECO;
+                            const double *ek = Ek + ((dr * (lsC + 1) + ic) * (lsD + 1) + id) * TCE_ECO;
+                            double val = 0.0;
+                            for (int n = 0; n <= ia + ib; ++n) {
+                                double sb = (n & 1) ? -eb[n] : eb[n];
+                                for (int kk = 0; kk <= ic + id; ++kk) val += sb * ek[kk] * gt[n + kk];
+                            }
+                            b.realb[((size_t)dr * cstride + cmb) * RS + k] = val;
+                        }
+                    }
+                }
+                __syncwarp();
+            }
+            const double fac = b.qfac[p];
+            const double *rowp = b.rows + (size_t)p * R * RS;
+            const int i = pq.x / Q.Ub.np2, j = pq.x % Q.Ub.np2;
+            const int kp = pq.y / Q.Uk.np2, lp = pq.y % Q.Uk.np2;
+            // The component quartets: sum_k w_k I_x I_y I_z per component.  G lanes
+            // share one component and split its nodes (G = 32 / next power of two of
+            // the component count, at most NQ), so that the warp holds 32 / G
+            // components at once and each needs log2(G) shuffles instead of a full
+            // warp reduction; each component's block entry has one owning lane.
+            const int G = cqg < NC ? cqg : NC;
+            const int slots = 32 / G, slot = lane / G, sub = lane - slot * G;
+            for (int c0 = 0; c0 < Q.ncq; c0 += slots) {
+                const int cq = c0 + slot;
+                double vK = 0.0, vG = 0.0;
+                int ca = 0, cb = 0, cc = 0, cd = 0;
+                if (cq < Q.ncq) {
+                    ca = cq % Q.nA;
+                    const int r1 = cq / Q.nA;
+                    cb = r1 % Q.nB;
+                    const int r2 = r1 / Q.nB;
+                    cc = r2 % Q.nC;
+                    cd = r2 / Q.nC;
+                    const int *pa = S.fn_pw + 3 * (S.sh_first[Q.SI] + ca);
+                    const int *pb = S.fn_pw + 3 * (S.sh_first[Q.SJ] + cb);
+                    const int *pc = S.fn_pw + 3 * (S.sh_first[Q.SK] + cc);
+                    const int *pd = S.fn_pw + 3 * (S.sh_first[Q.SL] + cd);
+                    const double *rw[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const int cm = pa[d] + (lsA + 1) * (pb[d] + (lsB + 1) * (pc[d] + (lsC + 1) * pd[d]));
+                        rw[d] = (d < ndp) ? rowp + ((size_t)d * ncomb + cm) * RS
+                                          : b.realb + ((size_t)(d - ndp) * cstride + cm) * RS;
+                    }
+                    // two partial sums per estimate: shorter dependent FMA chains
+                    double vK1 = 0.0, vG1 = 0.0;
+                    int k = sub;
+                    for (; k + G < kn; k += 2 * G) {
+                        const double p0 = rw[0][k] * rw[1][k] * rw[2][k];
+                        const double p1 = rw[0][k + G] * rw[1][k + G] * rw[2][k + G];
+                        vK = fma(Rv.wk[k0 + k], p0, vK);
+                        vK1 = fma(Rv.wk[k0 + k + G], p1, vK1);
+                        if (judge) {
+                            vG = fma(Rv.wg[k0 + k], p0, vG);
+                            vG1 = fma(Rv.wg[k0 + k + G], p1, vG1);
+                        }
+                    }
+                    if (k < kn) {
+                        const double p0 = rw[0][k] * rw[1][k] * rw[2][k];
+                        vK = fma(Rv.wk[k0 + k], p0, vK);
+                        if (judge) vG = fma(Rv.wg[k0 + k], p0, vG);
+                    }
+                    vK += vK1;
+                    vG += vG1;
+                }
+                for (int o = G >> 1; o > 0; o >>= 1) {
+                    vK += __shfl_xor_sync(0xffffffffu, vK, o);
+                    if (judge) vG += __shfl_xor_sync(0xffffffffu, vG, o);
+                }
+                if (cq < Q.ncq && sub == 0) {
+                    const double cf = S.sh_coef[S.sh_coff[Q.SI] + ca * npA + i] * S.sh_coef[S.sh_coff[Q.SJ] + cb * npB + j] *
+                                      S.sh_coef[S.sh_coff[Q.SK] + cc * npC + kp] * S.sh_coef[S.sh_coff[Q.SL] + cd * npD + lp];
+                    b.blkK[cq] += fac * cf * vK;
+                    if (judge) b.blkG[cq] += fac * cf * vG;
+                }
+            }
+            __syncwarp();
+        }
+    }
+}
+
 __device__ __forceinline__ void make_ctx(const DevSys &S, int4 q, QCtx &Q)
 {
     Q.SI = q.x; Q.SJ = q.y; Q.SK = q.z; Q.SL = q.w;
@@ -717,6 +853,10 @@ __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A
         b.dig[x] = (unsigned char)(ia | ib << 2 | (t2 % (Q.lsC + 1)) << 4 | (t2 / (Q.lsC + 1)) << 6);
     }
     __syncwarp();
+    auto batch = [&](int n) {
+        if (A.use_tc) process_batch<NQ, RO>(wofs, n, lane, A.cstride, accK, accG);
+        else process_batch_every<NQ, RO>(wofs, n, lane, A.cstride);
+    };
     int B = A.rowcap / Q.R;
     if (B < 1) B = 1;
     const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
@@ -761,14 +901,14 @@ __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A
             done += take;
             __syncwarp();
             if (nb == B) {
-                process_batch<NQ, RO>(wofs, nb, lane, A.cstride, A.use_tc != 0, accK, accG);
+                batch(nb);
                 nb = 0;
                 __syncwarp();
             }
         }
     }
-    if (nb > 0) process_batch<NQ, RO>(wofs, nb, lane, A.cstride, A.use_tc != 0, accK, accG);
-    if (Q.ncq <= 32) {
+    if (nb > 0) batch(nb);
+    if (A.use_tc && Q.ncq <= 32) {
         for (int o = Q.cqp; o < 32; o <<= 1) {
             accK += __shfl_xor_sync(0xffffffffu, accK, o);
             accG += __shfl_xor_sync(0xffffffffu, accG, o);
