@@ -115,7 +115,7 @@ struct QCtx {
 constexpr int TCE_NC = 32;        // nodes of a chunk
 constexpr int TCE_GT_ROWS = 12;   // rows of g_m(t) of the real directions: (NN + 1) x primitive quartets at once
 struct RowMeta {
-    int g, h;            // first elements of the bra and ket vectors, from the unit pairs' slabs
+    long long g, h;      // first elements of the bra and ket vectors, from the unit pairs' slabs
     double phi;
     float u, ap;         // 1/A_bra + 1/A_ket, |phi| in [0, pi]
 };
@@ -275,8 +275,8 @@ __device__ __noinline__ void row_setup(int wofs, int nb, int lane)
         const PairPrim &Pb = S.pp[Q.Ub.pp_off + pq.x];
         const PairPrim &Pk = S.pp[Q.Uk.pp_off + pq.y];
         RowMeta m;
-        m.g = (((d * (Q.lsA + 1) + ia) * (Q.lsB + 1) + ib) * 2 + 0) * Q.Ub.Nlen * nppb + pq.x;
-        m.h = (((d * (Q.lsC + 1) + ic) * (Q.lsD + 1) + id) * 2 + 1) * Q.Uk.Nlen * nppk + pq.y;
+        m.g = ((((long long)d * (Q.lsA + 1) + ia) * (Q.lsB + 1) + ib) * 2 + 0) * Q.Ub.Nlen * nppb + pq.x;
+        m.h = ((((long long)d * (Q.lsC + 1) + ic) * (Q.lsD + 1) + id) * 2 + 1) * Q.Uk.Nlen * nppk + pq.y;
         m.phi = S.a[d] * (Pb.cen[d] - (Pk.cen[d] + Q.Tsh[d]));
         m.u = 1.0f / (float)Pb.A[d] + 1.0f / (float)Pk.A[d];
         m.ap = tce_fold_phase(m.phi);
