@@ -824,6 +824,8 @@ def main():
                 "frac": (achieved / peak) if (achieved and peak) else None, "traffic": traffic,
                 "peak_source": "measured FP64 FMA throughput of this GPU (tce_fp64_peak probe); MEASURED_PEAKS.json "
                                "holds no FP64 figure",
+                # counted over every Bessel order of the reference's truncation; the kernels
+                # reach the same sums over a tenth of them, so the fraction is no pipe load
                 "algorithmic_flops_per_launch": lg_flops, "primitive_quartets": lg_nprim, "pass_ms": lg_kern,
                 "per_list": kernels}
     lg_err = lg_info["max_err_vs_oracle_table128"]

@@ -195,13 +195,14 @@ int tce_last_kernel_ms(void *handle, double *ms);
  * lists change.  Default off. */
 int tce_set_graph(void *handle, int32_t on);
 
-/* Node sums of the learned-grid pass on the FP64 tensor cores (mma.sync
- * m8n8k4, FP64 in and out) where a kernel has that form: the all-s quartets
- * and the s/p classes with one or two p shells of one periodic direction
- * (32- and 64-node rules, tile shapes from tce_lg_autotune), and the rows
- * (primitive quartet x power combination) of the generic kernel.  Default
- * on; off gives the FP64 CUDA-core kernels.  Same arithmetic type, different
- * summation order.  No reference counterpart. */
+/* Node sums of every method on the FP64 tensor cores (mma.sync m8n8k4, FP64 in
+ * and out): the all-s quartets, the s/p classes with one or two p shells of one
+ * periodic direction, and the rows (primitive quartet x power combination) of
+ * the generic kernel.  They sum the few Bessel orders that a sum's decay and
+ * the function's width leave, to rounding; off gives the FP64 CUDA-core
+ * kernels, which sum every order of the reference's truncation.  Default on.
+ * Shell blocks of tce_create_blocks handles (density fitting) always take
+ * every order.  No reference counterpart. */
 int tce_set_tensor_cores(void *handle, int32_t on);
 
 /* The learned-grid work lists of a pass as n chains (1 or 2; default 2): the
@@ -214,9 +215,9 @@ int tce_set_list_streams(void *handle, int32_t n);
 /* Kernel-form tuning of the learned-grid pass (after tce_lg_predict_rules /
  * tce_lg_set_item_rules): every work list that has both a CUDA-core and an
  * FP64 tensor-core kernel is timed in each of its forms (the CUDA-core
- * kernel, the tensor-core kernel, and for the all-s quartets each tile shape
- * of the tensor-core kernel: 16 primitive quartets x 32 nodes per pass, 32 x
- * 16, 16 x 16, 8 x 64) with reps launches each (CUDA events; the fastest
+ * kernel, the tensor-core kernel, and each tile shape of the all-s kernel of one
+ * periodic direction: 16 primitive quartets x 8 nodes per pass, 16 x 16, 8 x 8,
+ * 8 x 16, and of the s/p kernel: 8 x 16, 8 x 8) with reps launches each (CUDA events; the fastest
  * launch counts) and keeps the fastest, also when the lists are rebuilt later
  * (new rules, rejects moved to the plain list).
  * ntuned: lists timed; nswitched: lists whose choice differs from the built-in
@@ -385,7 +386,9 @@ int tce_lg_item_rules(void *handle, int32_t *rule);
  * direction) whose shell-pair Schwarz product Q(ij)Q(kl) is below thr sum
  * their periodic-direction node sums in FP32 (FP32 copy of the rule tables);
  * phases, Bessel vectors, real directions, weights, the judge and the J/K
- * accumulation stay FP64.  thr = 0 (default) turns it off; at most 1e-3. */
+ * accumulation stay FP64.  That is the lists' CUDA-core form (form 0, or tensor
+ * cores off); their default tensor-core form sums few orders in FP64, which is
+ * faster.  thr = 0 (default) turns it off; at most 1e-3. */
 int tce_set_fp32_threshold(void *handle, double thr);
 
 /* Quadrature method of tce_direct_jk[_device] (TCE_METHOD_*).  With
