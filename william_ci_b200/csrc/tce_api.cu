@@ -184,6 +184,12 @@ int ncomb_of(const Handle *h, int SI, int SJ, int SK, int SL)
     return (h->sh_l[SI] + 1) * (h->sh_l[SJ] + 1) * (h->sh_l[SK] + 1) * (h->sh_l[SL] + 1);
 }
 
+// Whether the shell blocks of a handle run on the tensor cores (few orders).
+// Blocks-only handles hold the power vectors of the d_k sums, which only the sums
+// over every order average well enough, and a fit follows the last bits of its
+// blocks: they always take the CUDA-core form.
+int block_tc(const Handle *h) { return h->use_tc && !h->blocks_only; }
+
 // run the quartet kernel on a host list of items in a block-output mode
 int run_blocks(Handle *h, const std::vector<int4> &items, const std::vector<int> *prim_sel, int mode, int prim_screen,
                std::vector<double> *blocks, std::vector<long long> *offs)
@@ -221,7 +227,7 @@ int run_blocks(Handle *h, const std::vector<int4> &items, const std::vector<int>
     a.max_ncq = h->max_ncq;
     a.fixed_gmax = h->d_gmax;
     a.num_sms = h->num_sms;
-    a.use_tc = !h->blocks_only;
+    a.use_tc = block_tc(h);
     CKS(h, tce_launch_quartets(h->S, a, h->st));
     if (blocks) {
         blocks->resize(off.back());
@@ -1233,6 +1239,7 @@ int tce_shell_block_noalloc(void *handle, const int32_t sh4[4], int32_t mode, do
     a.max_ncq = h->max_ncq;
     a.fixed_gmax = h->d_gmax;
     a.num_sms = h->num_sms;
+    a.use_tc = block_tc(h);
     CKS(h, tce_launch_quartets(h->S, a, h->st));
     CK(h, cudaMemcpyAsync(blk, base + TCE_STATIC_OFF_BLK, sizeof(double) * nblk, cudaMemcpyDeviceToHost, h->st));
     CK(h, cudaStreamSynchronize(h->st));
@@ -1311,6 +1318,7 @@ int tce_eri_stored(void *handle, int64_t eri_size, double *eri)
         a.max_ncq = h->max_ncq;
         a.fixed_gmax = h->d_gmax;
         a.num_sms = h->num_sms;
+        a.use_tc = h->use_tc;
         CKS(h, tce_launch_quartets(h->S, a, h->st));
     }
     if (!h->sao) CKS(h, tce_launch_sym_fill(h->nbas, h->nfuc, h->ncl, h->d_eri, h->st));

@@ -199,6 +199,7 @@ void dfree(Handle *h, void *p);
 // helpers defined in tce_api.cu
 int shift_to(const Handle *h, int idx, int refcell, int nblk);
 int generic_class(const Handle *h, const int4 &q);
+int block_tc(const Handle *h);
 float2 node_range(const double *t, int n);
 int ncomb_of(const Handle *h, int SI, int SJ, int SK, int SL);
 int make_lists(Handle *h, const std::vector<int4> &items);

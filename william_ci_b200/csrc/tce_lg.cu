@@ -1014,7 +1014,7 @@ int tce_rule_blocks(void *handle, int32_t rule, int32_t mode, int64_t n, const i
         a.dict_nq = h->rules_host[rule].nq;
     }
     if (rule == -2) a.method = TCE_METHOD_PLAIN;
-    a.use_tc = h->use_tc && !h->blocks_only;
+    a.use_tc = block_tc(h);
     CKS(h, tce_launch_quartets(h->S, a, h->st));
     CK(h, cudaMemcpyAsync(K, d_K, sizeof(double) * off.back(), cudaMemcpyDeviceToHost, h->st));
     if (d_G) CK(h, cudaMemcpyAsync(G, d_G, sizeof(double) * off.back(), cudaMemcpyDeviceToHost, h->st));

@@ -1404,6 +1404,7 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
     A.gk_wk = h.gk_wk;
     A.gk_wg = h.gk_wg;
     A.node_evals = h.node_evals;
+    if (h.use_tc < 0) return TCE_ERR_ARG;
     const bool plain = (h.method == TCE_METHOD_PLAIN);
     const bool dict = (h.method == TCE_METHOD_LEARNED) || h.rule_override >= 0;
     if (plain && (h.mode == TCE_MODE_PRIMTAB || !h.scratch || !h.gk_u)) return TCE_ERR_ARG;
