@@ -114,27 +114,29 @@ int shift_by(const Handle *h, int idx, int ct, int nblk)
     return (cx + ncl[0] * (cy + ncl[1] * cz)) * nblk + loc;
 }
 
+// The class of a quartet for the s/p kernels, bit i set when shell i of
+// (A, B | C, D) is p; -1 when one of its shells is none they take: s of one
+// function, or p of three in the reference's order px, py, pz.  (px alone is a
+// shell of one function, also when py and pz of other exponents come next.)
+int sp_class(const Handle *h, const int4 &q)
+{
+    int cls = 0, i = 0;
+    for (int S : {q.x, q.y, q.z, q.w}) {
+        const int l = h->sh_l[S];
+        if (l > 1 || h->sh_n[S] != 2 * l + 1) return -1;
+        for (int c = 0; l == 1 && c < 3; ++c)
+            if (h->lxyz[3 * (h->sh_first[S] + c) + c] != 1) return -1;
+        cls |= l << i++;
+    }
+    return cls;
+}
+
 // which kernel evaluates a quartet in J/K mode: key = kind * 16 + cls
 int route(const Handle *h, const int4 &q)
 {
-    const int l[4] = {h->sh_l[q.x], h->sh_l[q.y], h->sh_l[q.z], h->sh_l[q.w]};
-    int cls = 0;
-    bool sp = true;
-    for (int i = 0; i < 4; ++i) {
-        if (l[i] > 1) sp = false;
-        else cls |= l[i] << i;
-    }
-    if (sp) {
-        for (int i = 0; i < 4; ++i) {   // r1 needs the reference component order px, py, pz
-            int S = (&q.x)[i];
-            if (l[i] == 1)
-                for (int c = 0; c < 3; ++c)
-                    for (int d = 0; d < 3; ++d)
-                        if (h->lxyz[3 * (h->sh_first[S] + c) + d] != (c == d ? 1 : 0)) sp = false;
-        }
-    }
-    if (cls == 0 && sp) return 1 * 16;
-    if (sp && h->ndp == 1 && __builtin_popcount(cls) <= 2) return 2 * 16 + cls;
+    const int cls = sp_class(h, q);
+    if (cls == 0) return 1 * 16;
+    if (cls > 0 && h->ndp == 1 && __builtin_popcount(cls) <= 2) return 2 * 16 + cls;
     return generic_class(h, q);
 }
 

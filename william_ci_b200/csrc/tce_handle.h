@@ -198,6 +198,7 @@ void dfree(Handle *h, void *p);
 
 // helpers defined in tce_api.cu
 int shift_to(const Handle *h, int idx, int refcell, int nblk);
+int sp_class(const Handle *h, const int4 &q);
 int generic_class(const Handle *h, const int4 &q);
 int block_tc(const Handle *h);
 float2 node_range(const double *t, int n);

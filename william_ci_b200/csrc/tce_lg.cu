@@ -381,23 +381,9 @@ static bool lg_generic_cuda_core(const Handle::LgList &w)
 // order, 0 everything else)
 static int lg_route(const Handle *h, const int4 &q)
 {
-    const int l[4] = {h->sh_l[q.x], h->sh_l[q.y], h->sh_l[q.z], h->sh_l[q.w]};
-    int cls = 0;
-    bool sp = true;
-    for (int i = 0; i < 4; ++i) {
-        if (l[i] > 1) sp = false;
-        else cls |= l[i] << i;
-    }
-    if (!sp) return 0;
-    for (int i = 0; i < 4; ++i) {
-        const int S = (&q.x)[i];
-        if (l[i] == 1)
-            for (int c = 0; c < 3; ++c)
-                for (int d = 0; d < 3; ++d)
-                    if (h->lxyz[3 * (h->sh_first[S] + c) + d] != (c == d ? 1 : 0)) return 0;
-    }
+    const int cls = sp_class(h, q);
     if (cls == 0) return 16;
-    if (h->ndp == 1 && __builtin_popcount(cls) <= 2) return 32 + cls;
+    if (cls > 0 && h->ndp == 1 && __builtin_popcount(cls) <= 2) return 32 + cls;
     return 0;
 }
 
