@@ -82,6 +82,38 @@ def test_strided_orders_match_every_order(name, ncell, spacing, off, nquad):
     assert np.abs(K - K0).max() <= 1e-12 * scale, np.abs(K - K0).max() / scale
 
 
+# The CUDA-core kernels turn e^{i n phi} by a recurrence of 32 steps over some 170
+# orders: 32 eps per order, 170 orders, 1e-12 of a sum's peak; 1e-11 of the
+# density's sum with room for the sum over quartets.  (Not the long torus, whose
+# 1000 orders and phases take that past 1e-10.)
+EVERY = 1e-11
+
+
+@pytest.mark.parametrize("name,ncell,spacing,off,nquad",
+                         [c + (n,) for c in CASES if c[2] != 30.0 for n in (32, 40, 64)] + [c + (128,) for c in CASES[:3]])
+def test_tensor_cores_off(name, ncell, spacing, off, nquad):
+    """Every class through the CUDA-core kernels or the generic kernel's every-order
+    form: J and K direct, and from the stored integrals of the small systems."""
+    import pyoracle
+    from william_ci_b200.engine import Engine
+    s = _system(name, ncell, spacing, off)
+    P = random_density(s.nbas, 5) * 0.05
+    t, w = pyoracle.fast_quad(nquad)
+    J0, K0 = pyoracle.Oracle(s, t_nodes=t, t_weights=w).direct_jk(P)[:2]
+    scale = np.abs(P).sum()
+    with Engine(s, t_nodes=t, t_weights=w) as eng:
+        eng.set_tensor_cores(False)
+        got = [eng.direct_JK(P)]
+        if s.nbas < 70:
+            eng.ERI_integral_toroidal()
+            J, K = eng.stored_JK(P)
+            got.append((J[:s.nfuc], K[:s.nfuc]))
+        eng.set_tensor_cores(True)      # the lists are cut again for the tensor-core kernels
+        got.append(eng.direct_JK(P))
+    for J, K in got:
+        assert np.abs(J - J0[:len(J)]).max() <= EVERY * scale and np.abs(K - K0[:len(K)]).max() <= EVERY * scale
+
+
 @pytest.mark.parametrize("nquad", [32, 64])
 def test_shells_of_one_d_component(nquad):
     import pyoracle
@@ -96,11 +128,13 @@ def test_shells_of_one_d_component(nquad):
     assert np.abs(J - J0).max() <= 1e-12 * scale and np.abs(K - K0).max() <= 1e-12 * scale
 
 
+@pytest.mark.parametrize("cores", [True, False])
 @pytest.mark.parametrize("nquad", [32, 40, 64])
 @pytest.mark.parametrize("shells", ["sp", "spd"])
-def test_nuclear_attraction_few_orders(shells, nquad):
+def test_nuclear_attraction_few_orders(shells, nquad, cores):
     """One periodic direction, atoms off the axis, s to d shells: every element
-    within 1e-12 of the sum of charges times the largest s element's scale (1)."""
+    within 1e-12 (tensor cores off: EVERY) of the sum of charges times the largest
+    s element's scale (1)."""
     import pyoracle
     from william_ci_b200 import system as S
     from william_ci_b200.engine import Engine
@@ -113,9 +147,10 @@ def test_nuclear_attraction_few_orders(shells, nquad):
     t, w = pyoracle.fast_quad(nquad)
     V0 = pyoracle.Oracle(s, t_nodes=t, t_weights=w).one_electron()[2]
     with Engine(s, t_nodes=t, t_weights=w) as eng:
+        eng.set_tensor_cores(cores)
         V = eng.nuclear_attraction()
     assert np.abs(V0).max() > 0.1
-    assert np.abs(V - V0).max() <= 1e-12 * max(1.0, np.abs(V0).max()) * len(s.charges), np.abs(V - V0).max()
+    assert np.abs(V - V0).max() <= (1e-12 if cores else EVERY) * max(1.0, np.abs(V0).max()) * len(s.charges), np.abs(V - V0).max()
 
 
 @pytest.mark.parametrize("nquad", [32, 40, 64])

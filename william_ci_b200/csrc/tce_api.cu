@@ -131,19 +131,25 @@ int sp_class(const Handle *h, const int4 &q)
     return cls;
 }
 
-// which kernel evaluates a quartet in J/K mode: key = kind * 16 + cls
+// which kernel evaluates a quartet with the system's rule: key = kind * 16 + cls.
+// With the tensor cores off the all-s and one-p kernels are the CUDA-core ones,
+// built for 32 nodes (all-s: and 40).
 int route(const Handle *h, const int4 &q)
 {
     const int cls = sp_class(h, q);
-    if (cls == 0) return 1 * 16;
-    if (cls > 0 && h->ndp == 1 && __builtin_popcount(cls) <= 2) return 2 * 16 + cls;
+    if (cls == 0 && (h->use_tc || h->nq == 32 || h->nq == 40)) return 1 * 16;
+    if (cls > 0 && (h->use_tc ? h->ndp == 1 && __builtin_popcount(cls) <= 2 : tce_r1_supported(h->ndp, h->nq, cls)))
+        return 2 * 16 + cls;
     return generic_class(h, q);
 }
 
 // The generic kernel's lists, one per number of p and number of d shells
 // (0..14): each launches with its own combination count and block size, so that
 // no quartet carries the per-warp buffers of a larger class; the buffers decide
-// how many warps an SM holds (10 of 16 with the lists by d shells alone).
+// how many warps an SM holds (10 of 16 with the lists by d shells alone).  The
+// CUDA-core form has smaller buffers and more registers: one list per number of d
+// shells (0..4), whose single tail is worth more (2x2x2 cube, tensor cores off:
+// 26.9 ms with 5 lists, 23.5 with one).
 int generic_class(const Handle *h, const int4 &q)
 {
     int np = 0, nd = 0;
@@ -151,6 +157,7 @@ int generic_class(const Handle *h, const int4 &q)
         np += h->sh_l[S] == 1;
         nd += h->sh_l[S] > 1;
     }
+    if (!h->use_tc) return nd;
     return nd * 5 - nd * (nd - 1) / 2 + np;
 }
 
@@ -684,14 +691,13 @@ int build(Handle *h, const tce_system *sys)
 }
 
 // Every work list of the handle with the system's rule: J and K added up
-// (TCE_MODE_JK) or the integrals stored (TCE_MODE_STORE: dJ the array).
+// (TCE_MODE_JK) or, tensor cores on, the integrals stored (TCE_MODE_STORE: dJ the
+// array; the CUDA-core all-s and one-p kernels have no such form).
 static int fixed_lists(Handle *h, int mode, const double *dP, double *dJ, double *dK, cudaStream_t st)
 {
     for (const auto &w : h->lists) {
         if (w.n == 0) continue;
-        // the CUDA-core kernels of the all-s and one-p classes are built for 32 nodes (all-s: and 40) and J/K
-        const bool core = mode == TCE_MODE_JK && (w.kind == 1 ? (h->nq == 32 || h->nq == 40) : tce_r1_supported(h->ndp, h->nq, w.cls));
-        if (w.kind == 0 || (!h->use_tc && !core)) {   // every other class: generic kernel
+        if (w.kind == 0) {   // every other class: generic kernel
             QuartetHostArgs a;
             a.items = w.d;
             a.nitems = (int)w.n;
@@ -996,8 +1002,17 @@ int tce_set_tensor_cores(void *handle, int32_t on)
 {
     Handle *h = static_cast<Handle *>(handle);
     if (!h) return fail(h, TCE_ERR_ARG, "NULL handle");
+    const int was = h->use_tc;
     h->use_tc = on ? 1 : 0;
     ++h->work_version;   // a captured pass is re-captured
+    if (h->use_tc == was || h->items_host.empty()) return TCE_OK;
+    // the work lists are cut for the kernels that run them
+    std::vector<int4> mine;
+    mine.reserve(h->shard_idx.size());
+    for (long long i : h->shard_idx) mine.push_back(h->items_host[(size_t)i]);
+    int s;
+    if ((s = make_lists(h, mine)) || (s = lg_rebuild_lists(h))) return s;
+    CK(h, cudaStreamSynchronize(h->st));
     return TCE_OK;
 }
 
@@ -1302,11 +1317,12 @@ int tce_eri_stored(void *handle, int64_t eri_size, double *eri)
     }
     h->eri_size = esz;
     CK(h, cudaMemsetAsync(h->d_eri, 0, sizeof(double) * elems, h->st));
-    if (h->nitems > 0 && h->nitems_shard == h->nitems) {
+    if (h->nitems > 0 && h->nitems_shard == h->nitems && h->use_tc) {
         // the classes' own kernels over their lists, as a J/K pass
         int s = fixed_lists(h, TCE_MODE_STORE, nullptr, h->d_eri, nullptr, h->st);
         if (s) return s;
-    } else if (h->nitems > 0) {   // a shard's lists hold its quartets only: every quartet through the generic kernel
+    } else if (h->nitems > 0) {
+        // tensor cores off, or a shard, whose lists hold its quartets only: every quartet through the generic kernel
         QuartetHostArgs a;
         a.items = h->d_items;
         a.nitems = (int)h->nitems;

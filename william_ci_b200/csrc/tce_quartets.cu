@@ -111,7 +111,9 @@ struct QCtx {
 // tce_warp_doubles: rows of a chunk of 32 nodes at stride RS = 34 doubles (even,
 // so that two nodes load as one double2, and 16 bytes past a multiple of 128,
 // so that eight rows fall into different banks; 18 for the plain method's
-// 16-node panels).
+// 16-node panels).  The every-order form (process_batch_every) has lanes on rows
+// and no use for most of it: stride 33 (17), and a whole warp's 32 rows where the
+// tensor cores take 16 per direction.
 constexpr int TCE_NC = 32;        // nodes of a chunk
 constexpr int TCE_GT_ROWS = 12;   // rows of g_m(t) of the real directions: (NN + 1) x primitive quartets at once
 struct RowMeta {
@@ -133,27 +135,27 @@ struct WarpBuf {
 struct WarpLayout {              // offsets in doubles
     int qlist, qidx, qfac, rows, realb, gt, blkK, blkG, cf, wts, pqm, meta, plan, cs, cmap, dig, extra;
 };
-__host__ __device__ inline WarpLayout tce_warp_layout(int rowcap, int RS, int nreal, int cstride, int blkcap, int nhalf)
+__host__ __device__ inline WarpLayout tce_warp_layout(bool tc, int rowcap, int RS, int nreal, int cstride, int blkcap, int nhalf)
 {
     WarpLayout o;
     int at = ((int)(sizeof(QCtx) + 7) / 8 + 1) & ~1;   // the quartet at hand
     auto take = [&](int n) { const int r = at; at += (n + 1) & ~1; return r; };
     o.qlist = take(rowcap);
-    o.qidx = take(rowcap);
+    o.qidx = take(tc ? rowcap : 0);
     o.qfac = take(rowcap);
     o.rows = take(rowcap * RS);
     o.realb = take(nreal * cstride * RS);
-    o.gt = take(nreal * TCE_GT_ROWS * RS);
+    o.gt = take(tc ? nreal * TCE_GT_ROWS * RS : 0);
     o.blkK = take(blkcap);
     o.blkG = take(blkcap);
-    o.cf = take(72);
-    o.wts = take(64);
-    o.pqm = take(nreal > 0 ? 4 * rowcap : 0);
-    o.meta = take(rowcap * (int)(sizeof(RowMeta) / 8));
-    o.plan = take((rowcap / 16 + 3) * nhalf);
-    o.cs = take(2 * rowcap * nhalf);
-    o.cmap = take((blkcap + 1) / 2);
-    o.dig = take(12);
+    o.cf = take(tc ? 72 : 0);
+    o.wts = take(tc ? 64 : 0);
+    o.pqm = take(tc && nreal > 0 ? 4 * rowcap : 0);
+    o.meta = take(tc ? rowcap * (int)(sizeof(RowMeta) / 8) : 0);
+    o.plan = take(tc ? (rowcap / 16 + 3) * nhalf : 0);
+    o.cs = take(tc ? 2 * rowcap * nhalf : 0);
+    o.cmap = take(tc ? (blkcap + 1) / 2 : 0);
+    o.dig = take(tc ? 12 : 0);
     o.extra = at;
     return o;
 }
@@ -175,7 +177,6 @@ struct QuartetArgs {
     PairPrim *pp_rw;
     int rowcap, cstride, blkcap, warp_smem_doubles;
     WarpLayout lay;
-    int use_tc;
     const int *fixed_gmax;
     // learned grid
     const RuleDev *rules;
@@ -657,14 +658,13 @@ __device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstri
 // The fit's pivoted Cholesky follows the last bits of its integrals where
 // symmetric functions tie, so this form keeps its order of operations.
 template <int NQ, bool RO>
-__device__ __noinline__ void process_batch_every(int wofs, int nb, int lane, int cstride)
+__device__ __forceinline__ void process_batch_every(const DevSys &S, int wofs, int nb, int lane, int cstride)
 {
-    const DevSys &S = blk_sys();
     const QCtx &Q = warp_ctx(wofs);
     const RuleView &Rv = Q.R_;
     const WarpBuf b = warp_buf(wofs);
     constexpr int NC = NQ < TCE_NC ? NQ : TCE_NC;
-    constexpr int RS = NC + 2;
+    constexpr int RS = NC + 1;
     const int ndp = S.ndp, nreal = 3 - ndp;
     const int lsA = Q.lsA, lsB = Q.lsB, lsC = Q.lsC, lsD = Q.lsD, ncomb = Q.ncomb, R = Q.R;
     const int nppb = Q.Ub.npp, nppk = Q.Uk.npp;
@@ -829,7 +829,7 @@ __device__ __forceinline__ void make_ctx(const DevSys &S, int4 q, QCtx &Q)
 
 // The block of one shell quartet with its rule (Q.R_): screen and batch the primitive
 // quartets, accumulate into b.blkK (and b.blkG); both are zeroed first.
-template <int NQ, bool RO>
+template <int NQ, bool RO, bool TC>
 __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A, int wofs, int lane, int want)
 {
     const QCtx &Q = warp_ctx(wofs);
@@ -838,6 +838,7 @@ __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A
     for (int c = lane; c < Q.ncq; c += 32) {
         b.blkK[c] = 0.0;
         b.blkG[c] = 0.0;
+        if (!TC) continue;
         // the power combination of each direction
         const int ca = c % Q.nA, r1 = c / Q.nA, cb = r1 % Q.nB, r2 = r1 / Q.nB, cc = r2 % Q.nC, cd = r2 / Q.nC;
         const int *pa = S.fn_pw + 3 * (S.sh_first[Q.SI] + ca), *pb = S.fn_pw + 3 * (S.sh_first[Q.SJ] + cb);
@@ -848,14 +849,14 @@ __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A
             cm |= (unsigned)(pa[d] + (Q.lsA + 1) * (pb[d] + (Q.lsB + 1) * (pc[d] + (Q.lsC + 1) * pd[d]))) << (8 * d);
         b.cmap[c] = cm;
     }
-    for (int x = lane; x < Q.ncomb; x += 32) {
+    for (int x = lane; TC && x < Q.ncomb; x += 32) {
         const int ia = x % (Q.lsA + 1), t1 = x / (Q.lsA + 1), ib = t1 % (Q.lsB + 1), t2 = t1 / (Q.lsB + 1);
         b.dig[x] = (unsigned char)(ia | ib << 2 | (t2 % (Q.lsC + 1)) << 4 | (t2 / (Q.lsC + 1)) << 6);
     }
     __syncwarp();
     auto batch = [&](int n) {
-        if (A.use_tc) process_batch<NQ, RO>(wofs, n, lane, A.cstride, accK, accG);
-        else process_batch_every<NQ, RO>(wofs, n, lane, A.cstride);
+        if constexpr (TC) process_batch<NQ, RO>(wofs, n, lane, A.cstride, accK, accG);
+        else process_batch_every<NQ, RO>(S, wofs, n, lane, A.cstride);
     };
     int B = A.rowcap / Q.R;
     if (B < 1) B = 1;
@@ -893,8 +894,10 @@ __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A
             if (take > cnt - done) take = cnt - done;
             if (keep && pos >= done && pos < done + take) {
                 b.qlist[nb + pos - done] = make_int2(ipb, ipk);
-                const int i = ipb / Q.Ub.np2, k = ipk / Q.Uk.np2;
-                b.qidx[nb + pos - done] = make_short4((short)i, (short)(ipb - i * Q.Ub.np2), (short)k, (short)(ipk - k * Q.Uk.np2));
+                if (TC) {
+                    const int i = ipb / Q.Ub.np2, k = ipk / Q.Uk.np2;
+                    b.qidx[nb + pos - done] = make_short4((short)i, (short)(ipb - i * Q.Ub.np2), (short)k, (short)(ipk - k * Q.Uk.np2));
+                }
                 b.qfac[nb + pos - done] = fac;
             }
             nb += take;
@@ -908,7 +911,7 @@ __device__ __forceinline__ void eval_block(const DevSys &S, const QuartetArgs &A
         }
     }
     if (nb > 0) batch(nb);
-    if (A.use_tc && Q.ncq <= 32) {
+    if (TC && Q.ncq <= 32) {
         for (int o = Q.cqp; o < 32; o <<= 1) {
             accK += __shfl_xor_sync(0xffffffffu, accK, o);
             accG += __shfl_xor_sync(0xffffffffu, accG, o);
@@ -1004,8 +1007,13 @@ __device__ __forceinline__ int item_count(const QuartetArgs &A)
 
 // method 0: one fixed rule for every item (the system's rule, or dictionary rule
 // rule_override, judged when blk_out2 is set); method 1: the learned grid.
-template <int NQ>
-__global__ void __launch_bounds__(256, 2) k_quartets(DevSys S, QuartetArgs A)
+// TC: rows on the tensor cores over few orders, 128 registers; else every order
+// on the CUDA cores, whose 32 node sums per lane want 255.  With both in one kernel
+// of 128 registers and the tensor-core form's buffers the every-order form took
+// (16-cell chain, 40 nodes / 12 cells, 128 nodes / 3x2 sheet / 2x2x2 cube, ms)
+// 39.8 / 121 / 44.5 / 30.9; by itself 21.7 / 54.5 / 30.8 / 23.5.
+template <int NQ, bool TC>
+__global__ void __launch_bounds__(256, TC ? 2 : 1) k_quartets(DevSys S, QuartetArgs A)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     blk_header(S, A.lay);
@@ -1041,7 +1049,7 @@ __global__ void __launch_bounds__(256, 2) k_quartets(DevSys S, QuartetArgs A)
         __syncwarp();
         int want = -1;
         if (A.mode == TCE_MODE_PRIMTAB) want = A.prim_sel[2 * it] * Q.Ub.np2 + A.prim_sel[2 * it + 1];
-        eval_block<NQ, true>(S, A, wofs, lane, want);
+        eval_block<NQ, true, TC>(S, A, wofs, lane, want);
         if (lg) {
             const double e = block_judge(b.blkK, b.blkG, Q.ncq, lane);
             if (!(e <= A.judge_tol)) {      // the judge rejects the predicted rule
@@ -1189,7 +1197,8 @@ __device__ void plain_columns(const DevSys &S, const QuartetArgs &A, double *T, 
     __syncwarp();
 }
 
-__global__ void __launch_bounds__(128, 4) k_plain(DevSys S, QuartetArgs A)
+template <bool TC>
+__global__ void __launch_bounds__(128, TC ? 4 : 3) k_plain(DevSys S, QuartetArgs A)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     blk_header(S, A.lay);
@@ -1239,7 +1248,7 @@ __global__ void __launch_bounds__(128, 4) k_plain(DevSys S, QuartetArgs A)
         __syncwarp();
         auto eval_panel = [&](int slot, double a, double bnd) {
             plain_columns(S, A, T, nneed, a, bnd, tn, wk, wg, gmax, t2, lane);
-            eval_block<16, false>(S, A, wofs, lane, -1);
+            eval_block<16, false, TC>(S, A, wofs, lane, -1);
             const double e = block_judge(b.blkK, b.blkG, Q.ncq, lane);
             for (int c = lane; c < Q.ncq; c += 32) pblk[(size_t)slot * A.blkcap + c] = b.blkK[c];
             if (lane == 0) {
@@ -1284,10 +1293,10 @@ __global__ void __launch_bounds__(128, 4) k_plain(DevSys S, QuartetArgs A)
 // ---------------------------------------------------------------------------
 // launch
 // ---------------------------------------------------------------------------
-// Warps per block and blocks per SM of k_quartets<NQ> for a per-warp buffer of
+// Warps per block and blocks per SM of k_quartets<NQ, TC> for a per-warp buffer of
 // wbytes: the shape with the most warps resident on an SM (shared memory and
-// registers decide), found once per (NQ, wbytes) with the occupancy calculator.
-template <int NQ>
+// registers decide), found once per (NQ, TC, wbytes) with the occupancy calculator.
+template <int NQ, bool TC>
 static int2 quartet_shape(size_t wbytes)
 {
     static std::mutex mu;
@@ -1299,24 +1308,30 @@ static int2 quartet_shape(size_t wbytes)
     for (int w = 8; w >= 1; --w) {
         const size_t smem = TCE_HDR_DOUBLES * 8 + wbytes * (size_t)w;
         if (smem > 226 * 1024) continue;
-        cudaFuncSetAttribute(k_quartets<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        cudaFuncSetAttribute(k_quartets<NQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_quartets<NQ>, 32 * w, smem) != cudaSuccess) per = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_quartets<NQ, TC>, 32 * w, smem) != cudaSuccess) per = 0;
         if (per * w > best.x * best.y) best = make_int2(w, per);
     }
     known[wbytes] = best;
     return best;
 }
 
-template <int NQ>
-static cudaError_t launch_nq(const DevSys &S, const QuartetArgs &A, size_t wbytes, int nsm, cudaStream_t st)
+template <int NQ, bool TC>
+static cudaError_t launch_form(const DevSys &S, const QuartetArgs &A, size_t wbytes, int nsm, cudaStream_t st)
 {
-    const int2 sh = quartet_shape<NQ>(wbytes);
+    const int2 sh = quartet_shape<NQ, TC>(wbytes);
     if (sh.x < 1 || sh.y < 1) return cudaErrorInvalidConfiguration;
     const size_t smem = TCE_HDR_DOUBLES * 8 + wbytes * (size_t)sh.x;
-    cudaFuncSetAttribute(k_quartets<NQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_quartets<NQ><<<nsm * sh.y, 32 * sh.x, smem, st>>>(S, A);
+    cudaFuncSetAttribute(k_quartets<NQ, TC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    k_quartets<NQ, TC><<<nsm * sh.y, 32 * sh.x, smem, st>>>(S, A);
     return cudaGetLastError();
+}
+
+template <int NQ>
+static cudaError_t launch_nq(bool tc, const DevSys &S, const QuartetArgs &A, size_t wbytes, int nsm, cudaStream_t st)
+{
+    return tc ? launch_form<NQ, true>(S, A, wbytes, nsm, st) : launch_form<NQ, false>(S, A, wbytes, nsm, st);
 }
 
 // Debye polynomials u_k(t) (Abramowitz & Stegun 9.3.9-9.3.10):
@@ -1383,7 +1398,6 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
     A.eri_size = h.eri_size;
     A.physicist = h.physicist;
     A.pp_rw = h.pp_rw;
-    A.use_tc = h.use_tc;
     A.fixed_gmax = h.fixed_gmax;
     A.rules = h.rules;
     A.rule_T = h.rule_T;
@@ -1413,12 +1427,14 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
     if (!plain && !dict && !h.fixed_gmax) return TCE_ERR_ARG;
     const int nq = plain ? 16 : (dict ? h.dict_nq : S.nq);
     const int R = h.max_ncomb * S.ndp;
-    const int rowcap = std::max(R, 16 * S.ndp);   // at least a tile of rows per periodic direction
-    const int RS = (nq < TCE_NC ? nq : TCE_NC) + 2;   // rows of one chunk of at most 32 nodes
+    const bool tc = h.use_tc != 0;
+    const int rowcap = std::max(R, tc ? 16 * S.ndp : 32);   // at least a tile of rows per periodic direction, or a row per lane
+    const int RS = (nq < TCE_NC ? nq : TCE_NC) + (tc ? 2 : 1);   // rows of one chunk of at most 32 nodes
     const int nreal = 3 - S.ndp;
     const int blkcap = (h.max_ncq + 3) / 4 * 4;
-    const int cstride = h.max_ncomb > 16 ? h.max_ncomb : 16;   // real-direction rows: of one primitive quartet, or 32 / cqp small ones
-    A.lay = tce_warp_layout(rowcap, RS, nreal, cstride, blkcap, (nq + 15) / 16);
+    // real-direction rows: of one primitive quartet, or (tensor-core form) 32 / cqp small ones
+    const int cstride = tc && h.max_ncomb < 16 ? 16 : h.max_ncomb;
+    A.lay = tce_warp_layout(tc, rowcap, RS, nreal, cstride, blkcap, (nq + 15) / 16);
     long long wdoubles = A.lay.extra;
     if (plain) wdoubles += 3 * PLAIN_PMAX + 48 + 3 * TCE_MAXG / 2 + 4;
     wdoubles = (wdoubles + 31) / 32 * 32;
@@ -1438,9 +1454,10 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
         if (upload_debye() != TCE_OK) return TCE_ERR_CUDA;
         A.T_doubles = (long long)S.ndp * (S.ncap + 1) * 16;
         A.scratch_per_warp = tce_plain_scratch_per_warp(S, h.max_ncq);
-        cudaFuncSetAttribute(k_plain, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        auto kern = tc ? k_plain<true> : k_plain<false>;
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_plain, 32 * warps, smem);
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 32 * warps, smem);
         if (per < 1) per = 1;
         long long grid = (long long)nsm * per;
         if (grid * warps > h.scratch_warps) grid = h.scratch_warps / warps;
@@ -1449,24 +1466,31 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
         // would hold the registers and shared memory they need
         if (!h.nitems_dev && h.nitems > 0) grid = std::min<long long>(grid, (h.nitems + warps - 1) / warps);
         if (grid < 1) return TCE_ERR_NOMEM;
-        k_plain<<<(unsigned)grid, 32 * warps, smem, st>>>(S, A);
+        kern<<<(unsigned)grid, 32 * warps, smem, st>>>(S, A);
         e = cudaGetLastError();
-    } else if (nq == 32) e = launch_nq<32>(S, A, wbytes, nsm, st);
-    else if (nq == 40) e = launch_nq<40>(S, A, wbytes, nsm, st);
-    else if (nq == 64) e = launch_nq<64>(S, A, wbytes, nsm, st);
-    else if (nq == 128) e = launch_nq<128>(S, A, wbytes, nsm, st);
+    } else if (nq == 32) e = launch_nq<32>(tc, S, A, wbytes, nsm, st);
+    else if (nq == 40) e = launch_nq<40>(tc, S, A, wbytes, nsm, st);
+    else if (nq == 64) e = launch_nq<64>(tc, S, A, wbytes, nsm, st);
+    else if (nq == 128) e = launch_nq<128>(tc, S, A, wbytes, nsm, st);
     else return TCE_ERR_UNSUPPORTED;
     return e == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }
 
-int tce_preload_quartets(int nq)
+template <int NQ>
+static cudaError_t preload_nq()
 {
     cudaFuncAttributes fa;
+    const cudaError_t e = cudaFuncGetAttributes(&fa, k_quartets<NQ, true>);
+    return e == cudaSuccess ? cudaFuncGetAttributes(&fa, k_quartets<NQ, false>) : e;
+}
+
+int tce_preload_quartets(int nq)
+{
     cudaError_t e;
-    if (nq == 32) e = cudaFuncGetAttributes(&fa, k_quartets<32>);
-    else if (nq == 40) e = cudaFuncGetAttributes(&fa, k_quartets<40>);
-    else if (nq == 64) e = cudaFuncGetAttributes(&fa, k_quartets<64>);
-    else if (nq == 128) e = cudaFuncGetAttributes(&fa, k_quartets<128>);
+    if (nq == 32) e = preload_nq<32>();
+    else if (nq == 40) e = preload_nq<40>();
+    else if (nq == 64) e = preload_nq<64>();
+    else if (nq == 128) e = preload_nq<128>();
     else return TCE_ERR_UNSUPPORTED;
     return e == cudaSuccess ? TCE_OK : TCE_ERR_CUDA;
 }
