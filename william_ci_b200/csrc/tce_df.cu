@@ -40,6 +40,7 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
 namespace {
 
 struct DfHandle {
+    PoolUser pool;
     std::string err;
     void *eng = nullptr;      // blocks-only handle of the fit's system
     int N = 1, ncl[3] = {1, 1, 1}, nf = 0, nau = 0, nat = 0, nfc = 0;
@@ -49,8 +50,6 @@ struct DfHandle {
     int *d_crd = nullptr;     // [3 k + d] cell coordinates
     double *d_Vm = nullptr, *d_T3 = nullptr, *d_B = nullptr;
     double2 *d_W = nullptr;   // W(k)(x, q) = [sum_R T3(R) e^{ikR}] f(k), x = mu + nf nu
-    double2 *d_ws1 = nullptr, *d_wsF = nullptr, *d_wsC = nullptr;   // tce_dfmp2's workspaces
-    size_t n_ws1 = 0;
     std::vector<void *> mem;
 };
 
@@ -67,10 +66,8 @@ template <class T>
 int df_alloc(DfHandle *d, T **p, size_t n)
 {
     *p = nullptr;
-    if (cudaMalloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-        cudaGetLastError();
+    if (device_malloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess)
         return df_fail(d, TCE_ERR_NOMEM, "device allocation of " + std::to_string(n * sizeof(T)) + " bytes failed");
-    }
     d->mem.push_back(*p);
     return TCE_OK;
 }
@@ -777,29 +774,28 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     }
     const int no = ohi, nv = nf - vlo;
     if (no < 1 || nv < 1) return df_fail(d, TCE_ERR_ARG, "no occupied or no virtual bands");
-    int s;
-    // workspaces kept with the handle up to a gigabyte: G1 and the L vectors share one buffer (L after G1 is read)
     const long long nG1 = X * nau * N, nF = (long long)nf * nf * nau * N * N, nL = (long long)no * nv * nau * N * N;
-    const size_t need1 = (size_t)std::max(nG1, nL);
-    if (d->n_ws1 < need1) {
-        df_free(d, d->d_ws1);
-        d->n_ws1 = 0;
-        d->d_ws1 = nullptr;
-        if ((s = df_alloc(d, &d->d_ws1, need1))) return s;
-        d->n_ws1 = need1;
-    }
-    if (!d->d_wsF && (s = df_alloc(d, &d->d_wsF, (size_t)nF))) return s;
-    if (!d->d_wsC && (s = df_alloc(d, &d->d_wsC, (size_t)nbas * nbas))) return s;
-    double2 *d_G1 = d->d_ws1, *d_F = d->d_wsF, *d_C = d->d_wsC, *d_L = d->d_ws1;
+    double2 *d_G1 = nullptr, *d_F = nullptr, *d_C = nullptr, *d_L = nullptr;
+    CallMemory mem(d->st);
+    auto none = [&](long long n) {
+        return df_fail(d, TCE_ERR_NOMEM, "device allocation of " + std::to_string(n * sizeof(double2)) + " bytes failed");
+    };
+    if (!mem.get(&d_G1, (size_t)nG1)) return none(nG1);
+    if (!mem.get(&d_F, (size_t)nF)) return none(nF);
     const dim3 tiles(1, (unsigned)((N + DF_KT - 1) / DF_KT));
-    DCK(d, cudaMemcpyAsync(d_C, coeff, sizeof(double2) * nbas * nbas, cudaMemcpyHostToDevice, d->st));
     k_df_g1<<<dim3(nblk(X * nau, 128), tiles.y), 128, 0, d->st>>>(d->d_B, d->d_ph, X, N, nau, d_G1);
     DCK(d, cudaGetLastError());
     k_df_f<<<dim3(nblk((long long)nf * nf * nau * N, 128), tiles.y), 128, 0, d->st>>>(d_G1, d->d_ph, X, N, nf, nau, d_F);
     DCK(d, cudaGetLastError());
+    mem.drop(d_G1);
+    if (!mem.get(&d_C, (size_t)nbas * nbas)) return none(nbas * nbas);
+    if (!mem.get(&d_L, (size_t)nL)) return none(nL);
+    DCK(d, cudaMemcpyAsync(d_C, coeff, sizeof(double2) * nbas * nbas, cudaMemcpyHostToDevice, d->st));
     k_df_l<<<nblk(nL, 256), 256, 0, d->st>>>(d_F, d_C, d->d_crd, d->ncl[0], d->ncl[1], d->ncl[2], N, nf, nau, 0, no,
                                              vlo, nv, d_L);
     DCK(d, cudaGetLastError());
+    mem.drop(d_F);
+    mem.drop(d_C);
     DCK(d, cudaStreamSynchronize(d->st));
     std::vector<int32_t> crd(3 * (size_t)N), oo((size_t)N * no), ov((size_t)N * nv);
     std::vector<double> eo((size_t)N * no), ev((size_t)N * nv);
@@ -819,14 +815,8 @@ int tce_dfmp2(void *df, const double *coeff, const double *eps, const int32_t *o
     double a2d = 0.0, a2x = 0.0;
     int64_t nz = 0;
     double gz = 0.0, ms = 0.0;
-    s = tce_mp2_energy_on(N, d->ncl, crd.data(), no, nv, nau, reinterpret_cast<const double *>(d_L), true, eo.data(), oo.data(), ev.data(), ov.data(),
+    const int s = tce_mp2_energy_on(N, d->ncl, crd.data(), no, nv, nau, reinterpret_cast<const double *>(d_L), true, eo.data(), oo.data(), ev.data(), ov.data(),
                          mode, &a2d, &a2x, &nz, &gz, &ms);
-    if ((double)(d->n_ws1 + (size_t)nF) * sizeof(double2) > 1e9) {   // large ones are given back
-        df_free(d, d->d_ws1);
-        df_free(d, d->d_wsF);
-        d->d_ws1 = d->d_wsF = nullptr;
-        d->n_ws1 = 0;
-    }
     if (s) return df_fail(d, s, std::string("contraction: ") + tce_mp2_last_error());
     *e_mp2 = 2.0 * a2d - a2x;
     if (e2d) *e2d = a2d;

@@ -7,12 +7,14 @@
 #include <vector>
 
 #include "tce_kernels.h"
+#include "tce_pool.h"
 
 namespace tcehost {
 
 constexpr double kPi = 3.14159265358979323846;
 
 struct Handle {
+    PoolUser pool;
     std::string err;
     // system scalars
     int ndp = 0, nq = 0, ncap = 0, nbas = 0, nfuc = 0, nsh = 0, nshuc = 0, ncell = 1;
@@ -62,8 +64,6 @@ struct Handle {
     double *d_eri = nullptr;
     long long eri_elems = 0;
     int eri_size = 0;
-    double2 *d_kmo[5] = {};              // tce_ao_to_kmo: phases, coefficients, X1 / S, X2, output
-    size_t n_kmo[5] = {};
     double *d_blk = nullptr;
     long long *d_blkoff = nullptr;
     int4 *d_one = nullptr;
@@ -173,12 +173,10 @@ int dalloc(Handle *h, T **p, size_t n)
 {
     *p = nullptr;
     if (n == 0) n = 1;
-    cudaError_t e = cudaMalloc((void **)p, n * sizeof(T));
-    if (e != cudaSuccess) {
-        cudaGetLastError();
+    cudaError_t e = device_malloc((void **)p, n * sizeof(T));
+    if (e != cudaSuccess)
         return fail(h, TCE_ERR_NOMEM, "device allocation of " + std::to_string(n * sizeof(T)) + " bytes failed: " +
                                           cudaGetErrorString(e));
-    }
     h->allocs.push_back(*p);
     h->bytes += n * sizeof(T);
     return TCE_OK;

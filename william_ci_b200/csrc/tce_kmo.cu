@@ -13,7 +13,8 @@
 // The three sums over cells read every input once per KMO_T (x1: KMO_G) values of
 // k, phases as shared-memory broadcasts; reading it once per k they moved N
 // times the stored integrals, X1 and X2.  The groups follow each other on one
-// stream without waiting for the host, and the workspaces stay with the handle.
+// stream without waiting for the host; the workspaces come from the pool of call
+// memory (tce_pool.h).
 #include <vector>
 
 #include "tce_handle.h"
@@ -226,34 +227,24 @@ extern "C" int tce_ao_to_kmo(void *handle, const double *coeff, int32_t p_lo, in
     const size_t f4 = (size_t)nf * nf * nf * nf;
     const size_t n1 = (size_t)nf * nbas * nbas * nf, n2 = (size_t)nf * nbas * nf * nf * N, n3 = f4 * N * N;
     const size_t nout = (size_t)no * nv * no * nv * N * N * N, nC = (size_t)nbas * nbas, nph = (size_t)N * N;
-    // k4 per group: what a gigabyte of buffers takes (S shares X1's), at least one;
-    // one at a time also where the device has no room for more
-    const double keep = 1e9;
-    int G = std::min(KMO_G, N), s = TCE_OK;
-    while (G > 1 && (double)G * (std::max(n1, n3) + n2) * sizeof(double2) > keep) --G;
-    auto release = [&]() {
-        for (int i = 0; i < 5; ++i) {
-            dfree(h, h->d_kmo[i]);
-            h->d_kmo[i] = nullptr;
-            h->n_kmo[i] = 0;
-        }
+    // k4 per group (S shares X1's buffer): as many as the pool keeps the buffers
+    // of, at least one; one also where the device has no room for more
+    int G = std::min(KMO_G, N);
+    auto bytes = [&](int g) { return sizeof(double2) * ((size_t)g * (std::max(n1, n3) + n2) + nout + nC + nph); };
+    while (G > 1 && bytes(G) > TCE_POOL_KEEP) --G;
+    double2 *d_ph = nullptr, *d_C = nullptr, *d_X1 = nullptr, *d_X2 = nullptr, *d_out = nullptr;
+    CallMemory mem(h->st);
+    auto take = [&](int g) {
+        return mem.get(&d_ph, nph) && mem.get(&d_C, nC) && mem.get(&d_X1, g * std::max(n1, n3)) && mem.get(&d_X2, g * n2) &&
+               mem.get(&d_out, nout);
     };
-    for (;;) {
-        const size_t need[5] = {nph, nC, G * std::max(n1, n3), G * n2, nout};
-        s = TCE_OK;
-        for (int i = 0; i < 5 && s == TCE_OK; ++i) {   // workspaces grow with the largest call and stay with the handle
-            if (h->n_kmo[i] >= need[i]) continue;
-            dfree(h, h->d_kmo[i]);
-            h->d_kmo[i] = nullptr;
-            h->n_kmo[i] = 0;
-            if ((s = dalloc(h, &h->d_kmo[i], need[i])) == TCE_OK) h->n_kmo[i] = need[i];
-        }
-        if (s == TCE_OK) break;
-        release();
-        if (G == 1) return s;
+    if (!take(G)) {
+        mem.drop_all();
+        const int first = G;
         G = 1;
+        if (first == 1 || !take(1))
+            return fail(h, TCE_ERR_NOMEM, "device allocation of " + std::to_string(bytes(1)) + " bytes failed");
     }
-    double2 *d_ph = h->d_kmo[0], *d_C = h->d_kmo[1], *d_X1 = h->d_kmo[2], *d_X2 = h->d_kmo[3], *d_out = h->d_kmo[4];
     CK(h, cudaMemcpyAsync(d_ph, ph.data(), sizeof(double2) * nph, cudaMemcpyHostToDevice, h->st));
     CK(h, cudaMemcpyAsync(d_C, coeff, sizeof(double2) * nC, cudaMemcpyHostToDevice, h->st));
     CK(h, cudaFuncSetAttribute(k_kmo_q, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
@@ -269,6 +260,5 @@ extern "C" int tce_ao_to_kmo(void *handle, const double *coeff, int32_t p_lo, in
     }
     CK(h, cudaMemcpyAsync(out, d_out, sizeof(double2) * nout, cudaMemcpyDeviceToHost, h->st));
     CK(h, cudaStreamSynchronize(h->st));
-    if ((double)(h->n_kmo[2] + h->n_kmo[3] + h->n_kmo[4]) * sizeof(double2) > keep) release();   // large ones are given back
     return TCE_OK;
 }

@@ -22,6 +22,7 @@
 #include <vector>
 
 #include "../../include/tce.h"
+#include "tce_pool.h"
 
 using namespace nvcuda;
 
@@ -349,18 +350,6 @@ __global__ void k_mp2_energy(Mp2Dims D, const int *crd, const double2 *G, const 
     }
 }
 
-template <class T>
-int dmalloc(T **p, size_t n, std::vector<void *> &keep)
-{
-    *p = nullptr;
-    if (cudaMalloc((void **)p, (n ? n : 1) * sizeof(T)) != cudaSuccess) {
-        cudaGetLastError();
-        return mp2_fail(TCE_ERR_NOMEM, "device allocation of " + std::to_string(n * sizeof(T)) + " bytes failed");
-    }
-    keep.push_back(*p);
-    return TCE_OK;
-}
-
 }  // namespace
 
 extern "C" {
@@ -392,32 +381,20 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
     Mp2Dims D{ncell, no, nv, nau, ov, {ncl[0], ncl[1], ncl[2]}};
     const size_t nL = (size_t)ov * nau * ncell * ncell;
     const size_t nG = (size_t)ov * ov * ncell * ncell * ncell;
-    std::vector<void *> keep;
-    auto cleanup = [&]() {
-        for (void *p : keep) cudaFree(p);
-    };
+    tcehost::CallMemory mem(nullptr);   // the legacy stream, on which all of this runs
     int *d_crd = nullptr, *d_oo = nullptr, *d_ov = nullptr;
     double2 *d_L = nullptr, *d_G = nullptr;
     double *d_eo = nullptr, *d_ev = nullptr, *d_acc = nullptr;
     unsigned long long *d_nz = nullptr;
-    int s = 0;
-    if (!s) s = dmalloc(&d_crd, 3 * (size_t)ncell, keep);
-    if (!s) s = dmalloc(&d_oo, (size_t)ncell * no, keep);
-    if (!s) s = dmalloc(&d_ov, (size_t)ncell * nv, keep);
+    bool ok = mem.get(&d_crd, 3 * (size_t)ncell) && mem.get(&d_oo, (size_t)ncell * no) && mem.get(&d_ov, (size_t)ncell * nv) &&
+              mem.get(&d_eo, (size_t)ncell * no) && mem.get(&d_ev, (size_t)ncell * nv) && mem.get(&d_acc, 3) && mem.get(&d_nz, 1);
+    if (l_dev) d_L = reinterpret_cast<double2 *>(const_cast<double *>(L));
+    else ok = ok && mem.get(&d_L, nL);
     // the fused FP64 kernel where its tiles fit a block's shared memory, else G in memory
     const size_t fsmem = sizeof(double2) * MP2_FW * ((size_t)4 * ov * nau + (size_t)2 * ov * ov);
     const bool fused = mode == 0 && fsmem <= 200 * 1024;
-    if (l_dev) d_L = reinterpret_cast<double2 *>(const_cast<double *>(L));
-    else if (!s) s = dmalloc(&d_L, nL, keep);
-    if (!s && !fused) s = dmalloc(&d_G, nG, keep);
-    if (!s) s = dmalloc(&d_eo, (size_t)ncell * no, keep);
-    if (!s) s = dmalloc(&d_ev, (size_t)ncell * nv, keep);
-    if (!s) s = dmalloc(&d_acc, 3, keep);
-    if (!s) s = dmalloc(&d_nz, 1, keep);
-    if (s) {
-        cleanup();
-        return s;
-    }
+    ok = ok && (fused || mem.get(&d_G, nG));
+    if (!ok) return mp2_fail(TCE_ERR_NOMEM, "device allocation of " + std::to_string(sizeof(double2) * (fused ? nL : nL + nG)) + " bytes failed");
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
@@ -429,12 +406,15 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
     cudaMemcpy(d_ev, eps_v, sizeof(double) * ncell * nv, cudaMemcpyHostToDevice);
     cudaMemset(d_acc, 0, sizeof(double) * 3);
     cudaMemset(d_nz, 0, sizeof(unsigned long long));
+    int dev = 0, nsm = 148;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
     cudaEventRecord(e0);
     if (fused) {
         cudaFuncSetAttribute(k_mp2_fused, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem);
         int per = 0;
         cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_mp2_fused, 32 * MP2_FW, fsmem);
-        const long long blocks = std::min<long long>((long long)ncell * ncell, 148LL * std::max(per, 1));
+        const long long blocks = std::min<long long>((long long)ncell * ncell, (long long)nsm * std::max(per, 1));
         k_mp2_fused<<<(unsigned)blocks, 32 * MP2_FW, fsmem>>>(D, d_crd, d_L, d_eo, d_oo, d_ev, d_ov, d_acc, d_nz);
     } else if (mode == 0) {
         k_ovov_fp64<<<148 * 16, 256>>>(D, d_crd, d_L, d_G);
@@ -445,7 +425,8 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
         const size_t smem = sizeof(__nv_bfloat16) * ((size_t)2 * MP * KP + (size_t)4 * NP * KP) +
                             sizeof(float) * MP2_WARPS * 2 * 256;
         if (smem > 200 * 1024) {
-            cleanup();
+            cudaEventDestroy(e0);
+            cudaEventDestroy(e1);
             return mp2_fail(TCE_ERR_UNSUPPORTED, "nau too large for the tensor-core tile");
         }
         cudaFuncSetAttribute(k_ovov_bf16, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -458,7 +439,6 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
     cudaEventRecord(e1);
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) {
-        cleanup();
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
         return mp2_fail(TCE_ERR_CUDA, std::string("DF-MP2 kernels: ") + cudaGetErrorString(e));
@@ -474,7 +454,6 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
     if (nzero) *nzero = (int64_t)nz;
     if (gzero) *gzero = acc[2];
     if (ms) *ms = t;
-    cleanup();
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     return TCE_OK;
