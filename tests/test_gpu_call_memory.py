@@ -106,17 +106,21 @@ def test_dfmp2_peak_memory():
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-def test_dfmp2_energy_without_room_for_g(mode):
-    """Where the 354 MB of G do not fit, the FP64 energy comes from the kernel that
-    holds no G, and the split-BF16 one is refused with an error, not a fault."""
+@pytest.mark.parametrize("ncl,no,nv,nau,room", [((96, 1, 1), 1, 5, 16, 200), ((3, 3, 3), 2, 3, 7, 8)])
+def test_dfmp2_energy_without_room_for_g(ncl, no, nv, nau, room, mode):
+    """Where G (354 and 11 MB) does not fit, the FP64 energy comes from the kernel
+    that holds no G, and the split-BF16 one is refused with an error."""
     from william_ci_b200.engine import TCEError, dfmp2_energy
     rng = np.random.default_rng(2)
-    N, nv, nau = 96, 5, 16
-    L = (rng.standard_normal((1, nv, nau, N, N)) + 1j * rng.standard_normal((1, nv, nau, N, N))) * 0.05
-    args = ((N, 1, 1), L, np.full((N, 1), -0.5), np.full((N, 1), 2, dtype=np.int32), 0.2 + rng.random((N, nv)),
+    N = int(np.prod(ncl))
+    L = (rng.standard_normal((no, nv, nau, N, N)) + 1j * rng.standard_normal((no, nv, nau, N, N))) * 0.05
+    args = (ncl, L, -0.5 - rng.random((N, no)), np.full((N, no), 2, dtype=np.int32), 0.2 + rng.random((N, nv)),
             np.zeros((N, nv), dtype=np.int32))
+    args[2][:, 0] = args[4][:, 0] = 0.0                        # zero-gap terms: left out and counted
+    args[3][2, no - 1] = 0
     ref = dfmp2_energy(*args, mode=mode)
-    with _Filled(200 * MB):
+    assert ref["nzero"] > 0
+    with _Filled(room * MB):
         if mode == 0:
             got = dfmp2_energy(*args, mode=0)
             assert abs(got["emp2"] - ref["emp2"]) <= 1e-12 * abs(ref["emp2"]) and got["nzero"] == ref["nzero"]

@@ -99,13 +99,13 @@ __global__ void k_ovov_fp64(Mp2Dims D, const int *crd, const double2 *L, double2
     }
 }
 
-// FP64 contraction and energy in one kernel, no G array: the exchange partner of
-// triple (ki, ka, kj) is the direct block of (ki, kb, kj), kb = ki - ka + kj, whose
-// own partner is ka.  A block takes one (ki, kj); its warps take the pairs
-// {ka, kb}: the four L tiles of a pair go to shared memory, both direct blocks
-// G(ka), G(kb) are formed there and both triples' energies follow.
-// G through memory cost 354 MB written and read (and allocated) per call on 96
-// cells with 5 bands; L (12 MB) stays in the L2.
+// FP64 contraction and energy in one kernel, no G array (systems whose G does not
+// fit the device): the exchange partner of triple (ki, ka, kj) is the direct block
+// of (ki, kb, kj), kb = ki - ka + kj, whose own partner is ka.  A block takes one
+// (ki, kj); its warps take the pairs {ka, kb}: the four L tiles of a pair go to
+// shared memory, both direct blocks G(ka), G(kb) are formed there and both triples'
+// energies follow.  Bound by the tiles' index arithmetic and the lanes that ov^2
+// leaves idle; with large tiles by four warps per SM.
 constexpr int MP2_FW = 4;   // warps per block
 __global__ void __launch_bounds__(32 * MP2_FW) k_mp2_fused(Mp2Dims D, const int *crd, const double2 *__restrict__ L, const double *eo,
                                                            const int *oo, const double *ev, const int *ov_,
@@ -390,10 +390,14 @@ int tce_mp2_energy_on(int32_t ncell, const int32_t ncl[3], const int32_t *kcoord
               mem.get(&d_eo, (size_t)ncell * no) && mem.get(&d_ev, (size_t)ncell * nv) && mem.get(&d_acc, 3) && mem.get(&d_nz, 1);
     if (l_dev) d_L = reinterpret_cast<double2 *>(const_cast<double *>(L));
     else ok = ok && mem.get(&d_L, nL);
-    // the fused FP64 kernel where its tiles fit a block's shared memory, else G in memory
+    // G through memory; where the device has no room for it, the FP64 kernel that
+    // holds none, if its tiles fit a block.  (That kernel is the slower one: ms of
+    // the kernels with G / without, 96 cells ov 5 nau 16 0.86 / 1.22, 200 cells 8.2 /
+    // 10.5, 32 cells ov 12 nau 24 0.26 / 0.45, 48 cells ov 4 nau 64 0.17 / 0.53, 64
+    // cells ov 16 nau 32 4.2 / 9.3.)
     const size_t fsmem = sizeof(double2) * MP2_FW * ((size_t)4 * ov * nau + (size_t)2 * ov * ov);
-    const bool fused = mode == 0 && fsmem <= 200 * 1024;
-    ok = ok && (fused || mem.get(&d_G, nG));
+    bool fused = false;
+    if (ok && !mem.get(&d_G, nG)) ok = fused = mode == 0 && fsmem <= 200 * 1024;
     if (!ok) return mp2_fail(TCE_ERR_NOMEM, "device allocation of " + std::to_string(sizeof(double2) * (fused ? nL : nL + nG)) + " bytes failed");
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
