@@ -652,8 +652,9 @@ def main():
     # kernel form (CUDA cores or FP64 tensor cores) per work list, chosen by timing both
     tune = eng.lg_autotune(3) if world == 1 else None
     if tune is not None:
-        names = {0: "generic", 1: "all-s", 2: "one-p"}
-        shapes = {1: {1: "16x32", 2: "32x16", 3: "16x16", 4: "8x64", 5: "8x32"}, 2: {1: "8x32", 2: "16x32", 3: "8x64"}}
+        names = {0: "generic", 1: "all-s", 2: "s/p"}
+        # primitive quartets x nodes per pass
+        shapes = {1: {1: "16x8", 2: "16x16", 3: "8x8", 4: "8x16"}, 2: {1: "8x16", 2: "8x8"}}
 
         def form(w):
             if not w["tc"]:

@@ -416,10 +416,9 @@ def test_learned_grid_setup_from_the_c_abi(systems):
 
 def test_every_all_s_tile_shape_gives_the_same_jk(chain16_lg):
     """The all-s tensor-core kernel in each tile shape the autotuner can pick
-    (16 x 32, 32 x 16, 16 x 16, 8 x 64, 8 x 32 primitive quartets x nodes per
-    pass),
-    set by hand on every all-s list: J/K equal the CUDA-core kernel's to 1e-12
-    of the density scale."""
+    (16 x 8, 16 x 16, 8 x 8, 8 x 16 primitive quartets x nodes per pass; 5 is
+    taken as 2), set by hand on every all-s list: J/K equal the CUDA-core
+    kernel's to 1e-12 of the density scale."""
     from william_ci_b200.engine import TCE_METHOD_LEARNED
     sysm, eng, net = chain16_lg
     P = random_density(sysm.nbas, 9) * 0.05
@@ -438,6 +437,7 @@ def test_every_all_s_tile_shape_gives_the_same_jk(chain16_lg):
     for shape in (1, 2, 3, 4, 5):
         for i in alls:
             eng.lg_set_list_form(i, shape)
+            assert eng.lg_lists()[i]["tc"] == (2 if shape == 5 else shape)   # one number per kernel
         J, K = eng.direct_JK(P)
         assert np.abs(J - J0).max() <= 1e-12 * scale and np.abs(K - K0).max() <= 1e-12 * scale, shape
     for i in alls:
@@ -445,10 +445,10 @@ def test_every_all_s_tile_shape_gives_the_same_jk(chain16_lg):
 
 
 def test_every_one_p_tile_shape_gives_the_same_jk(chain16_lg):
-    """The one-p tensor-core kernel (both power combinations per step loop,
+    """The s/p tensor-core kernel (every power combination in one step loop,
     the real directions by moments) in each tile shape the autotuner can pick
-    (8 x 32, 16 x 32 and, for 64-node rules, 8 x 64 primitive quartets x nodes
-    per pass), set by hand on every one-p list: J/K equal the CUDA-core
+    (8 x 16 and 8 x 8 primitive quartets x nodes per pass; 3 is taken as 2 for
+    64-node rules), set by hand on every s/p list: J/K equal the CUDA-core
     kernel's to 1e-12 of the density scale, with no more judge rejects."""
     from william_ci_b200.engine import TCE_METHOD_LEARNED
     sysm, eng, net = chain16_lg
@@ -468,6 +468,7 @@ def test_every_one_p_tile_shape_gives_the_same_jk(chain16_lg):
     for shape in (1, 2, 3):
         for i, nq in onep:
             eng.lg_set_list_form(i, shape if shape <= (3 if nq == 64 else 2) else 1)
+            assert eng.lg_lists()[i]["tc"] <= 2
         J, K = eng.direct_JK(P)
         assert eng.lg_stats()["rejected"] == 0
         assert np.abs(J - J0).max() <= 1e-12 * scale and np.abs(K - K0).max() <= 1e-12 * scale, shape

@@ -101,9 +101,14 @@ int tce_launch_quartets_sp_tc(const DevSys &S, int cls, const SArgsHost &h, int 
 int tce_tc_shapes_sp(int nq);
 // Default tile shapes by the torus' length (in orders, ncap): on long ones the
 // strides differ much from node to node, and passes of 8 nodes need fewer orders
-// than passes of 16, which build fewer fragments.  Measured (ms, 8 against 16
-// nodes per pass): 64 cells (ncap 592) all-s 64-node list 6.4 / 7.4, one-p lists
-// 1.3 / 1.5; 16 cells (ncap 166) 1.45 / 1.30 and 0.36 / 0.32.
+// than passes of 16, which build fewer fragments.  The line lies where the two
+// cross on the chain (ms, 8 against 16 nodes per pass; all-s 32-node lists / all-s
+// 64-node lists / all one-p lists; three spacings and exponent seeds agree):
+//   ncap 166   0.90, 0.88    1.62, 1.44    1.85, 1.64
+//        237   1.25, 1.29    2.33, 2.21    2.51, 2.34
+//        308   1.48, 1.65    3.22, 3.18    3.15, 3.11
+//        379   1.66, 1.99    4.14, 4.30    3.78, 4.01
+//        592   2.48, 3.42    6.88, 8.00    5.82, 6.86
 inline int tce_tc_shape_s(const DevSys &S) { return S.ndp > 1 || S.ncap >= 300 ? 1 : 2; }
 inline int tce_tc_shape_sp(const DevSys &S) { return S.ncap >= 300 ? 2 : 1; }
 inline bool tce_r1_supported(int ndp, int nq, int cls)

@@ -1,7 +1,7 @@
 // tce_kernels_sp2.cu -- the s/p tensor-core kernel (k_quartets_sp_tc,
 // tce_kernels_tc.cuh) for the six classes with two p shells of one periodic
 // direction (four power combinations per step loop), learned grid and system
-// rule: 8 primitive quartets x 16 (shape 1) or 8 (shapes 2 and 3) nodes per pass.
+// rule: 8 primitive quartets x 16 (shape 1) or 8 (shape 2) nodes per pass.
 #include "tce_kernels_tc.cuh"
 
 template <int NT, bool LG>

@@ -329,10 +329,10 @@ __global__ void __launch_bounds__(256, 2) k_quartets_s_tc(DevSys S, SArgs A)
 
 int tce_tc_shapes_sp(int nq)
 {
-    return nq == 64 ? 3 : nq == 32 ? 2 : 0;
+    return (nq == 32 || nq == 64) ? 2 : 0;
 }
 
-// one p shell.  shape 1: 8 rows x 16 nodes per pass, 2 and 3: 8 x 8
+// one p shell.  shape 1: 8 rows x 16 nodes per pass, 2: 8 x 8
 template <bool LG>
 static int sp1_launch(const DevSys &S, int cls, const SArgs &A, int shape, int nsm, cudaStream_t st)
 {
@@ -355,7 +355,7 @@ int tce_launch_quartets_sp_tc(const DevSys &S, int cls, const SArgsHost &h, int 
     if (lg && (!h.rules || !h.rule_T || !h.fb_items || !h.fb_count)) return TCE_ERR_ARG;
     if (S.ndp != 1) return TCE_ERR_UNSUPPORTED;
     if (lg && (nq != 32 && nq != 64)) return TCE_ERR_UNSUPPORTED;
-    if (shape < 1 || shape > 3) return TCE_ERR_ARG;
+    if (shape < 1 || shape > 2) return TCE_ERR_ARG;
     const int np = __builtin_popcount(cls & 15);
     if (cls < 1 || cls > 15 || np > 2) return TCE_ERR_UNSUPPORTED;
     SArgs A{};
@@ -371,16 +371,16 @@ int tce_launch_quartets_sp_tc(const DevSys &S, int cls, const SArgsHost &h, int 
 
 int tce_tc_shapes_s(int nq)
 {
-    return (nq == 32 || nq == 64) ? 5 : 0;
+    return (nq == 32 || nq == 64) ? 4 : 0;
 }
 
-// shape 1: 16 rows x 8 nodes per pass, 2 and 5: 16 x 16, 3: 8 x 8, 4: 8 x 16
+// shape 1: 16 rows x 8 nodes per pass, 2: 16 x 16, 3: 8 x 8, 4: 8 x 16
 int tce_launch_quartets_s_tc(const DevSys &S, const SArgsHost &h, int nq, int shape, cudaStream_t st)
 {
     const bool lg = h.item_rule != nullptr;
     if (lg && (!h.rules || !h.rule_T || !h.fb_items || !h.fb_count)) return TCE_ERR_ARG;
     if (lg && (nq != 32 && nq != 64)) return TCE_ERR_UNSUPPORTED;
-    if (shape < 1 || shape > 5) return TCE_ERR_ARG;
+    if (shape < 1 || shape > 4) return TCE_ERR_ARG;
     SArgs A{};
     tc_args(A, h);
     if (cudaMemsetAsync(h.next, 0, sizeof(unsigned int), st) != cudaSuccess) return TCE_ERR_CUDA;
@@ -399,9 +399,9 @@ int tce_launch_quartets_s_tc(const DevSys &S, const SArgsHost &h, int nq, int sh
     } else {
         switch (shape) {
         case 1: TCE_S_TC(1, 2, 1, true); break;
+        case 2: TCE_S_TC(1, 2, 2, true); break;
         case 3: TCE_S_TC(1, 1, 1, true); break;
-        case 4: TCE_S_TC(1, 1, 2, true); break;
-        default: TCE_S_TC(1, 2, 2, true); break;
+        default: TCE_S_TC(1, 1, 2, true); break;
         }
     }
 #undef TCE_S_TC

@@ -1478,6 +1478,9 @@ int tce_lg_set_list_form(void *handle, int32_t list, int32_t form)
     if (!h) return fail(h, TCE_ERR_ARG, "NULL handle");
     if (list < 0 || list >= (int32_t)h->lg_lists.size()) return fail(h, TCE_ERR_ARG, "no such work list");
     auto &w = h->lg_lists[(size_t)list];
+    // 5 (all-s) and 3 (s/p, 64 nodes) were shapes of their own: still taken, as the 16-node shapes they run
+    if (h->ndp == 1 && w.kind == 1 && form == 5 && lg_nforms(h, w) > 1) form = 2;
+    if (w.kind == 2 && form == 3 && w.nq == 64 && lg_nforms(h, w) > 1) form = 2;
     if (form < 0 || form >= lg_nforms(h, w)) return fail(h, TCE_ERR_ARG, "the list has no such kernel form");
     const int key = ((w.kind * 16 + w.cls) * 2 + (w.nq == 64 ? 1 : 0)) * 2 + (w.fp32 ? 1 : 0);
     h->tc_choice[key] = form;
