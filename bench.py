@@ -51,7 +51,7 @@ NAMED = {"li_cube": {"shard": 256, "train": 6000,
          "h2_sheet": {"shard": 1024, "train": 3000,
                       "workload": "Tori2D H2 sheet, 8x8 cells, d=2.0, L=16x16 bohr, 2s+1p+1d per H, nbas=1408"}}
 L2_FLUSH_BYTES = 512 << 20
-FP32_THRESHOLD = 1e-6        # Schwarz product below which the node sums run in FP32
+FP32_THRESHOLD = 1e-6        # Schwarz product below which a list may run its node sums in FP32 (where that is faster)
 
 
 def parse():
@@ -641,11 +641,17 @@ def main():
         return float(t[0]) / steps, float(t[1])
 
     nq_total = info["n_func_quartets"]
-    # FP32 panels (Schwarz product < 1e-6): their J/K error against the all-FP64 pass
+    # FP32 panels (Schwarz product < 1e-6), the CUDA-core form of their lists: their J/K error
+    # against the all-FP64 pass
     eng.set_method(TCE_METHOD_LEARNED)
     J64, K64 = eng.direct_JK(Ph)
     eng.set_fp32_threshold(FP32_THRESHOLD)
+    panels = {i: w["tc"] for i, w in enumerate(eng.lg_lists()) if w["fp32"]}
+    for i in panels:
+        eng.lg_set_list_form(i, 0)
     J32, K32 = eng.direct_JK(Ph)
+    for i, form_ in panels.items():
+        eng.lg_set_list_form(i, form_)
     fp32 = {"threshold": FP32_THRESHOLD, "quartets": eng.lg_stats()["fp32"],
             "max_abs_jk_diff_vs_fp64": float(max(np.abs(J32 - J64).max(), np.abs(K32 - K64).max())),
             "density_abs_sum": float(np.abs(Ph).sum())}
@@ -715,8 +721,8 @@ def main():
     single_err, single_rej = pass_error(eng, ho, np.full(len(ho), single), T_ho, offs_ho)
     single_plain = eng.lg_stats()["plain_direct"]
     eng.lg_set_item_rules(net_rules)
-    # the reference's own rules on the learned grid's kernels (tensor cores, FP32 panels,
-    # autotuned forms; the 40-node rule padded to 64 nodes): a one-rule dictionary whose Gauss
+    # the reference's own rules on the learned grid's kernels (tensor cores, autotuned forms;
+    # the 40-node rule padded to 64 nodes): a one-rule dictionary whose Gauss
     # weights are its own weights, so that the judge accepts every block; the blocks are those
     # of the fixed_rule and rule_40_node arms
     from william_ci_b200 import learned_grid as LGm
@@ -837,7 +843,8 @@ def main():
                                     if world > 1 else "single GPU",
                                     "quadrature": "learned grid: per-quartet Gauss-Kronrod rule (K15..K61, 21 map "
                                                   "scales) picked by the network, judge <= 1e-10, plain fallback; "
-                                                  "FP32 node sums below Schwarz 1e-6",
+                                                  "few Bessel orders in FP64, lists below Schwarz 1e-6 in FP32 "
+                                                  "panels where those are faster",
                                     "shell_quartets": info["n_shell_quartets"],
                                     "function_quartets": nq_total}),
             "plain": {"value": nq_total / (plain_ms * 1e-3), "ms_per_step": plain_ms, "steps": plain_steps,
@@ -858,7 +865,7 @@ def main():
             "fixed_rule_tensor_cores": {"value": nq_total / (r32tc_ms * 1e-3), "ms_per_step": r32tc_ms,
                                         "max_err_vs_oracle_table128": err32tc,
                                         "method": "the reference's default 32-node rule on the learned grid's "
-                                                  "kernels (FP64 tensor cores, FP32 panels, autotuned forms)"},
+                                                  "kernels (FP64 tensor cores, autotuned forms)"},
             "list_chains": {"two_chains_ms_per_step": ms_step, "one_chain_ms_per_step": one_chain_ms,
                             "note": "the learned-grid lists split into two cost-balanced chains on two streams "
                                     "(the default, the headline) or run one after another on one stream"},

@@ -257,8 +257,11 @@ def test_one_and_two_list_chains_give_the_same_jk(chain16_lg):
 
 
 def test_fp32_panels_error_vs_fp64(chain16_lg):
-    """FP32 node sums for quartets with Schwarz product below 1e-6: the J/K
-    difference from the all-FP64 pass stays below 1e-10 per unit density."""
+    """FP32 node sums for quartets with Schwarz product below a threshold, in the
+    lists' CUDA-core form (their default form sums few orders in FP64): below 1e-6
+    the J/K difference from the all-FP64 pass stays within 1e-10 per unit density.
+    That the sums are FP32 shows at the largest threshold, 1e-3, against a control:
+    the FP64 CUDA-core form of the same classes, whose difference is rounding."""
     from william_ci_b200.engine import TCE_METHOD_LEARNED
     sysm, eng, net = chain16_lg
     P = random_density(sysm.nbas, 4) * 0.05
@@ -266,13 +269,25 @@ def test_fp32_panels_error_vs_fp64(chain16_lg):
     eng.set_method(TCE_METHOD_LEARNED)
     eng.set_fp32_threshold(0.0)
     J0, K0 = eng.direct_JK(P)
-    eng.set_fp32_threshold(1e-6)
-    J1, K1 = eng.direct_JK(P)
-    st = eng.lg_stats()
+    err = {}
+    for thr in (0.0, 1e-6, 1e-3):
+        eng.set_fp32_threshold(thr)
+        lists = eng.lg_lists()
+        core = [i for i, w in enumerate(lists) if (w["fp32"] if thr else w["kind"])]
+        assert core
+        default = {i: lists[i]["tc"] for i in core}
+        assert all(default.values())
+        for i in core:
+            eng.lg_set_list_form(i, 0)
+        J1, K1 = eng.direct_JK(P)
+        st = eng.lg_stats()
+        assert st["fp32"] > 0.2 * st["learned"] if thr else st["fp32"] == 0
+        err[thr] = max(np.abs(J1 - J0).max(), np.abs(K1 - K0).max())
+        for i in core:
+            eng.lg_set_list_form(i, default[i])
     eng.set_fp32_threshold(0.0)
-    assert st["fp32"] > 0.2 * st["learned"]
-    err = max(np.abs(J1 - J0).max(), np.abs(K1 - K0).max())
-    assert err <= 1e-10 * scale, err
+    assert err[1e-6] <= 1e-10 * scale, err
+    assert err[1e-3] > 10 * err[0.0], err
 
 
 def test_graph_on_the_legacy_stream(chain16_lg):
