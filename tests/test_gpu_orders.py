@@ -54,6 +54,17 @@ def _split_p(name, ncell):
     return s
 
 
+def _with_d(name, ncell):
+    """The chain with the sheet's s, p, d basis and its second atom off the axis."""
+    import pyoracle
+    from william_ci_b200 import system as S
+    cell, _ = S.workload(name)
+    cell = dataclasses.replace(cell, atoms=cell.atoms + [(cell.atoms[0][0], (0.7, 0.9, -0.4))])
+    s = S.build_system(S.scaled_down(cell, ncell), S.workload("h2_sheet")[1])
+    pyoracle.normalize(s)
+    return s
+
+
 CASES = [
     ("h2_ring", (2, 1, 1), None, False),        # antipodal pairs: Bessel argument 0
     ("h_chain64", (1, 1, 1), 3.0, False),       # one cell, small arguments
@@ -62,6 +73,12 @@ CASES = [
     ("h_chain64", (7, 1, 1), 30.0, True),       # long torus: large strides, phases past the width
     ("h2_sheet", (2, 2, 1), None, False),
     ("li_cube", (2, 2, 2), None, False),
+]
+LONG = [    # long tori of two and three directions, one of them ragged: strides above 1, phases past the width
+    ("h2_sheet", (3, 1, 1), 25.0, False),
+    ("h2_sheet", (2, 2, 1), 25.0, True),
+    ("li_cube", (3, 1, 2), 25.0, False),
+    ("li_cube", (2, 2, 1), 25.0, True),
 ]
 
 
@@ -112,6 +129,41 @@ def test_tensor_cores_off(name, ncell, spacing, off, nquad):
         got.append(eng.direct_JK(P))
     for J, K in got:
         assert np.abs(J - J0[:len(J)]).max() <= EVERY * scale and np.abs(K - K0[:len(K)]).max() <= EVERY * scale
+
+
+@pytest.mark.parametrize("nquad", [32, 64])
+@pytest.mark.parametrize("name,ncell,spacing,off", LONG)
+def test_long_tori_of_two_and_three_directions(name, ncell, spacing, off, nquad):
+    """Strided sums against every order on the same power vectors (the engine's
+    CUDA-core form).  Not against the oracle: at Bessel arguments of 1e4 its d_k
+    sums, and not the orders, set the difference (1.1e-12 of the density's sum on
+    the ragged sheet, where these two forms agree to 1e-17)."""
+    from william_ci_b200.engine import Engine
+    s = _system(name, ncell, spacing, off)
+    P = random_density(s.nbas, 5) * 0.05
+    with Engine(s, nquad=nquad) as eng:
+        J, K = eng.direct_JK(P)
+        eng.set_tensor_cores(False)
+        J0, K0 = eng.direct_JK(P)
+    scale = np.abs(P).sum()
+    assert np.abs(J0).max() > 0
+    assert np.abs(J - J0).max() <= 1e-12 * scale and np.abs(K - K0).max() <= 1e-12 * scale
+
+
+@pytest.mark.parametrize("cores", [True, False])
+def test_d_shells_of_one_direction_off_the_axis(cores):
+    """J and K of s, p and d shells with one periodic direction and R != 0 in the real ones."""
+    import pyoracle
+    from william_ci_b200.engine import Engine
+    s = _with_d("h_chain64", (2, 1, 1))
+    P = random_density(s.nbas, 5) * 0.05
+    t, w = pyoracle.fast_quad(32)
+    J0, K0 = pyoracle.Oracle(s, t_nodes=t, t_weights=w).direct_jk(P)[:2]
+    with Engine(s, t_nodes=t, t_weights=w) as eng:
+        eng.set_tensor_cores(cores)
+        J, K = eng.direct_JK(P)
+    tol = (1e-12 if cores else EVERY) * np.abs(P).sum()
+    assert np.abs(J - J0).max() <= tol and np.abs(K - K0).max() <= tol
 
 
 @pytest.mark.parametrize("nquad", [32, 64])
@@ -189,3 +241,9 @@ def _learned_against_plain(s):
 
 def test_learned_grid_p_functions_that_are_no_full_shell():
     assert 2 not in _learned_against_plain(_split_p("h_chain64", (6, 1, 1)))
+
+
+def test_learned_grid_pairs_of_p_shells_off_the_axis():
+    """(pp|ss) and (ss|pp) with R != 0: the (1,0) and (0,1) power vectors of a pair
+    differ, and the s/p kernel takes each for its own component."""
+    assert 2 in _learned_against_plain(_system("h_chain64", (6, 1, 1), None, True))
