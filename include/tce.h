@@ -201,8 +201,11 @@ int tce_set_graph(void *handle, int32_t on);
  * the generic kernel.  They sum the few Bessel orders that a sum's decay and
  * the function's width leave, to rounding; off gives the FP64 CUDA-core
  * kernels, which sum every order of the reference's truncation.  Default on.
- * Shell blocks of tce_create_blocks handles (density fitting) always take
- * every order.  No reference counterpart. */
+ * J/K, stored integrals, shell blocks and the nuclear attraction follow it; the
+ * blocks of tce_create_blocks handles (density fitting) always take every order.
+ * A change cuts the work lists again for the kernels that run them (the indices of
+ * tce_lg_lists change, the forms set for each setting are kept).  No reference
+ * counterpart. */
 int tce_set_tensor_cores(void *handle, int32_t on);
 
 /* The learned-grid work lists of a pass as n chains (1 or 2; default 2): the

@@ -56,3 +56,23 @@ def test_stored_integrals_of_a_shard_follow_the_switch(systems, name, ncell):
         eng.set_shard(1, 2)
         got = eng.ERI_integral_toroidal()
     assert np.array_equal(got, ref), np.abs(got - ref).max()
+
+
+def test_list_forms_of_each_setting_are_kept_apart(systems):
+    """The generic classes are numbered by p and d shells with the tensor cores on, by
+    d shells with them off: a form set for one is no form of the other's lists."""
+    from william_ci_b200.engine import TCE_METHOD_LEARNED, Engine
+    with Engine(systems("h2_sheet", (2, 2, 1))) as eng:
+        eng.lg_setup(n_train=1500, seed=2026, epochs=20)
+        eng.set_method(TCE_METHOD_LEARNED)
+        generic = [i for i, w in enumerate(eng.lg_lists()) if w["kind"] == 0]
+        eng.lg_set_list_form(generic[-1], 0)          # kept over the other setting
+        chosen = eng.lg_lists()
+        assert chosen[generic[-1]]["tc"] == 0
+        eng.set_tensor_cores(False)
+        for i, w in enumerate(eng.lg_lists()):
+            if w["kind"] == 0:
+                assert w["cls"] <= 4
+                eng.lg_set_list_form(i, 0)
+        eng.set_tensor_cores(True)
+        assert eng.lg_lists() == chosen

@@ -414,6 +414,13 @@ static void fill_common(Handle *h, QuartetHostArgs &a)
     a.pp_rw = h->d_pp;
 }
 
+// A list's key in tc_choice.  The generic classes are other ones with the tensor
+// cores off (generic_class), so their choices are kept apart.
+static int lg_choice_key(const Handle *h, const Handle::LgList &w)
+{
+    return (((w.kind * 16 + w.cls) * 2 + (w.nq == 64 ? 1 : 0)) * 2 + (w.fp32 ? 1 : 0)) * 2 + (h->use_tc ? 0 : 1);
+}
+
 int lg_rebuild_lists(Handle *h)
 {
     int s;
@@ -494,7 +501,7 @@ int lg_rebuild_lists(Handle *h)
         w.nq = ((key / 2) & 1) ? 64 : 32;
         w.fp32 = key & 1;
         {
-            auto tcit = h->tc_choice.find(key);
+            auto tcit = h->tc_choice.find(lg_choice_key(h, w));
             if (tcit != h->tc_choice.end()) w.tc = tcit->second;
         }
         w.n = (long long)lg[key].size();
@@ -1385,8 +1392,7 @@ int tce_lg_autotune(void *handle, int32_t reps, int32_t *ntuned, int32_t *nswitc
             if (f != dflt && best[f] < best[alt]) alt = f;
         const double alt_t = best[alt], def_t = best[dflt];
         const int choice = (alt_t < 0.97 * def_t && def_t - alt_t > 0.02) ? alt : dflt;
-        const int key = ((w.kind * 16 + w.cls) * 2 + (w.nq == 64 ? 1 : 0)) * 2 + (w.fp32 ? 1 : 0);
-        h->tc_choice[key] = choice;
+        h->tc_choice[lg_choice_key(h, w)] = choice;
         w.tc = choice;
         ++nt;
         if (choice != dflt) ++nsw;
@@ -1482,8 +1488,7 @@ int tce_lg_set_list_form(void *handle, int32_t list, int32_t form)
     if (h->ndp == 1 && w.kind == 1 && form == 5 && lg_nforms(h, w) > 1) form = 2;
     if (w.kind == 2 && form == 3 && w.nq == 64 && lg_nforms(h, w) > 1) form = 2;
     if (form < 0 || form >= lg_nforms(h, w)) return fail(h, TCE_ERR_ARG, "the list has no such kernel form");
-    const int key = ((w.kind * 16 + w.cls) * 2 + (w.nq == 64 ? 1 : 0)) * 2 + (w.fp32 ? 1 : 0);
-    h->tc_choice[key] = form;
+    h->tc_choice[lg_choice_key(h, w)] = form;
     w.tc = form;
     // the captured pass is re-captured with the new form; rejects of the last
     // pass stay valid (same items and rules)
