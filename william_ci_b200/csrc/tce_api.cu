@@ -522,8 +522,8 @@ int build(Handle *h, const tce_system *sys)
     double2 *d_vec = nullptr;
     if ((s = dalloc(h, &d_vec, (size_t)v_tot))) return s;
     S.vec = d_vec;
-    double *d_rvec = nullptr;
-    if ((s = dalloc(h, &d_rvec, (size_t)r_tot))) return s;
+    double *d_rvec = nullptr;   // read by the all-s and s/p kernels: not by blocks
+    if (!h->blocks_only && (s = dalloc(h, &d_rvec, (size_t)r_tot))) return s;
     S.rvec = d_rvec;
     {
         int stride = h->ncap + 2 * TCE_LMAX + 2;

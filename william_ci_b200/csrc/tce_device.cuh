@@ -274,6 +274,14 @@ __device__ __forceinline__ double2 tce_power_coef(const PowerSeries &ps, const d
     return make_double2(re, im);
 }
 
+// one 8 x 8 tile and step of four on the FP64 tensor cores
+__device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
 __device__ __forceinline__ double tce_warp_sum(double v)
 {
 #pragma unroll

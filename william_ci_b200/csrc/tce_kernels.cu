@@ -217,7 +217,7 @@ __global__ void k_pair_vectors(DevSys S, long long npp_tot, const int *pp_unit, 
                 }
         }
         out[(long long)n * U.npp + loc] = val;
-        if (M == 0 && s == 0) rvec[U.r_off + ((long long)d * U.Nlen + n) * U.npp + loc] = val.x;
+        if (M == 0 && s == 0 && rvec) rvec[U.r_off + ((long long)d * U.Nlen + n) * U.npp + loc] = val.x;
     }
 }
 

@@ -1,18 +1,10 @@
 // tce_kernels_tc.cuh -- pieces shared by the FP64 tensor-core quartet kernels:
-// the mma.sync.m8n8k4 (FP64) wrapper, the primitive pool fill and its order, the
-// rule view, the launch helpers, and the s/p kernel of one periodic direction
+// the primitive pool fill and its order, the rule view, the launch helpers, and the s/p kernel of one periodic direction
 // k_quartets_sp_tc (one or two p shells), instantiated per class in
 // tce_kernels_tc.cu (one p) and tce_kernels_sp2.cu (two p).
 #pragma once
 #include "tce_kernels_s.cuh"
 #include "tce_orders.cuh"
-
-__device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
 
 // Screen the primitive quartets base + lane of a shell quartet (as
 // k_quartets_s) and append the kept ones to the warp's pool: pair indices,

@@ -202,13 +202,6 @@ __global__ void __launch_bounds__(NA_WARPS_MAX * 32) k_nuclear(DevSys S, NaArgs 
     if (lane == 0) A.V[A.plist ? pair : fi + (long long)S.nfuc * fj] = fabs(V) < 1e-14 ? 0.0 : V;
 }
 
-__device__ __forceinline__ void na_dmma(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // One periodic direction: a block per function pair, its warps over the
 // primitive pairs.  Per primitive pair the node sums of every atom,
 //     X(atom, k) = h sum_j F_{h j}(atom) T[h j][k],
@@ -221,9 +214,10 @@ __device__ __forceinline__ void na_dmma(double &d0, double &d1, double a, double
 // What bounds it: with every order (about 250) and powers by pow() it was the
 // epilogue, then the order loop, and 576 of 2304 warps had a 16-fold share.
 // 1 / (p + t^2) is found once per node and primitive pair, the powers are
-// multiplied out.  64-cell chain, 32 nodes: 15.5 -> 3.0 ms per call.
-// A primitive pair whose prefactor leaves nothing above 1e-28 (elements below
-// 1e-14 are set to zero) is skipped.
+// multiplied out.  64-cell chain, 32 nodes: kernel 15 -> 0.48 ms, call 15.5 -> 0.66.
+// A primitive pair whose prefactor times the charges is below 1e-36 is skipped:
+// with powers of distances up to 1e8 it adds less than 1e-28, and elements below
+// 1e-14 are set to zero.
 constexpr int NA_TC_WARPS = 4;
 __global__ void __launch_bounds__(NA_TC_WARPS * 32) k_nuclear_tc(DevSys S, NaArgs A)
 {
@@ -388,11 +382,7 @@ __global__ void __launch_bounds__(NA_TC_WARPS * 32) k_nuclear_tc(DevSys S, NaArg
                 for (int m = 0; m < MT; ++m) {
                     const int src = (lane & ~3) | (2 * m + (hf & 1));
                     const double c = __shfl_sync(0xffffffffu, cs, src), s = __shfl_sync(0xffffffffu, sn, src);
-                    const double c2 = fma(-2.0 * s, s, 1.0), s2 = 2.0 * s * c;
-                    cc[m] = cq == 0 ? 1.0 : cq == 1 ? c : cq == 2 ? c2 : fma(c2, c, -s2 * s);
-                    ss[m] = cq == 0 ? 0.0 : cq == 1 ? s : cq == 2 ? s2 : fma(s2, c, c2 * s);
-                    c4[m] = fma(-2.0 * s2, s2, 1.0);
-                    s4[m] = 2.0 * s2 * c2;
+                    tce_phase_start(c, s, cq, cc[m], ss[m], c4[m], s4[m]);
                 }
                 const double *T = S.Tt + 16 * hf + rq;
                 const int t1 = ntile > 1 ? 8 : 0;
@@ -405,11 +395,9 @@ __global__ void __launch_bounds__(NA_TC_WARPS * 32) k_nuclear_tc(DevSys S, NaArg
 #pragma unroll
                     for (int m = 0; m < MT; ++m) {
                         const double F = g.x * cc[m] - g.y * ss[m];
-                        const double t = cc[m];
-                        cc[m] = fma(t, c4[m], -ss[m] * s4[m]);
-                        ss[m] = fma(ss[m], c4[m], t * s4[m]);
-                        na_dmma(acc[0][m][0], acc[0][m][1], F, T0);
-                        na_dmma(acc[1][m][0], acc[1][m][1], F, T1);
+                        tce_phase_step(cc[m], ss[m], c4[m], s4[m]);
+                        tce_dmma(acc[0][m][0], acc[0][m][1], F, T0);
+                        tce_dmma(acc[1][m][0], acc[1][m][1], F, T1);
                     }
                 }
                 // epilogue: acc[t][m][i] = X(atom 8 m + rq, node 16 hf + 8 t + 2 cq + i) / h

@@ -239,13 +239,6 @@ __device__ __forceinline__ void blk_header(const DevSys &S, const WarpLayout &la
     __syncthreads();
 }
 
-__device__ __forceinline__ void tce_dmma(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 __device__ __forceinline__ double tce_ipow(double x, int k)
 {
     double r = 1.0;
@@ -395,11 +388,7 @@ __device__ __noinline__ void tc_rows(int wofs, int nb, int lane, int g0c)
 #pragma unroll
             for (int m = 0; m < MT; ++m) {
                 const double2 z = cs[m][half];
-                const double c2 = fma(-2.0 * z.y, z.y, 1.0), s2 = 2.0 * z.y * z.x;
-                cc[m] = cq == 0 ? 1.0 : cq == 1 ? z.x : cq == 2 ? c2 : fma(c2, z.x, -s2 * z.y);
-                sc[m] = cq == 0 ? 0.0 : cq == 1 ? z.y : cq == 2 ? s2 : fma(s2, z.x, c2 * z.y);
-                c4[m] = fma(-2.0 * s2, s2, 1.0);
-                s4[m] = 2.0 * s2 * c2;
+                tce_phase_start(z.x, z.y, cq, cc[m], sc[m], c4[m], s4[m]);
             }
 #pragma unroll 1
             for (int n0 = 0; n0 <= last; n0 += h4) {
@@ -414,11 +403,7 @@ __device__ __noinline__ void tc_rows(int wofs, int nb, int lane, int g0c)
                 n += h4;
                 load();
 #pragma unroll
-                for (int m = 0; m < MT; ++m) {
-                    const double t = cc[m];
-                    cc[m] = fma(t, c4[m], -sc[m] * s4[m]);
-                    sc[m] = fma(sc[m], c4[m], t * s4[m]);
-                }
+                for (int m = 0; m < MT; ++m) tce_phase_step(cc[m], sc[m], c4[m], s4[m]);
 #pragma unroll
                 for (int t = T0; t < T1; ++t)
 #pragma unroll
@@ -590,63 +575,63 @@ __device__ __noinline__ void process_batch(int wofs, int nb, int lane, int cstri
                 __syncwarp();
             }
 #pragma unroll 1
-          for (int p0 = q0; p0 < q0 + qn; p0 += PW) {
-            const int pn = q0 + qn - p0 < PW ? q0 + qn - p0 : PW;
-            if (!few) {   // the primitive quartet's coefficient products of bra and ket components
-                const short4 ix = b.qidx[p0];
-                const double fac = b.qfac[p0];
-                for (int x = lane; x < nAB + nCD; x += 32) {
-                    const int z = x - nAB;
-                    if (x < nAB) {
-                        const int ca = x % Q.nA, cb = x / Q.nA;
-                        b.cf[x] = fac * (coA[ca * npA + ix.x] * apow(Q.SI, ca)) * (coB[cb * npB + ix.y] * apow(Q.SJ, cb));
+            for (int p0 = q0; p0 < q0 + qn; p0 += PW) {
+                const int pn = q0 + qn - p0 < PW ? q0 + qn - p0 : PW;
+                if (!few) {   // the primitive quartet's coefficient products of bra and ket components
+                    const short4 ix = b.qidx[p0];
+                    const double fac = b.qfac[p0];
+                    for (int x = lane; x < nAB + nCD; x += 32) {
+                        const int z = x - nAB;
+                        if (x < nAB) {
+                            const int ca = x % Q.nA, cb = x / Q.nA;
+                            b.cf[x] = fac * (coA[ca * npA + ix.x] * apow(Q.SI, ca)) * (coB[cb * npB + ix.y] * apow(Q.SJ, cb));
+                        } else {
+                            const int cc = z % Q.nC, cd = z / Q.nC;
+                            b.cf[36 + z] = (coC[cc * npC + ix.z] * apow(Q.SK, cc)) * (coD[cd * npD + ix.w] * apow(Q.SL, cd));
+                        }
+                    }
+                    __syncwarp();
+                }
+                // sum_k w_k I_x I_y I_z per component: one lane per component (and primitive
+                // quartet), two nodes per load
+                const int p = p0 + pl;
+                for (int c = cl; c < Q.ncq && pl < pn; c += 32) {
+                    const unsigned cm = few ? cm0 : b.cmap[c];
+                    const double2 *rw[3];
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const int x = (cm >> (8 * d)) & 255;
+                        rw[d] = reinterpret_cast<const double2 *>(d < ndp ? b.rows + (size_t)(d * per + p * ncomb + x) * RS
+                                                                          : b.realb + (size_t)((d - ndp) * cstride + (p - q0) * ncomb + x) * RS);
+                    }
+                    const double2 *wk2 = reinterpret_cast<const double2 *>(b.wts), *wg2 = wk2 + 16;
+                    double vK = 0.0, vG = 0.0, vK1 = 0.0, vG1 = 0.0;
+#pragma unroll 4
+                    for (int k = 0; k < (kn >> 1); ++k) {
+                        const double2 x = rw[0][k], y = rw[1][k], z = rw[2][k], w = wk2[k];
+                        const double a0 = x.x * y.x * z.x, a1 = x.y * y.y * z.y;
+                        vK = fma(w.x, a0, vK);
+                        vK1 = fma(w.y, a1, vK1);
+                        if (judge) {
+                            const double2 g = wg2[k];
+                            vG = fma(g.x, a0, vG);
+                            vG1 = fma(g.y, a1, vG1);
+                        }
+                    }
+                    if (few) {
+                        const short4 ix = b.qidx[p];
+                        const double f = b.qfac[p] * f0 * (coA[ix.x] * coB[ix.y] * coC[ix.z] * coD[ix.w]);
+                        accK = fma(f, vK + vK1, accK);
+                        if (judge) accG = fma(f, vG + vG1, accG);
                     } else {
-                        const int cc = z % Q.nC, cd = z / Q.nC;
-                        b.cf[36 + z] = (coC[cc * npC + ix.z] * apow(Q.SK, cc)) * (coD[cd * npD + ix.w] * apow(Q.SL, cd));
+                        const int cd = c / nAB;
+                        const double f = b.cf[c - cd * nAB] * b.cf[36 + cd];
+                        b.blkK[c] = fma(f, vK + vK1, b.blkK[c]);
+                        if (judge) b.blkG[c] = fma(f, vG + vG1, b.blkG[c]);
                     }
                 }
                 __syncwarp();
             }
-            // sum_k w_k I_x I_y I_z per component: one lane per component (and primitive
-            // quartet), two nodes per load
-            const int p = p0 + pl;
-            for (int c = cl; c < Q.ncq && pl < pn; c += 32) {
-                const unsigned cm = few ? cm0 : b.cmap[c];
-                const double2 *rw[3];
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const int x = (cm >> (8 * d)) & 255;
-                    rw[d] = reinterpret_cast<const double2 *>(d < ndp ? b.rows + (size_t)(d * per + p * ncomb + x) * RS
-                                                                      : b.realb + (size_t)((d - ndp) * cstride + (p - q0) * ncomb + x) * RS);
-                }
-                const double2 *wk2 = reinterpret_cast<const double2 *>(b.wts), *wg2 = wk2 + 16;
-                double vK = 0.0, vG = 0.0, vK1 = 0.0, vG1 = 0.0;
-#pragma unroll 4
-                for (int k = 0; k < (kn >> 1); ++k) {
-                    const double2 x = rw[0][k], y = rw[1][k], z = rw[2][k], w = wk2[k];
-                    const double a0 = x.x * y.x * z.x, a1 = x.y * y.y * z.y;
-                    vK = fma(w.x, a0, vK);
-                    vK1 = fma(w.y, a1, vK1);
-                    if (judge) {
-                        const double2 g = wg2[k];
-                        vG = fma(g.x, a0, vG);
-                        vG1 = fma(g.y, a1, vG1);
-                    }
-                }
-                if (few) {
-                    const short4 ix = b.qidx[p];
-                    const double f = b.qfac[p] * f0 * (coA[ix.x] * coB[ix.y] * coC[ix.z] * coD[ix.w]);
-                    accK = fma(f, vK + vK1, accK);
-                    if (judge) accG = fma(f, vG + vG1, accG);
-                } else {
-                    const int cd = c / nAB;
-                    const double f = b.cf[c - cd * nAB] * b.cf[36 + cd];
-                    b.blkK[c] = fma(f, vK + vK1, b.blkK[c]);
-                    if (judge) b.blkG[c] = fma(f, vG + vG1, b.blkG[c]);
-                }
-            }
-            __syncwarp();
-          }
         }
     }
     accK_ += accK;
