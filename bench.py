@@ -519,8 +519,9 @@ def named_shape_stage(name, flush, steps=5):
             "fixed_rule": {"value": nfq / (fixed_ms * 1e-3), "ms_per_pass": fixed_ms},
             "plain": {"value": nfq / (plain_ms * 1e-3), "ms_per_pass": plain_ms},
             "lg_over_plain": plain_ms / lg_ms,
-            "roofline": {"bound": "fp64", "achieved": flops / (lg_ms * 1e-3) / 1e12, "peak": peak,
-                         "unit": "TFLOP/s", "frac": flops / (lg_ms * 1e-3) / 1e12 / peak,
+            "roofline": {"bound": "load latency, L1 data pipe", "achieved": flops / (lg_ms * 1e-3) / 1e12, "peak": peak,
+                         "unit": "TFLOP/s of the reference's operations (every Bessel order)", "frac": None,
+                         "reference_operations_over_peak": flops / (lg_ms * 1e-3) / 1e12 / peak,
                          "algorithmic_flops_per_pass": flops, "primitive_quartets": nprim},
             "setup": lg}
 
@@ -800,10 +801,12 @@ def main():
     peak = _fp64_peak()
     lg_flops, lg_nprim = eng.lg_work() if world == 1 else (None, None)
     achieved = lg_flops / (lg_kern * 1e-3) / 1e12 if world == 1 else None
-    traffic = None
+    traffic = pipes = None
     if os.path.exists(PROFILE_TRAFFIC):
         try:
-            traffic = json.load(open(PROFILE_TRAFFIC)).get("dram_bytes_per_pass")
+            prof = json.load(open(PROFILE_TRAFFIC))
+            traffic = prof.get("dram_bytes_per_pass")
+            pipes = prof.get("fp64_pipe_fraction", 0.0) + prof.get("dmma_pipe_fraction", 0.0) or None
         except Exception:
             traffic = None
     kernels = None
@@ -823,16 +826,19 @@ def main():
             kernels.append({"kernel": nm + (" fp32" if w["fp32"] else ""), "cls": w["cls"], "quartets": w["n"],
                             "ms": w["ms"], "flops": w["flops"],
                             "tflops": w["flops"] / (w["ms"] * 1e-3) / 1e12 if w["ms"] > 0 else None,
-                            "frac": w["flops"] / (w["ms"] * 1e-3) / 1e12 / peak if w["ms"] > 0 else None})
-    roofline = {"bound": "fp64", "kernel": "the learned-grid J/K pass, one CUDA graph: k_quartets<32|64>, "
+                            "reference_operations_over_peak":
+                                w["flops"] / (w["ms"] * 1e-3) / 1e12 / peak if w["ms"] > 0 else None})
+    # The operations are the reference's, counted over every Bessel order of its truncation; the
+    # kernels reach the same sums over a tenth of them.  Their rate over the FP64 peak is a speed
+    # and no load: frac is the load of the FP64 and FP64 tensor pipes in the captured pass.
+    roofline = {"bound": "L1 data pipe (all-s lists), load latency (the others)", "kernel": "the learned-grid J/K pass, one CUDA graph: k_quartets<32|64>, "
                                            "k_quartets_s[_tc], k_quartets_sp_tc, k_quartets_r1 (per-quartet rule, judge, fused "
                                            "J/K scatter) and the plain launches",
-                "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
-                "frac": (achieved / peak) if (achieved and peak) else None, "traffic": traffic,
+                "achieved": achieved, "peak": peak, "unit": "TFLOP/s of the reference's operations (every Bessel order)",
+                "reference_operations_over_peak": (achieved / peak) if (achieved and peak) else None,
+                "frac": pipes, "frac_of": "FP64 pipe plus FP64 tensor pipe cycles of the pass's kernels, from profiles/", "traffic": traffic,
                 "peak_source": "measured FP64 FMA throughput of this GPU (tce_fp64_peak probe); MEASURED_PEAKS.json "
                                "holds no FP64 figure",
-                # counted over every Bessel order of the reference's truncation; the kernels
-                # reach the same sums over a tenth of them, so the fraction is no pipe load
                 "algorithmic_flops_per_launch": lg_flops, "primitive_quartets": lg_nprim, "pass_ms": lg_kern,
                 "per_list": kernels}
     lg_err = lg_info["max_err_vs_oracle_table128"]
@@ -914,7 +920,8 @@ def main():
                                        "lg_over_plain": v["lg_over_plain"],
                                        "lg_max_err_vs_oracle_table128":
                                            v["setup"]["max_err_vs_oracle_table128"]["learned_grid"],
-                                       "roofline_frac": v["roofline"]["frac"]}
+                                       "reference_operations_over_peak":
+                                           v["roofline"]["reference_operations_over_peak"]}
                                    for k, v in line["named_shapes"].items()}
     if "cpu_baseline" in line:
         summary["cpu_baseline_timing_build"] = line["cpu_baseline"]["value"]

@@ -49,7 +49,7 @@ def test_ao_to_kmo_ragged_cells(systems, name, ncell, pr, qr):
         coeff[k * nf:(k + 1) * nf, k * nf:(k + 1) * nf] = C[k]
     with Engine(ao) as eng:
         eri = eng.ERI_integral_toroidal()
-        for _ in range(2):      # the second call on the kept workspaces
+        for _ in range(2):      # the second call on the first one's workspaces
             got = eng.ao_to_kmo(C, pr, qr)
             ref = kmo_ref.ao_to_kmo(eri, coeff, tuple(ncell), nf, pr[0] + 1, pr[1], qr[0] + 1, qr[1])
             assert np.abs(got - ref).max() <= 1e-12 * N * max(1.0, np.abs(ref).max())
