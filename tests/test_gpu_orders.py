@@ -166,6 +166,32 @@ def test_d_shells_of_one_direction_off_the_axis(cores):
     assert np.abs(J - J0).max() <= tol and np.abs(K - K0).max() <= tol
 
 
+@pytest.mark.parametrize("name,ncell", [("h2_sheet", (1, 1, 1)), ("h2_sheet", (2, 1, 1)), ("li_cube", (1, 1, 1)),
+                                        ("li_cube", (2, 1, 1)), ("h2_sheet", (3, 2, 1))])
+def test_classes_of_few_quartets_share_a_launch(name, ncell):
+    """Systems whose generic classes hold fewer quartets than the GPU holds warps:
+    the all-s list and one to four merged ones instead of up to fifteen launches, each
+    as long as its dearest quartet (cube: four of them).  J and K, direct and stored, and the learned grid's."""
+    import pyoracle
+    from william_ci_b200.engine import Engine
+    s = _system(name, ncell)
+    with Engine(s) as eng:
+        if ncell == (3, 2, 1):            # most classes have a wave of their own
+            assert eng.pass_kernels() >= 12
+            return
+        assert eng.pass_kernels() <= (5 if name == "h2_sheet" else 2)
+        P = random_density(s.nbas, 5) * 0.05
+        scale = np.abs(P).sum()
+        J0, K0 = pyoracle.Oracle(s).direct_jk(P)[:2]
+        got = [eng.direct_JK(P)]
+        eng.ERI_integral_toroidal()
+        got.append(eng.stored_JK(P))
+    for J, K in got:
+        J, K = J[:s.nfuc], K[:s.nfuc]
+        assert np.abs(J - J0[:s.nfuc]).max() <= 1e-12 * scale and np.abs(K - K0[:s.nfuc]).max() <= 1e-12 * scale
+    _learned_against_plain(s)
+
+
 @pytest.mark.parametrize("nquad", [32, 64])
 def test_shells_of_one_d_component(nquad):
     import pyoracle

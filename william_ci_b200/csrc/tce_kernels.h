@@ -63,6 +63,10 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
 int tce_preload_quartets(int nq);
 
 // all-s shell quartets, J/K mode (k_quartets_s)
+// warps of k_quartets (system's rule, tensor-core form) that the GPU holds at once
+// with buffers for max_ncomb combinations and max_ncq components
+long long tce_quartet_resident(const DevSys &S, int max_ncomb, int max_ncq, int nsm);
+
 struct SArgsHost {
     const int4 *items = nullptr;
     int nitems = 0;

@@ -1362,6 +1362,38 @@ long long tce_plain_scratch_per_warp(const DevSys &S, int max_ncq)
     return (long long)S.ndp * (S.ncap + 1) * 16 + (long long)PLAIN_PMAX * blkcap;
 }
 
+// The per-warp buffers of a launch: layout and capacities into A, their bytes
+static size_t quartet_buffers(const DevSys &S, int nq, bool tc, bool plain, int max_ncomb, int max_ncq, QuartetArgs &A)
+{
+    const int R = max_ncomb * S.ndp;
+    const int rowcap = std::max(R, tc ? 16 * S.ndp : 32);   // at least a tile of rows per periodic direction, or a row per lane
+    const int RS = (nq < TCE_NC ? nq : TCE_NC) + (tc ? 2 : 1);   // rows of one chunk of at most 32 nodes
+    const int nreal = 3 - S.ndp;
+    const int blkcap = (max_ncq + 3) / 4 * 4;
+    // real-direction rows: of one primitive quartet, or (tensor-core form) 32 / cqp small ones
+    const int cstride = tc && max_ncomb < 16 ? 16 : max_ncomb;
+    A.lay = tce_warp_layout(tc, rowcap, RS, nreal, cstride, blkcap, (nq + 15) / 16);
+    long long wdoubles = A.lay.extra;
+    if (plain) wdoubles += 3 * PLAIN_PMAX + 48 + 3 * TCE_MAXG / 2 + 4;
+    wdoubles = (wdoubles + 31) / 32 * 32;
+    A.rowcap = rowcap;
+    A.cstride = cstride;
+    A.blkcap = blkcap;
+    A.warp_smem_doubles = (int)wdoubles;
+    return (size_t)wdoubles * sizeof(double);
+}
+
+long long tce_quartet_resident(const DevSys &S, int max_ncomb, int max_ncq, int nsm)
+{
+    QuartetArgs A;
+    const size_t wbytes = quartet_buffers(S, S.nq, true, false, max_ncomb, max_ncq, A);
+    const int2 sh = S.nq == 32   ? quartet_shape<32, true>(wbytes)
+                    : S.nq == 40 ? quartet_shape<40, true>(wbytes)
+                    : S.nq == 64 ? quartet_shape<64, true>(wbytes)
+                                 : quartet_shape<128, true>(wbytes);
+    return (long long)sh.x * sh.y * (nsm > 0 ? nsm : 148);
+}
+
 int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t st)
 {
     QuartetArgs A;
@@ -1411,23 +1443,8 @@ int tce_launch_quartets(const DevSys &S, const QuartetHostArgs &h, cudaStream_t 
     if (h.method == TCE_METHOD_LEARNED && (!h.item_rule || !h.fb_items || !h.fb_count)) return TCE_ERR_ARG;
     if (!plain && !dict && !h.fixed_gmax) return TCE_ERR_ARG;
     const int nq = plain ? 16 : (dict ? h.dict_nq : S.nq);
-    const int R = h.max_ncomb * S.ndp;
     const bool tc = h.use_tc != 0;
-    const int rowcap = std::max(R, tc ? 16 * S.ndp : 32);   // at least a tile of rows per periodic direction, or a row per lane
-    const int RS = (nq < TCE_NC ? nq : TCE_NC) + (tc ? 2 : 1);   // rows of one chunk of at most 32 nodes
-    const int nreal = 3 - S.ndp;
-    const int blkcap = (h.max_ncq + 3) / 4 * 4;
-    // real-direction rows: of one primitive quartet, or (tensor-core form) 32 / cqp small ones
-    const int cstride = tc && h.max_ncomb < 16 ? 16 : h.max_ncomb;
-    A.lay = tce_warp_layout(tc, rowcap, RS, nreal, cstride, blkcap, (nq + 15) / 16);
-    long long wdoubles = A.lay.extra;
-    if (plain) wdoubles += 3 * PLAIN_PMAX + 48 + 3 * TCE_MAXG / 2 + 4;
-    wdoubles = (wdoubles + 31) / 32 * 32;
-    A.rowcap = rowcap;
-    A.cstride = cstride;
-    A.blkcap = blkcap;
-    A.warp_smem_doubles = (int)wdoubles;
-    const size_t wbytes = (size_t)wdoubles * sizeof(double);
+    const size_t wbytes = quartet_buffers(S, nq, tc, plain, h.max_ncomb, h.max_ncq, A);
     int warps = 4;
     while (warps > 1 && wbytes * warps > 220 * 1024) --warps;
     if (wbytes > 220 * 1024) return TCE_ERR_UNSUPPORTED;
