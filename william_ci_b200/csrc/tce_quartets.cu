@@ -1182,8 +1182,11 @@ __device__ void plain_columns(const DevSys &S, const QuartetArgs &A, double *T, 
     __syncwarp();
 }
 
+// 168 registers: the columns' recurrences and the panels' bookkeeping spill at 128
+// (plain method, 24-cell chain 185 / 177 ms at 128 / 168; learned grid of the 2x1x1
+// cube, which waits for its plain list, 6.6 / 6.0).
 template <bool TC>
-__global__ void __launch_bounds__(128, TC ? 4 : 3) k_plain(DevSys S, QuartetArgs A)
+__global__ void __launch_bounds__(128, 3) k_plain(DevSys S, QuartetArgs A)
 {
     const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
     blk_header(S, A.lay);
