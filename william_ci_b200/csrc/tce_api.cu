@@ -140,7 +140,7 @@ int route(const Handle *h, const int4 &q)
     if (cls == 0 && (h->use_tc || h->nq == 32 || h->nq == 40)) return 1 * 16;
     if (cls > 0 && (h->use_tc ? h->ndp == 1 && __builtin_popcount(cls) <= 2 : tce_r1_supported(h->ndp, h->nq, cls)))
         return 2 * 16 + cls;
-    return generic_class(h, q, false);
+    return generic_class(h, q);
 }
 
 // The generic kernel's lists, one per number of p and number of d shells
@@ -150,7 +150,7 @@ int route(const Handle *h, const int4 &q)
 // CUDA-core form has smaller buffers and more registers: one list per number of d
 // shells (0..4), whose single tail is worth more (2x2x2 cube, tensor cores off:
 // 26.9 ms with 5 lists, 23.5 with one).
-int full_class(const Handle *h, const int4 &q)
+int generic_class(const Handle *h, const int4 &q)
 {
     int np = 0, nd = 0;
     for (int S : {q.x, q.y, q.z, q.w}) {
@@ -160,28 +160,25 @@ int full_class(const Handle *h, const int4 &q)
     if (!h->use_tc) return nd;
     return nd * 5 - nd * (nd - 1) / 2 + np;
 }
-int generic_class(const Handle *h, const int4 &q, bool lg) { return h->gen_class[lg][full_class(h, q)]; }
-
-// Classes of few quartets share a list with the next smaller ones: while a list
-// has fewer quartets than the GPU holds warps for it, its launch takes the time of
-// its dearest quartet, and fifteen such launches one after the other take fifteen
-// times that.  The learned grid's lists run as two chains next to each other: half
-// as many.  Measured (32 nodes, ms with one list per class / merged at half the
-// warps / at the warps / at twice; in brackets the learned grid): 1x1 sheet 3.3 /
-// 0.72 / 0.73 / 0.76 (4.6 / 3.7 / 3.7 / 3.7), 2x1 sheet 3.7 / 1.9 / 1.6 / 1.6 (3.5 /
-// 2.1 / 2.3 / 2.6), 2x2 sheet 7.9 / 7.5 / 7.5 / 7.4 (12.1 / 11.9 / 12.9 / 12.9), 3x2
-// sheet 21.0 / 20.7 / 20.7 / 21.3, 2x1x1 cube 2.4 / 0.97 / 1.0 / 0.97, 2x2x1 cube
-// 3.3 / 2.9 / 2.5 / 2.5 (8.9 / 8.1 / 7.4 / 7.5).  By number of d shells, unmerged,
-// the small ones took 2.2, 2.5, 10.3, 32, 1.4 and 3.7.
+// The system's rule: classes of few quartets share a list with the next smaller
+// ones.  While a list has fewer quartets than the GPU holds warps for it, its launch
+// takes the time of its dearest quartet, and fifteen such launches one after the
+// other take fifteen times that.  Measured (32 nodes, ms with one list per class /
+// merged at half the warps / at the warps / at twice): 1x1 sheet 3.3 / 0.72 / 0.73 /
+// 0.76, 2x1 sheet 3.7 / 1.9 / 1.6 / 1.6, 2x2 sheet 7.9 / 7.5 / 7.5 / 7.4, 3x2 sheet
+// 21.0 / 20.7 / 20.7 / 21.3, 2x1x1 cube 2.4 / 0.97 / 1.0 / 0.97, 2x2x1 cube 3.3 / 2.9
+// / 2.5 / 2.5; by number of d shells, unmerged, they took 2.2, 2.5, 10.3, 32, 1.4 and
+// 3.7.  Not the learned grid's lists: they run as two chains next to each other, and
+// merged ones balance worse (16-cell chain 4.43 -> 4.79 ms).
 void merge_classes(Handle *h, const std::vector<int4> &items)
 {
-    for (int c = 0; c < 16; ++c) h->gen_class[0][c] = h->gen_class[1][c] = c;
+    for (int c = 0; c < 16; ++c) h->gen_class[c] = c;
     if (!h->use_tc) return;
     long long cnt[16] = {};
     int ncomb[16] = {}, ncq[16] = {};
     for (const int4 &q : items) {
-        if (route(h, q) >= 16) continue;
-        const int c = full_class(h, q);
+        const int c = route(h, q);
+        if (c >= 16) continue;
         ++cnt[c];
         ncomb[c] = std::max(ncomb[c], ncomb_of(h, q.x, q.y, q.z, q.w));
         ncq[c] = std::max(ncq[c], h->sh_n[q.x] * h->sh_n[q.y] * h->sh_n[q.z] * h->sh_n[q.w]);
@@ -189,19 +186,17 @@ void merge_classes(Handle *h, const std::vector<int4> &items)
     int order[16];
     std::iota(order, order + 16, 0);
     std::sort(order, order + 16, [&](int x, int y) { return ncomb[x] != ncomb[y] ? ncomb[x] > ncomb[y] : x > y; });
-    for (int lg = 0; lg < 2; ++lg) {
-        int head = -1;
-        long long have = 0, room = 0;
-        for (int c : order) {
-            if (cnt[c] == 0) continue;
-            if (head < 0 || have >= room) {
-                head = c;
-                have = 0;
-                room = tce_quartet_resident(h->S, ncomb[c], ncq[c], h->num_sms) / (lg ? 2 : 1);
-            }
-            h->gen_class[lg][c] = head;
-            have += cnt[c];
+    int head = -1;
+    long long have = 0, room = 0;
+    for (int c : order) {
+        if (cnt[c] == 0) continue;
+        if (head < 0 || have >= room) {
+            head = c;
+            have = 0;
+            room = tce_quartet_resident(h->S, ncomb[c], ncq[c], h->num_sms);
         }
+        h->gen_class[c] = head;
+        have += cnt[c];
     }
 }
 
@@ -213,7 +208,10 @@ int make_lists(Handle *h, const std::vector<int4> &items)
     h->lists.clear();
     merge_classes(h, items);
     std::vector<std::vector<int4>> by(3 * 16);
-    for (const int4 &q : items) by[route(h, q)].push_back(q);
+    for (const int4 &q : items) {
+        const int key = route(h, q);
+        by[key < 16 ? h->gen_class[key] : key].push_back(q);
+    }
     h->nitems_shard = 0;
     for (int key = 0; key < 3 * 16; ++key) {
         if (by[key].empty()) continue;

@@ -57,7 +57,7 @@ struct Handle {
     // (generic lists: cls = generic_class; max_ncomb / max_ncq of the list's quartets)
     struct WorkList { int kind, cls; int4 *d = nullptr; long long n = 0; int max_ncomb = 1, max_ncq = 1; };
     std::vector<WorkList> lists;
-    int gen_class[2][16] = {};           // [learned grid][generic class]: the class whose list takes its quartets
+    int gen_class[16] = {};              // generic class -> the class whose list takes its quartets (merge_classes)
     long long nitems_shard = 0;
     int *d_tnmax = nullptr;
     unsigned int *d_next = nullptr;
@@ -198,7 +198,7 @@ void dfree(Handle *h, void *p);
 // helpers defined in tce_api.cu
 int shift_to(const Handle *h, int idx, int refcell, int nblk);
 int sp_class(const Handle *h, const int4 &q);
-int generic_class(const Handle *h, const int4 &q, bool lg);
+int generic_class(const Handle *h, const int4 &q);
 int block_tc(const Handle *h);
 float2 node_range(const double *t, int n);
 int ncomb_of(const Handle *h, int SI, int SJ, int SK, int SL);

@@ -455,7 +455,7 @@ int lg_rebuild_lists(Handle *h)
         const int4 &q = h->items_host[(size_t)i];
         if (r >= 0 && r < h->lg_nrules) {
             int route = lg_route(h, q);
-            if (route == 0) route = generic_class(h, q, true);
+            if (route == 0) route = generic_class(h, q);
             // (no FP32 form for two p shells: their CUDA-core form is the generic kernel)
             const bool f32 = h->fp32_thr > 0.0 && route >= 16 && h->ndp == 1 && h->d_rule_T32 &&
                              __builtin_popcount(route & 15) <= 1 &&
