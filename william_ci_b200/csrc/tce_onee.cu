@@ -23,6 +23,7 @@
 // coalesced), reduced over the warp.
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <vector>
 
 #include "tce_handle.h"
@@ -455,21 +456,24 @@ static int nuclear_elements(Handle *h, int natoms, const double *geo, const int3
     const long long npairs = plist.empty() ? (long long)nfuc * nbas : (long long)plist.size();
     std::vector<double> g(geo, geo + (size_t)natoms * 3);
     std::vector<int> z(Z, Z + natoms);
-    int2 *d_fsh = nullptr, *d_pl = nullptr;
-    double *d_geo = nullptr, *d_V = nullptr;
-    int *d_Z = nullptr;
+    // one buffer, one copy: out[npairs] | geometry | function table | pairs | charges
+    const size_t np = (size_t)npairs, ng = g.size(), nf = fsh.size(), npl = plist.size();
+    std::vector<double> in(ng + nf + npl + (z.size() + 1) / 2);
+    static_assert(sizeof(int2) == sizeof(double), "tables packed as doubles");
+    std::memcpy(in.data(), g.data(), sizeof(double) * ng);
+    std::memcpy(in.data() + ng, fsh.data(), sizeof(int2) * nf);
+    if (npl) std::memcpy(in.data() + ng + nf, plist.data(), sizeof(int2) * npl);
+    std::memcpy(in.data() + ng + nf + npl, z.data(), sizeof(int) * z.size());
+    double *d_V = nullptr;
     int s;
-    auto cleanup = [&]() {
-        dfree(h, d_fsh);
-        dfree(h, d_pl);
-        dfree(h, d_geo);
-        dfree(h, d_Z);
+    if ((s = dalloc(h, &d_V, np + in.size()))) return s;
+    double *d_geo = d_V + np;
+    int2 *d_fsh = reinterpret_cast<int2 *>(d_geo + ng), *d_pl = d_fsh + nf;
+    int *d_Z = reinterpret_cast<int *>(d_pl + npl);
+    cudaError_t e = cudaMemcpyAsync(d_geo, in.data(), sizeof(double) * in.size(), cudaMemcpyHostToDevice, h->st);
+    if (e != cudaSuccess) {
         dfree(h, d_V);
-    };
-    if ((s = upload(h, &d_fsh, fsh)) || (!plist.empty() && (s = upload(h, &d_pl, plist))) ||
-        (s = upload(h, &d_geo, g)) || (s = upload(h, &d_Z, z)) || (s = dalloc(h, &d_V, (size_t)npairs))) {
-        cleanup();
-        return s;
+        return fail(h, TCE_ERR_CUDA, std::string("nuclear attraction: ") + cudaGetErrorString(e));
     }
     NaArgs A;
     A.fsh = d_fsh;
@@ -494,7 +498,7 @@ static int nuclear_elements(Handle *h, int natoms, const double *geo, const int3
         int warps = NA_WARPS_MAX;
         while (warps > 1 && wbytes * warps > 200 * 1024) --warps;
         if (wbytes > 200 * 1024) {
-            cleanup();
+            dfree(h, d_V);
             return fail(h, TCE_ERR_UNSUPPORTED, "truncation order too large for the nuclear-attraction kernel");
         }
         const size_t smem = wbytes * (size_t)warps;
@@ -502,11 +506,11 @@ static int nuclear_elements(Handle *h, int natoms, const double *geo, const int3
         cudaFuncSetAttribute(k_nuclear, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_nuclear<<<grid, 32 * warps, smem, h->st>>>(h->S, A);
     }
-    cudaError_t e = cudaGetLastError();
+    e = cudaGetLastError();
     out.assign((size_t)npairs, 0.0);
     if (e == cudaSuccess) e = cudaMemcpyAsync(out.data(), d_V, sizeof(double) * out.size(), cudaMemcpyDeviceToHost, h->st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(h->st);
-    cleanup();
+    dfree(h, d_V);
     if (e != cudaSuccess) return fail(h, TCE_ERR_CUDA, std::string("nuclear attraction: ") + cudaGetErrorString(e));
     return TCE_OK;
 }
